@@ -1,0 +1,968 @@
+// f4j_crt.cuh -- the split GEMM's residue form: the same fixed-point operands,
+// multiplied modulo small coprime numbers instead of slice by slice.
+//
+// The operands become the slice form's integers Y = round(x 2^(F - e)),
+// F = 4 + 5 (s - 1) bits for the same s.  Their product C' = Y_A Y_B is an
+// integer below k 2^(2F), so it is known once it is known modulo pairwise
+// coprime p_1 .. p_L with p_1 ... p_L > 2 k 2^(2F) (Chinese remainder theorem;
+// the residue-number form of error-free GEMM emulation, Ozaki, Uchino and
+// Imamura 2025).  Residues here are E4M3 numbers:
+//  - b odd, b <= 49, or b <= 32: each residue mod b has a representative d with
+//    |d| <= 16, or even and |d| <= 32, which E4M3 holds exactly.  C' mod b is
+//    one FP8 product.
+//  - b^2: with x = x0 + b x1 (digits as above), x y = x0 y0 + b (x0 y1 + x1 y0)
+//    modulo b^2 (b^2 x1 y1 vanishes): three FP8 products in two accumulators.
+// A product of 8192 terms at F = 49 needs 112 bits: eight squares and seven
+// single moduli, 31 FP8 products where the slices take 55 (66 -> 34 or 35 at
+// F = 54), and no slice product is dropped: C' is exact and C is C' 2^(..)
+// rounded once.
+//
+//  k_crt_planes   Y of each element, then its residues' digits, one E4M3 plane
+//                 per digit (K-major, as the slice planes).
+//  k_crt_gemm     for each modulus and 256 x 256 tile of C, the FP8 products on
+//                 CTA pairs (tcgen05 cta_group::2), exact in FP32 (|sum| <= 2^24
+//                 over at most 8192 terms), reduced mod p and multiplied by the
+//                 modulus's weight (M / p)^-1: an int16 plane per modulus.
+//  k_crt_combine  sum_l y_l (M / p_l) in 31-bit limbs, reduced mod M, rounded to
+//                 double once and scaled.
+//
+// Included by f4j_split.cu.
+#pragma once
+
+namespace {
+
+// ------------------------------------------------------------------ moduli
+constexpr int CRT_NB = 15;     // bases; a configuration squares the first nsq and drops some of the last
+constexpr int CRT_LIMBS = 5;   // 31-bit limbs of M
+constexpr int CRT_NG = 7;      // groups of moduli in the reconstruction: pairs, and the last three
+constexpr int CRT_CFGS = 48;
+constexpr int CRT_KC = 8192;   // terms per accumulation: 2 * 8192 * 32 * 32 = 2^24
+__host__ __device__ constexpr int crt_base(int i) {
+    // pairwise coprime; the large ones first, as the order in which they are squared
+    constexpr int b[CRT_NB] = {49, 47, 43, 41, 37, 32, 31, 29, 27, 25, 23, 19, 17, 13, 11};
+    return b[i];
+}
+
+// Residue weights of the eight bytes of Y + 2^60: 256^i = wh b + wl (mod b^2),
+// packed for dp4a.  The two sums start at kl and kh, the bits of floats 2^23 +
+// k0 and 2^23 + k1, so each is a float without a conversion; k0 and k1 make
+// the 2^23 and the 2^60 vanish modulo b (and b^2 for the two together).
+struct CrtMod {
+    uint32_t wl[2] = {0, 0}, wh[2] = {0, 0};
+    uint32_t kl = 0, kh = 0;
+    float b = 0, inv = 0;  // b, 1 / b
+};
+struct CrtMods {
+    CrtMod m[CRT_NB] = {};
+    constexpr CrtMods() {
+        for (int i = 0; i < CRT_NB; i++) {
+            const uint32_t b = (uint32_t)crt_base(i), p = b * b;
+            uint32_t pw = 1;
+            for (int u = 0; u < 8; u++) {
+                m[i].wl[u / 4] |= (pw % b) << (8 * (u % 4));
+                m[i].wh[u / 4] |= (pw / b) << (8 * (u % 4));
+                pw = pw * 256 % p;
+            }
+            uint32_t c = 8388608u % p, c60 = 1;
+            for (int u = 0; u < 60; u++) c60 = c60 * 2 % p;
+            c = (c + c60) % p;
+            const uint32_t k0 = (b - c % b) % b;          // 2^23 + 2^60 + k0 = g b (mod b^2)
+            const uint32_t g = (c + k0) % p / b;
+            const uint32_t k1 = (2 * b - g - 8388608u % b) % b;  // 2^23 + k1 = -g (mod b)
+            m[i].kl = 0x4B000000u + k0;
+            m[i].kh = 0x4B000000u + k1;
+            m[i].b = (float)b;
+            m[i].inv = 1.0f / (float)b;
+        }
+    }
+};
+__constant__ CrtMods c_crt{};
+
+// One configuration: which moduli, and the constants of the reconstruction.
+struct CrtCfg {
+    int nmod, nsq;   // moduli; the first nsq are squares
+    int cost;        // FP8 products: nmod + 2 nsq
+    int limbs;       // limbs of the reconstruction: 4 while M < 2^124, else 5
+    float bits;      // log2 M
+    int sh;          // the limbs below hold 2^sh times their number: 2^sh M in [2^(31 limbs - 1), 2^(31 limbs))
+    float qinv;      // 2^(31 limbs - 18) / (2^sh M), for the quotient by M
+    int pad;
+    float p[CRT_NB], invp[CRT_NB], u[CRT_NB];  // modulus, 1 / p, (M / p)^-1 mod p (balanced)
+    int32_t c[CRT_NB];                         // P / p, P the product of the group's moduli
+    int32_t W[CRT_NG][CRT_LIMBS];              // M / P, 31-bit limbs
+    int32_t M[CRT_LIMBS];
+};
+__host__ __device__ constexpr int crt_group(int l) { return l / 2 < CRT_NG ? l / 2 : CRT_NG - 1; }
+
+constexpr float CRT_MAGIC = 12582912.0f;  // 1.5 * 2^23: x + CRT_MAGIC rounds |x| < 2^22 to an integer
+
+// ------------------------------------------------------------------ residue planes
+typedef unsigned long long f32x2;  // two floats in a register pair
+__device__ __forceinline__ f32x2 pack2(uint32_t a, uint32_t b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 dup2(float a) { return pack2(__float_as_uint(a), __float_as_uint(a)); }
+__device__ __forceinline__ void unpack2(f32x2 v, uint32_t& a, uint32_t& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(a), "=r"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// Eight digits, |d| <= 16, as E4M3 bytes.
+__device__ __forceinline__ uint2 crt_e4m3(const f32x2 (&f)[4]) {
+    uint32_t w[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        uint32_t x0, x1;
+        uint16_t h;
+        unpack2(f[u], x0, x1);
+        asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(h) : "f"(__uint_as_float(x1)), "f"(__uint_as_float(x0)));
+        w[u] = h;
+    }
+    return make_uint2(__byte_perm(w[0], w[1], 0x5410), __byte_perm(w[2], w[3], 0x5410));
+}
+
+// Eight digits as bytes d + 64.
+__device__ __forceinline__ uint2 crt_bytes64(const f32x2 (&f)[4]) {
+    uint32_t x[8], h[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        unpack2(add2(f[u], dup2(CRT_MAGIC + 64.0f)), x[2 * u], x[2 * u + 1]);
+        h[u] = __byte_perm(x[2 * u], x[2 * u + 1], 0x0040);
+    }
+    return make_uint2(__byte_perm(h[0], h[1], 0x5410), __byte_perm(h[2], h[3], 0x5410));
+}
+
+// Four bytes g = d + 64, |d| <= 26: an odd d beyond 16 is not an E4M3 number
+// and becomes the even d -+ b; up / down flag those bytes (d above 16: up).
+__device__ __forceinline__ uint32_t crt_even(uint32_t g, uint32_t b, uint32_t& up, uint32_t& down) {
+    up = ((g + 0x2F2F2F2Fu) >> 7) & g & 0x01010101u;    // g >= 81, odd
+    down = ((0xAFAFAFAFu - g) >> 7) & g & 0x01010101u;  // g <= 47, odd
+    return g + down * b - up * b;
+}
+
+// Four bytes d + 64 as E4M3 bytes, by way of halves 1024 + (d + 64).
+__device__ __forceinline__ uint32_t crt_e4m3_of64(uint32_t g) {
+    uint32_t a = __byte_perm(g, 0x64646464u, 0x4140), c = __byte_perm(g, 0x64646464u, 0x4342);
+    const uint32_t off = 0xE440E440u;  // -1088, twice
+    uint16_t h0, h1;
+    asm("add.rn.f16x2 %0, %0, %1;" : "+r"(a) : "r"(off));
+    asm("add.rn.f16x2 %0, %0, %1;" : "+r"(c) : "r"(off));
+    asm("cvt.rn.satfinite.e4m3x2.f16x2 %0, %1;" : "=h"(h0) : "r"(a));
+    asm("cvt.rn.satfinite.e4m3x2.f16x2 %0, %1;" : "=h"(h1) : "r"(c));
+    return __byte_perm((uint32_t)h0, (uint32_t)h1, 0x5410);
+}
+
+struct CrtDst {
+    uint8_t* a;   // first copy
+    uint8_t* b;   // second copy, or null
+    uint32_t xb;  // xor of the second copy's bytes (0x80808080: negated)
+};
+
+__device__ __forceinline__ void crt_store(const CrtDst& d, int64_t off, uint2 v) {
+    *reinterpret_cast<uint2*>(d.a + off) = v;
+    if (d.b) *reinterpret_cast<uint2*>(d.b + off) = make_uint2(v.x ^ d.xb, v.y ^ d.xb);
+}
+
+// The residue digits of eight integers Yb = Y + 2^60 (lo, hi words), plane i at
+// d + i * plane.
+__device__ __forceinline__ void crt_digits8(const uint32_t (&lo)[8], const uint32_t (&hi)[8], int nmod, int nsq,
+                                            const CrtDst& d, int64_t plane) {
+    const f32x2 magic = dup2(CRT_MAGIC), unmagic = dup2(-CRT_MAGIC);
+#pragma unroll 1
+    for (int i = 0; i < nmod; i++) {
+        const CrtMod& c = c_crt.m[i];
+        const f32x2 nb = dup2(-c.b), inv = dup2(c.inv);
+        const bool wide = c.b > 33.0f;
+        const uint32_t bi = (uint32_t)c.b;
+        f32x2 f[4], q[4];
+        uint2 up = make_uint2(0, 0), down = make_uint2(0, 0);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const f32x2 t = pack2(__dp4a(hi[2 * j], c.wl[1], __dp4a(lo[2 * j], c.wl[0], c.kl)),
+                                  __dp4a(hi[2 * j + 1], c.wl[1], __dp4a(lo[2 * j + 1], c.wl[0], c.kl)));
+            q[j] = add2(fma2(t, inv, magic), unmagic);
+            f[j] = fma2(nb, q[j], t);
+        }
+        if (wide) {
+            uint2 g = crt_bytes64(f);
+            g.x = crt_even(g.x, bi, up.x, down.x);
+            g.y = crt_even(g.y, bi, up.y, down.y);
+            crt_store(d, (int64_t)i * plane, make_uint2(crt_e4m3_of64(g.x), crt_e4m3_of64(g.y)));
+        } else {
+            crt_store(d, (int64_t)i * plane, crt_e4m3(f));
+        }
+        if (i < nsq) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const f32x2 t = add2(pack2(__dp4a(hi[2 * j], c.wh[1], __dp4a(lo[2 * j], c.wh[0], c.kh)),
+                                           __dp4a(hi[2 * j + 1], c.wh[1], __dp4a(lo[2 * j + 1], c.wh[0], c.kh))),
+                                     q[j]);
+                f[j] = fma2(nb, add2(fma2(t, inv, magic), unmagic), t);
+            }
+            if (wide) {  // the first digit's d -+ b leaves +-1 for this one
+                uint2 g = crt_bytes64(f);
+                g.x = g.x + up.x - down.x;
+                g.y = g.y + up.y - down.y;
+                g.x = crt_even(g.x, bi, up.x, down.x);
+                g.y = crt_even(g.y, bi, up.y, down.y);
+                crt_store(d, (int64_t)(nmod + i) * plane, make_uint2(crt_e4m3_of64(g.x), crt_e4m3_of64(g.y)));
+            } else {
+                crt_store(d, (int64_t)(nmod + i) * plane, crt_e4m3(f));
+            }
+        }
+    }
+}
+
+// One operand: planes[i] is rows_out x Kp bytes at out + i * rows_out * Kp.
+//   real, and A of a complex product (role 0): as k_split writes its planes
+//   B of a complex product (role 1): out[r][q] = re, out[r][Kh+q] = -im,
+//     out[half+r][q] = im, out[half+r][Kh+q] = re
+struct CrtOperand {
+    const double* X;
+    int64_t scols;
+    int transposed, conj, role;
+    int64_t targets, rows_out, half;
+    const int* e_t;
+    uint8_t* out;
+};
+
+template <bool CPLX>
+__device__ __forceinline__ void crt_planes_body(const CrtOperand& o, int64_t klen, int64_t Kh, int64_t Kp,
+                                                int s, int nmod, int nsq, double (*sre)[SP_TQ + 1],
+                                                double (*sim)[SP_TQ + 1]) {
+    const int64_t q0 = (int64_t)blockIdx.x * SP_TQ;
+    const int F = 4 + 5 * (s - 1);
+    const int rr = threadIdx.x / 8, qs = (threadIdx.x % 8) * 8;
+    const int64_t plane = o.rows_out * Kp;
+    const bool staged = CPLX || o.transposed;
+    for (int by = blockIdx.y; (int64_t)by * SP_TR < o.targets; by += gridDim.y) {
+        const int64_t r0 = (int64_t)by * SP_TR;
+        if (staged) {
+            for (int e = threadIdx.x; e < SP_TR * SP_TQ; e += 256) {
+                int tr, tq;
+                if (!o.transposed) { tr = e / SP_TQ; tq = e % SP_TQ; }
+                else { tq = e / SP_TR; tr = e % SP_TR; }
+                const int64_t r = r0 + tr, q = q0 + tq;
+                double re = 0, im = 0;
+                if (r < o.targets && q < klen) {
+                    const int64_t idx = o.transposed ? (q * o.scols + r) : (r * o.scols + q);
+                    if constexpr (CPLX) {
+                        re = o.X[2 * idx];
+                        im = o.X[2 * idx + 1];
+                        if (o.conj) im = -im;
+                    } else {
+                        re = o.X[idx];
+                    }
+                }
+                sre[tr][tq] = re;
+                if constexpr (CPLX) sim[tr][tq] = im;
+            }
+            __syncthreads();
+        }
+        const int64_t r = r0 + rr;
+        if (r < o.targets) {
+            const int e = o.e_t[r];
+#pragma unroll 1
+            for (int part = 0; part < (CPLX ? 2 : 1); part++) {
+                uint32_t lo[8], hi[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    double v;
+                    if (staged) {
+                        v = sre[rr][qs + j];
+                        if constexpr (CPLX) v = part ? sim[rr][qs + j] : v;
+                    } else {
+                        v = q0 + qs + j < klen ? __ldg(o.X + r * o.scols + q0 + qs + j) : 0.0;
+                    }
+                    const unsigned long long y = (unsigned long long)(fixed_of(v, e, F) + (1ll << 60));
+                    lo[j] = (uint32_t)y;
+                    hi[j] = (uint32_t)(y >> 32);
+                }
+                CrtDst d{o.out + r * Kp + q0 + qs, nullptr, 0};
+                if constexpr (CPLX) {
+                    if (o.role == 0) {
+                        if (part) d.a += Kh;
+                    } else if (part == 0) {
+                        d.b = d.a + o.half * Kp + Kh;
+                    } else {
+                        d.b = d.a + Kh;
+                        d.xb = 0x80808080u;
+                        d.a += o.half * Kp;
+                    }
+                }
+                crt_digits8(lo, hi, nmod, nsq, d, plane);
+            }
+        }
+        if (staged) __syncthreads();
+    }
+}
+
+// Both operands' residue planes in one launch (blockIdx.z picks the operand).
+template <bool CPLX>
+__global__ void __launch_bounds__(256, 4) k_crt_planes(const CrtOperand a, const CrtOperand b, int64_t klen,
+                                                       int64_t Kh, int64_t Kp, const SplitPlan* __restrict__ plan,
+                                                       const CrtCfg* __restrict__ cfgs) {
+    __shared__ double sre[SP_TR][SP_TQ + 1];
+    __shared__ double sim[CPLX ? SP_TR : 1][SP_TQ + 1];
+    if (plan->nonfinite) return;
+    const int s = plan->s, nmod = cfgs[plan->crt].nmod, nsq = cfgs[plan->crt].nsq;
+    if (blockIdx.z == 0) crt_planes_body<CPLX>(a, klen, Kh, Kp, s, nmod, nsq, sre, sim);
+    else crt_planes_body<CPLX>(b, klen, Kh, Kp, s, nmod, nsq, sre, sim);
+}
+
+// ------------------------------------------------------------------ GEMM
+constexpr int CG_T = 256;                   // output tile of a CTA pair; each CTA holds 128 rows of A, 128 of B
+constexpr int CG_BK = 128;                  // K bytes per ring slot (one 128-byte swizzle row)
+constexpr int CG_TILE = 128 * CG_BK;        // 16 KB
+constexpr int CG_SLOT = 2 * CG_TILE;        // an A tile and a B tile
+constexpr int CG_RING = 7;
+constexpr int CG_THREADS = 320;             // warp 0 TMA, warp 1 MMA, warps 2..9 epilogue
+constexpr int CG_KB = CRT_KC / CG_BK;       // K blocks per accumulation
+constexpr int CG_GROUP_M = 8;
+
+struct CrtGemmParams {
+    int M, N, nkb;          // rows of A, (padded) rows of B^T, K blocks of CG_BK bytes
+    int tm0, tm1, tn0, tn1; // tile rows and columns of C the launch covers
+    int row0, rows;         // rows of C in y: [row0, row0 + rows)
+    int64_t ldy;            // columns of y (multiple of 8, >= N)
+    int16_t* y;             // [nmod][rows][ldy]
+    int* status;
+    const SplitPlan* plan;
+    const CrtCfg* cfgs;
+};
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// shared::cluster address of the same variable in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t cluster_map(const void* p, uint32_t rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// mbar_wait for a barrier that threads of the other CTA arrive on
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, int* status, int code) {
+    if (mbar_try_wait_cluster(bar, parity)) return true;
+    const uint64_t t0 = f4j_globaltimer_ns();
+    for (uint32_t it = 0; it < F4J_WAIT_LIMIT; ++it) {
+        if (mbar_try_wait_cluster(bar, parity)) return true;
+        if ((it & 255) == 255 && f4j_globaltimer_ns() - t0 > F4J_WAIT_NS) break;
+    }
+    if (status) atomicExch(status, code);
+    return false;
+}
+__device__ __forceinline__ void tma_load_3d_pair(void* dst, const CUtensorMap* map, uint32_t bar, int c0, int c1,
+                                                 int c2) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 "
+        "[%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
+        : "memory");
+}
+// D (+)= A B^T over one 128-byte K block: four K = 32 steps on the CTA pair.
+__device__ __forceinline__ void umma2_f8_k128(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc,
+                                              uint32_t acc) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+            "setp.ne.b32 p, %5, 0;\n\t"
+            "mov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
+            "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], da, db, %4, p;\n\t}" ::"r"(d),
+            "r"(a_lo + 2 * k), "r"(b_lo + 2 * k), "r"(hi), "r"(idesc), "r"(k == 0 ? acc : 1u)
+            : "memory");
+    }
+}
+// Arrive on the barrier of both CTAs once this thread's MMAs have completed.
+__device__ __forceinline__ void umma2_commit(uint64_t* bar) {
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+            smem_u32(bar)),
+        "h"((uint16_t)3)
+        : "memory");
+}
+
+// Tile `t` of a tiles_m x tiles_n block, bands of CG_GROUP_M tile rows,
+// column-major inside a band (see tile_origin).
+__device__ __forceinline__ void crt_tile(int t, int tiles_m, int tiles_n, int& tm, int& tn) {
+    const int per = CG_GROUP_M * tiles_n;
+    const int g = t / per, first = g * CG_GROUP_M;
+    const int gm = tiles_m - first < CG_GROUP_M ? tiles_m - first : CG_GROUP_M;
+    const int r = t - g * per;
+    tm = first + r % gm;
+    tn = r / gm;
+}
+
+// Balanced x mod p for an integer |x| <= 2^24.
+__device__ __forceinline__ float crt_mod(float x, float p, float invp) {
+    const float q = __fmaf_rn(x, invp, CRT_MAGIC) - CRT_MAGIC;
+    return __fmaf_rn(-p, q, x);
+}
+
+// A unit is one modulus of one 256 x 256 tile: squares first (modulus-major,
+// so the pairs running together share operand tiles in L2), then the singles.
+// Ring slots carry (A digit, B digit) tile pairs: one per K block of a single
+// modulus, (A0, B0) and (A1, B1) of a square.  TMEM holds two accumulators of
+// 256 columns: X (x0 y0) and Y (x0 y1 + x1 y0) of a square, in turn the
+// singles'.  Y's products run one K block behind X's, so at the end of a
+// square X is drained under Y's last products and Y under the next unit's
+// first.
+__global__ void __launch_bounds__(CG_THREADS, 1) __cluster_dims__(2, 1, 1)
+    k_crt_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+               const __grid_constant__ CrtGemmParams p) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char* ring = reinterpret_cast<unsigned char*>(
+        (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    __shared__ __align__(8) uint64_t full[CG_RING], empty[CG_RING], accfull[2], accempty[2], mma_done;
+    __shared__ uint32_t tmem_slot;
+    __shared__ int abort_flag;
+
+    if (p.plan->nonfinite) return;  // the gated plain path computes this product (both CTAs of a pair)
+    const CrtCfg* __restrict__ cfg = p.cfgs + p.plan->crt;
+    const int nmod = cfg->nmod, nsq = cfg->nsq;
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const uint32_t rank = cluster_rank();
+    const int tiles_m = p.tm1 - p.tm0, tiles_n = p.tn1 - p.tn0, ntiles = tiles_m * tiles_n;
+    const int nunits = ntiles * nmod;
+    const int pair = blockIdx.x / 2, npairs = gridDim.x / 2;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < CG_RING; i++) {
+            mbar_init(&full[i], 1);
+            mbar_init(&empty[i], 1);
+        }
+        for (int i = 0; i < 2; i++) {
+            mbar_init(&accfull[i], 1);
+            mbar_init(&accempty[i], 16);  // eight epilogue warps in each CTA
+        }
+        mbar_init(&mma_done, 1);
+        abort_flag = 0;
+        fence_barrier_init();
+    }
+    if (warp == 0 && lane == 0) {
+        prefetch_tmap(&tmA);
+        prefetch_tmap(&tmB);
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
+                     "r"(512u)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+
+    if (warp == 0) {
+        // ---------------- TMA producer: lane 0 loads the slot's A tile, lane 1 its B tile
+        int st = 0;
+        bool ok = true;
+        for (int u = pair; u < nunits && ok; u += npairs) {
+            const int l = u / ntiles;
+            int tm, tn;
+            crt_tile(u - l * ntiles, tiles_m, tiles_n, tm, tn);
+            const int row = lane == 0 ? (p.tm0 + tm) * CG_T + (int)rank * 128 : (p.tn0 + tn) * CG_T + (int)rank * 128;
+            const int nd = l < nsq ? 2 : 1;
+            for (int kb = 0; kb < p.nkb && ok; kb++) {
+                for (int d = 0; d < nd; d++, st++) {
+                    const int s = st % CG_RING;
+                    if (lane == 0) {
+                        if (st >= CG_RING)
+                            ok = mbar_wait(&empty[s], ((st / CG_RING) & 1) ^ 1, p.status, 21) &&
+                                 !*(volatile int*)&abort_flag;
+                        if (!ok) abort_flag = 1;
+                        else if (rank == 0) mbar_arrive_expect_tx(&full[s], 2 * CG_SLOT);
+                    }
+                    ok = __shfl_sync(0xffffffffu, ok, 0);
+                    if (!ok) break;
+                    if (lane < 2)
+                        tma_load_3d_pair(ring + s * CG_SLOT + lane * CG_TILE, lane == 0 ? &tmA : &tmB,
+                                         cluster_map(&full[s], 0), kb * CG_BK, row, d ? nmod + l : l);
+                }
+            }
+        }
+        // copies still in flight signal the first CTA's barriers: it waits for them (bounded), and the
+        // cluster barrier below keeps both CTAs until then
+        if (rank == 0 && lane == 0)
+            for (int q = st > CG_RING ? st - CG_RING : 0; q < st; q++)
+                mbar_wait(&full[q % CG_RING], (q / CG_RING) & 1, nullptr, 0);
+    } else if (warp == 1) {
+        // ---------------- MMA issuer: one thread of the pair's first CTA
+        if (rank == 0 && lane == 0) {
+            const uint64_t desc0 = umma_desc_sw128(ring);
+            const uint32_t hi = (uint32_t)(desc0 >> 32), lo0 = (uint32_t)desc0;
+            const uint32_t idesc = umma_idesc_e4m3_f32(256, 256);
+            constexpr uint32_t SLOT16 = CG_SLOT >> 4, TILE16 = CG_TILE >> 4;
+            int st = 0, turn = 0;
+            uint32_t fills[2] = {0, 0};
+            bool ok = true;
+            auto acquire = [&](int a) {
+                if (ok && fills[a] > 0) ok = mbar_wait_cluster(&accempty[a], (fills[a] - 1) & 1, p.status, 22);
+                tc_fence_after();
+            };
+            auto landed = [&](int i) {
+                if (ok) ok = mbar_wait_cluster(&full[i % CG_RING], (i / CG_RING) & 1, p.status, 23) &&
+                             !*(volatile int*)&abort_flag;
+                tc_fence_after();
+            };
+            auto mma = [&](int acc, int ia, int ib, bool first) {
+                umma2_f8_k128(tmem + acc * 256, lo0 + (uint32_t)(ia % CG_RING) * SLOT16,
+                              lo0 + (uint32_t)(ib % CG_RING) * SLOT16 + TILE16, hi, idesc, first ? 0u : 1u);
+            };
+            for (int u = pair; u < nunits && ok; u += npairs) {
+                const int l = u / ntiles;
+                for (int k0 = 0; k0 < p.nkb && ok; k0 += CG_KB) {
+                    const int nk = p.nkb - k0 < CG_KB ? p.nkb - k0 : CG_KB;
+                    if (l < nsq) {
+                        acquire(0);
+                        landed(st);
+                        if (!ok) break;
+                        mma(0, st, st, true);
+                        if (nk == 1) umma2_commit(&accfull[0]);
+                        for (int kb = 0; kb < nk; kb++) {
+                            const int s0 = st + 2 * kb;
+                            if (kb + 1 < nk) {
+                                landed(s0 + 2);
+                                if (!ok) break;
+                                mma(0, s0 + 2, s0 + 2, false);
+                                if (kb + 2 == nk) umma2_commit(&accfull[0]);
+                            }
+                            if (kb == 0) acquire(1);
+                            landed(s0 + 1);
+                            if (!ok) break;
+                            mma(1, s0 + 1, s0, kb == 0);
+                            mma(1, s0, s0 + 1, false);
+                            umma2_commit(&empty[s0 % CG_RING]);
+                            umma2_commit(&empty[(s0 + 1) % CG_RING]);
+                        }
+                        if (!ok) break;
+                        umma2_commit(&accfull[1]);
+                        fills[0]++;
+                        fills[1]++;
+                        st += 2 * nk;
+                    } else {
+                        acquire(turn);
+                        for (int kb = 0; kb < nk; kb++) {
+                            landed(st + kb);
+                            if (!ok) break;
+                            mma(turn, st + kb, st + kb, kb == 0);
+                            umma2_commit(&empty[(st + kb) % CG_RING]);
+                        }
+                        if (!ok) break;
+                        umma2_commit(&accfull[turn]);
+                        fills[turn]++;
+                        turn ^= 1;
+                        st += nk;
+                    }
+                }
+            }
+            if (!ok) abort_flag = 1;
+            umma2_commit(&mma_done);
+            mbar_wait_cluster(&mma_done, 0, p.status, 24);
+        }
+    } else {
+        // ---------------- epilogue warps: lane quarter q of the CTA's 128 rows, column half h
+        const int q = warp % 4, h = (warp - 2) / 4;
+        const uint32_t tq = tmem + ((uint32_t)(32 * q) << 16) + h * 128;
+        uint32_t filled[2] = {0, 0};
+        int turn = 0;
+        bool ok = true;
+        const uint32_t empty_addr[2] = {cluster_map(&accempty[0], 0), cluster_map(&accempty[1], 0)};
+        auto wait_full = [&](int a) {
+            bool w = true;
+            if (lane == 0) w = mbar_wait_cluster(&accfull[a], filled[a] & 1, p.status, 25);
+            filled[a]++;
+            ok = __shfl_sync(0xffffffffu, w, 0) && !*(volatile int*)&abort_flag;
+            if (!ok) abort_flag = 1;
+            tc_fence_after();
+        };
+        auto release = [&](int a) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(empty_addr[a]);
+        };
+        for (int u = pair; u < nunits && ok; u += npairs) {
+            const int l = u / ntiles;
+            int tm, tn;
+            crt_tile(u - l * ntiles, tiles_m, tiles_n, tm, tn);
+            const int row = (p.tm0 + tm) * CG_T + (int)rank * 128 + 32 * q + lane;
+            const int col0 = (p.tn0 + tn) * CG_T + h * 128;
+            const float pm = cfg->p[l], ip = cfg->invp[l], uw = cfg->u[l];
+            int16_t* yrow = p.y + ((int64_t)l * p.rows + (row - p.row0)) * p.ldy + col0;
+            // 32 reduced values (c: an integer below 2^22 / |uw| + ..) times the weight, plus what earlier
+            // K chunks left, mod p, to y
+            auto put = [&](int part, const float (&c)[32], bool add) {
+                if (row >= p.M) return;
+#pragma unroll
+                for (int g = 0; g < 4; g++) {
+                    if (col0 + part * 32 + g * 8 >= p.ldy) break;
+                    uint4* dst = reinterpret_cast<uint4*>(yrow + part * 32 + g * 8);
+                    uint32_t old[4] = {0, 0, 0, 0}, w[4];
+                    if (add) {
+                        const uint4 o4 = *dst;
+                        old[0] = o4.x, old[1] = o4.y, old[2] = o4.z, old[3] = o4.w;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        float z0 = c[g * 8 + 2 * i], z1 = c[g * 8 + 2 * i + 1];
+                        const float o0 = __int_as_float(0x4B400000 + (int)(int16_t)(old[i] & 0xffff)) - CRT_MAGIC;
+                        const float o1 = __int_as_float(0x4B400000 + ((int)old[i] >> 16)) - CRT_MAGIC;
+                        z0 = crt_mod(__fmaf_rn(z0, uw, o0), pm, ip) + CRT_MAGIC;
+                        z1 = crt_mod(__fmaf_rn(z1, uw, o1), pm, ip) + CRT_MAGIC;
+                        w[i] = __byte_perm(__float_as_uint(z0), __float_as_uint(z1), 0x5410);
+                    }
+                    *dst = make_uint4(w[0], w[1], w[2], w[3]);
+                }
+            };
+            for (int k0 = 0; k0 < p.nkb && ok; k0 += CG_KB) {
+                if (l < nsq) {
+                    const float b = c_crt.m[l].b, ib = c_crt.m[l].inv;
+                    uint32_t xr[64];
+                    wait_full(0);
+                    if (!ok) break;
+#pragma unroll
+                    for (int part = 0; part < 4; part++) {
+                        uint32_t v[32];
+                        tmem_ld32(tq + part * 32, v);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 16; i++) {
+                            const float x0 = crt_mod(__uint_as_float(v[2 * i]), pm, ip) + CRT_MAGIC;
+                            const float x1 = crt_mod(__uint_as_float(v[2 * i + 1]), pm, ip) + CRT_MAGIC;
+                            xr[part * 16 + i] = __byte_perm(__float_as_uint(x0), __float_as_uint(x1), 0x5410);
+                        }
+                    }
+                    release(0);
+                    wait_full(1);
+                    if (!ok) break;
+#pragma unroll
+                    for (int part = 0; part < 4; part++) {
+                        uint32_t v[32];
+                        float c[32];
+                        __syncwarp();  // rows past M skip their stores
+                        tmem_ld32(tq + 256 + part * 32, v);
+                        tmem_ld_wait();
+                        if (part == 3) release(1);
+#pragma unroll
+                        for (int i = 0; i < 32; i++) {
+                            const uint32_t w = xr[part * 16 + i / 2];
+                            const int xi = i % 2 ? (int)w >> 16 : (int)(int16_t)(w & 0xffff);
+                            const float x = __int_as_float(0x4B400000 + xi) - CRT_MAGIC;
+                            c[i] = __fmaf_rn(b, crt_mod(__uint_as_float(v[i]), b, ib), x);
+                        }
+                        put(part, c, k0 > 0);
+                    }
+                } else {
+                    wait_full(turn);
+                    if (!ok) break;
+#pragma unroll
+                    for (int part = 0; part < 4; part++) {
+                        uint32_t v[32];
+                        float c[32];
+                        __syncwarp();  // rows past M skip their stores
+                        tmem_ld32(tq + turn * 256 + part * 32, v);
+                        tmem_ld_wait();
+                        if (part == 3) release(turn);
+#pragma unroll
+                        for (int i = 0; i < 32; i++) c[i] = crt_mod(__uint_as_float(v[i]), pm, ip);
+                        put(part, c, k0 > 0);
+                    }
+                    turn ^= 1;
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    }
+}
+
+// ------------------------------------------------------------------ reconstruction
+// round(sign mag 2^X) of a 192-bit magnitude (w2, w1, w0), to nearest even.
+__device__ __forceinline__ double crt_round(unsigned long long w2, unsigned long long w1, unsigned long long w0,
+                                            bool neg, int X) {
+    if (w2) {  // five-limb sums only
+        const int z = 64 - __clzll((long long)w2);  // 1..64 bits to drop from the bottom
+        const unsigned long long lost = z == 64 ? w0 : w0 << (64 - z);
+        w0 = z == 64 ? w1 : (w0 >> z) | (w1 << (64 - z));
+        w1 = z == 64 ? w2 : (w1 >> z) | (w2 << (64 - z));
+        w0 |= lost ? 1ull : 0ull;
+        X += z;
+    }
+    if (!w1) {
+        if (!w0) return 0.0;
+        w1 = w0;
+        w0 = 0;
+        X -= 64;
+    }
+    const int z = __clzll((long long)w1);
+    const unsigned long long top = z ? (w1 << z) | (w0 >> (64 - z)) : w1;
+    const bool sticky = (w0 << z) != 0;
+    unsigned long long m = top >> 11;  // 53 bits
+    const uint32_t rem = ((uint32_t)top & 0x7FFu) << 1 | (sticky ? 1u : 0u);
+    m += rem > 0x800u || (rem == 0x800u && (m & 1ull));
+    // value = m 2^(X + 64 - z + 11), m in [2^52, 2^53]
+    const int E = X + 75 - z + 1075 - 1;  // biased exponent - 1 of m = 2^52..: the hidden bit adds 1
+    if (E >= 0 && E < 2045) {
+        const unsigned long long bits = ((unsigned long long)E << 52) + m;
+        return __longlong_as_double((long long)(bits | (neg ? 1ull << 63 : 0ull)));
+    }
+    const double v = (double)m;
+    return scale_pow2(neg ? -v : v, X + 75 - z);
+}
+
+// C' = sum - q M (limbs scaled by 2^sh), q = round(sum / M) from the top limb
+// (|sum| < 8 M): its 2^-17 of M is far inside what |C'| < 0.497 M leaves.
+template <int LIMBS>
+__device__ __forceinline__ double crt_value(long long (&acc)[LIMBS], float qinv, const int32_t* __restrict__ Ml,
+                                            int X) {
+    const long long t = acc[LIMBS - 1] + (acc[LIMBS - 2] >> 31);
+    const float tf = __int_as_float(0x4B400000 + (int)(t >> 13)) - CRT_MAGIC;
+    const int q = __float_as_int(__fmaf_rn(tf, qinv, CRT_MAGIC)) - 0x4B400000;
+#pragma unroll
+    for (int j = 0; j < LIMBS; j++) acc[j] -= (long long)q * Ml[j];
+#pragma unroll
+    for (int j = 0; j + 1 < LIMBS; j++) {
+        acc[j + 1] += acc[j] >> 31;
+        acc[j] &= 0x7FFFFFFFll;
+    }
+    unsigned long long w0, w1, w2 = 0;
+    const bool neg = acc[LIMBS - 1] < 0;
+    w0 = (unsigned long long)acc[0] | (unsigned long long)acc[1] << 31 | (unsigned long long)acc[2] << 62;
+    w1 = (unsigned long long)acc[2] >> 2 | (unsigned long long)acc[3] << 29;  // |C'| < 2^127: acc[3] << 29 keeps its sign
+    if constexpr (LIMBS == 5) {
+        w1 |= (unsigned long long)acc[4] << 60;
+        w2 = (unsigned long long)(acc[4] >> 4);
+    }
+    if (neg) {
+        w0 = ~w0 + 1;
+        w1 = ~w1 + (w0 == 0);
+        if constexpr (LIMBS == 5) w2 = ~w2 + (w0 == 0 && w1 == 0);
+    }
+    return crt_round(w2, w1, w0, neg, X);
+}
+
+struct CrtCombineParams {
+    int yrow0, row0;     // the first row in y; y's first row in C
+    int rows, yrows;     // rows to combine; rows of a plane of y
+    int c0, c1, n;       // columns [c0, c1) of C's n (complex: complex columns)
+    int64_t half, ldy;   // complex: column of the imaginary half in y
+    const int16_t* y;
+    const int* ea;
+    const int* eb;
+    double* C;
+    int cplx;
+    const SplitPlan* plan;
+    const CrtCfg* cfgs;
+};
+
+template <int LIMBS>
+__device__ __forceinline__ void crt_combine_body(const CrtCombineParams& p, const CrtCfg& c, int row, int j0,
+                                                 int ubits) {
+    // four values: columns j0 .. j0 + 3, or (re, im) of columns j0, j0 + 1
+    const int nmod = c.nmod;
+    const int64_t plane = (int64_t)p.yrows * p.ldy;
+    const int16_t* src = p.y + (int64_t)(p.yrow0 + row) * p.ldy + j0;
+    uint2 v[CRT_NB];
+#pragma unroll
+    for (int l = 0; l < CRT_NB; l++) {
+        v[l] = make_uint2(0, 0);
+        if (l < nmod) {
+            if (!p.cplx) {
+                v[l] = *reinterpret_cast<const uint2*>(src + l * plane);
+            } else {
+                const uint32_t re = *reinterpret_cast<const uint32_t*>(src + l * plane);
+                const uint32_t im = *reinterpret_cast<const uint32_t*>(src + l * plane + p.half);
+                v[l] = make_uint2(__byte_perm(re, im, 0x5410), __byte_perm(re, im, 0x7632));
+            }
+        }
+    }
+    long long acc[4][LIMBS];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < LIMBS; j++) acc[i][j] = 0;
+    // a group's residues first become one number modulo P (|z| < 2^24), so the
+    // wide multiplies are per group: 7 x LIMBS of them instead of 15 x LIMBS
+#pragma unroll
+    for (int g = 0; g < CRT_NG; g++) {
+        int z[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int l = 2 * g; l < (g + 1 < CRT_NG ? 2 * g + 2 : CRT_NB); l++) {
+            const int cl = c.c[l];
+            z[0] += (int)(int16_t)(v[l].x & 0xffff) * cl;
+            z[1] += ((int)v[l].x >> 16) * cl;
+            z[2] += (int)(int16_t)(v[l].y & 0xffff) * cl;
+            z[3] += ((int)v[l].y >> 16) * cl;
+        }
+#pragma unroll
+        for (int j = 0; j < LIMBS; j++) {
+            const int32_t wj = c.W[g][j];
+#pragma unroll
+            for (int i = 0; i < 4; i++) acc[i][j] += (long long)z[i] * wj;
+        }
+    }
+    const int64_t r = p.row0 + p.yrow0 + row;
+    const int X = ubits + p.ea[r] - c.sh;
+    double out[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int col = p.cplx ? j0 + i / 2 : j0 + i;
+        out[i] = col < p.c1 ? crt_value<LIMBS>(acc[i], c.qinv, c.M, X + p.eb[col]) : 0.0;
+    }
+    double* dst = p.C + (p.cplx ? 2 * (r * p.n + j0) : r * p.n + j0);
+    const int cnt = p.cplx ? 2 * (p.c1 - j0 < 2 ? p.c1 - j0 : 2) : (p.c1 - j0 < 4 ? p.c1 - j0 : 4);
+    if (cnt == 4 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+        reinterpret_cast<double2*>(dst)[0] = make_double2(out[0], out[1]);
+        reinterpret_cast<double2*>(dst)[1] = make_double2(out[2], out[3]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            if (i < cnt) dst[i] = out[i];
+    }
+}
+
+// Blocks of blockDim.x x blockDim.y = 256 threads over (columns, rows), four
+// values each along a row of C; blocks stride over the rows.
+__global__ void __launch_bounds__(256, 2) k_crt_combine(const __grid_constant__ CrtCombineParams p) {
+    __shared__ CrtCfg c;
+    if (p.plan->nonfinite) return;
+    {
+        const int* src = reinterpret_cast<const int*>(p.cfgs + p.plan->crt);
+        for (int i = threadIdx.y * blockDim.x + threadIdx.x; i < (int)(sizeof(CrtCfg) / 4); i += 256)
+            reinterpret_cast<int*>(&c)[i] = src[i];
+    }
+    __syncthreads();
+    const int ubits = -2 * (4 + 5 * (p.plan->s - 1));
+    const int j0 = p.c0 + (int)(blockIdx.x * blockDim.x + threadIdx.x) * (p.cplx ? 2 : 4);
+    if (j0 >= p.c1) return;
+    for (int row = blockIdx.y * blockDim.y + threadIdx.y; row < p.rows; row += gridDim.y * blockDim.y) {
+        if (c.limbs == 4) crt_combine_body<4>(p, c, row, j0, ubits);
+        else crt_combine_body<5>(p, c, row, j0, ubits);
+    }
+}
+
+// ------------------------------------------------------------------ host side
+// Every configuration worth having, by rising cost: squares of the first nsq
+// bases, the last `drop` bases left out.  Exact 192-bit arithmetic on 31-bit
+// limbs: M and M / p are products of the other moduli.
+struct CrtTable {
+    CrtCfg cfg[CRT_CFGS];
+    int n = 0;
+};
+
+static void crt_limbs_mul(int64_t (&a)[CRT_LIMBS + 1], int m) {
+    int64_t carry = 0;
+    for (int j = 0; j <= CRT_LIMBS; j++) {
+        const int64_t t = a[j] * m + carry;
+        a[j] = t & 0x7FFFFFFF;
+        carry = t >> 31;
+    }
+}
+
+static const CrtTable& crt_table() {
+    static const CrtTable table = [] {
+        CrtTable T;
+        float best = 0;
+        for (int cost = 9; cost <= 3 * CRT_NB; cost++) {
+            int bj = -1, bd = 0;
+            double bbits = 0;
+            for (int d = 0; d <= 6; d++) {
+                const int nmod = CRT_NB - d, j2 = cost - nmod;
+                if (j2 < 0 || j2 % 2 || j2 / 2 > nmod) continue;
+                double bits = 0;
+                for (int i = 0; i < nmod; i++) bits += (i < j2 / 2 ? 2 : 1) * log2((double)crt_base(i));
+                if (bits > bbits) bbits = bits, bj = j2 / 2, bd = d;
+            }
+            if (bj < 0 || bbits <= best || T.n >= CRT_CFGS) continue;
+            best = (float)bbits;
+            CrtCfg& c = T.cfg[T.n++];
+            c = CrtCfg{};
+            c.nmod = CRT_NB - bd;
+            c.nsq = bj;
+            c.cost = cost;
+            c.bits = (float)bbits;
+            c.limbs = bbits < 124.0 ? 4 : 5;
+            const auto mod = [&](int l) { return l < c.nsq ? crt_base(l) * crt_base(l) : crt_base(l); };
+            const int top = 31 * c.limbs;
+            c.sh = top - (int)ceil(bbits);  // M is never a power of two
+            const auto store = [&](int64_t(&a)[CRT_LIMBS + 1], int32_t* out) {
+                for (int i = 0; i < c.sh; i++) crt_limbs_mul(a, 2);
+                for (int j = 0; j < CRT_LIMBS; j++) out[j] = (int32_t)a[j];
+            };
+            int64_t M[CRT_LIMBS + 1] = {1};
+            for (int l = 0; l < c.nmod; l++) {
+                const int pl = mod(l);
+                crt_limbs_mul(M, pl);
+                int inv = 1, r = 1, cl = 1;
+                for (int i = 0; i < c.nmod; i++) {
+                    if (i == l) continue;
+                    r = (int)((int64_t)r * mod(i) % pl);  // M / p mod p
+                    if (crt_group(i) == crt_group(l)) cl *= mod(i);
+                }
+                while ((int64_t)inv * r % pl != 1 % pl) inv++;
+                c.p[l] = (float)pl;
+                c.invp[l] = 1.0f / (float)pl;
+                c.u[l] = (float)(2 * inv > pl ? inv - pl : inv);
+                c.c[l] = cl;
+            }
+            store(M, c.M);
+            for (int g = 0; g < CRT_NG; g++) {
+                int64_t W[CRT_LIMBS + 1] = {1};
+                for (int i = 0; i < c.nmod; i++)
+                    if (crt_group(i) != g) crt_limbs_mul(W, mod(i));
+                if (2 * g < c.nmod) store(W, c.W[g]);  // else no modulus: z is 0
+            }
+            c.qinv = (float)exp2((double)(top - 18) - bbits - c.sh);
+        }
+        return T;
+    }();
+    return table;
+}
+
+// The cheapest configuration that holds a sum of klen products of F-bit
+// integers with its sign (|C'| <= klen 2^(2F) < M / 2), or -1.
+static int crt_config(int s, int64_t klen) {
+    const CrtTable& T = crt_table();
+    const double need = 2.0 * (4 + 5 * (s - 1)) + log2((double)(klen > 1 ? klen : 1)) + 1.01;
+    for (int i = 0; i < T.n; i++)
+        if (T.cfg[i].bits >= need) return i;
+    return -1;
+}
+}  // namespace

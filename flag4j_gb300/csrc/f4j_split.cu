@@ -113,10 +113,17 @@ struct SplitPlan {
     int ngroups;    // groups per K chunk
     int nkb;        // K blocks of BKB bytes
     int kcb;        // K blocks per chunk
+    int crt;        // residue form: its configuration (the rounds and groups below are then unused)
+    int pad[3];
     Round rounds[MAX_ROUNDS];
     Group groups[MAX_GROUPS];
     Load loads[MAX_LOADS];
     Op ops[MAX_OPS];
+};
+
+// Residue-form configuration of each slice count, for k_finalize_pick.
+struct CrtPick {
+    int8_t cfg[S_MAX + 1];
 };
 
 struct SplitGemmParams {
@@ -423,14 +430,28 @@ __global__ void k_plan_table(int64_t Kp, int64_t klen_cat, int band, int kcb_cap
     P->nrounds = n;
 }
 
+// Plan header of a residue-form product (the slice program stays unused).
+__device__ __forceinline__ void crt_header(SplitPlan* plan, int s, const CrtPick& pick, float spread, int bad) {
+    plan->s = s;
+    plan->nrounds = 1;
+    plan->crt = pick.cfg[s];
+    plan->spread = spread;
+    plan->nonfinite = (bad != 0 || pick.cfg[s] < 0) ? 1 : 0;
+}
+
 // One block of 128 threads: k_plan's result from a plan table (the slice count
-// from the statistics, that plan copied, the header filled in).
+// from the statistics, that plan copied, the header filled in); for the
+// residue form (tab null) the header alone.
 __global__ void k_plan_pick(const int* __restrict__ misc, int64_t k, int64_t klen_cat, int s_req,
-                            const SplitPlan* __restrict__ tab, SplitPlan* __restrict__ plan) {
+                            const SplitPlan* __restrict__ tab, const CrtPick pick, SplitPlan* __restrict__ plan) {
     if (blockIdx.x != 0) return;
     const double spread = (misc[1] > misc[2] ? misc[1] : misc[2]) / 256.0;
     const int s = s_req > 0 ? (s_req > S_MAX ? S_MAX : (s_req < 2 ? 2 : s_req))
                             : slices_for(misc[1] / 256.0, misc[2] / 256.0, k, klen_cat);
+    if (!tab) {
+        if (threadIdx.x == 0) crt_header(plan, s, pick, (float)spread, misc[0]);
+        return;
+    }
     const uint4* src = reinterpret_cast<const uint4*>(&tab[s]);
     uint4* dst = reinterpret_cast<uint4*>(plan);
 #pragma unroll 4
@@ -449,8 +470,9 @@ __global__ void k_plan_pick(const int* __restrict__ misc, int64_t k, int64_t kle
 // blocks [0, cdiv(ta, 256)) finalise op(A)'s targets, the rest op(B)'s (dupb:
 // the complex B_cat's targets appear twice).  Each block counts itself done
 // on misc[4] (zeroed with misc before the statistics); the block that counts
-// last has seen every spread and picks the plan as k_plan_pick does.  No
-// block waits for another.
+// last has seen every spread and picks the plan as k_plan_pick does; for the
+// residue form (tab null) only the header, with the slice count's
+// configuration.  No block waits for another.
 __global__ void __launch_bounds__(256) k_finalize_pick(int64_t ta, int64_t tb, int dupb,
                                                        const unsigned long long* __restrict__ mxa,
                                                        const long long* __restrict__ esa,
@@ -461,7 +483,7 @@ __global__ void __launch_bounds__(256) k_finalize_pick(int64_t ta, int64_t tb, i
                                                        int* __restrict__ eb, int* misc, int64_t k,
                                                        int64_t klen_cat, int s_req,
                                                        const SplitPlan* __restrict__ tab,
-                                                       SplitPlan* __restrict__ plan) {
+                                                       const CrtPick pick, SplitPlan* __restrict__ plan) {
     const int64_t nba = (ta + 255) / 256;
     const bool is_b = (int64_t)blockIdx.x >= nba;
     const int64_t t = ((int64_t)blockIdx.x - (is_b ? nba : 0)) * 256 + threadIdx.x;
@@ -482,6 +504,10 @@ __global__ void __launch_bounds__(256) k_finalize_pick(int64_t ta, int64_t tb, i
     const double spread = (sa > sb ? sa : sb) / 256.0;
     const int s = s_req > 0 ? (s_req > S_MAX ? S_MAX : (s_req < 2 ? 2 : s_req))
                             : slices_for(sa / 256.0, sb / 256.0, k, klen_cat);
+    if (!tab) {
+        if (threadIdx.x == 0) crt_header(plan, s, pick, (float)spread, bad);
+        return;
+    }
     const uint4* src = reinterpret_cast<const uint4*>(&tab[s]);
     uint4* dst = reinterpret_cast<uint4*>(plan);
     for (int i = threadIdx.x; i < (int)(sizeof(SplitPlan) / 16); i += blockDim.x) dst[i] = src[i];
@@ -1303,6 +1329,14 @@ static int plan_table(f4j_ctx* ctx, int64_t Kp, int64_t klen_cat, int kcb_cap, S
     return F4J_OK;
 }
 
+// The static scratch of f4j_dgemm_split_noalloc and what a call needs of it
+// (see there).
+#define F4J_NOALLOC_SCRATCH_BYTES (32u << 20)
+#define F4J_NOALLOC_NEED(m, n, Kp) \
+    ((size_t)12 * (size_t)((m) + (n)) * (size_t)(Kp) + (size_t)24 * (size_t)((m) + (n)) + (size_t)16384)
+
+#include "f4j_crt.cuh"
+
 static int split_prepare(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, const double* A, int opA,
                          const double* B, int opB, double* C, int slices_req, SplitLaunch* L) {
     const int64_t M = m, N = cplx ? 2 * n : n;
@@ -1367,7 +1401,8 @@ static int split_prepare(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t 
         const unsigned blocks = (unsigned)(f4j_cdiv(M, 256) + f4j_cdiv(n, 256));
         k_finalize_pick<<<blocks, 256, 0, ctx->stream>>>(M, n, cplx ? 1 : 0, mxa, esa, cna, mxb, esb, cnb, ea, eb,
                                                          misc, k, klen_cat,
-                                                         slices_req > 0 ? slices_req : env_slices(), tab, plan);
+                                                         slices_req > 0 ? slices_req : env_slices(), tab, CrtPick{},
+                                                         plan);
         F4J_LAUNCHED(ctx);
     }
     {   // both operands' slice planes in one launch.  A: targets = rows of op(A),
@@ -1470,9 +1505,229 @@ static int split_report(f4j_ctx* ctx, const SplitPlan* plan, f4j_report* rep) {
     return F4J_OK;
 }
 
+// ------------------------------------------------------------------ residue form, host side
+// Whether a split product takes the residue form: a function of the shape
+// alone, so the device and the host-buffer path agree.  Not the shapes that
+// f4j_dgemm_split_noalloc accepts (its result is f4j_dgemm's bit for bit and
+// its scratch holds slice planes only), nor a forced small slice count.
+// Narrow and short products stay with the slices: the residue planes cost
+// about twice as much per element, the tiles are 256 wide, and reconstructing
+// C is work per entry that the slices do not have.  Measured on GB300, slices
+// / residues, us: 8192 x 8192 x 512 1731 / 2400, 3000 x 3000 x 500 316 / 402,
+// 1500 x 1500 x 1000 180 / 193, 2048 x 2048 x 1024 291 / 275, 700 x 700 x 2500
+// 208 / 158, 384 x 8192 x 8192 1750 / 1492, 8192^3 19200 / 11900; complex
+// 384 x 192 x 300 90 / 72, 1000 x 1000 x 300 200 / 171.
+static bool crt_wanted(bool cplx, int64_t m, int64_t n, int64_t k, int slices_req) {
+    const int req = slices_req > 0 ? slices_req : env_slices();
+    if (req > 0 && req < 8) return false;
+    const int64_t N = cplx ? 2 * n : n, klen = cplx ? 2 * k : k;
+    if (m < 384 || N < 384 || klen < (cplx ? 512 : 1024) || klen > (1 << 22)) return false;
+    if (!cplx && F4J_NOALLOC_NEED(m, n, f4j_cdiv(k, BKB) * BKB) <= F4J_NOALLOC_SCRATCH_BYTES) return false;
+    return crt_config(S_MAX, klen) >= 0;
+}
+
+static int make_crt_map(CUtensorMap* map, const void* base, uint64_t Kp, uint64_t rows, uint64_t planes) {
+    f4j_encode_tiled_fn enc = f4j_encode_fn();
+    if (!enc) return f4j_fail(F4J_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled unavailable");
+    cuuint64_t dims[3] = {Kp, rows, planes};
+    cuuint64_t strides[2] = {Kp, Kp * rows};
+    cuuint32_t box[3] = {CG_BK, 128, 1};
+    cuuint32_t es[3] = {1, 1, 1};
+    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box, es,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return f4j_fail(F4J_ERR_CUDA, "cuTensorMapEncodeTiled (residues) failed (%d)", (int)r);
+    return F4J_OK;
+}
+
+// The configurations' constants on the device, uploaded on the context's first use.
+static int crt_device_table(f4j_ctx* ctx, const CrtCfg** out) {
+    if (!ctx->crt_tab) {
+        const CrtTable& T = crt_table();
+        F4J_CUDA(cudaMalloc(&ctx->crt_tab, sizeof T.cfg));
+        cudaError_t e = cudaMemcpy(ctx->crt_tab, T.cfg, sizeof T.cfg, cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) {
+            cudaFree(ctx->crt_tab);
+            ctx->crt_tab = nullptr;
+            return f4j_cuda_fail(e, "residue constants");
+        }
+    }
+    *out = (const CrtCfg*)ctx->crt_tab;
+    return F4J_OK;
+}
+
+// Residues of C (2 bytes per modulus and entry) up to this size are kept for
+// all of C; a larger product goes in row blocks of it.
+constexpr size_t CRT_Y_BYTES = size_t(4) << 30;
+
+// A residue-form product's sizes and workspace.
+struct CrtSetup {
+    int64_t half, M, N, Kh, Kp, klen, ldy, blk, yrows;  // blk: tile rows per row block of C, yrows its rows
+    int tiles_m, tiles_n, planes, nmod;
+    CrtPick pick;
+    const CrtCfg* cfgs;
+    SmallLayout Lo;
+    size_t plane_a, plane_b;
+    char* w;
+    unsigned long long *mxa, *mxb;
+    long long *esa, *esb;
+    int *cna, *cnb, *ea, *eb, *misc;
+    SplitPlan* plan;
+    uint8_t *plA, *plB;
+    int16_t* y;
+    CUtensorMap ta, tb;
+    size_t smem;
+};
+
+static int crt_setup(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, CrtSetup* S) {
+    S->half = cplx ? f4j_cdiv(n, 8) * 8 : 0;  // the imaginary half's first row of B_cat^T
+    S->M = m;
+    S->N = cplx ? 2 * S->half : n;
+    S->Kh = f4j_cdiv(k, BKB) * BKB;
+    S->Kp = cplx ? 2 * S->Kh : S->Kh;
+    S->klen = cplx ? 2 * k : k;
+    if (S->M > INT32_MAX || S->N > INT32_MAX || S->Kp > INT32_MAX)
+        return f4j_fail(F4J_ERR_ARG, "split GEMM too large");
+    const int req = env_slices();
+    const int s_max = req > 0 ? (req > S_MAX ? S_MAX : req) : S_MAX;
+    S->planes = S->nmod = 0;  // the most any slice count needs
+    for (int s = 0; s <= S_MAX; s++) {
+        S->pick.cfg[s] = (int8_t)(s < 2 || s > s_max ? -1 : crt_config(s, S->klen));
+        if (S->pick.cfg[s] < 0) continue;
+        const CrtCfg& c = crt_table().cfg[S->pick.cfg[s]];
+        S->planes = c.nmod + c.nsq > S->planes ? c.nmod + c.nsq : S->planes;
+        S->nmod = c.nmod > S->nmod ? c.nmod : S->nmod;
+    }
+    int rc = crt_device_table(ctx, &S->cfgs);
+    if (rc) return rc;
+    S->Lo = small_layout(S->M, n, cplx ? 2 * n : n);
+    S->plane_a = (size_t)S->M * S->Kp;
+    S->plane_b = (size_t)S->N * S->Kp;
+    S->ldy = f4j_cdiv(S->N, 8) * 8;
+    S->tiles_m = (int)f4j_cdiv(S->M, CG_T);
+    S->tiles_n = (int)f4j_cdiv(S->N, CG_T);
+    const int64_t fit = (int64_t)(CRT_Y_BYTES / ((size_t)S->nmod * S->ldy * 2)) / CG_T;
+    S->blk = fit < 1 ? 1 : (fit > S->tiles_m ? S->tiles_m : fit);
+    S->yrows = S->blk * CG_T < S->M ? S->blk * CG_T : S->M;
+    void *ws1, *ws0;
+    rc = f4j_workspace(ctx, ctx->ws_base + 1, S->Lo.total, &ws1);
+    if (rc) return rc;
+    const size_t pa = al1k(S->plane_a * S->planes), pb = al1k(S->plane_b * S->planes);
+    rc = f4j_workspace(ctx, ctx->ws_base, pa + pb + (size_t)S->nmod * S->yrows * S->ldy * 2, &ws0);
+    if (rc) return rc;
+    char* w = S->w = (char*)ws1;
+    S->mxa = (unsigned long long*)(w + S->Lo.mxa);
+    S->esa = (long long*)(w + S->Lo.esa);
+    S->cna = (int*)(w + S->Lo.cna);
+    S->mxb = (unsigned long long*)(w + S->Lo.mxb);
+    S->esb = (long long*)(w + S->Lo.esb);
+    S->cnb = (int*)(w + S->Lo.cnb);
+    S->ea = (int*)(w + S->Lo.ea);
+    S->eb = (int*)(w + S->Lo.eb);
+    S->misc = (int*)(w + S->Lo.misc);
+    S->plan = (SplitPlan*)(w + S->Lo.plan);
+    S->plA = (uint8_t*)ws0;
+    S->plB = S->plA + pa;
+    S->y = (int16_t*)(S->plB + pb);
+    rc = make_crt_map(&S->ta, S->plA, S->Kp, S->M, S->planes);
+    if (rc) return rc;
+    rc = make_crt_map(&S->tb, S->plB, S->Kp, S->N, S->planes);
+    if (rc) return rc;
+    S->smem = (size_t)CG_RING * CG_SLOT + 1024;
+    F4J_CUDA(cudaFuncSetAttribute(k_crt_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S->smem));
+    return F4J_OK;
+}
+
+// The products of tile rows [tm0, tm1) x tile columns [tn0, tn1) and their
+// reconstruction into C, on `stream`; y holds rows [row0, row0 + S.yrows).
+static int crt_launch(f4j_ctx* ctx, const CrtSetup& S, bool cplx, int64_t n, double* C, cudaStream_t stream, int tm0,
+                      int tm1, int tn0, int tn1, int row0) {
+    const int64_t r0 = (int64_t)tm0 * CG_T, r1 = (int64_t)tm1 * CG_T < S.M ? (int64_t)tm1 * CG_T : S.M;
+    // complex launches cover every tile column
+    const int64_t c0 = cplx ? 0 : (int64_t)tn0 * CG_T, c1 = cplx || (int64_t)tn1 * CG_T > n ? n : (int64_t)tn1 * CG_T;
+    if (tm0 < 0 || tm1 > S.tiles_m || tm0 >= tm1 || tn0 < 0 || tn1 > S.tiles_n || tn0 >= tn1 || r0 < row0 ||
+        r1 > row0 + S.yrows || (cplx && (tn0 != 0 || tn1 != S.tiles_n)))
+        return f4j_fail(F4J_ERR_ARG, "residue GEMM tile range [%d, %d) x [%d, %d)", tm0, tm1, tn0, tn1);
+    CrtGemmParams g{(int)S.M, (int)S.N, (int)f4j_cdiv(S.Kp, CG_BK), tm0, tm1, tn0, tn1, row0, (int)S.yrows, S.ldy, S.y,
+                    ctx->d_status + F4J_ST_TIMEOUT, S.plan, S.cfgs};
+    const int64_t units = (int64_t)(tm1 - tm0) * (tn1 - tn0) * S.nmod;
+    const int pairs = (int)(units < ctx->sm_count / 2 ? units : ctx->sm_count / 2);
+    const cudaStream_t saved = ctx->stream;
+    ctx->stream = stream;
+    f4j_prof_begin(ctx);
+    k_crt_gemm<<<2 * pairs, CG_THREADS, S.smem, stream>>>(S.ta, S.tb, g);
+    f4j_prof_end(ctx);
+    ctx->stream = saved;
+    F4J_LAUNCHED(ctx);
+    CrtCombineParams cp{(int)(r0 - row0), row0, (int)(r1 - r0), (int)S.yrows, (int)c0, (int)c1, (int)n, S.half, S.ldy,
+                        S.y, S.ea, S.eb, C, cplx ? 1 : 0, S.plan, S.cfgs};
+    const int64_t per_row = f4j_cdiv(c1 - c0, cplx ? 2 : 4);
+    unsigned bx = 32;  // threads along a row
+    while (bx < 256 && bx < per_row) bx *= 2;
+    const int64_t gx = f4j_cdiv(per_row, bx), gy = f4j_cdiv(r1 - r0, 256 / bx);
+    int64_t cap = 16 * (int64_t)ctx->sm_count / gx;  // a few blocks per resident slot, each over several rows
+    cap = cap < 1 ? 1 : (cap > 65535 ? 65535 : cap);
+    k_crt_combine<<<dim3((unsigned)gx, (unsigned)(gy < cap ? gy : cap)), dim3(bx, 256 / bx), 0, stream>>>(cp);
+    F4J_LAUNCHED(ctx);
+    return F4J_OK;
+}
+
+// Asynchronous residue-form GEMM: statistics -> device plan -> residue planes
+// -> products -> reconstruction, queued on the context stream as
+// f4j_gemm_split's slice form is.
+static int crt_gemm(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, const double* A, int opA,
+                    const double* B, int opB, double* C, const SplitPlan** plan_out) {
+    CrtSetup S;
+    int rc = crt_setup(ctx, cplx, m, n, k, &S);
+    if (rc) return rc;
+    const int64_t M = S.M;
+    F4J_CUDA(cudaMemsetAsync(S.w, 0, S.Lo.plan, ctx->stream));
+    const bool a_rows = opA == F4J_OP_N, b_rows = opB != F4J_OP_N;
+    f4j_prof_begin(ctx, F4J_PROF_PREP);
+    if (a_rows)
+        k_stats_rows<<<(unsigned)f4j_cdiv(M, 8), 256, 0, ctx->stream>>>(A, M, k, cplx, S.mxa, S.esa, S.cna, S.misc);
+    else
+        launch_stats_cols(A, k, M, M, cplx, ctx->sm_count, S.mxa, S.esa, S.cna, S.misc, ctx->stream);
+    F4J_LAUNCHED(ctx);
+    if (b_rows)
+        k_stats_rows<<<(unsigned)f4j_cdiv(n, 8), 256, 0, ctx->stream>>>(B, n, k, cplx, S.mxb, S.esb, S.cnb, S.misc);
+    else
+        launch_stats_cols(B, k, n, n, cplx, ctx->sm_count, S.mxb, S.esb, S.cnb, S.misc, ctx->stream);
+    F4J_LAUNCHED(ctx);
+    k_finalize_pick<<<(unsigned)(f4j_cdiv(M, 256) + f4j_cdiv(n, 256)), 256, 0, ctx->stream>>>(
+        M, n, 0, S.mxa, S.esa, S.cna, S.mxb, S.esb, S.cnb, S.ea, S.eb, S.misc, k, S.klen, env_slices(), nullptr,
+        S.pick, S.plan);
+    F4J_LAUNCHED(ctx);
+    {
+        const CrtOperand oa{A, a_rows ? k : M, a_rows ? 0 : 1, opA == F4J_OP_C ? 1 : 0, 0, M, M, 0, S.ea, S.plA};
+        const CrtOperand ob{B, b_rows ? k : n, b_rows ? 0 : 1, opB == F4J_OP_C ? 1 : 0, 1, n, S.N, S.half, S.eb, S.plB};
+        const dim3 grid((unsigned)(S.Kh / SP_TQ), slice_grid_y(M > n ? M : n), 2);
+        if (cplx) k_crt_planes<true><<<grid, 256, 0, ctx->stream>>>(oa, ob, k, S.Kh, S.Kp, S.plan, S.cfgs);
+        else k_crt_planes<false><<<grid, 256, 0, ctx->stream>>>(oa, ob, k, S.Kh, S.Kp, S.plan, S.cfgs);
+        F4J_LAUNCHED(ctx);
+    }
+    f4j_prof_end(ctx);
+    for (int t0 = 0; t0 < S.tiles_m; t0 += (int)S.blk) {
+        const int t1 = t0 + (int)S.blk < S.tiles_m ? t0 + (int)S.blk : S.tiles_m;
+        rc = crt_launch(ctx, S, cplx, n, C, ctx->stream, t0, t1, 0, S.tiles_n, t0 * CG_T);
+        if (rc) return rc;
+    }
+    *plan_out = S.plan;
+    return F4J_OK;
+}
+
 int f4j_gemm_split(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, const double* A, int opA,
                    const double* B, int opB, double* C, int slices_req, f4j_report* rep, const int** gate) {
     *gate = nullptr;
+    if (crt_wanted(cplx, m, n, k, slices_req)) {
+        const SplitPlan* plan = nullptr;
+        const int rc = crt_gemm(ctx, cplx, m, n, k, A, opA, B, opB, C, &plan);
+        if (rc != F4J_ERR_OOM) {
+            if (rc) return rc;
+            *gate = &plan->nonfinite;
+            return rep ? split_report(ctx, plan, rep) : F4J_OK;
+        }  // no room for the residue planes: the slice form needs less than half
+    }
     SplitLaunch L;
     int rc = split_prepare(ctx, cplx, m, n, k, A, opA, B, opB, C, slices_req, &L);
     if (rc) return rc;
@@ -1490,11 +1745,11 @@ int f4j_gemm_split(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, con
 // quarter of A when that is less), the second as many, the last 1/8 of the
 // tile rows and the rest is cut into equal middle parts; every part keeps at
 // least one tile row.
-static void host_part_bounds(int tiles_m, int parts, int* bound) {
+static void host_part_bounds(int tiles_m, int parts, int* bound, int first = 8) {
     bound[0] = 0;
     bound[1] = tiles_m;
     if (parts < 2) return;
-    const int a0 = tiles_m / 4 < 1 ? 1 : (tiles_m / 4 > 8 ? 8 : tiles_m / 4);
+    const int a0 = tiles_m / 4 < 1 ? 1 : (tiles_m / 4 > first ? first : tiles_m / 4);
     const int last = tiles_m / 8 < 1 ? 1 : tiles_m / 8;
     bound[parts] = tiles_m;
     bound[1] = a0;
@@ -1523,7 +1778,8 @@ static void host_part_bounds(int tiles_m, int parts, int* bound) {
 // caller then runs the ordinary path.  When the counts agree, every exponent,
 // slice, plan and tile sum is the ordinary path's, and so is every bit of C.
 // Waits for everything it queued before returning; *spread_out receives the
-// spread all of A and B give.
+// spread all of A and B give.  `crt`: the residue form, the same pipeline with
+// residue planes, 256 x 256 tiles and a reconstruction behind each product.
 //
 // Part sizes.  A's first part has up to 8 tile rows (all of A in one part
 // when parts == 1): its product with one of
@@ -1538,9 +1794,10 @@ static void host_part_bounds(int tiles_m, int parts, int* bound) {
 // beside a slice GEMM (its CTA fills two of an SM's four register files and
 // all but ~1 KB of its shared memory), so they wait for SMs whenever the
 // products before them hold every SM; these sizes keep that wait short.
+constexpr int CRT_HOST_FIRST = 4;  // A's first part in 256-row tiles: as many rows as the slice form's 8
 static int host_split_pipelined(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, const double* A,
-                                const double* B, int opB, double* C, double* dA, double* dB, double* dC, int parts,
-                                int bparts, bool* recompute, const SplitPlan** plan_out, float* spread_out) {
+                                const double* B, int opB, double* C, double* dA, double* dB, double* dC, bool crt,
+                                int parts, int bparts, bool* recompute, const SplitPlan** plan_out, float* spread_out) {
     *recompute = false;
     // complex: the [Re | Im] concatenation of the ordinary path (2n slice rows
     // of B, K of 2 Kh), interleaved (re, im) doubles in host and device memory
@@ -1550,14 +1807,24 @@ static int host_split_pipelined(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, i
     const int64_t klen_cat = cplx ? 2 * k : k;
     const int64_t w2 = cplx ? 2 : 1;  // doubles per element
     if (M > INT32_MAX || N > INT32_MAX || Kp > INT32_MAX) return f4j_fail(F4J_ERR_ARG, "host-buffer split GEMM too large");
+    // the residue form (crt) has workspace and tensor maps of its own
+    CrtSetup R;
+    int rc = F4J_OK;
+    if (crt) {
+        rc = crt_setup(ctx, cplx, m, n, k, &R);
+        if (rc) return rc;
+        if (R.blk < R.tiles_m) return f4j_fail(F4J_ERR_ARG, "residue-form product in parts and row blocks");
+    }
     const SmallLayout Lo = small_layout(M, n, N);
-    void *ws1, *ws0;
-    int rc = f4j_workspace(ctx, ctx->ws_base + 1, Lo.total, &ws1);
-    if (rc) return rc;
+    void *ws1 = nullptr, *ws0 = nullptr;
     const size_t plane_a = (size_t)M * Kp, plane_b = (size_t)N * Kp;
-    rc = f4j_workspace(ctx, ctx->ws_base, al1k(plane_a * S_MAX) + al1k(plane_b * S_MAX), &ws0);
-    if (rc) return rc;
-    char* w = (char*)ws1;
+    if (!crt) {
+        rc = f4j_workspace(ctx, ctx->ws_base + 1, Lo.total, &ws1);
+        if (rc) return rc;
+        rc = f4j_workspace(ctx, ctx->ws_base, al1k(plane_a * S_MAX) + al1k(plane_b * S_MAX), &ws0);
+        if (rc) return rc;
+    }
+    char* w = crt ? R.w : (char*)ws1;  // both forms lay it out alike
     unsigned long long* mxa = (unsigned long long*)(w + Lo.mxa);
     long long* esa = (long long*)(w + Lo.esa);
     int* cna = (int*)(w + Lo.cna);
@@ -1568,23 +1835,26 @@ static int host_split_pipelined(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, i
     int* eb = (int*)(w + Lo.eb);
     int* misc = (int*)(w + Lo.misc);  // [0] non-finite, [1] spread of A so far, [2] of B, [5] the check
     SplitPlan* plan = (SplitPlan*)(w + Lo.plan);
-    uint8_t* slA = (uint8_t*)ws0;
-    uint8_t* slB = slA + al1k(plane_a * S_MAX);
+    uint8_t* slA = crt ? R.plA : (uint8_t*)ws0;
+    uint8_t* slB = crt ? R.plB : slA + al1k(plane_a * S_MAX);
     const bool b_rows = opB != F4J_OP_N;  // columns of op(B) are stored rows of B (n x k)
     const int conjb = cplx && opB == F4J_OP_C ? 1 : 0;
     const auto split_k = cplx ? k_split<true> : k_split<false>;
+    const auto planes_k = cplx ? k_crt_planes<true> : k_crt_planes<false>;
     const int s_req = env_slices();
     // the same K-chunk cap the ordinary path plans with (no split K here)
     int kchunks = 0;
-    const int kcb_cap = split_kcb_cap(f4j_cdiv(M, BM) * f4j_cdiv(N, BN), Kp / BKB, &kchunks);
+    const int kcb_cap = crt ? 0 : split_kcb_cap(f4j_cdiv(M, BM) * f4j_cdiv(N, BN), Kp / BKB, &kchunks);
     if (kchunks) return f4j_fail(F4J_ERR_ARG, "split-K product in parts");
     const cudaStream_t st = ctx->stream;
 
     SplitLaunch L;
-    rc = make_slice_map(&L.ta, slA, Kp, M, S_MAX);
-    if (rc) return rc;
-    rc = make_slice_map(&L.tb, slB, Kp, N, S_MAX);
-    if (rc) return rc;
+    if (!crt) {
+        rc = make_slice_map(&L.ta, slA, Kp, M, S_MAX);
+        if (rc) return rc;
+        rc = make_slice_map(&L.tb, slB, Kp, N, S_MAX);
+        if (rc) return rc;
+    }
     SplitGemmParams& prm = L.prm;
     prm = SplitGemmParams{};
     prm.M = (int)M;
@@ -1598,8 +1868,10 @@ static int host_split_pipelined(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, i
     prm.status = ctx->d_status + F4J_ST_TIMEOUT;
     prm.plan = plan;
     prm.wpart = nullptr;
-    L.tiles_m = (int)f4j_cdiv(M, BM);
-    L.tiles_n = (int)f4j_cdiv(N, BN);
+    const int64_t tile = crt ? CG_T : BM;  // parts are whole tiles of C
+    static_assert(BM == BN, "square tiles");
+    L.tiles_m = (int)f4j_cdiv(M, tile);
+    L.tiles_n = crt ? R.tiles_n : (int)f4j_cdiv(N, tile);
     L.kchunks = 0;
     prm.tm0 = 0;
     prm.tm1 = L.tiles_m;
@@ -1611,7 +1883,7 @@ static int host_split_pipelined(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, i
     if (parts < 1 || parts > tiles_m || parts > F4J_HOST_PARTS_MAX)
         return f4j_fail(F4J_ERR_ARG, "%d row parts of %d tile rows", parts, tiles_m);
     int bound[F4J_HOST_PARTS_MAX + 1];
-    host_part_bounds(tiles_m, parts, bound);
+    host_part_bounds(tiles_m, parts, bound, crt ? CRT_HOST_FIRST : 8);
     // complex: B whole (its column parts would fall on both halves of the
     // concatenation)
     const int qb = cplx ? 1 : (bparts < tiles_n ? bparts : tiles_n);
@@ -1625,7 +1897,7 @@ static int host_split_pipelined(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, i
     auto queue = [&]() -> int {
         F4J_CUDA(cudaMemsetAsync(w, 0, Lo.plan, st));
         SplitPlan* tab = nullptr;
-        rc = plan_table(ctx, Kp, klen_cat, kcb_cap, &tab);
+        if (!crt) rc = plan_table(ctx, Kp, klen_cat, kcb_cap, &tab);
         if (rc) return rc;
 
         // Every upload goes up back to back on the upload stream, in the order the
@@ -1636,12 +1908,12 @@ static int host_split_pipelined(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, i
         F4J_CUDA(cudaStreamWaitEvent(up, ctx->up_start, 0));
         {
             int u = 0;
-            const int64_t r1 = (int64_t)bound[1] * BM < m ? (int64_t)bound[1] * BM : m;
+            const int64_t r1 = (int64_t)bound[1] * tile < m ? (int64_t)bound[1] * tile : m;
             F4J_CUDA(cudaMemcpyAsync(dA, A, (size_t)r1 * k * 8 * w2, cudaMemcpyHostToDevice, up));
             F4J_CUDA(cudaEventRecord(ctx->up_ev[u++], up));
             for (int j = 0; j < qb; j++) {
-                const int64_t c0 = (int64_t)cbound[j] * BN;
-                const int64_t c1 = (int64_t)cbound[j + 1] * BN < n ? (int64_t)cbound[j + 1] * BN : n;
+                const int64_t c0 = (int64_t)cbound[j] * tile;
+                const int64_t c1 = (int64_t)cbound[j + 1] * tile < n ? (int64_t)cbound[j + 1] * tile : n;
                 if (b_rows)  // stored rows [c0, c1) of B (n x k)
                     F4J_CUDA(cudaMemcpyAsync(dB + c0 * k * w2, B + c0 * k * w2, (size_t)(c1 - c0) * k * 8 * w2,
                                              cudaMemcpyHostToDevice, up));
@@ -1651,8 +1923,8 @@ static int host_split_pipelined(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, i
                 F4J_CUDA(cudaEventRecord(ctx->up_ev[u++], up));
             }
             for (int p = 1; p < parts; p++) {
-                const int64_t r0 = (int64_t)bound[p] * BM;
-                const int64_t re = (int64_t)bound[p + 1] * BM < m ? (int64_t)bound[p + 1] * BM : m;
+                const int64_t r0 = (int64_t)bound[p] * tile;
+                const int64_t re = (int64_t)bound[p + 1] * tile < m ? (int64_t)bound[p + 1] * tile : m;
                 F4J_CUDA(cudaMemcpyAsync(dA + r0 * k * w2, A + r0 * k * w2, (size_t)(re - r0) * k * 8 * w2,
                                          cudaMemcpyHostToDevice, up));
                 F4J_CUDA(cudaEventRecord(ctx->up_ev[u++], up));
@@ -1672,8 +1944,14 @@ static int host_split_pipelined(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, i
         };
         // its slice planes: target t of the part is row r0 + t
         auto a_part_split = [&](int64_t r0, int64_t rows) -> int {
-            split_k<<<dim3((unsigned)(Kh / SP_TQ), slice_grid_y(rows)), 256, 0, st>>>(
-                dA + r0 * k * w2, rows, k, 0, 0, 0, rows, k, Kh, Kp, M, ea + r0, plan, slA + r0 * Kp);
+            const dim3 grid((unsigned)(Kh / SP_TQ), slice_grid_y(rows));
+            if (crt) {
+                const CrtOperand o{dA + r0 * k * w2, k, 0, 0, 0, rows, M, 0, ea + r0, slA + r0 * Kp};
+                planes_k<<<grid, 256, 0, st>>>(o, o, k, Kh, Kp, plan, R.cfgs);
+            } else {
+                split_k<<<grid, 256, 0, st>>>(dA + r0 * k * w2, rows, k, 0, 0, 0, rows, k, Kh, Kp, M, ea + r0, plan,
+                                              slA + r0 * Kp);
+            }
             F4J_LAUNCHED(ctx);
             return F4J_OK;
         };
@@ -1685,10 +1963,11 @@ static int host_split_pipelined(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, i
             const cudaStream_t ps = ctx->part_stream[id];
             F4J_CUDA(cudaStreamWaitEvent(ps, ctx->part_prep_ev[id], 0));
             launched = id + 1;
-            int r = split_launch(ctx, L, ps, tm0, tm1, tn0, tn1);
+            int r = crt ? crt_launch(ctx, R, cplx, n, dC, ps, tm0, tm1, tn0, tn1, 0)
+                        : split_launch(ctx, L, ps, tm0, tm1, tn0, tn1);
             if (r) return r;
-            const int64_t r0 = (int64_t)tm0 * BM, r1 = (int64_t)tm1 * BM < m ? (int64_t)tm1 * BM : m;
-            const int64_t c0 = (int64_t)tn0 * BN, c1 = (int64_t)tn1 * BN < n ? (int64_t)tn1 * BN : n;
+            const int64_t r0 = (int64_t)tm0 * tile, r1 = (int64_t)tm1 * tile < m ? (int64_t)tm1 * tile : m;
+            const int64_t c0 = (int64_t)tn0 * tile, c1 = (int64_t)tn1 * tile < n ? (int64_t)tn1 * tile : n;
             F4J_CUDA(cudaMemcpy2DAsync(C + (r0 * n + c0) * w2, (size_t)n * 8 * w2, dC + (r0 * n + c0) * w2,
                                        (size_t)n * 8 * w2, (size_t)(c1 - c0) * 8 * w2, (size_t)(r1 - r0),
                                        cudaMemcpyDeviceToHost, ps));
@@ -1697,11 +1976,11 @@ static int host_split_pipelined(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, i
         };
 
         // A's first rows, then B's column parts, each multiplied by those rows
-        const int64_t a0_rows = (int64_t)bound[1] * BM < m ? (int64_t)bound[1] * BM : m;
+        const int64_t a0_rows = (int64_t)bound[1] * tile < m ? (int64_t)bound[1] * tile : m;
         rc = a_part_stats(0, 0, a0_rows);
         for (int j = 0; j < qb && !rc; j++) {
-            const int64_t c0 = (int64_t)cbound[j] * BN;
-            const int64_t c1 = (int64_t)cbound[j + 1] * BN < n ? (int64_t)cbound[j + 1] * BN : n;
+            const int64_t c0 = (int64_t)cbound[j] * tile;
+            const int64_t c1 = (int64_t)cbound[j + 1] * tile < n ? (int64_t)cbound[j + 1] * tile : n;
             const int64_t cw = c1 - c0;
             F4J_CUDA(cudaStreamWaitEvent(st, ctx->up_ev[1 + j], 0));
             if (b_rows) {  // stored rows [c0, c1) of B (n x k)
@@ -1717,21 +1996,28 @@ static int host_split_pipelined(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, i
                                                                            cnb + c0, eb + c0, misc + 2);
             F4J_LAUNCHED(ctx);
             if (j == 0) {  // the plan from A's first rows and B's first columns, then those rows' slices
-                k_plan_pick<<<1, 128, 0, st>>>(misc, k, klen_cat, s_req, tab, plan);
+                k_plan_pick<<<1, 128, 0, st>>>(misc, k, klen_cat, s_req, tab, crt ? R.pick : CrtPick{}, plan);
                 F4J_LAUNCHED(ctx);
                 rc = a_part_split(0, a0_rows);
                 if (rc) break;
             }
-            split_k<<<dim3((unsigned)(Kh / SP_TQ), slice_grid_y(cw)), 256, 0, st>>>(
-                b_rows ? dB + c0 * k * w2 : dB + c0 * w2, b_rows ? cw : k, b_rows ? k : n, b_rows ? 0 : 1, conjb, 1,
-                cw, k, Kh, Kp, N, eb + c0, plan, slB + c0 * Kp);
+            const dim3 grid((unsigned)(Kh / SP_TQ), slice_grid_y(cw));
+            const double* src = b_rows ? dB + c0 * k * w2 : dB + c0 * w2;
+            if (crt) {
+                const CrtOperand o{src, b_rows ? k : n, b_rows ? 0 : 1, conjb, 1, cw, R.N, R.half, eb + c0,
+                                   slB + c0 * Kp};
+                planes_k<<<grid, 256, 0, st>>>(o, o, k, Kh, Kp, plan, R.cfgs);
+            } else {
+                split_k<<<grid, 256, 0, st>>>(src, b_rows ? cw : k, b_rows ? k : n, b_rows ? 0 : 1, conjb, 1, cw, k,
+                                              Kh, Kp, N, eb + c0, plan, slB + c0 * Kp);
+            }
             F4J_LAUNCHED(ctx);
             rc = product(j, 0, bound[1], cbound[j], cbound[j + 1]);
         }
         // the rest of A, each row part multiplied by all of B
         for (int p = 1; p < parts && !rc; p++) {
-            const int64_t r0 = (int64_t)bound[p] * BM;
-            const int64_t r1 = (int64_t)bound[p + 1] * BM < m ? (int64_t)bound[p + 1] * BM : m;
+            const int64_t r0 = (int64_t)bound[p] * tile;
+            const int64_t r1 = (int64_t)bound[p + 1] * tile < m ? (int64_t)bound[p + 1] * tile : m;
             rc = a_part_stats(qb + p, r0, r1 - r0);
             if (!rc) rc = a_part_split(r0, r1 - r0);
             if (!rc) rc = product(qb + p - 1, bound[p], bound[p + 1], 0, tiles_n);
@@ -1834,27 +2120,32 @@ static int gemm_host(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, c
     if (rc) return rc;
     // n == 1 runs the device path's matrix-vector kernel
     const bool split = k > 0 && n > 1 && f4j_resolve_mode(cplx, m, n, k, mode) == F4J_MODE_SPLIT;
-    const int tiles_m = (int)f4j_cdiv(m, BM);
+    // the residue form's parts are whole 256 x 256 tiles and need all of C's residues at once
+    const bool crt = split && crt_wanted(cplx, m, n, k, 0);
+    const int tile = crt ? CG_T : BM;
+    const int tiles_m = (int)f4j_cdiv(m, tile);
     const int want = env_host_parts("F4J_HOST_PARTS", F4J_HOST_PARTS);
     const int parts = tiles_m < want ? tiles_m : want;
     const int bparts = env_host_parts("F4J_HOST_BPARTS", F4J_HOST_BPARTS);
     const int64_t ncat = cplx ? 2 * n : n;  // slice rows of B (the [Re | Im] concatenation when complex)
-    const int tiles_n = (int)f4j_cdiv(ncat, BN);
+    const int tiles_n = (int)f4j_cdiv(ncat, tile);
     // pipelined when A has two row parts or B two column parts (real only)
     const bool piped = parts >= 2 || (!cplx && bparts >= 2 && tiles_n >= 2);
     int kchunks = 0;
-    split_kcb_cap(tiles_m * (int64_t)tiles_n, (cplx ? 2 : 1) * f4j_cdiv(k, BKB), &kchunks);
-    if (!split || opA != F4J_OP_N || !piped || kchunks) {  // split K runs as one launch
+    if (!crt) split_kcb_cap(tiles_m * (int64_t)tiles_n, (cplx ? 2 : 1) * f4j_cdiv(k, BKB), &kchunks);
+    const bool blocks = crt && (size_t)CRT_NB * 2 * (m + CG_T) * (ncat + 16) > CRT_Y_BYTES;
+    auto in_turn = [&]() -> int {  // upload, multiply, download
         if (ab) F4J_CUDA(cudaMemcpyAsync(dA, A, ab, cudaMemcpyHostToDevice, ctx->stream));
         if (bb) F4J_CUDA(cudaMemcpyAsync(dB, B, bb, cudaMemcpyHostToDevice, ctx->stream));
-        rc = f4j_gemm_impl(ctx, cplx, m, n, k, (const double*)dA, opA, (const double*)dB, opB, (double*)dC, mode,
-                           rep);
-        if (rc) return rc;
+        int r = f4j_gemm_impl(ctx, cplx, m, n, k, (const double*)dA, opA, (const double*)dB, opB, (double*)dC, mode,
+                              rep);
+        if (r) return r;
         F4J_CUDA(cudaMemcpyAsync(C, dC, cb, cudaMemcpyDeviceToHost, ctx->stream));
         F4J_CUDA(cudaStreamSynchronize(ctx->stream));
         return f4j_report_accuracy(ctx, cplx, m, n, k, (const double*)dA, opA, (const double*)dB, opB,
                                    (const double*)dC, check_samples, check_flags, rep);
-    }
+    };
+    if (!split || opA != F4J_OP_N || !piped || kchunks || blocks) return in_turn();  // split K runs as one launch
     if (!ctx->parts_init) {
         for (int i = 0; i < F4J_HOST_STREAMS; i++) {
             F4J_CUDA(cudaStreamCreateWithFlags(&ctx->part_stream[i], cudaStreamNonBlocking));
@@ -1870,8 +2161,9 @@ static int gemm_host(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, c
     bool recompute = false;
     const SplitPlan* plan = nullptr;
     float spread = 0.0f;
-    rc = host_split_pipelined(ctx, cplx, m, n, k, A, B, opB, C, (double*)dA, (double*)dB, (double*)dC, parts, bparts,
-                              &recompute, &plan, &spread);
+    rc = host_split_pipelined(ctx, cplx, m, n, k, A, B, opB, C, (double*)dA, (double*)dB, (double*)dC, crt, parts,
+                              bparts, &recompute, &plan, &spread);
+    if (rc == F4J_ERR_OOM && crt) return in_turn();  // no room for the residue planes
     if (rc) return rc;
     if (recompute) {
         // all of A and B ask for another slice count than their first parts
@@ -1929,9 +2221,6 @@ extern "C" int f4j_zgemm_host(f4j_ctx* ctx, int64_t m, int64_t n, int64_t k, con
 // exponents per row of op(A) and column of op(B), and under 16 KiB for the
 // plan, the status words and the 1 KiB roundings of each part.  The call is
 // rejected exactly when that formula exceeds the array.
-#define F4J_NOALLOC_SCRATCH_BYTES (32u << 20)
-#define F4J_NOALLOC_NEED(m, n, Kp) \
-    ((size_t)12 * (size_t)((m) + (n)) * (size_t)(Kp) + (size_t)24 * (size_t)((m) + (n)) + (size_t)16384)
 static_assert(sizeof(SplitPlan) <= 4096, "the no-allocation bound's fixed part counts the plan as at most 4 KiB");
 static __device__ __align__(256) unsigned char g_f4j_noalloc_scratch[F4J_NOALLOC_SCRATCH_BYTES];
 
