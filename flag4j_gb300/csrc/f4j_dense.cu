@@ -15,6 +15,7 @@
 //    modes, FP64 FMA dot products reading A once.
 //  * k_gemm_check: double-double (Dot2) evaluation of sampled entries.
 #include <cstring>
+#include <type_traits>
 
 #include "f4j_internal.cuh"
 #include "f4j_ptx.cuh"
@@ -37,81 +38,96 @@ __device__ __forceinline__ void ld_op(const double* __restrict__ X, int64_t ld, 
 }
 
 // ------------------------------------------------------------------ EXACT
-constexpr int EX_BM = 64, EX_BN = 64, EX_BK = 16, EX_T = 256;  // 16x16 threads, 4x4 each
-
-template <bool CPLX>
-__global__ void __launch_bounds__(EX_T) k_gemm_exact(int64_t m, int64_t n, int64_t k,
-                                                     const double* __restrict__ A, int64_t lda, int opA,
-                                                     const double* __restrict__ B, int64_t ldb, int opB,
-                                                     double* __restrict__ C) {
-    __shared__ double sAr[EX_BK][EX_BM + 1], sBr[EX_BK][EX_BN + 1];
-    __shared__ double sAi[CPLX ? EX_BK : 1][EX_BM + 1], sBi[CPLX ? EX_BK : 1][EX_BN + 1];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    const int64_t m0 = (int64_t)blockIdx.y * EX_BM, n0 = (int64_t)blockIdx.x * EX_BN;
-    double cr[4][4], ci[4][4];
+// One output per thread, TM x TN of them per block, K in slabs of BK staged in
+// shared memory, the next slab's loads in flight under the current one's
+// arithmetic.  Two separately rounded FP64 operations per term on GB300's two
+// FP64 lanes per SM and clock bound it: shared-memory reads cost nothing beside
+// them, so a thread holds one output and the tiles stay small enough that a
+// product of a few thousand entries reaches every SM (64 x 64 tiles with 4 x 4
+// outputs per thread left most SMs idle below 1024^2).
+template <bool CPLX, int TM, int TN>
+__global__ void __launch_bounds__(TM * TN) k_gemm_exact(int64_t m, int64_t n, int64_t k,
+                                                        const double* __restrict__ A, int64_t lda, int opA,
+                                                        const double* __restrict__ B, int64_t ldb, int opB,
+                                                        double* __restrict__ C) {
+    constexpr int T = TM * TN, BK = CPLX ? 16 : 32;
+    constexpr int NA = (TM * BK + T - 1) / T, NB = (TN * BK + T - 1) / T;
+    using V = typename std::conditional<CPLX, double2, double>::type;
+    __shared__ V sA[BK][TM + 1], sB[BK][TN + 1];
+    const int tx = threadIdx.x % TN, ty = threadIdx.x / TN;
+    const int tiles_n = (int)((n + TN - 1) / TN);
+    const int64_t m0 = (int64_t)(blockIdx.x / tiles_n) * TM, n0 = (int64_t)(blockIdx.x % tiles_n) * TN;
+    V ra[NA], rb[NB];
+    // slab element e of op(A): consecutive threads along the stored rows
+    auto a_at = [&](int e, int& kk, int& r) {
+        if (opA == F4J_OP_N) kk = e % BK, r = e / BK;
+        else r = e % TM, kk = e / TM;
+    };
+    auto b_at = [&](int e, int& kk, int& c) {
+        if (opB == F4J_OP_N) c = e % TN, kk = e / TN;
+        else kk = e % BK, c = e / BK;
+    };
+    auto fetch = [&](int64_t k0) {
 #pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) cr[i][j] = ci[i][j] = 0.0;
-
-    for (int64_t k0 = 0; k0 < k; k0 += EX_BK) {
-        for (int e = threadIdx.x; e < EX_BK * EX_BM; e += EX_T) {
-            int kk = e / EX_BM, r = e % EX_BM;
+        for (int i = 0; i < NA; i++) {
+            int kk, r;
+            a_at(threadIdx.x + i * T, kk, r);
             double re = 0, im = 0;
-            if (m0 + r < m && k0 + kk < k) ld_op<CPLX>(A, lda, opA, m0 + r, k0 + kk, re, im);
-            sAr[kk][r] = re;
-            if (CPLX) sAi[kk][r] = im;
+            if (m0 + r < m && k0 + kk < k && r < TM) ld_op<CPLX>(A, lda, opA, m0 + r, k0 + kk, re, im);
+            if constexpr (CPLX) ra[i] = make_double2(re, im);
+            else ra[i] = re;
         }
-        for (int e = threadIdx.x; e < EX_BK * EX_BN; e += EX_T) {
-            int kk = e / EX_BN, c = e % EX_BN;
+#pragma unroll
+        for (int i = 0; i < NB; i++) {
+            int kk, c;
+            b_at(threadIdx.x + i * T, kk, c);
             double re = 0, im = 0;
-            if (n0 + c < n && k0 + kk < k) ld_op<CPLX>(B, ldb, opB, k0 + kk, n0 + c, re, im);
-            sBr[kk][c] = re;
-            if (CPLX) sBi[kk][c] = im;
+            if (n0 + c < n && k0 + kk < k && c < TN) ld_op<CPLX>(B, ldb, opB, k0 + kk, n0 + c, re, im);
+            if constexpr (CPLX) rb[i] = make_double2(re, im);
+            else rb[i] = re;
+        }
+    };
+    double cr = 0.0, ci = 0.0;
+    fetch(0);
+    for (int64_t k0 = 0; k0 < k; k0 += BK) {
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < NA; i++) {
+            int kk, r;
+            a_at(threadIdx.x + i * T, kk, r);
+            if (kk < BK && r < TM) sA[kk][r] = ra[i];
+        }
+#pragma unroll
+        for (int i = 0; i < NB; i++) {
+            int kk, c;
+            b_at(threadIdx.x + i * T, kk, c);
+            if (kk < BK && c < TN) sB[kk][c] = rb[i];
         }
         __syncthreads();
-        const int kmax = (int)((k - k0) < EX_BK ? (k - k0) : EX_BK);
-        for (int kk = 0; kk < kmax; kk++) {
-            double ar[4], br[4], ai[4], bi[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                ar[i] = sAr[kk][ty + 16 * i];
-                br[i] = sBr[kk][tx + 16 * i];
-                if (CPLX) {
-                    ai[i] = sAi[kk][ty + 16 * i];
-                    bi[i] = sBi[kk][tx + 16 * i];
-                }
+        if (k0 + BK < k) fetch(k0 + BK);
+        auto step = [&](int kk) {
+            if constexpr (CPLX) {
+                const double2 a = sA[kk][ty], b = sB[kk][tx];
+                const double pr = __dsub_rn(__dmul_rn(a.x, b.x), __dmul_rn(a.y, b.y));
+                const double pi = __dadd_rn(__dmul_rn(a.x, b.y), __dmul_rn(a.y, b.x));
+                cr = __dadd_rn(cr, pr);
+                ci = __dadd_rn(ci, pi);
+            } else {
+                cr = __dadd_rn(cr, __dmul_rn(sA[kk][ty], sB[kk][tx]));
             }
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    if (CPLX) {
-                        double pr = __dsub_rn(__dmul_rn(ar[i], br[j]), __dmul_rn(ai[i], bi[j]));
-                        double pi = __dadd_rn(__dmul_rn(ar[i], bi[j]), __dmul_rn(ai[i], br[j]));
-                        cr[i][j] = __dadd_rn(cr[i][j], pr);
-                        ci[i][j] = __dadd_rn(ci[i][j], pi);
-                    } else {
-                        cr[i][j] = __dadd_rn(cr[i][j], __dmul_rn(ar[i], br[j]));
-                    }
-                }
+        };
+        if (k - k0 >= BK) {
+#pragma unroll 8
+            for (int kk = 0; kk < BK; kk++) step(kk);
+        } else {
+            for (int kk = 0; kk < (int)(k - k0); kk++) step(kk);
         }
-        __syncthreads();
     }
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            int64_t r = m0 + ty + 16 * i, c = n0 + tx + 16 * j;
-            if (r < m && c < n) {
-                if (CPLX) {
-                    C[2 * (r * n + c)] = cr[i][j];
-                    C[2 * (r * n + c) + 1] = ci[i][j];
-                } else {
-                    C[r * n + c] = cr[i][j];
-                }
-            }
-        }
+    const int64_t r = m0 + ty, c = n0 + tx;
+    if (r < m && c < n) {
+        if constexpr (CPLX) reinterpret_cast<double2*>(C)[r * n + c] = make_double2(cr, ci);
+        else C[r * n + c] = cr;
+    }
 }
 
 // ------------------------------------------------------------------ DMMA
@@ -526,20 +542,46 @@ __global__ void k_gemv_sum(int64_t len, int64_t nchunk, const double* __restrict
 }  // namespace
 
 // ------------------------------------------------------------------ host side
-int f4j_gemm_exact(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, const double* A, int opA,
-                   const double* B, int opB, double* C) {
-    int64_t lda = (opA == F4J_OP_N) ? k : m;
-    int64_t ldb = (opB == F4J_OP_N) ? n : k;
-    dim3 grid((unsigned)f4j_cdiv(n, EX_BN), (unsigned)f4j_cdiv(m, EX_BM));
-    if (grid.y > 65535) return f4j_fail(F4J_ERR_ARG, "m too large for the exact kernel grid");
+template <bool CPLX, int TM, int TN>
+static int launch_exact(f4j_ctx* ctx, int64_t m, int64_t n, int64_t k, const double* A, int opA, const double* B,
+                        int opB, double* C) {
+    const int64_t lda = (opA == F4J_OP_N) ? k : m, ldb = (opB == F4J_OP_N) ? n : k;
+    const int64_t tiles = f4j_cdiv(m, TM) * f4j_cdiv(n, TN);
+    if (tiles > INT32_MAX) return f4j_fail(F4J_ERR_ARG, "product too large for the exact kernel grid");
     f4j_prof_begin(ctx);
-    if (cplx)
-        k_gemm_exact<true><<<grid, EX_T, 0, ctx->stream>>>(m, n, k, A, lda, opA, B, ldb, opB, C);
-    else
-        k_gemm_exact<false><<<grid, EX_T, 0, ctx->stream>>>(m, n, k, A, lda, opA, B, ldb, opB, C);
+    k_gemm_exact<CPLX, TM, TN><<<(unsigned)tiles, TM * TN, 0, ctx->stream>>>(m, n, k, A, lda, opA, B, ldb, opB, C);
     f4j_prof_end(ctx);
     F4J_LAUNCHED(ctx);
     return F4J_OK;
+}
+
+// The FP64 units bound this kernel whatever the tile (1024^3: 4.09 ms for every
+// tile from 4 x 8 to 64 x 1), so the tile only has to put warps on every SM
+// sub-partition and leave few lanes idle: 8 x 8 (two warps) unless one side is
+// at most 6, where a tile of that side's width keeps the lanes busy.  Measured,
+// us, the earlier 64 x 64 tile / 8 x 8: 96 x 80 x 64 162 / 8.7, 700 x 500 x 600
+// 1497 / 849, 1024^3 4894 / 4090.  8 x 8 / 16 x 2 or 2 x 16: 8192 x 1 x 1000
+// 264 / 99, 2 x 8192 x 500 134 / 58, 4000 x 6 x 400 66 / 53, 4000 x 12 x 400
+// 109 / 81 but 1000 x 1 x 1000 92 / 96.  16 x 2 / 32 x 1: 30000 x 1 x 300
+// 80 / 52, 8192 x 1 x 1000 99 / 103.
+template <bool CPLX>
+static int pick_exact(f4j_ctx* ctx, int64_t m, int64_t n, int64_t k, const double* A, int opA, const double* B,
+                      int opB, double* C) {
+    if (n <= 6 && m > n) {
+        if (n == 1 && m >= 16384) return launch_exact<CPLX, 32, 1>(ctx, m, n, k, A, opA, B, opB, C);
+        return launch_exact<CPLX, 16, 2>(ctx, m, n, k, A, opA, B, opB, C);
+    }
+    if (m <= 6 && n > m) {
+        if (m == 1 && n >= 16384) return launch_exact<CPLX, 1, 32>(ctx, m, n, k, A, opA, B, opB, C);
+        return launch_exact<CPLX, 2, 16>(ctx, m, n, k, A, opA, B, opB, C);
+    }
+    return launch_exact<CPLX, 8, 8>(ctx, m, n, k, A, opA, B, opB, C);
+}
+
+int f4j_gemm_exact(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, const double* A, int opA,
+                   const double* B, int opB, double* C) {
+    if (f4j_cdiv(m, 64) > 65535) return f4j_fail(F4J_ERR_ARG, "m too large for the exact kernel grid");
+    return cplx ? pick_exact<true>(ctx, m, n, k, A, opA, B, opB, C) : pick_exact<false>(ctx, m, n, k, A, opA, B, opB, C);
 }
 
 static int make_map_2d(CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer, uint32_t box_inner,

@@ -805,3 +805,23 @@ def test_herm_pos_def_product_chain(f4j, oracle, n):
     ref = oracle.zgemm(oracle.zgemm(UH, D.astype(np.complex128)), U)
     assert np.array_equal(got.view(np.uint64), ref.view(np.uint64))
     assert np.max(np.abs(got - got.conj().T)) < 1e-13
+
+
+@pytest.mark.parametrize("m,n,k", [
+    (1, 1, 1), (7, 9, 33), (8, 8, 32), (9, 8, 31), (17, 65, 64),          # 8 x 8 tiles, slabs of 32 and their edges
+    (17, 2, 40), (33, 6, 95), (16385, 1, 3), (100, 1, 1000),              # 16 x 2 and 32 x 1
+    (2, 17, 40), (6, 33, 95), (1, 16385, 3), (1, 100, 1000), (6, 6, 64),  # 2 x 16 and 1 x 32
+])
+@pytest.mark.parametrize("cp", [False, True])
+def test_exact_tiles_bit_identical(f4j, oracle, m, n, k, cp):
+    """Every tile shape of the EXACT kernel, at its edges and with transposed operands: bit for bit the
+    oracle's k-ascending loops."""
+    from flag4j_gb300 import synth
+    mk = lambda r, c, s: synth.normal(r, c, s) + 1j * synth.normal(r, c, s + 1) if cp else synth.normal(r, c, s)
+    A, B = mk(m, k, 301), mk(k, n, 303)
+    ref = oracle.zgemm(A, B) if cp else oracle.dgemm(A, B)
+    for opA, opB in ((0, 0), (1, 1)):
+        a = A if opA == 0 else np.ascontiguousarray(A.T)
+        b = B if opB == 0 else np.ascontiguousarray(B.T)
+        C, _ = run_gemm(f4j, a, b, mode="exact", opA=opA, opB=opB)
+        assert np.array_equal(C, ref), (opA, opB)
