@@ -23,7 +23,7 @@
 //                 CTA pairs (tcgen05 cta_group::2), exact in FP32 (|sum| <= 2^24
 //                 over at most 8192 terms), reduced mod p and multiplied by the
 //                 modulus's weight (M / p)^-1: an int16 plane per modulus.
-//  k_crt_combine  sum_l y_l (M / p_l) in 31-bit limbs, reduced mod M, rounded to
+//  k_crt_combine  sum_l y_l (M / p_l) in 32-bit words, reduced mod M, rounded to
 //                 double once and scaled.
 //
 // Included by f4j_split.cu.
@@ -33,7 +33,7 @@ namespace {
 
 // ------------------------------------------------------------------ moduli
 constexpr int CRT_NB = 15;     // bases; a configuration squares the first nsq and drops some of the last
-constexpr int CRT_LIMBS = 5;   // 31-bit limbs of M
+constexpr int CRT_WORDS = 5;   // 32-bit words of M, at most
 constexpr int CRT_NG = 7;      // groups of moduli in the reconstruction: pairs, and the last three
 constexpr int CRT_CFGS = 48;
 constexpr int CRT_KC = 8192;   // terms per accumulation: 2 * 8192 * 32 * 32 = 2^24
@@ -50,7 +50,8 @@ __host__ __device__ constexpr int crt_base(int i) {
 struct CrtMod {
     uint32_t wl[2] = {0, 0}, wh[2] = {0, 0};
     uint32_t kl = 0, kh = 0;
-    float b = 0, inv = 0;  // b, 1 / b
+    alignas(8) float nb[2] = {0, 0};  // -b and 1 / b, twice for the paired arithmetic
+    alignas(8) float inv[2] = {0, 0};
 };
 struct CrtMods {
     CrtMod m[CRT_NB] = {};
@@ -71,8 +72,8 @@ struct CrtMods {
             const uint32_t k1 = (2 * b - g - 8388608u % b) % b;  // 2^23 + k1 = -g (mod b)
             m[i].kl = 0x4B000000u + k0;
             m[i].kh = 0x4B000000u + k1;
-            m[i].b = (float)b;
-            m[i].inv = 1.0f / (float)b;
+            m[i].nb[0] = m[i].nb[1] = -(float)b;
+            m[i].inv[0] = m[i].inv[1] = 1.0f / (float)b;
         }
     }
 };
@@ -82,15 +83,16 @@ __constant__ CrtMods c_crt{};
 struct CrtCfg {
     int nmod, nsq;   // moduli; the first nsq are squares
     int cost;        // FP8 products: nmod + 2 nsq
-    int limbs;       // limbs of the reconstruction: 4 while M < 2^124, else 5
+    int words;       // words of the reconstruction: 4 while M < 2^127, else 5
     float bits;      // log2 M
-    int sh;          // the limbs below hold 2^sh times their number: 2^sh M in [2^(31 limbs - 1), 2^(31 limbs))
-    float qinv;      // 2^(31 limbs - 18) / (2^sh M), for the quotient by M
+    int sh;          // the words below hold 2^sh times their number: 2^sh M in [2^(32 words - 2), 2^(32 words - 1))
+    float qinv;      // 2^(32 words - 18) / (2^sh M), for the quotient by M
     int pad;
     float p[CRT_NB], invp[CRT_NB], u[CRT_NB];  // modulus, 1 / p, (M / p)^-1 mod p (balanced)
     int32_t c[CRT_NB];                         // P / p, P the product of the group's moduli
-    int32_t W[CRT_NG][CRT_LIMBS];              // M / P, 31-bit limbs
-    int32_t M[CRT_LIMBS];
+    int32_t z0[CRT_NG];                        // 2 P: makes a group's sum positive, and vanishes modulo M
+    uint32_t W[CRT_NG][CRT_WORDS];             // M / P
+    uint32_t NM[CRT_WORDS];                    // 2^(32 words) - M
 };
 __host__ __device__ constexpr int crt_group(int l) { return l / 2 < CRT_NG ? l / 2 : CRT_NG - 1; }
 
@@ -179,12 +181,16 @@ __device__ __forceinline__ void crt_store(const CrtDst& d, int64_t off, uint2 v)
 __device__ __forceinline__ void crt_digits8(const uint32_t (&lo)[8], const uint32_t (&hi)[8], int nmod, int nsq,
                                             const CrtDst& d, int64_t plane) {
     const f32x2 magic = dup2(CRT_MAGIC), unmagic = dup2(-CRT_MAGIC);
-#pragma unroll 1
-    for (int i = 0; i < nmod; i++) {
+    // unrolled: the weights are constant-bank operands and the kinds of moduli
+    // compile-time (a rolled loop spent an eighth of its instructions on loading
+    // them)
+#pragma unroll
+    for (int i = 0; i < CRT_NB; i++) {
+        if (i >= nmod) break;
         const CrtMod& c = c_crt.m[i];
-        const f32x2 nb = dup2(-c.b), inv = dup2(c.inv);
-        const bool wide = c.b > 33.0f;
-        const uint32_t bi = (uint32_t)c.b;
+        const f32x2 nb = *reinterpret_cast<const f32x2*>(c.nb), inv = *reinterpret_cast<const f32x2*>(c.inv);
+        const bool wide = crt_base(i) > 33;
+        const uint32_t bi = (uint32_t)crt_base(i);
         f32x2 f[4], q[4];
         uint2 up = make_uint2(0, 0), down = make_uint2(0, 0);
 #pragma unroll
@@ -648,7 +654,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) __cluster_dims__(2, 1, 1)
             };
             for (int k0 = 0; k0 < p.nkb && ok; k0 += CG_KB) {
                 if (l < nsq) {
-                    const float b = c_crt.m[l].b, ib = c_crt.m[l].inv;
+                    const float b = -c_crt.m[l].nb[0], ib = c_crt.m[l].inv[0];
                     uint32_t xr[64];
                     wait_full(0);
                     if (!ok) break;
@@ -747,35 +753,50 @@ __device__ __forceinline__ double crt_round(unsigned long long w2, unsigned long
     return scale_pow2(neg ? -v : v, X + 75 - z);
 }
 
-// C' = sum - q M (limbs scaled by 2^sh), q = round(sum / M) from the top limb
-// (|sum| < 8 M): its 2^-17 of M is far inside what |C'| < 0.497 M leaves.
-template <int LIMBS>
-__device__ __forceinline__ double crt_value(long long (&acc)[LIMBS], float qinv, const int32_t* __restrict__ Ml,
-                                            int X) {
-    const long long t = acc[LIMBS - 1] + (acc[LIMBS - 2] >> 31);
-    const float tf = __int_as_float(0x4B400000 + (int)(t >> 13)) - CRT_MAGIC;
-    const int q = __float_as_int(__fmaf_rn(tf, qinv, CRT_MAGIC)) - 0x4B400000;
+// The value of one entry from its sum S = C' + q M (words a, each a 64-bit sum
+// of the products at its place; scaled by 2^sh): q = round(S / M) from the top
+// (0 < S < 25 M: an error of 2^-16 M is far inside what |C'| < 0.497 M leaves),
+// C' = S - q M modulo 2^(32 L), rounded once.
+template <int L>
+__device__ __forceinline__ double crt_value(unsigned long long (&a)[L], const CrtCfg& c, int X) {
+    const unsigned long long t = a[L - 1] + (a[L - 2] >> 32);
+    const float tf = __uint_as_float(0x4B000000u + (uint32_t)(t >> 14)) - 8388608.0f;
+    const uint32_t q = __float_as_uint(__fmaf_rn(tf, c.qinv, 8388608.0f)) - 0x4B000000u;
+    uint32_t x[L];
 #pragma unroll
-    for (int j = 0; j < LIMBS; j++) acc[j] -= (long long)q * Ml[j];
+    for (int j = 0; j < L; j++) a[j] += (unsigned long long)q * c.NM[j];
 #pragma unroll
-    for (int j = 0; j + 1 < LIMBS; j++) {
-        acc[j + 1] += acc[j] >> 31;
-        acc[j] &= 0x7FFFFFFFll;
+    for (int j = 0; j < L; j++) {
+        x[j] = (uint32_t)a[j];
+        if (j + 1 < L) a[j + 1] += a[j] >> 32;
     }
-    unsigned long long w0, w1, w2 = 0;
-    const bool neg = acc[LIMBS - 1] < 0;
-    w0 = (unsigned long long)acc[0] | (unsigned long long)acc[1] << 31 | (unsigned long long)acc[2] << 62;
-    w1 = (unsigned long long)acc[2] >> 2 | (unsigned long long)acc[3] << 29;  // |C'| < 2^127: acc[3] << 29 keeps its sign
-    if constexpr (LIMBS == 5) {
-        w1 |= (unsigned long long)acc[4] << 60;
-        w2 = (unsigned long long)(acc[4] >> 4);
-    }
+    const bool neg = (int)x[L - 1] < 0;
     if (neg) {
-        w0 = ~w0 + 1;
-        w1 = ~w1 + (w0 == 0);
-        if constexpr (LIMBS == 5) w2 = ~w2 + (w0 == 0 && w1 == 0);
+        uint32_t carry = 1;
+#pragma unroll
+        for (int j = 0; j < L; j++) {
+            x[j] = ~x[j] + carry;
+            carry = carry && x[j] == 0;
+        }
     }
-    return crt_round(w2, w1, w0, neg, X);
+    if (x[L - 1] == 0) {  // much cancellation, or zero
+        const unsigned long long w2 = L == 5 ? x[L - 1] : 0ull;
+        return crt_round(w2, (unsigned long long)x[3] << 32 | x[2], (unsigned long long)x[1] << 32 | x[0], neg, X);
+    }
+    // top 64 bits, 53 of them to nearest even
+    const int z = __clz((int)x[L - 1]);
+    const uint32_t y3 = __funnelshift_l(x[L - 2], x[L - 1], z), y2 = __funnelshift_l(x[L - 3], x[L - 2], z);
+    uint32_t below = (x[L - 3] << z) | x[L - 4];
+    if (L == 5) below |= x[0];
+    unsigned long long m = ((unsigned long long)y3 << 32 | y2) >> 11;
+    const uint32_t rem = (y2 & 0x7FFu) << 1 | (below ? 1u : 0u);
+    m += (rem + ((uint32_t)m & 1u)) > 0x800u;  // above half, or half and odd
+    const int Y = X + 32 * (L - 2) - z + 11;   // value = m 2^Y, m in [2^52, 2^53]
+    const int E = Y + 1074;                    // its exponent field less one (m's top bit adds it)
+    if (E >= 0 && E < 2045)
+        return __longlong_as_double((long long)((((unsigned long long)E << 52) + m) | (neg ? 1ull << 63 : 0ull)));
+    const double v = (double)m;
+    return scale_pow2(neg ? -v : v, Y);
 }
 
 struct CrtCombineParams {
@@ -787,80 +808,81 @@ struct CrtCombineParams {
     const int* ea;
     const int* eb;
     double* C;
-    int cplx;
     const SplitPlan* plan;
     const CrtCfg* cfgs;
 };
 
-template <int LIMBS>
-__device__ __forceinline__ void crt_combine_body(const CrtCombineParams& p, const CrtCfg& c, int row, int j0,
-                                                 int ubits) {
-    // four values: columns j0 .. j0 + 3, or (re, im) of columns j0, j0 + 1
+// Two adjacent entries of C (X: exponent of the row's unit, eb: the columns').
+template <int L>
+__device__ __forceinline__ void crt_two(const int16_t* __restrict__ src, int64_t plane, const CrtCfg& c, int X, int eb0,
+                                        int eb1, double& out0, double& out1) {
     const int nmod = c.nmod;
-    const int64_t plane = (int64_t)p.yrows * p.ldy;
-    const int16_t* src = p.y + (int64_t)(p.yrow0 + row) * p.ldy + j0;
-    uint2 v[CRT_NB];
+    int v[CRT_NB];
 #pragma unroll
     for (int l = 0; l < CRT_NB; l++) {
-        v[l] = make_uint2(0, 0);
-        if (l < nmod) {
-            if (!p.cplx) {
-                v[l] = *reinterpret_cast<const uint2*>(src + l * plane);
-            } else {
-                const uint32_t re = *reinterpret_cast<const uint32_t*>(src + l * plane);
-                const uint32_t im = *reinterpret_cast<const uint32_t*>(src + l * plane + p.half);
-                v[l] = make_uint2(__byte_perm(re, im, 0x5410), __byte_perm(re, im, 0x7632));
-            }
-        }
+        v[l] = 0;
+        if (l < nmod) v[l] = __ldg(reinterpret_cast<const int*>(src));
+        src += plane;
     }
-    long long acc[4][LIMBS];
+    unsigned long long a0[L], a1[L];
 #pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < LIMBS; j++) acc[i][j] = 0;
-    // a group's residues first become one number modulo P (|z| < 2^24), so the
-    // wide multiplies are per group: 7 x LIMBS of them instead of 15 x LIMBS
+    for (int j = 0; j < L; j++) a0[j] = a1[j] = 0;
+    // a group's residues first become one number modulo P (0 < z < 2^25), so the
+    // wide multiplies are per group: 7 x L of them instead of 15 x L
 #pragma unroll
     for (int g = 0; g < CRT_NG; g++) {
-        int z[4] = {0, 0, 0, 0};
+        int z0 = c.z0[g], z1 = z0;
 #pragma unroll
         for (int l = 2 * g; l < (g + 1 < CRT_NG ? 2 * g + 2 : CRT_NB); l++) {
-            const int cl = c.c[l];
-            z[0] += (int)(int16_t)(v[l].x & 0xffff) * cl;
-            z[1] += ((int)v[l].x >> 16) * cl;
-            z[2] += (int)(int16_t)(v[l].y & 0xffff) * cl;
-            z[3] += ((int)v[l].y >> 16) * cl;
+            z0 += (int)(int16_t)(v[l] & 0xffff) * c.c[l];
+            z1 += (v[l] >> 16) * c.c[l];
         }
 #pragma unroll
-        for (int j = 0; j < LIMBS; j++) {
-            const int32_t wj = c.W[g][j];
-#pragma unroll
-            for (int i = 0; i < 4; i++) acc[i][j] += (long long)z[i] * wj;
+        for (int j = 0; j < L; j++) {
+            a0[j] += (unsigned long long)(uint32_t)z0 * c.W[g][j];
+            a1[j] += (unsigned long long)(uint32_t)z1 * c.W[g][j];
         }
     }
+    out0 = crt_value<L>(a0, c, X + eb0);
+    out1 = crt_value<L>(a1, c, X + eb1);
+}
+
+// Entries j0, j0 + 1 of a row (complex: both parts).
+template <int L, bool CPLX>
+__device__ __forceinline__ void crt_combine_body(const CrtCombineParams& p, const CrtCfg& c, int row, int j0,
+                                                 int ubits, int eb0, int eb1) {
+    const int64_t plane = (int64_t)p.yrows * p.ldy;
+    const int16_t* src = p.y + (int64_t)(p.yrow0 + row) * p.ldy + j0;
     const int64_t r = p.row0 + p.yrow0 + row;
-    const int X = ubits + p.ea[r] - c.sh;
-    double out[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int col = p.cplx ? j0 + i / 2 : j0 + i;
-        out[i] = col < p.c1 ? crt_value<LIMBS>(acc[i], c.qinv, c.M, X + p.eb[col]) : 0.0;
-    }
-    double* dst = p.C + (p.cplx ? 2 * (r * p.n + j0) : r * p.n + j0);
-    const int cnt = p.cplx ? 2 * (p.c1 - j0 < 2 ? p.c1 - j0 : 2) : (p.c1 - j0 < 4 ? p.c1 - j0 : 4);
-    if (cnt == 4 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-        reinterpret_cast<double2*>(dst)[0] = make_double2(out[0], out[1]);
-        reinterpret_cast<double2*>(dst)[1] = make_double2(out[2], out[3]);
+    const int X = ubits + __ldg(p.ea + r) - c.sh;
+    const bool two = j0 + 1 < p.c1;
+    if constexpr (!CPLX) {
+        double v0, v1;
+        crt_two<L>(src, plane, c, X, eb0, eb1, v0, v1);
+        double* dst = p.C + r * p.n + j0;
+        if (two && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+            *reinterpret_cast<double2*>(dst) = make_double2(v0, v1);
+        } else {
+            dst[0] = v0;
+            if (two) dst[1] = v1;
+        }
     } else {
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-            if (i < cnt) dst[i] = out[i];
+        double2 u0{0, 0}, u1{0, 0};
+#pragma unroll 1  // one copy of the code, in 64 registers
+        for (int part = 0; part < 2; part++) {
+            u0.x = u0.y, u1.x = u1.y;
+            crt_two<L>(src + part * p.half, plane, c, X, eb0, eb1, u0.y, u1.y);
+        }
+        double2* dst = reinterpret_cast<double2*>(p.C) + r * p.n + j0;  // complex buffers are 16-byte aligned
+        dst[0] = u0;
+        if (two) dst[1] = u1;
     }
 }
 
-// Blocks of blockDim.x x blockDim.y = 256 threads over (columns, rows), four
-// values each along a row of C; blocks stride over the rows.
-__global__ void __launch_bounds__(256, 2) k_crt_combine(const __grid_constant__ CrtCombineParams p) {
+// Blocks of blockDim.x x blockDim.y = 256 threads over (columns, rows), two
+// entries each along a row of C; blocks stride over the rows.
+template <bool CPLX>
+__global__ void __launch_bounds__(256, 4) k_crt_combine(const __grid_constant__ CrtCombineParams p) {
     __shared__ CrtCfg c;
     if (p.plan->nonfinite) return;
     {
@@ -870,29 +892,30 @@ __global__ void __launch_bounds__(256, 2) k_crt_combine(const __grid_constant__ 
     }
     __syncthreads();
     const int ubits = -2 * (4 + 5 * (p.plan->s - 1));
-    const int j0 = p.c0 + (int)(blockIdx.x * blockDim.x + threadIdx.x) * (p.cplx ? 2 : 4);
+    const int j0 = p.c0 + (int)(blockIdx.x * blockDim.x + threadIdx.x) * 2;
     if (j0 >= p.c1) return;
+    const int eb0 = __ldg(p.eb + j0), eb1 = j0 + 1 < p.c1 ? __ldg(p.eb + j0 + 1) : 0;
     for (int row = blockIdx.y * blockDim.y + threadIdx.y; row < p.rows; row += gridDim.y * blockDim.y) {
-        if (c.limbs == 4) crt_combine_body<4>(p, c, row, j0, ubits);
-        else crt_combine_body<5>(p, c, row, j0, ubits);
+        if (c.words == 4) crt_combine_body<4, CPLX>(p, c, row, j0, ubits, eb0, eb1);
+        else crt_combine_body<5, CPLX>(p, c, row, j0, ubits, eb0, eb1);
     }
 }
 
 // ------------------------------------------------------------------ host side
 // Every configuration worth having, by rising cost: squares of the first nsq
-// bases, the last `drop` bases left out.  Exact 192-bit arithmetic on 31-bit
-// limbs: M and M / p are products of the other moduli.
+// bases, the last `drop` bases left out.  Exact arithmetic on 32-bit words: M
+// and M / P are products of the other moduli.
 struct CrtTable {
     CrtCfg cfg[CRT_CFGS];
     int n = 0;
 };
 
-static void crt_limbs_mul(int64_t (&a)[CRT_LIMBS + 1], int m) {
-    int64_t carry = 0;
-    for (int j = 0; j <= CRT_LIMBS; j++) {
-        const int64_t t = a[j] * m + carry;
-        a[j] = t & 0x7FFFFFFF;
-        carry = t >> 31;
+static void crt_words_mul(uint32_t (&a)[CRT_WORDS], uint32_t m) {
+    uint64_t carry = 0;
+    for (int j = 0; j < CRT_WORDS; j++) {
+        const uint64_t t = (uint64_t)a[j] * m + carry;
+        a[j] = (uint32_t)t;
+        carry = t >> 32;
     }
 }
 
@@ -918,18 +941,14 @@ static const CrtTable& crt_table() {
             c.nsq = bj;
             c.cost = cost;
             c.bits = (float)bbits;
-            c.limbs = bbits < 124.0 ? 4 : 5;
+            c.words = bbits < 127.0 ? 4 : 5;
             const auto mod = [&](int l) { return l < c.nsq ? crt_base(l) * crt_base(l) : crt_base(l); };
-            const int top = 31 * c.limbs;
-            c.sh = top - (int)ceil(bbits);  // M is never a power of two
-            const auto store = [&](int64_t(&a)[CRT_LIMBS + 1], int32_t* out) {
-                for (int i = 0; i < c.sh; i++) crt_limbs_mul(a, 2);
-                for (int j = 0; j < CRT_LIMBS; j++) out[j] = (int32_t)a[j];
-            };
-            int64_t M[CRT_LIMBS + 1] = {1};
+            const int top = 32 * c.words;
+            c.sh = top - 1 - (int)ceil(bbits);  // M is never a power of two
+            uint32_t M[CRT_WORDS] = {1};
             for (int l = 0; l < c.nmod; l++) {
                 const int pl = mod(l);
-                crt_limbs_mul(M, pl);
+                crt_words_mul(M, (uint32_t)pl);
                 int inv = 1, r = 1, cl = 1;
                 for (int i = 0; i < c.nmod; i++) {
                     if (i == l) continue;
@@ -942,12 +961,24 @@ static const CrtTable& crt_table() {
                 c.u[l] = (float)(2 * inv > pl ? inv - pl : inv);
                 c.c[l] = cl;
             }
-            store(M, c.M);
+            for (int i = 0; i < c.sh; i++) crt_words_mul(M, 2);
+            uint64_t borrow = 1;  // two's complement over `words` words
+            for (int j = 0; j < c.words; j++) {
+                const uint64_t t = (uint64_t)(uint32_t)~M[j] + borrow;
+                c.NM[j] = (uint32_t)t;
+                borrow = t >> 32;
+            }
             for (int g = 0; g < CRT_NG; g++) {
-                int64_t W[CRT_LIMBS + 1] = {1};
-                for (int i = 0; i < c.nmod; i++)
-                    if (crt_group(i) != g) crt_limbs_mul(W, mod(i));
-                if (2 * g < c.nmod) store(W, c.W[g]);  // else no modulus: z is 0
+                uint32_t W[CRT_WORDS] = {1};
+                int P = 1;
+                for (int i = 0; i < c.nmod; i++) {
+                    if (crt_group(i) == g) P *= mod(i);
+                    else crt_words_mul(W, (uint32_t)mod(i));
+                }
+                if (2 * g >= c.nmod) continue;  // no modulus: z stays 0
+                for (int i = 0; i < c.sh; i++) crt_words_mul(W, 2);
+                c.z0[g] = 2 * P;
+                for (int j = 0; j < CRT_WORDS; j++) c.W[g][j] = W[j];
             }
             c.qinv = (float)exp2((double)(top - 18) - bbits - c.sh);
         }

@@ -1660,14 +1660,14 @@ static int crt_launch(f4j_ctx* ctx, const CrtSetup& S, bool cplx, int64_t n, dou
     ctx->stream = saved;
     F4J_LAUNCHED(ctx);
     CrtCombineParams cp{(int)(r0 - row0), row0, (int)(r1 - r0), (int)S.yrows, (int)c0, (int)c1, (int)n, S.half, S.ldy,
-                        S.y, S.ea, S.eb, C, cplx ? 1 : 0, S.plan, S.cfgs};
-    const int64_t per_row = f4j_cdiv(c1 - c0, cplx ? 2 : 4);
+                        S.y, S.ea, S.eb, C, S.plan, S.cfgs};
+    const int64_t per_row = f4j_cdiv(c1 - c0, 2);
     unsigned bx = 32;  // threads along a row
     while (bx < 256 && bx < per_row) bx *= 2;
     const int64_t gx = f4j_cdiv(per_row, bx), gy = f4j_cdiv(r1 - r0, 256 / bx);
     int64_t cap = 16 * (int64_t)ctx->sm_count / gx;  // a few blocks per resident slot, each over several rows
     cap = cap < 1 ? 1 : (cap > 65535 ? 65535 : cap);
-    k_crt_combine<<<dim3((unsigned)gx, (unsigned)(gy < cap ? gy : cap)), dim3(bx, 256 / bx), 0, stream>>>(cp);
+    (cplx ? k_crt_combine<true> : k_crt_combine<false>)<<<dim3((unsigned)gx, (unsigned)(gy < cap ? gy : cap)), dim3(bx, 256 / bx), 0, stream>>>(cp);
     F4J_LAUNCHED(ctx);
     return F4J_OK;
 }
