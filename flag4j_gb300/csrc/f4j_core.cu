@@ -487,6 +487,7 @@ int f4j_gemm_impl(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, cons
     // AUTO follows the dispatcher configuration: the reference's small-product
     // rule and products of a few microseconds of work run Flag4j's own order
     // (bit-identical); larger ones take the configured GPU path (f4j_config.cu).
+    const bool any_form = mode == F4J_MODE_AUTO;
     if (mode == F4J_MODE_AUTO) {
         mode = f4j_resolve_mode(cplx, m, n, k, mode);
         if (mode == F4J_MODE_AUTO) mode = F4J_MODE_SPLIT;
@@ -509,7 +510,7 @@ int f4j_gemm_impl(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, cons
         // and the gated DMMA launch (a no-op otherwise) propagates them like
         // the reference.  Nothing here waits for the GPU.
         const int* gate = nullptr;
-        rc = f4j_gemm_split(ctx, cplx, m, n, k, A, opA, B, opB, C, 0, rep, &gate);
+        rc = f4j_gemm_split(ctx, cplx, m, n, k, A, opA, B, opB, C, 0, any_form, rep, &gate);
         if (gate_out) *gate_out = gate;
         used = F4J_MODE_SPLIT;
         if (rc == F4J_OK) rc = f4j_gemm_dmma(ctx, cplx, m, n, k, A, opA, B, opB, C, gate);

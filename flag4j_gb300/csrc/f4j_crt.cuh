@@ -341,7 +341,7 @@ struct CrtGemmParams {
     int M, N, nkb;          // rows of A, (padded) rows of B^T, K blocks of CG_BK bytes
     int tm0, tm1, tn0, tn1; // tile rows and columns of C the launch covers
     int row0, rows;         // rows of C in y: [row0, row0 + rows)
-    int64_t ldy;            // columns of y (multiple of 8, >= N)
+    int64_t ldy;            // columns of y (multiple of 16, >= N)
     int16_t* y;             // [nmod][rows][ldy]
     int* status;
     const SplitPlan* plan;
@@ -429,10 +429,20 @@ __device__ __forceinline__ void crt_tile(int t, int tiles_m, int tiles_n, int& t
     tn = r / gm;
 }
 
-// Balanced x mod p for an integer |x| <= 2^24.
-__device__ __forceinline__ float crt_mod(float x, float p, float invp) {
-    const float q = __fmaf_rn(x, invp, CRT_MAGIC) - CRT_MAGIC;
-    return __fmaf_rn(-p, q, x);
+// Balanced x mod p for integers |x| <= 2^24 (a pair; p and 1 / p twice).
+__device__ __forceinline__ f32x2 crt_mod2(f32x2 x, f32x2 np, f32x2 invp) {
+    const f32x2 q = add2(fma2(x, invp, dup2(CRT_MAGIC)), dup2(-CRT_MAGIC));
+    return fma2(np, q, x);
+}
+// Two integers |x| < 2^15 as 16-bit halves x + 2^15, and back.
+__device__ __forceinline__ uint32_t crt_halves(f32x2 x) {
+    uint32_t a, b;
+    unpack2(add2(x, dup2(8388608.0f + 32768.0f)), a, b);
+    return __byte_perm(a, b, 0x5410);
+}
+__device__ __forceinline__ f32x2 crt_floats(uint32_t h) {
+    return add2(pack2(__byte_perm(h, 0x4B000000u, 0x7610), __byte_perm(h, 0x4B000000u, 0x7632)),
+                dup2(-8388608.0f - 32768.0f));
 }
 
 // A unit is one modulus of one 256 x 256 tile: squares first (modulus-major,
@@ -440,9 +450,9 @@ __device__ __forceinline__ float crt_mod(float x, float p, float invp) {
 // Ring slots carry (A digit, B digit) tile pairs: one per K block of a single
 // modulus, (A0, B0) and (A1, B1) of a square.  TMEM holds two accumulators of
 // 256 columns: X (x0 y0) and Y (x0 y1 + x1 y0) of a square, in turn the
-// singles'.  Y's products run one K block behind X's, so at the end of a
-// square X is drained under Y's last products and Y under the next unit's
-// first.
+// singles'.  X's products run two K blocks ahead of Y's at the start and the end of
+// a square, so X is drained under Y's last products and Y under the next
+// unit's first.
 __global__ void __launch_bounds__(CG_THREADS, 1) __cluster_dims__(2, 1, 1)
     k_crt_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ CrtGemmParams p) {
@@ -493,104 +503,129 @@ __global__ void __launch_bounds__(CG_THREADS, 1) __cluster_dims__(2, 1, 1)
 
     if (warp == 0) {
         // ---------------- TMA producer: lane 0 loads the slot's A tile, lane 1 its B tile
-        int st = 0;
+        int s = 0, round = 0;  // next slot, and how often the ring has been filled
         bool ok = true;
+        const uint32_t full0 = cluster_map(&full[0], 0);
+        const CUtensorMap* map = lane == 0 ? &tmA : &tmB;
         for (int u = pair; u < nunits && ok; u += npairs) {
             const int l = u / ntiles;
             int tm, tn;
             crt_tile(u - l * ntiles, tiles_m, tiles_n, tm, tn);
-            const int row = lane == 0 ? (p.tm0 + tm) * CG_T + (int)rank * 128 : (p.tn0 + tn) * CG_T + (int)rank * 128;
+            const int row = (lane == 0 ? p.tm0 + tm : p.tn0 + tn) * CG_T + (int)rank * 128;
             const int nd = l < nsq ? 2 : 1;
             for (int kb = 0; kb < p.nkb && ok; kb++) {
-                for (int d = 0; d < nd; d++, st++) {
-                    const int s = st % CG_RING;
+                for (int d = 0; d < nd; d++) {
                     if (lane == 0) {
-                        if (st >= CG_RING)
-                            ok = mbar_wait(&empty[s], ((st / CG_RING) & 1) ^ 1, p.status, 21) &&
-                                 !*(volatile int*)&abort_flag;
+                        if (round > 0)
+                            ok = mbar_wait(&empty[s], (round & 1) ^ 1, p.status, 21) && !*(volatile int*)&abort_flag;
                         if (!ok) abort_flag = 1;
                         else if (rank == 0) mbar_arrive_expect_tx(&full[s], 2 * CG_SLOT);
                     }
                     ok = __shfl_sync(0xffffffffu, ok, 0);
                     if (!ok) break;
                     if (lane < 2)
-                        tma_load_3d_pair(ring + s * CG_SLOT + lane * CG_TILE, lane == 0 ? &tmA : &tmB,
-                                         cluster_map(&full[s], 0), kb * CG_BK, row, d ? nmod + l : l);
+                        tma_load_3d_pair(ring + s * CG_SLOT + lane * CG_TILE, map, full0 + 8 * s, kb * CG_BK, row,
+                                         d ? nmod + l : l);
+                    if (++s == CG_RING) s = 0, round++;
                 }
             }
         }
         // copies still in flight signal the first CTA's barriers: it waits for them (bounded), and the
         // cluster barrier below keeps both CTAs until then
         if (rank == 0 && lane == 0)
-            for (int q = st > CG_RING ? st - CG_RING : 0; q < st; q++)
-                mbar_wait(&full[q % CG_RING], (q / CG_RING) & 1, nullptr, 0);
+            for (int q = 0; q < CG_RING; q++) {
+                const int fills = round + (q < s ? 1 : 0);
+                if (fills) mbar_wait(&full[q], (fills - 1) & 1, nullptr, 0);
+            }
     } else if (warp == 1) {
-        // ---------------- MMA issuer: one thread of the pair's first CTA
+        // ---------------- MMA issuer: one thread of the pair's first CTA.  The
+        // tensor pipe queues only a couple of MMAs, so what this thread does
+        // between them (waits, slot arithmetic, commits) shows as idle pipe: ring
+        // cursors instead of divisions, one barrier test per slot on the fast path.
         if (rank == 0 && lane == 0) {
             const uint64_t desc0 = umma_desc_sw128(ring);
             const uint32_t hi = (uint32_t)(desc0 >> 32), lo0 = (uint32_t)desc0;
             const uint32_t idesc = umma_idesc_e4m3_f32(256, 256);
             constexpr uint32_t SLOT16 = CG_SLOT >> 4, TILE16 = CG_TILE >> 4;
-            int st = 0, turn = 0;
-            uint32_t fills[2] = {0, 0};
+            struct Cursor {
+                uint32_t s = 0, par = 0;
+                __device__ __forceinline__ void next() {
+                    if (++s == CG_RING) s = 0, par ^= 1;
+                }
+            };
+            Cursor cur;  // first slot not yet consumed
+            uint32_t turn = 0, fill0 = 0, fill1 = 0;
             bool ok = true;
-            auto acquire = [&](int a) {
-                if (ok && fills[a] > 0) ok = mbar_wait_cluster(&accempty[a], (fills[a] - 1) & 1, p.status, 22);
+            auto acquire = [&](uint32_t a, uint32_t fills) {  // the epilogue has drained accumulator a
+                if (fills > 0) ok = ok && mbar_wait_cluster(&accempty[a], (fills - 1) & 1, p.status, 22);
                 tc_fence_after();
             };
-            auto landed = [&](int i) {
-                if (ok) ok = mbar_wait_cluster(&full[i % CG_RING], (i / CG_RING) & 1, p.status, 23) &&
-                             !*(volatile int*)&abort_flag;
-                tc_fence_after();
+            auto landed = [&](const Cursor& c) {
+                if (!mbar_try_wait(&full[c.s], c.par)) {
+                    ok = ok && mbar_wait(&full[c.s], c.par, p.status, 23) && !*(volatile int*)&abort_flag;
+                }
             };
-            auto mma = [&](int acc, int ia, int ib, bool first) {
-                umma2_f8_k128(tmem + acc * 256, lo0 + (uint32_t)(ia % CG_RING) * SLOT16,
-                              lo0 + (uint32_t)(ib % CG_RING) * SLOT16 + TILE16, hi, idesc, first ? 0u : 1u);
+            auto mma = [&](uint32_t acc, uint32_t sa, uint32_t sb, bool first) {
+                umma2_f8_k128(tmem + acc * 256, lo0 + sa * SLOT16, lo0 + sb * SLOT16 + TILE16, hi, idesc,
+                              first ? 0u : 1u);
             };
             for (int u = pair; u < nunits && ok; u += npairs) {
                 const int l = u / ntiles;
                 for (int k0 = 0; k0 < p.nkb && ok; k0 += CG_KB) {
                     const int nk = p.nkb - k0 < CG_KB ? p.nkb - k0 : CG_KB;
                     if (l < nsq) {
-                        acquire(0);
-                        landed(st);
-                        if (!ok) break;
-                        mma(0, st, st, true);
-                        if (nk == 1) umma2_commit(&accfull[0]);
-                        for (int kb = 0; kb < nk; kb++) {
-                            const int s0 = st + 2 * kb;
-                            if (kb + 1 < nk) {
-                                landed(s0 + 2);
-                                if (!ok) break;
-                                mma(0, s0 + 2, s0 + 2, false);
-                                if (kb + 2 == nk) umma2_commit(&accfull[0]);
+                        acquire(0, fill0);
+                        Cursor cx = cur;
+                        auto step_x = [&](bool first) {
+                            landed(cx);
+                            if (!ok) return;
+                            mma(0, cx.s, cx.s, first);
+                            cx.next();
+                            cx.next();
+                        };
+                        step_x(true);
+                        int x = 1;  // K blocks of X issued
+                        for (int kb = 0; kb < nk && ok; kb++) {
+                            // X ahead of Y by two blocks at the start and the end only: in between a
+                            // K block's slots are freed at once, so more of the ring is loads in flight
+                            const int lead = kb == 0 ? 3 : kb + 2 < nk ? kb + 1 : nk;
+                            const int xend = lead < nk ? lead : nk;
+                            if (x < xend) {
+                                for (; x < xend && ok; x++) step_x(false);
+                                if (ok && x == nk) umma2_commit(&accfull[0]);
                             }
-                            if (kb == 0) acquire(1);
-                            landed(s0 + 1);
+                            if (kb == 0) {
+                                if (ok && nk == 1) umma2_commit(&accfull[0]);
+                                acquire(1, fill1);
+                            }
+                            const uint32_t s0 = cur.s;
+                            cur.next();
+                            landed(cur);
                             if (!ok) break;
-                            mma(1, s0 + 1, s0, kb == 0);
-                            mma(1, s0, s0 + 1, false);
-                            umma2_commit(&empty[s0 % CG_RING]);
-                            umma2_commit(&empty[(s0 + 1) % CG_RING]);
+                            mma(1, s0, cur.s, kb == 0);
+                            mma(1, cur.s, s0, false);
+                            umma2_commit(&empty[s0]);
+                            umma2_commit(&empty[cur.s]);
+                            cur.next();
                         }
                         if (!ok) break;
                         umma2_commit(&accfull[1]);
-                        fills[0]++;
-                        fills[1]++;
-                        st += 2 * nk;
+                        fill0++;
+                        fill1++;
                     } else {
-                        acquire(turn);
+                        acquire(turn, turn ? fill1 : fill0);
                         for (int kb = 0; kb < nk; kb++) {
-                            landed(st + kb);
+                            landed(cur);
                             if (!ok) break;
-                            mma(turn, st + kb, st + kb, kb == 0);
-                            umma2_commit(&empty[(st + kb) % CG_RING]);
+                            mma(turn, cur.s, cur.s, kb == 0);
+                            umma2_commit(&empty[cur.s]);
+                            cur.next();
                         }
                         if (!ok) break;
                         umma2_commit(&accfull[turn]);
-                        fills[turn]++;
+                        if (turn) fill1++;
+                        else fill0++;
                         turn ^= 1;
-                        st += nk;
                     }
                 }
             }
@@ -625,37 +660,36 @@ __global__ void __launch_bounds__(CG_THREADS, 1) __cluster_dims__(2, 1, 1)
             crt_tile(u - l * ntiles, tiles_m, tiles_n, tm, tn);
             const int row = (p.tm0 + tm) * CG_T + (int)rank * 128 + 32 * q + lane;
             const int col0 = (p.tn0 + tn) * CG_T + h * 128;
-            const float pm = cfg->p[l], ip = cfg->invp[l], uw = cfg->u[l];
+            const f32x2 np = dup2(-cfg->p[l]), ip = dup2(cfg->invp[l]), uw = dup2(cfg->u[l]);
             int16_t* yrow = p.y + ((int64_t)l * p.rows + (row - p.row0)) * p.ldy + col0;
-            // 32 reduced values (c: an integer below 2^22 / |uw| + ..) times the weight, plus what earlier
-            // K chunks left, mod p, to y
-            auto put = [&](int part, const float (&c)[32], bool add) {
-                if (row >= p.M) return;
+            // sixteen reduced values times the weight, plus what earlier K chunks
+            // left, mod p, to columns c16 .. c16 + 15 of y: one whole 32-byte
+            // sector a lane (two 16-byte stores each touched half a sector)
+            auto put = [&](int c16, const f32x2 (&c)[8], bool add) {
+                if (row >= p.M || col0 + c16 >= p.ldy) return;
+                int16_t* dst = yrow + c16;
+                uint32_t w[8];
+                if (add) {
+                    const uint4 o0 = reinterpret_cast<const uint4*>(dst)[0], o1 = reinterpret_cast<const uint4*>(dst)[1];
+                    const uint32_t old[8] = {o0.x, o0.y, o0.z, o0.w, o1.x, o1.y, o1.z, o1.w};
 #pragma unroll
-                for (int g = 0; g < 4; g++) {
-                    if (col0 + part * 32 + g * 8 >= p.ldy) break;
-                    uint4* dst = reinterpret_cast<uint4*>(yrow + part * 32 + g * 8);
-                    uint32_t old[4] = {0, 0, 0, 0}, w[4];
-                    if (add) {
-                        const uint4 o4 = *dst;
-                        old[0] = o4.x, old[1] = o4.y, old[2] = o4.z, old[3] = o4.w;
-                    }
+                    for (int i = 0; i < 8; i++)  // signed halves: flip the top bit for the unsigned form
+                        w[i] = crt_halves(crt_mod2(fma2(c[i], uw, crt_floats(old[i] ^ 0x80008000u)), np, ip));
+                } else {
 #pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        float z0 = c[g * 8 + 2 * i], z1 = c[g * 8 + 2 * i + 1];
-                        const float o0 = __int_as_float(0x4B400000 + (int)(int16_t)(old[i] & 0xffff)) - CRT_MAGIC;
-                        const float o1 = __int_as_float(0x4B400000 + ((int)old[i] >> 16)) - CRT_MAGIC;
-                        z0 = crt_mod(__fmaf_rn(z0, uw, o0), pm, ip) + CRT_MAGIC;
-                        z1 = crt_mod(__fmaf_rn(z1, uw, o1), pm, ip) + CRT_MAGIC;
-                        w[i] = __byte_perm(__float_as_uint(z0), __float_as_uint(z1), 0x5410);
-                    }
-                    *dst = make_uint4(w[0], w[1], w[2], w[3]);
+                    for (int i = 0; i < 8; i++) w[i] = crt_halves(crt_mod2(fma2(c[i], uw, 0ull), np, ip));
                 }
+                asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst),
+                             "r"(w[0] ^ 0x80008000u), "r"(w[1] ^ 0x80008000u), "r"(w[2] ^ 0x80008000u),
+                             "r"(w[3] ^ 0x80008000u), "r"(w[4] ^ 0x80008000u), "r"(w[5] ^ 0x80008000u),
+                             "r"(w[6] ^ 0x80008000u), "r"(w[7] ^ 0x80008000u)
+                             : "memory");
             };
             for (int k0 = 0; k0 < p.nkb && ok; k0 += CG_KB) {
                 if (l < nsq) {
-                    const float b = -c_crt.m[l].nb[0], ib = c_crt.m[l].inv[0];
-                    uint32_t xr[64];
+                    const f32x2 nb = dup2(c_crt.m[l].nb[0]), b = dup2(-c_crt.m[l].nb[0]), ib = dup2(c_crt.m[l].inv[0]);
+                    // both accumulators are reduced to halves first, so TMEM is free again early
+                    uint32_t xr[64], yr[64];
                     wait_full(0);
                     if (!ok) break;
 #pragma unroll
@@ -664,11 +698,8 @@ __global__ void __launch_bounds__(CG_THREADS, 1) __cluster_dims__(2, 1, 1)
                         tmem_ld32(tq + part * 32, v);
                         tmem_ld_wait();
 #pragma unroll
-                        for (int i = 0; i < 16; i++) {
-                            const float x0 = crt_mod(__uint_as_float(v[2 * i]), pm, ip) + CRT_MAGIC;
-                            const float x1 = crt_mod(__uint_as_float(v[2 * i + 1]), pm, ip) + CRT_MAGIC;
-                            xr[part * 16 + i] = __byte_perm(__float_as_uint(x0), __float_as_uint(x1), 0x5410);
-                        }
+                        for (int i = 0; i < 16; i++)
+                            xr[part * 16 + i] = crt_halves(crt_mod2(pack2(v[2 * i], v[2 * i + 1]), np, ip));
                     }
                     release(0);
                     wait_full(1);
@@ -676,37 +707,45 @@ __global__ void __launch_bounds__(CG_THREADS, 1) __cluster_dims__(2, 1, 1)
 #pragma unroll
                     for (int part = 0; part < 4; part++) {
                         uint32_t v[32];
-                        float c[32];
-                        __syncwarp();  // rows past M skip their stores
                         tmem_ld32(tq + 256 + part * 32, v);
                         tmem_ld_wait();
-                        if (part == 3) release(1);
 #pragma unroll
-                        for (int i = 0; i < 32; i++) {
-                            const uint32_t w = xr[part * 16 + i / 2];
-                            const int xi = i % 2 ? (int)w >> 16 : (int)(int16_t)(w & 0xffff);
-                            const float x = __int_as_float(0x4B400000 + xi) - CRT_MAGIC;
-                            c[i] = __fmaf_rn(b, crt_mod(__uint_as_float(v[i]), b, ib), x);
-                        }
-                        put(part, c, k0 > 0);
+                        for (int i = 0; i < 16; i++)
+                            yr[part * 16 + i] = crt_halves(crt_mod2(pack2(v[2 * i], v[2 * i + 1]), nb, ib));
+                    }
+                    release(1);
+#pragma unroll
+                    for (int g = 0; g < 8; g++) {
+                        f32x2 c[8];
+#pragma unroll
+                        for (int i = 0; i < 8; i++)
+                            c[i] = fma2(b, crt_floats(yr[g * 8 + i]), crt_floats(xr[g * 8 + i]));
+                        put(g * 16, c, k0 > 0);
                     }
                 } else {
+                    uint32_t xr[64];
                     wait_full(turn);
                     if (!ok) break;
 #pragma unroll
                     for (int part = 0; part < 4; part++) {
                         uint32_t v[32];
-                        float c[32];
-                        __syncwarp();  // rows past M skip their stores
                         tmem_ld32(tq + turn * 256 + part * 32, v);
                         tmem_ld_wait();
-                        if (part == 3) release(turn);
 #pragma unroll
-                        for (int i = 0; i < 32; i++) c[i] = crt_mod(__uint_as_float(v[i]), pm, ip);
-                        put(part, c, k0 > 0);
+                        for (int i = 0; i < 16; i++)
+                            xr[part * 16 + i] = crt_halves(crt_mod2(pack2(v[2 * i], v[2 * i + 1]), np, ip));
+                    }
+                    release(turn);
+#pragma unroll
+                    for (int g = 0; g < 8; g++) {
+                        f32x2 c[8];
+#pragma unroll
+                        for (int i = 0; i < 8; i++) c[i] = crt_floats(xr[g * 8 + i]);
+                        put(g * 16, c, k0 > 0);
                     }
                     turn ^= 1;
                 }
+                __syncwarp();  // rows past M skip their stores; the TMEM reads are warp-wide
             }
         }
     }

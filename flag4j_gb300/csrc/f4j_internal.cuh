@@ -186,6 +186,8 @@ int f4j_check_sampled(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, 
                       double* max_rel);
 int f4j_gemm_exact(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, const double* A,
                    int opA, const double* B, int opB, double* C);
+// any_form: the caller did not ask for F4J_MODE_SPLIT itself, so the faster of
+// the split forms may run also where f4j_dgemm_split_noalloc fixes the bits.
 int f4j_gemm_split(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, const double* A,
-                   int opA, const double* B, int opB, double* C, int slices_req,
+                   int opA, const double* B, int opB, double* C, int slices_req, bool any_form,
                    f4j_report* rep, const int** gate);

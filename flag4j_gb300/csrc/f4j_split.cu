@@ -152,12 +152,22 @@ __device__ __forceinline__ void stat_elem(double x, unsigned long long& mx, long
     }
 }
 
-// One warp per stored row: stats of stored rows (block blk covers rows 8 blk .. 8 blk + 7).
-__device__ __forceinline__ void stats_rows_body(const double* __restrict__ X, int64_t rows, int64_t cols, int cplx,
-                                                int64_t blk, unsigned long long* __restrict__ mx_out,
-                                                long long* __restrict__ esum_out, int* __restrict__ cnt_out,
-                                                int* __restrict__ bad_out) {
-    int64_t r = blk * (blockDim.x / 32) + threadIdx.x / 32;
+// Lanes' statistics to lane 0.
+__device__ __forceinline__ void stats_warp_sum(unsigned long long& mx, long long& es, int& cnt, int& bad) {
+    for (int off = 16; off; off >>= 1) {
+        unsigned long long o = __shfl_xor_sync(0xffffffffu, mx, off);
+        mx = o > mx ? o : mx;
+        es += __shfl_xor_sync(0xffffffffu, es, off);
+        cnt += __shfl_xor_sync(0xffffffffu, cnt, off);
+        bad |= __shfl_xor_sync(0xffffffffu, bad, off);
+    }
+}
+
+// One warp per stored row.
+__global__ void k_stats_rows(const double* __restrict__ X, int64_t rows, int64_t cols, int cplx,
+                             unsigned long long* __restrict__ mx_out, long long* __restrict__ esum_out,
+                             int* __restrict__ cnt_out, int* __restrict__ bad_out) {
+    int64_t r = (int64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     int lane = threadIdx.x % 32;
     if (r >= rows) return;
     unsigned long long mx = 0;
@@ -166,13 +176,7 @@ __device__ __forceinline__ void stats_rows_body(const double* __restrict__ X, in
     int64_t w = cplx ? 2 * cols : cols;
     const double* row = X + r * w;
     for (int64_t c = lane; c < w; c += 32) stat_elem(row[c], mx, es, cnt, bad);
-    for (int off = 16; off; off >>= 1) {
-        unsigned long long o = __shfl_xor_sync(0xffffffffu, mx, off);
-        mx = o > mx ? o : mx;
-        es += __shfl_xor_sync(0xffffffffu, es, off);
-        cnt += __shfl_xor_sync(0xffffffffu, cnt, off);
-        bad |= __shfl_xor_sync(0xffffffffu, bad, off);
-    }
+    stats_warp_sum(mx, es, cnt, bad);
     if (lane == 0) {
         mx_out[r] = mx;
         esum_out[r] = es;
@@ -181,10 +185,37 @@ __device__ __forceinline__ void stats_rows_body(const double* __restrict__ X, in
     }
 }
 
-__global__ void k_stats_rows(const double* __restrict__ X, int64_t rows, int64_t cols, int cplx,
-                             unsigned long long* __restrict__ mx_out, long long* __restrict__ esum_out,
-                             int* __restrict__ cnt_out, int* __restrict__ bad_out) {
-    stats_rows_body(X, rows, cols, cplx, blockIdx.x, mx_out, esum_out, cnt_out, bad_out);
+// One block of 256 threads per stored row.
+__global__ void __launch_bounds__(256) k_stats_row_blocks(const double* __restrict__ X, int64_t cols, int cplx,
+                                                          unsigned long long* __restrict__ mx_out,
+                                                          long long* __restrict__ esum_out, int* __restrict__ cnt_out,
+                                                          int* __restrict__ bad_out) {
+    __shared__ unsigned long long smx[8];
+    __shared__ long long ses[8];
+    __shared__ int scnt[8], sbad[8];
+    const int64_t r = blockIdx.x;
+    const int warp = threadIdx.x / 32;
+    unsigned long long mx = 0;
+    long long es = 0;
+    int cnt = 0, bad = 0;
+    const int64_t w = cplx ? 2 * cols : cols;
+    const double* row = X + r * w;
+#pragma unroll 4
+    for (int64_t c = threadIdx.x; c < w; c += 256) stat_elem(row[c], mx, es, cnt, bad);
+    stats_warp_sum(mx, es, cnt, bad);
+    if (threadIdx.x % 32 == 0) smx[warp] = mx, ses[warp] = es, scnt[warp] = cnt, sbad[warp] = bad;
+    __syncthreads();
+    if (threadIdx.x) return;
+    for (int i = 1; i < 8; i++) {
+        mx = smx[i] > mx ? smx[i] : mx;
+        es += ses[i];
+        cnt += scnt[i];
+        bad |= sbad[i];
+    }
+    mx_out[r] = mx;
+    esum_out[r] = es;
+    cnt_out[r] = cnt;
+    if (bad) atomicExch(bad_out, 1);
 }
 
 // Thread per stored column, block (bx, by) over chunks of `chunk` rows: stats
@@ -237,9 +268,11 @@ __device__ __forceinline__ int finalize_target(int64_t t, int64_t targets, int d
             // in the fixed-point form instead of being rounded at 2^(-1022 - F)
             int E = (int)(b >> 52);
             e = E ? E - 1022 : (63 - __clzll((long long)b)) - 1073;
-            double mean = (double)esum[t] / (double)cnt[t];
-            double s = (double)(e - 1) - mean;
-            sp = s > 0 ? (int)(s * 256.0 + 0.5) : 0;
+            // (e - 1) - mean exponent, from its exact numerator: 32 bits carry it to
+            // 2^-8 for any spread, and GB300's FP64 division would be the longest
+            // wait of this kernel
+            const long long num = (long long)(e - 1) * cnt[t] - esum[t];
+            sp = num > 0 ? (int)((float)num / (float)cnt[t] * 256.0f + 0.5f) : 0;
         }
         e_out[t] = e;
         if (dup) e_out[t + targets] = e;
@@ -275,13 +308,20 @@ __global__ void k_stats_finalize(int64_t targets, int dup, const unsigned long l
 //   F >= 51.74 + 0.81 (sa + sb) - 0.36 log2 k.
 // A second floor, F >= 54 + max(sa, sb) - floor(log2 k), keeps short sums
 // within the componentwise bound 2 k u |A||B|.
-__host__ __device__ inline int slices_for(double sa, double sb, int64_t k, int64_t klen) {
-    sa = sa > 0 ? sa : 0.0;
-    sb = sb > 0 ? sb : 0.0;
+// What the model takes from the lengths, evaluated on the host: the two floors'
+// constant parts.
+struct SliceModel {
+    double accuracy, bound;
+};
+inline SliceModel slice_model(int64_t k, int64_t klen) {
     int lk = 0;
     while (lk < 62 && (2ll << lk) <= k) lk++;  // floor(log2 k)
-    const double lklen = log2((double)(klen > 1 ? klen : 1));
-    const double need = fmax(51.74 + 0.81 * (sa + sb) - 0.36 * lklen, 54.0 + fmax(sa, sb) - (double)lk);
+    return SliceModel{51.74 - 0.36 * log2((double)(klen > 1 ? klen : 1)), 54.0 - (double)lk};
+}
+__host__ __device__ inline int slices_for(double sa, double sb, const SliceModel& m) {
+    sa = sa > 0 ? sa : 0.0;
+    sb = sb > 0 ? sb : 0.0;
+    const double need = fmax(m.accuracy + 0.81 * (sa + sb), m.bound + fmax(sa, sb));
     int s = 1 + (int)ceil((need - 4.0) / 5.0);
     return s < 2 ? 2 : (s > S_MAX ? S_MAX : s);
 }
@@ -405,12 +445,12 @@ __host__ __device__ inline int plan_build(int s, int64_t Kp, int64_t klen_cat, S
 
 // One thread: slice count and the group / round / MMA program from the
 // statistics.  misc: [0] non-finite flag, [1] spread of A x256, [2] of B.
-__global__ void k_plan(const int* __restrict__ misc, int64_t k, int64_t Kp, int64_t klen_cat, int s_req,
+__global__ void k_plan(const int* __restrict__ misc, const SliceModel model, int64_t Kp, int64_t klen_cat, int s_req,
                        int band, int kcb_cap, SplitPlan* __restrict__ plan) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     const double spread = (misc[1] > misc[2] ? misc[1] : misc[2]) / 256.0;
     int s = s_req > 0 ? (s_req > S_MAX ? S_MAX : (s_req < 2 ? 2 : s_req))
-                      : slices_for(misc[1] / 256.0, misc[2] / 256.0, k, klen_cat);
+                      : slices_for(misc[1] / 256.0, misc[2] / 256.0, model);
     int n = plan_build(s, Kp, klen_cat, plan, band, kcb_cap);
     plan->s = s;
     plan->nrounds = n < 0 ? 0 : n;
@@ -442,12 +482,12 @@ __device__ __forceinline__ void crt_header(SplitPlan* plan, int s, const CrtPick
 // One block of 128 threads: k_plan's result from a plan table (the slice count
 // from the statistics, that plan copied, the header filled in); for the
 // residue form (tab null) the header alone.
-__global__ void k_plan_pick(const int* __restrict__ misc, int64_t k, int64_t klen_cat, int s_req,
+__global__ void k_plan_pick(const int* __restrict__ misc, const SliceModel model, int s_req,
                             const SplitPlan* __restrict__ tab, const CrtPick pick, SplitPlan* __restrict__ plan) {
     if (blockIdx.x != 0) return;
     const double spread = (misc[1] > misc[2] ? misc[1] : misc[2]) / 256.0;
     const int s = s_req > 0 ? (s_req > S_MAX ? S_MAX : (s_req < 2 ? 2 : s_req))
-                            : slices_for(misc[1] / 256.0, misc[2] / 256.0, k, klen_cat);
+                            : slices_for(misc[1] / 256.0, misc[2] / 256.0, model);
     if (!tab) {
         if (threadIdx.x == 0) crt_header(plan, s, pick, (float)spread, misc[0]);
         return;
@@ -480,8 +520,7 @@ __global__ void __launch_bounds__(256) k_finalize_pick(int64_t ta, int64_t tb, i
                                                        const unsigned long long* __restrict__ mxb,
                                                        const long long* __restrict__ esb,
                                                        const int* __restrict__ cnb, int* __restrict__ ea,
-                                                       int* __restrict__ eb, int* misc, int64_t k,
-                                                       int64_t klen_cat, int s_req,
+                                                       int* __restrict__ eb, int* misc, const SliceModel model, int s_req,
                                                        const SplitPlan* __restrict__ tab,
                                                        const CrtPick pick, SplitPlan* __restrict__ plan) {
     const int64_t nba = (ta + 255) / 256;
@@ -503,7 +542,7 @@ __global__ void __launch_bounds__(256) k_finalize_pick(int64_t ta, int64_t tb, i
     const int sa = atomicAdd(&misc[1], 0), sb = atomicAdd(&misc[2], 0), bad = atomicAdd(&misc[0], 0);
     const double spread = (sa > sb ? sa : sb) / 256.0;
     const int s = s_req > 0 ? (s_req > S_MAX ? S_MAX : (s_req < 2 ? 2 : s_req))
-                            : slices_for(sa / 256.0, sb / 256.0, k, klen_cat);
+                            : slices_for(sa / 256.0, sb / 256.0, model);
     if (!tab) {
         if (threadIdx.x == 0) crt_header(plan, s, pick, (float)spread, bad);
         return;
@@ -526,11 +565,11 @@ __global__ void __launch_bounds__(256) k_finalize_pick(int64_t ta, int64_t tb, i
 // picked with (from part of op(A)), or an operand holds a NaN / Inf, or the
 // plan stood down; 0 when the product sliced with `plan` is the one k_plan
 // would have planned.
-__global__ void k_spec_check(int* __restrict__ misc, int64_t k, int64_t klen_cat, int s_req,
+__global__ void k_spec_check(int* __restrict__ misc, const SliceModel model, int s_req,
                              const SplitPlan* __restrict__ plan) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     const int s = s_req > 0 ? (s_req > S_MAX ? S_MAX : (s_req < 2 ? 2 : s_req))
-                            : slices_for(misc[1] / 256.0, misc[2] / 256.0, k, klen_cat);
+                            : slices_for(misc[1] / 256.0, misc[2] / 256.0, model);
     misc[5] = (s != plan->s || misc[0] != 0 || plan->nonfinite) ? 1 : 0;
 }
 
@@ -1271,6 +1310,18 @@ static int split_kcb_cap(int64_t tiles, int64_t nkb, int* nchunks) {
     return (int)best;
 }
 
+// Row statistics of a stored rows x cols operand.  A block per row while a warp
+// per row would leave SMs without a block of eight rows: a few hundred rows then
+// wait for their own loads, one after the other.  Measured, us, warp / block per
+// row: 700 x 2500 14.7 / 8.4, 2111 x 1543 11.0 / 13.0.
+static void launch_stats_rows(const double* X, int64_t rows, int64_t cols, int cplx, int sm_count,
+                              unsigned long long* mx, long long* es, int* cn, int* bad, cudaStream_t st) {
+    if (rows < 8 * (int64_t)sm_count && cols >= 512)
+        k_stats_row_blocks<<<(unsigned)rows, 256, 0, st>>>(X, cols, cplx, mx, es, cn, bad);
+    else
+        k_stats_rows<<<(unsigned)f4j_cdiv(rows, 8), 256, 0, st>>>(X, rows, cols, cplx, mx, es, cn, bad);
+}
+
 // Column statistics of a stored rows x cols operand whose rows are ld elements
 // apart.  Row chunks of 256, halved (down to 16) while the grid has fewer than
 // four blocks per SM: a 1024-wide operand otherwise runs as 16 blocks.  The
@@ -1381,13 +1432,13 @@ static int split_prepare(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t 
     // statistics, one launch per operand (one launch for both measured 233 us
     // against 91 + 85 us at 8192^3, and the same at 1024^3)
     if (a_rows) {
-        k_stats_rows<<<(unsigned)f4j_cdiv(M, 8), 256, 0, ctx->stream>>>(A, M, k, cplx, mxa, esa, cna, misc);
+        launch_stats_rows(A, M, k, cplx, ctx->sm_count, mxa, esa, cna, misc, ctx->stream);
     } else {
         launch_stats_cols(A, k, M, M, cplx, ctx->sm_count, mxa, esa, cna, misc, ctx->stream);
     }
     F4J_LAUNCHED(ctx);
     if (b_rows) {
-        k_stats_rows<<<(unsigned)f4j_cdiv(n, 8), 256, 0, ctx->stream>>>(B, n, k, cplx, mxb, esb, cnb, misc);
+        launch_stats_rows(B, n, k, cplx, ctx->sm_count, mxb, esb, cnb, misc, ctx->stream);
     } else {
         launch_stats_cols(B, k, n, n, cplx, ctx->sm_count, mxb, esb, cnb, misc, ctx->stream);
     }
@@ -1400,7 +1451,7 @@ static int split_prepare(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t 
         if (rc) return rc;
         const unsigned blocks = (unsigned)(f4j_cdiv(M, 256) + f4j_cdiv(n, 256));
         k_finalize_pick<<<blocks, 256, 0, ctx->stream>>>(M, n, cplx ? 1 : 0, mxa, esa, cna, mxb, esb, cnb, ea, eb,
-                                                         misc, k, klen_cat,
+                                                         misc, slice_model(k, klen_cat),
                                                          slices_req > 0 ? slices_req : env_slices(), tab, CrtPick{},
                                                          plan);
         F4J_LAUNCHED(ctx);
@@ -1506,23 +1557,29 @@ static int split_report(f4j_ctx* ctx, const SplitPlan* plan, f4j_report* rep) {
 }
 
 // ------------------------------------------------------------------ residue form, host side
-// Whether a split product takes the residue form: a function of the shape
-// alone, so the device and the host-buffer path agree.  Not the shapes that
-// f4j_dgemm_split_noalloc accepts (its result is f4j_dgemm's bit for bit and
-// its scratch holds slice planes only), nor a forced small slice count.
+// Whether a split product takes the residue form: a function of the shape and
+// the mode asked for, so the device and the host-buffer path agree.  Not a
+// forced small slice count, and with F4J_MODE_SPLIT (any_form false) not the
+// shapes f4j_dgemm_split_noalloc accepts: its result is that mode's bit for
+// bit, and its scratch holds slice planes only.
 // Narrow and short products stay with the slices: the residue planes cost
 // about twice as much per element, the tiles are 256 wide, and reconstructing
-// C is work per entry that the slices do not have.  Measured on GB300, slices
-// / residues, us: 8192 x 8192 x 512 1731 / 2400, 3000 x 3000 x 500 316 / 402,
-// 1500 x 1500 x 1000 180 / 193, 2048 x 2048 x 1024 291 / 275, 700 x 700 x 2500
-// 208 / 158, 384 x 8192 x 8192 1750 / 1492, 8192^3 19200 / 11900; complex
-// 384 x 192 x 300 90 / 72, 1000 x 1000 x 300 200 / 171.
-static bool crt_wanted(bool cplx, int64_t m, int64_t n, int64_t k, int slices_req) {
+// C is work per entry that the slices do not have.  Measured on GB300, us,
+// slices / residues: 256^3 68 / 52, 512^3 74 / 60, 1024^3 123 / 108, 1024 x
+// 1024 x 512 95 / 92, 1500 x 1500 x 512 113 / 131, 4096 x 4096 x 512 503 / 528,
+// 2500 x 700 x 600 200 / 130, 4096 x 4096 x 768 774 / 584, 256 x 256 x 4096
+// 91 / 98, 300 x 3000 x 1000 133 / 140, 256 x 8192 x 8192 1107 / 1097, 384 x
+// 8192 x 8192 1750 / 1410, 8192^3 19200 / 12000; complex 384 x 192 x 300
+// 86 / 69, 2000 x 2000 x 100 259 / 284.
+static bool crt_wanted(bool cplx, int64_t m, int64_t n, int64_t k, int slices_req, bool any_form) {
     const int req = slices_req > 0 ? slices_req : env_slices();
     if (req > 0 && req < 8) return false;
     const int64_t N = cplx ? 2 * n : n, klen = cplx ? 2 * k : k;
-    if (m < 384 || N < 384 || klen < (cplx ? 512 : 1024) || klen > (1 << 22)) return false;
-    if (!cplx && F4J_NOALLOC_NEED(m, n, f4j_cdiv(k, BKB) * BKB) <= F4J_NOALLOC_SCRATCH_BYTES) return false;
+    const int64_t lo = m < N ? m : N, hi = m < N ? N : m;
+    if (lo < 384 && !(lo >= 256 && hi <= 1024 && klen <= 2048)) return false;
+    if (klen < (lo * hi <= (1 << 20) ? 256 : 576) || klen > (1 << 22)) return false;
+    if (!any_form && !cplx && F4J_NOALLOC_NEED(m, n, f4j_cdiv(k, BKB) * BKB) <= F4J_NOALLOC_SCRATCH_BYTES)
+        return false;
     return crt_config(S_MAX, klen) >= 0;
 }
 
@@ -1603,7 +1660,7 @@ static int crt_setup(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, C
     S->Lo = small_layout(S->M, n, cplx ? 2 * n : n);
     S->plane_a = (size_t)S->M * S->Kp;
     S->plane_b = (size_t)S->N * S->Kp;
-    S->ldy = f4j_cdiv(S->N, 8) * 8;
+    S->ldy = f4j_cdiv(S->N, 16) * 16;  // rows of y start on 32-byte sectors
     S->tiles_m = (int)f4j_cdiv(S->M, CG_T);
     S->tiles_n = (int)f4j_cdiv(S->N, CG_T);
     const int64_t fit = (int64_t)(CRT_Y_BYTES / ((size_t)S->nmod * S->ldy * 2)) / CG_T;
@@ -1665,9 +1722,11 @@ static int crt_launch(f4j_ctx* ctx, const CrtSetup& S, bool cplx, int64_t n, dou
     unsigned bx = 32;  // threads along a row
     while (bx < 256 && bx < per_row) bx *= 2;
     const int64_t gx = f4j_cdiv(per_row, bx), gy = f4j_cdiv(r1 - r0, 256 / bx);
-    int64_t cap = 16 * (int64_t)ctx->sm_count / gx;  // a few blocks per resident slot, each over several rows
+    // at least three rows a block (its constants are loaded once), and a few blocks per resident slot
+    int64_t by = f4j_cdiv(gy, 3), cap = 16 * (int64_t)ctx->sm_count / gx;
     cap = cap < 1 ? 1 : (cap > 65535 ? 65535 : cap);
-    (cplx ? k_crt_combine<true> : k_crt_combine<false>)<<<dim3((unsigned)gx, (unsigned)(gy < cap ? gy : cap)), dim3(bx, 256 / bx), 0, stream>>>(cp);
+    by = by < cap ? by : cap;
+    (cplx ? k_crt_combine<true> : k_crt_combine<false>)<<<dim3((unsigned)gx, (unsigned)by), dim3(bx, 256 / bx), 0, stream>>>(cp);
     F4J_LAUNCHED(ctx);
     return F4J_OK;
 }
@@ -1685,17 +1744,17 @@ static int crt_gemm(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, co
     const bool a_rows = opA == F4J_OP_N, b_rows = opB != F4J_OP_N;
     f4j_prof_begin(ctx, F4J_PROF_PREP);
     if (a_rows)
-        k_stats_rows<<<(unsigned)f4j_cdiv(M, 8), 256, 0, ctx->stream>>>(A, M, k, cplx, S.mxa, S.esa, S.cna, S.misc);
+        launch_stats_rows(A, M, k, cplx, ctx->sm_count, S.mxa, S.esa, S.cna, S.misc, ctx->stream);
     else
         launch_stats_cols(A, k, M, M, cplx, ctx->sm_count, S.mxa, S.esa, S.cna, S.misc, ctx->stream);
     F4J_LAUNCHED(ctx);
     if (b_rows)
-        k_stats_rows<<<(unsigned)f4j_cdiv(n, 8), 256, 0, ctx->stream>>>(B, n, k, cplx, S.mxb, S.esb, S.cnb, S.misc);
+        launch_stats_rows(B, n, k, cplx, ctx->sm_count, S.mxb, S.esb, S.cnb, S.misc, ctx->stream);
     else
         launch_stats_cols(B, k, n, n, cplx, ctx->sm_count, S.mxb, S.esb, S.cnb, S.misc, ctx->stream);
     F4J_LAUNCHED(ctx);
     k_finalize_pick<<<(unsigned)(f4j_cdiv(M, 256) + f4j_cdiv(n, 256)), 256, 0, ctx->stream>>>(
-        M, n, 0, S.mxa, S.esa, S.cna, S.mxb, S.esb, S.cnb, S.ea, S.eb, S.misc, k, S.klen, env_slices(), nullptr,
+        M, n, 0, S.mxa, S.esa, S.cna, S.mxb, S.esb, S.cnb, S.ea, S.eb, S.misc, slice_model(k, S.klen), env_slices(), nullptr,
         S.pick, S.plan);
     F4J_LAUNCHED(ctx);
     {
@@ -1717,9 +1776,10 @@ static int crt_gemm(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, co
 }
 
 int f4j_gemm_split(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, const double* A, int opA,
-                   const double* B, int opB, double* C, int slices_req, f4j_report* rep, const int** gate) {
+                   const double* B, int opB, double* C, int slices_req, bool any_form, f4j_report* rep,
+                   const int** gate) {
     *gate = nullptr;
-    if (crt_wanted(cplx, m, n, k, slices_req)) {
+    if (crt_wanted(cplx, m, n, k, slices_req, any_form)) {
         const SplitPlan* plan = nullptr;
         const int rc = crt_gemm(ctx, cplx, m, n, k, A, opA, B, opB, C, &plan);
         if (rc != F4J_ERR_OOM) {
@@ -1842,6 +1902,7 @@ static int host_split_pipelined(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, i
     const auto split_k = cplx ? k_split<true> : k_split<false>;
     const auto planes_k = cplx ? k_crt_planes<true> : k_crt_planes<false>;
     const int s_req = env_slices();
+    const SliceModel model = slice_model(k, klen_cat);
     // the same K-chunk cap the ordinary path plans with (no split K here)
     int kchunks = 0;
     const int kcb_cap = crt ? 0 : split_kcb_cap(f4j_cdiv(M, BM) * f4j_cdiv(N, BN), Kp / BKB, &kchunks);
@@ -1934,8 +1995,8 @@ static int host_split_pipelined(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, i
         // one row part of A (upload u): statistics, exponents (spread into misc[1])
         auto a_part_stats = [&](int u, int64_t r0, int64_t rows) -> int {
             F4J_CUDA(cudaStreamWaitEvent(st, ctx->up_ev[u], 0));
-            k_stats_rows<<<(unsigned)f4j_cdiv(rows, 8), 256, 0, st>>>(dA + r0 * k * w2, rows, k, cplx ? 1 : 0,
-                                                                      mxa + r0, esa + r0, cna + r0, misc);
+            launch_stats_rows(dA + r0 * k * w2, rows, k, cplx ? 1 : 0, ctx->sm_count, mxa + r0, esa + r0, cna + r0,
+                              misc, st);
             F4J_LAUNCHED(ctx);
             k_stats_finalize<<<(unsigned)f4j_cdiv(rows, 256), 256, 0, st>>>(rows, 0, mxa + r0, esa + r0, cna + r0,
                                                                              ea + r0, misc + 1);
@@ -1984,8 +2045,8 @@ static int host_split_pipelined(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, i
             const int64_t cw = c1 - c0;
             F4J_CUDA(cudaStreamWaitEvent(st, ctx->up_ev[1 + j], 0));
             if (b_rows) {  // stored rows [c0, c1) of B (n x k)
-                k_stats_rows<<<(unsigned)f4j_cdiv(cw, 8), 256, 0, st>>>(dB + c0 * k * w2, cw, k, cplx ? 1 : 0,
-                                                                        mxb + c0, esb + c0, cnb + c0, misc);
+                launch_stats_rows(dB + c0 * k * w2, cw, k, cplx ? 1 : 0, ctx->sm_count, mxb + c0, esb + c0, cnb + c0,
+                                  misc, st);
             } else {       // stored columns [c0, c1) of B (k x n)
                 launch_stats_cols(dB + c0 * w2, k, cw, n, cplx ? 1 : 0, ctx->sm_count, mxb + c0, esb + c0, cnb + c0,
                                   misc, st);
@@ -1996,7 +2057,7 @@ static int host_split_pipelined(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, i
                                                                            cnb + c0, eb + c0, misc + 2);
             F4J_LAUNCHED(ctx);
             if (j == 0) {  // the plan from A's first rows and B's first columns, then those rows' slices
-                k_plan_pick<<<1, 128, 0, st>>>(misc, k, klen_cat, s_req, tab, crt ? R.pick : CrtPick{}, plan);
+                k_plan_pick<<<1, 128, 0, st>>>(misc, model, s_req, tab, crt ? R.pick : CrtPick{}, plan);
                 F4J_LAUNCHED(ctx);
                 rc = a_part_split(0, a0_rows);
                 if (rc) break;
@@ -2027,7 +2088,7 @@ static int host_split_pipelined(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, i
     rc = queue();
     int hm[6] = {0, 0, 0, 0, 0, 0};
     if (!rc) {
-        k_spec_check<<<1, 32, 0, st>>>(misc, k, klen_cat, s_req, plan);
+        k_spec_check<<<1, 32, 0, st>>>(misc, model, s_req, plan);
         cudaError_t e = cudaGetLastError();
         if (e == cudaSuccess) {
             ctx->launches++;
@@ -2121,7 +2182,7 @@ static int gemm_host(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, c
     // n == 1 runs the device path's matrix-vector kernel
     const bool split = k > 0 && n > 1 && f4j_resolve_mode(cplx, m, n, k, mode) == F4J_MODE_SPLIT;
     // the residue form's parts are whole 256 x 256 tiles and need all of C's residues at once
-    const bool crt = split && crt_wanted(cplx, m, n, k, 0);
+    const bool crt = split && crt_wanted(cplx, m, n, k, 0, mode == F4J_MODE_AUTO);
     const int tile = crt ? CG_T : BM;
     const int tiles_m = (int)f4j_cdiv(m, tile);
     const int want = env_host_parts("F4J_HOST_PARTS", F4J_HOST_PARTS);
@@ -2299,15 +2360,15 @@ extern "C" int f4j_dgemm_split_noalloc(int64_t m, int64_t n, int64_t k, const do
     F4J_CUDA(cudaMemsetAsync(w + off_misc, 0, 1024, st));
 
     const bool a_rows = (opA == F4J_OP_N), b_rows = (opB != F4J_OP_N);
-    if (a_rows) k_stats_rows<<<(unsigned)f4j_cdiv(M, 8), 256, 0, st>>>(A, M, k, 0, mxa, esa, cna, misc);
+    if (a_rows) launch_stats_rows(A, M, k, 0, sms, mxa, esa, cna, misc, st);
     else launch_stats_cols(A, k, M, M, 0, sms, mxa, esa, cna, misc, st);
-    if (b_rows) k_stats_rows<<<(unsigned)f4j_cdiv(N, 8), 256, 0, st>>>(B, N, k, 0, mxb, esb, cnb, misc);
+    if (b_rows) launch_stats_rows(B, N, k, 0, sms, mxb, esb, cnb, misc, st);
     else launch_stats_cols(B, k, N, N, 0, sms, mxb, esb, cnb, misc, st);
     k_stats_finalize<<<(unsigned)f4j_cdiv(M, 256), 256, 0, st>>>(M, 0, mxa, esa, cna, ea, misc + 1);
     k_stats_finalize<<<(unsigned)f4j_cdiv(N, 256), 256, 0, st>>>(N, 0, mxb, esb, cnb, eb, misc + 2);
     int kchunks_na = 0;  // the same chunks as f4j_dgemm plans for this shape, run in turn
     const int kcb_cap = split_kcb_cap(f4j_cdiv(M, BM) * f4j_cdiv(N, BN), Kp / BKB, &kchunks_na);
-    k_plan<<<1, 32, 0, st>>>(misc, k, Kp, k, env_slices(), env_band(), kcb_cap, plan);
+    k_plan<<<1, 32, 0, st>>>(misc, slice_model(k, k), Kp, k, env_slices(), env_band(), kcb_cap, plan);
     F4J_CUDA(cudaGetLastError());
     // The slicing and slice GEMM kernels read the plan's verdict on the device
     // and return at once for a NaN/Inf operand or a plan that does not fit.
