@@ -369,21 +369,37 @@ __global__ void k_count(int64_t n, const int* __restrict__ idx, int* __restrict_
 
 // COO -> CSR row count with the row range check of SparseValidation.validateCoo:
 // one count per in-range row index in counts_plus1[r + 1], and the first
-// position of an out-of-range one in *first_bad.  Lanes of a warp holding the
-// same row add together (COO input is usually row-sorted, so a warp's 32
-// entries fall in a few rows).
+// position of an out-of-range one in *first_bad.  A thread takes eight
+// consecutive entries and adds each run of equal rows at once (COO input is
+// usually row-sorted): 16.8 M entries of 16 a row 71 -> 25 us against one entry
+// a lane with equal rows matched across the warp.  VEC: 16-byte loads.
+template <bool VEC>
 __global__ void k_count_rows_checked(int64_t n, const int* __restrict__ idx, int64_t limit,
                                      int* __restrict__ counts_plus1, int* __restrict__ first_bad) {
-    const int lane = threadIdx.x & 31;
-    const int64_t stride = ((int64_t)gridDim.x * blockDim.x) & ~(int64_t)31;
-    for (int64_t base = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~(int64_t)31; base < n; base += stride) {
-        const int64_t i = base + lane;
-        const bool in = i < n;
-        const int v = in ? idx[i] : -1;
-        const bool ok = in && v >= 0 && v < limit;
-        if (in && !ok) atomicMin(first_bad, (int)i);
-        const unsigned peers = __match_any_sync(0xffffffffu, ok ? v : -1);
-        if (ok && lane == __ffs(peers) - 1) atomicAdd(&counts_plus1[v + 1], __popc(peers));
+    const int64_t i0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
+    if (i0 >= n) return;
+    const int m = n - i0 < 8 ? (int)(n - i0) : 8;
+    int v[8];
+    if (VEC && m == 8) {
+        const int4 a = reinterpret_cast<const int4*>(idx + i0)[0], b = reinterpret_cast<const int4*>(idx + i0)[1];
+        v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+    } else {
+#pragma unroll
+        for (int u = 0; u < 8; u++) v[u] = u < m ? idx[i0 + u] : -1;
+    }
+    int run = 0;
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+        if (u >= m) break;
+        if (v[u] < 0 || v[u] >= limit) {
+            atomicMin(first_bad, (int)(i0 + u));
+            continue;
+        }
+        run++;
+        if (u + 1 >= m || v[u + 1] != v[u]) {
+            atomicAdd(&counts_plus1[v[u] + 1], run);
+            run = 0;
+        }
     }
 }
 
@@ -434,11 +450,27 @@ __global__ void k_validate_csr(int64_t rows, int64_t cols, int64_t nnz, const in
     }
 }
 
+// Row of each nonzero.  A warp covers 32 consecutive rows: their nonzeros are
+// written in order, each lane finding its row among the 32 by bisection over
+// the lanes (a warp per row left half its lanes idle at 16 nonzeros a row and
+// started 2^20 warps: 93 us for 16.8 M nonzeros).
 __global__ void k_expand_rows(int64_t rows, const int* __restrict__ rowptr, int* __restrict__ rowidx) {
-    const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
+    const int64_t w0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32) * 32;
     const int lane = threadIdx.x % 32;
-    if (row >= rows) return;
-    for (int q = rowptr[row] + lane; q < rowptr[row + 1]; q += 32) rowidx[q] = (int)row;
+    if (w0 >= rows) return;
+    const int64_t r = w0 + lane;
+    const int end = __ldg(rowptr + (r < rows ? r + 1 : rows));  // rows past the last end where it ends
+    const int q1 = __shfl_sync(0xffffffffu, end, 31);
+    for (int base = __ldg(rowptr + w0); base < q1; base += 32) {
+        const int q = base + lane;
+        int lo = 0;  // first row of the 32 that ends after q
+#pragma unroll
+        for (int step = 16; step; step >>= 1) {
+            const int e = __shfl_sync(0xffffffffu, end, lo + step - 1);
+            if (e <= q) lo += step;
+        }
+        if (q < q1) rowidx[q] = (int)(w0 + lo);
+    }
 }
 
 __global__ void k_iota(int64_t n, int* __restrict__ v) {
@@ -454,10 +486,11 @@ __global__ void k_flip_copy(int64_t n, const int* __restrict__ perm, const int* 
     if (i < n) keys[i] = (unsigned)src[perm ? perm[i] : i] ^ (flip ? 0x80000000u : 0u);
 }
 
+// perm and dst pass through once and are marked so, which leaves L2 to src.
 template <typename T>
 __global__ void k_gather(int64_t n, const int* __restrict__ perm, const T* __restrict__ src, T* __restrict__ dst) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        dst[i] = src[perm[i]];
+        __stcs(dst + i, __ldg(src + __ldcs(perm + i)));
 }
 
 // ---------------- inclusive scan (int32), 1024 threads x 4 items per block
@@ -574,6 +607,265 @@ __global__ void __launch_bounds__(RS_T) k_radix_scatter(int64_t n, const unsigne
         }
         __syncthreads();
     }
+}
+
+// ---------------- transpose structure: stable order by column in two passes
+// A stable sort of the nonzeros by column, most significant bits first.  Pass 1
+// (k_tp_hist, a scan, k_tp_scatter) moves each nonzero, as one 64-bit word of
+// its low column bits, row and source index, into at most TP_NB buckets of
+// 2^shift columns, in storage order inside each; pass 2 (k_tp_bucket, a block
+// per bucket) counts the bucket's columns, which gives its part of the row
+// pointers, and orders it by column.  Both rank stably the same way: each warp
+// owns a contiguous part of the items and a counter per bucket (column); the
+// counters are summed over the warps before, so a warp then only walks its own
+// items in order.  The lanes holding equal keys are found with one ballot per
+// key bit (__match_any_sync took ~130 clocks an SM for 32 mostly different
+// keys).  Items are placed in shared memory and leave in runs: gathering them
+// from global memory by their place instead took half of both passes.
+// Against an LSD radix sort of (column, index) pairs, three passes of two random
+// 4-byte writes at 2^20 columns, and the rows gathered after it: 2^20 rows and
+// columns, 16.8 M nonzeros, 0.93 -> 0.42 ms (scatter 148, bucket 185, histogram
+// and scan 67, rows 19 us).
+constexpr int TP_NB = 1024, TP_BITS = 10;
+constexpr int TP1_T = 256, TP1_WARPS = TP1_T / 32, TP1_TILE = 4096;  // pass 1: items per block
+constexpr int TP2_T = 512, TP2_WARPS = TP2_T / 32;
+constexpr int TP2_CNT = TP2_WARPS * TP_NB;
+constexpr int TP2_CAP = 18432;           // bucket items that pass 2 places in shared memory
+
+__global__ void __launch_bounds__(512) k_tp_hist(int64_t n, const int* __restrict__ col, int shift, int nb,
+                                                 int* __restrict__ hist, int nblocks) {
+    __shared__ int h[TP_NB];
+    for (int i = threadIdx.x; i < nb; i += 512) h[i] = 0;
+    __syncthreads();
+    const int64_t base = (int64_t)blockIdx.x * TP1_TILE;
+    const int cnt = (int)(n - base < TP1_TILE ? n - base : TP1_TILE);
+#pragma unroll 8
+    for (int i = threadIdx.x; i < cnt; i += 512) atomicAdd(&h[__ldg(col + base + i) >> shift], 1);
+    __syncthreads();
+    for (int i = threadIdx.x; i < nb; i += 512) hist[(int64_t)i * nblocks + blockIdx.x] = h[i];
+}
+
+// Exclusive prefix of v over the block's WARPS warps; *total their sum.
+template <int WARPS>
+__device__ __forceinline__ int tp_block_excl(int v, int* sh, int* total) {
+    const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+    int x = v;
+    for (int off = 1; off < 32; off <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, x, off);
+        if (lane >= off) x += o;
+    }
+    if (lane == 31) sh[warp] = x;
+    __syncthreads();
+    int before = 0, all = 0;
+    for (int w = 0; w < WARPS; w++) {
+        if (w < warp) before += sh[w];
+        all += sh[w];
+    }
+    __syncthreads();
+    *total = all;
+    return before + x - v;
+}
+
+// cnt[w * nkp + key]: how many of warp w's items have the key (nkp: keys rounded
+// up to a multiple of four, the rest zero).  Turns it into the place of the
+// warp's first one in (key, item) order; start(key, first, count) sees each
+// key's first place and count.  A thread takes four adjacent keys, so that one
+// block scan covers 4 x threads of them.
+template <int WARPS, typename F>
+__device__ __forceinline__ void tp_places(int* cnt, int nw, int nkp, int* sh, F start) {
+    int run = 0;
+    for (int k0 = 0; k0 < nkp; k0 += WARPS * 128) {
+        const int key = k0 + 4 * (int)threadIdx.x;
+        const bool in = key < nkp;
+        int4 c = make_int4(0, 0, 0, 0);
+        if (in)
+            for (int w = 0; w < nw; w++) {
+                const int4 t = *reinterpret_cast<const int4*>(cnt + w * nkp + key);
+                c.x += t.x, c.y += t.y, c.z += t.z, c.w += t.w;
+            }
+        int total;
+        int4 at;
+        at.x = run + tp_block_excl<WARPS>(c.x + c.y + c.z + c.w, sh, &total);
+        at.y = at.x + c.x, at.z = at.y + c.y, at.w = at.z + c.z;
+        if (in) {
+            start(key, at, c);
+            for (int w = 0; w < nw; w++) {
+                int4* p = reinterpret_cast<int4*>(cnt + w * nkp + key);
+                const int4 t = *p;
+                *p = at;
+                at.x += t.x, at.y += t.y, at.z += t.z, at.w += t.w;
+            }
+        }
+        run += total;
+    }
+    __syncthreads();
+}
+
+// The place of this lane's item (key < 0: none), stably after the warp's
+// earlier items; all lanes call.  keys below 2^bits.
+__device__ __forceinline__ int tp_rank(int* mine, int key, int bits) {
+    const int lane = threadIdx.x % 32;
+    unsigned peers = __ballot_sync(0xffffffffu, key >= 0);
+    for (int b = 0; b < bits; b++) {
+        const unsigned one = __ballot_sync(0xffffffffu, (key >> b) & 1);
+        peers &= (key >> b) & 1 ? one : ~one;
+    }
+    int at = 0;
+    if (key >= 0) at = mine[key];
+    const int r = __popc(peers & ((1u << lane) - 1));
+    __syncwarp();
+    if (key >= 0 && r == 0) mine[key] = at + __popc(peers);
+    __syncwarp();
+    return at + r;
+}
+
+// Item words: source index in the low qbits, row in the next rbits, column
+// within the bucket above.
+__global__ void __launch_bounds__(TP1_T) k_tp_scatter(int64_t n, const int* __restrict__ col,
+                                                      const int* __restrict__ row, int shift, int nb, int qbits,
+                                                      int rbits, const int* __restrict__ incl, int nblocks,
+                                                      unsigned long long* __restrict__ items, int* __restrict__ perm,
+                                                      int* __restrict__ t_row) {
+    extern __shared__ unsigned long long tp_smem[];
+    unsigned long long* place = tp_smem;                      // (column, row) at each place of the tile
+    int* cnt = reinterpret_cast<int*>(place + TP1_TILE);       // [warp][bucket]
+    int* delta = cnt + TP1_WARPS * TP_NB;                     // place in the output less place in the tile
+    uint16_t* order = reinterpret_cast<uint16_t*>(delta + TP_NB);  // tile item at each place
+    __shared__ int sh[TP1_WARPS];
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int64_t base = (int64_t)blockIdx.x * TP1_TILE;
+    const int m = (int)(n - base < TP1_TILE ? n - base : TP1_TILE);
+    // a lane's items are loaded once, all in flight together
+    constexpr int PART = TP1_TILE / TP1_WARPS, PER = PART / 32;
+    const int nkp = (nb + 3) & ~3;
+    int* mine = cnt + warp * nkp;
+    const int i0 = warp * PART + lane;
+    // this block's last place of four buckets, for tp_places (nb <= 4 x threads)
+    static_assert(TP_NB <= 4 * TP1_T, "four buckets a thread");
+    int last[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const int b = 4 * threadIdx.x + u;
+        last[u] = b < nb ? __ldg(incl + (int64_t)b * nblocks + blockIdx.x) : 0;
+    }
+    int c[PER], r[PER];
+#pragma unroll
+    for (int u = 0; u < PER; u++) {
+        const bool in = i0 + 32 * u < m;
+        c[u] = in ? __ldg(col + base + i0 + 32 * u) : -1;
+        r[u] = in ? __ldg(row + base + i0 + 32 * u) : 0;
+    }
+    for (int i = threadIdx.x; i < TP1_WARPS * nkp / 4; i += TP1_T)
+        reinterpret_cast<int4*>(cnt)[i] = make_int4(0, 0, 0, 0);
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < PER; u++)
+        if (c[u] >= 0) atomicAdd(&mine[c[u] >> shift], 1);
+    __syncthreads();
+    tp_places<TP1_WARPS>(cnt, TP1_WARPS, nkp, sh, [&](int b, int4 first, int4 k) {
+        *reinterpret_cast<int4*>(delta + b) = make_int4(last[0] - k.x - first.x, last[1] - k.y - first.y,
+                                                        last[2] - k.z - first.z, last[3] - k.w - first.w);
+    });
+#pragma unroll
+    for (int u = 0; u < PER; u++) {
+        const int at = tp_rank(mine, c[u] >= 0 ? c[u] >> shift : -1, TP_BITS);
+        if (c[u] >= 0) {
+            place[at] = (unsigned long long)(unsigned)c[u] << 32 | (unsigned)r[u];
+            order[at] = (uint16_t)(i0 + 32 * u);
+        }
+    }
+    __syncthreads();
+    for (int p = threadIdx.x; p < m; p += TP1_T) {
+        const unsigned long long w = place[p];
+        const int cc = (int)(w >> 32);
+        const unsigned long long q = (unsigned long long)(base + order[p]);
+        const int64_t dst = (int64_t)p + delta[cc >> shift];
+        if (items) {
+            items[dst] = q | (w & 0xffffffffull) << qbits |
+                         (unsigned long long)(cc & ((1 << shift) - 1)) << (qbits + rbits);
+        } else {  // one column a bucket: this is the whole order
+            perm[dst] = (int)q;
+            t_row[dst] = (int)w;
+        }
+    }
+}
+
+// Bucket blockIdx.x: columns [b << shift, (b + 1) << shift), items
+// [incl[b nblocks - 1], incl[(b + 1) nblocks - 1]) of the pass 1 output.
+__global__ void __launch_bounds__(TP2_T) k_tp_bucket(int64_t cols, int shift, int qbits, int rbits, int nw,
+                                                     const int* __restrict__ incl, int nblocks,
+                                                     const unsigned long long* __restrict__ items,
+                                                     int* __restrict__ t_rowptr, int* __restrict__ perm,
+                                                     int* __restrict__ t_row) {
+    extern __shared__ unsigned long long tp_smem[];
+    unsigned long long* place = tp_smem;                 // item at each place of the bucket
+    int* cnt = reinterpret_cast<int*>(place + TP2_CAP);   // [warp][column]
+    __shared__ int sh[TP2_WARPS];
+    const int b = blockIdx.x, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int64_t s0 = b ? __ldg(incl + (int64_t)b * nblocks - 1) : 0, s1 = __ldg(incl + (int64_t)(b + 1) * nblocks - 1);
+    const int m = (int)(s1 - s0);
+    const int64_t c0 = (int64_t)b << shift;
+    const int nk = (int)(cols - c0 < (1 << shift) ? cols - c0 : 1 << shift);
+    const int nkp = (nk + 3) & ~3;
+    const unsigned long long* in = items + s0;
+    for (int i = threadIdx.x; i < nw * nkp / 4; i += TP2_T) reinterpret_cast<int4*>(cnt)[i] = make_int4(0, 0, 0, 0);
+    __syncthreads();
+    // nw warps (all of them up to 2^10 columns a bucket) rank; each takes a multiple of 32 items
+    const int part = ((m + nw - 1) / nw + 31) & ~31;
+    int* mine = cnt + warp * nkp;
+    const int i0 = warp < nw ? (int)((int64_t)warp * part < m ? warp * part : m) : m;
+    const int i1 = (int64_t)i0 + part < m ? i0 + part : m;
+    const int up = qbits + rbits;
+    constexpr int U = 8;  // loads in flight per lane
+    for (int i = i0 + lane; i < i1; i += 32 * U) {
+        int key[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) key[u] = i + 32 * u < i1 ? (int)(__ldg(in + i + 32 * u) >> up) : -1;
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (key[u] >= 0) atomicAdd(&mine[key[u]], 1);
+    }
+    __syncthreads();
+    tp_places<TP2_WARPS>(cnt, nw, nkp, sh, [&](int c, int4 first, int4) {
+        const int f[4] = {first.x, first.y, first.z, first.w};
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (c + u < nk) t_rowptr[c0 + c + u] = (int)s0 + f[u];
+    });
+    if (b == gridDim.x - 1 && threadIdx.x == 0) t_rowptr[cols] = (int)s1;
+    const bool placed = m <= TP2_CAP;
+    const unsigned long long qmask = (1ull << qbits) - 1, rmask = (1ull << rbits) - 1;
+    for (int i = i0; i < i1; i += 32 * U) {
+        unsigned long long w[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) w[u] = i + 32 * u + lane < i1 ? __ldg(in + i + 32 * u + lane) : ~0ull;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const bool has = i + 32 * u + lane < i1;
+            const int at = tp_rank(mine, has ? (int)(w[u] >> up) : -1, shift);
+            if (!has) continue;
+            if (placed) {
+                place[at] = w[u];
+            } else {  // more items than shared memory holds: straight to their places
+                perm[s0 + at] = (int)(w[u] & qmask);
+                t_row[s0 + at] = (int)(w[u] >> qbits & rmask);
+            }
+        }
+    }
+    if (!placed) return;
+    __syncthreads();
+    for (int p = threadIdx.x; p < m; p += TP2_T) {
+        const unsigned long long w = place[p];
+        perm[s0 + p] = (int)(w & qmask);
+        t_row[s0 + p] = (int)(w >> qbits & rmask);
+    }
+}
+
+// Row pointers when every bucket is one column (shift 0).
+__global__ void k_tp_rowptr(int nb, const int* __restrict__ incl, int nblocks, int* __restrict__ t_rowptr) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c > nb) return;
+    t_rowptr[c] = c ? incl[(int64_t)c * nblocks - 1] : 0;
 }
 
 // ---------------- COO sort by (row, col), stable
@@ -921,50 +1213,117 @@ static int bits_for(int64_t maxval) {
     return b;
 }
 
+// Stable order of S's nonzeros by column and its row pointers, by
+// most-significant-bits-first buckets (see k_tp_scatter); shift: columns per
+// bucket, qbits / rbits: bits of a source index and of a row.
+static int transpose_buckets(f4j_ctx* ctx, f4j_csr S, int shift, int qbits, int rbits, const int* rowidx, int* trp,
+                             int* perm, int* trow) {
+    const int64_t nnz = S->nnz, cols = S->cols;
+    const int* col = (const int*)S->colidx->ptr;
+    const int nb = (int)((cols - 1) >> shift) + 1;
+    const int nblocks = (int)f4j_cdiv(nnz, TP1_TILE);
+    const size_t smem1 = (size_t)TP1_TILE * 10 + (size_t)(TP1_WARPS + 1) * TP_NB * 4;
+    const size_t smem2 = (size_t)TP2_CAP * 8 + (size_t)TP2_CNT * 4;
+    F4J_CUDA(cudaFuncSetAttribute(k_tp_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1));
+    F4J_CUDA(cudaFuncSetAttribute(k_tp_bucket, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));
+    int* hist = nullptr;
+    unsigned long long* items = nullptr;
+    int rc = f4j_dev_alloc(ctx, (size_t)nb * nblocks * 4, (void**)&hist);
+    if (!rc && shift) rc = f4j_dev_alloc(ctx, (size_t)nnz * 8, (void**)&items);
+    if (!rc) {
+        k_tp_hist<<<nblocks, 512, 0, ctx->stream>>>(nnz, col, shift, nb, hist, nblocks);
+        ctx->launches++;
+        rc = scan_inclusive(ctx, hist, (int64_t)nb * nblocks);
+    }
+    if (!rc) {
+        k_tp_scatter<<<nblocks, TP1_T, smem1, ctx->stream>>>(nnz, col, rowidx, shift, nb, qbits, rbits, hist, nblocks,
+                                                             items, perm, trow);
+        if (shift) {
+            const int nw = TP2_WARPS < TP2_CNT >> shift ? TP2_WARPS : TP2_CNT >> shift;
+            k_tp_bucket<<<nb, TP2_T, smem2, ctx->stream>>>(cols, shift, qbits, rbits, nw, hist, nblocks, items, trp,
+                                                           perm, trow);
+        } else {
+            k_tp_rowptr<<<grid1(nb + 1), 256, 0, ctx->stream>>>(nb, hist, nblocks, trp);
+        }
+        ctx->launches += 2;
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) rc = f4j_cuda_fail(e, "transpose structure");
+    }
+    f4j_dev_free(ctx, hist);
+    f4j_dev_free(ctx, items);
+    return rc;
+}
+
+// The same by an LSD radix sort of (column, index) pairs: past 2^22 columns
+// (4096 a bucket), where a block's counters leave fewer than four warps to rank,
+// and where an item does not fit 64 bits.
+static int transpose_radix(f4j_ctx* ctx, f4j_csr S, const int* rowidx, int* trp, int* perm, int* trow) {
+    const int64_t nnz = S->nnz, cols = S->cols;
+    unsigned* keys = nullptr;
+    int rc = f4j_dev_alloc(ctx, (size_t)nnz * 4, (void**)&keys);
+    if (rc) return rc;
+    // pointers of S^T: column counts, inclusive scan (as RealCsrOps.transpose :203-211)
+    cudaMemsetAsync(trp, 0, (size_t)(cols + 1) * 4, ctx->stream);
+    k_count<<<grid1(nnz), 256, 0, ctx->stream>>>(nnz, (const int*)S->colidx->ptr, trp);
+    ctx->launches++;
+    rc = scan_inclusive(ctx, trp + 1, cols);
+    if (!rc) {
+        // stable order by column == scatter in storage order (:216-222)
+        cudaMemcpyAsync(keys, S->colidx->ptr, (size_t)nnz * 4, cudaMemcpyDeviceToDevice, ctx->stream);
+        k_iota<<<grid1(nnz), 256, 0, ctx->stream>>>(nnz, perm);
+        ctx->launches++;
+        rc = radix_sort_pairs(ctx, keys, perm, nnz, bits_for(cols - 1));
+    }
+    if (!rc) {
+        k_gather<int><<<grid1(nnz), 256, 0, ctx->stream>>>(nnz, perm, rowidx, trow);
+        ctx->launches++;
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) rc = f4j_cuda_fail(e, "transpose structure");
+    }
+    f4j_dev_free(ctx, keys);
+    return rc;
+}
+
 // Builds the cached transpose structure of S (RealCsrOps.transpose order).
 static int ensure_transpose(f4j_ctx* ctx, f4j_csr S) {
     if (S->t_perm) return F4J_OK;
     const int64_t nnz = S->nnz, rows = S->rows, cols = S->cols;
-    int *trp = nullptr, *perm = nullptr, *trow = nullptr;
-    unsigned* keys = nullptr;
-    int* rowidx = nullptr;
+    int *trp = nullptr, *perm = nullptr, *trow = nullptr, *ri = nullptr;
     int rc = f4j_dev_alloc(ctx, (size_t)(cols + 1) * 4, (void**)&trp);
     if (!rc) rc = f4j_dev_alloc(ctx, (size_t)nnz * 4, (void**)&perm);
     if (!rc) rc = f4j_dev_alloc(ctx, (size_t)nnz * 4, (void**)&trow);
-    if (!rc) rc = f4j_dev_alloc(ctx, (size_t)nnz * 4, (void**)&keys);
-    if (!rc) rc = f4j_dev_alloc(ctx, (size_t)nnz * 4, (void**)&rowidx);
-    if (rc) goto fail;
-    // pointers of S^T: column counts, inclusive scan (as RealCsrOps.transpose :203-211)
-    F4J_CUDA(cudaMemsetAsync(trp, 0, (size_t)(cols + 1) * 4, ctx->stream));
-    if (nnz) {
-        k_count<<<grid1(nnz), 256, 0, ctx->stream>>>(nnz, (const int*)S->colidx->ptr, trp);
-        F4J_LAUNCHED(ctx);
-        rc = scan_inclusive(ctx, trp + 1, cols);
-        if (rc) goto fail;
-        // stable order by column == scatter in storage order (:216-222)
-        F4J_CUDA(cudaMemcpyAsync(keys, S->colidx->ptr, (size_t)nnz * 4, cudaMemcpyDeviceToDevice, ctx->stream));
-        k_iota<<<grid1(nnz), 256, 0, ctx->stream>>>(nnz, perm);
-        F4J_LAUNCHED(ctx);
-        rc = radix_sort_pairs(ctx, keys, perm, nnz, bits_for(cols - 1));
-        if (rc) goto fail;
-        k_expand_rows<<<grid1(rows * 32), 256, 0, ctx->stream>>>(rows, (const int*)S->rowptr->ptr, rowidx);
-        F4J_LAUNCHED(ctx);
-        k_gather<int><<<grid1(nnz), 256, 0, ctx->stream>>>(nnz, perm, rowidx, trow);
-        F4J_LAUNCHED(ctx);
+    if (!rc && nnz == 0) {
+        const cudaError_t e = cudaMemsetAsync(trp, 0, (size_t)(cols + 1) * 4, ctx->stream);
+        if (e != cudaSuccess) rc = f4j_cuda_fail(e, "transpose structure");
+    } else if (!rc) {
+        const int* rowidx = (const int*)S->rowidx;  // cached by f4j_sddmm, or made here
+        if (!rowidx) {
+            rc = f4j_dev_alloc(ctx, (size_t)nnz * 4, (void**)&ri);
+            if (!rc) {
+                k_expand_rows<<<(unsigned)f4j_cdiv(rows, 256), 256, 0, ctx->stream>>>(rows, (const int*)S->rowptr->ptr, ri);
+                ctx->launches++;
+            }
+            rowidx = ri;
+        }
+        int shift = 0;
+        while (((cols - 1) >> shift) >= TP_NB) shift++;
+        const int qbits = bits_for(nnz - 1), rbits = bits_for(rows - 1);
+        if (!rc)
+            rc = shift <= 12 && qbits + rbits + shift <= 64
+                     ? transpose_buckets(ctx, S, shift, qbits, rbits, rowidx, trp, perm, trow)
+                     : transpose_radix(ctx, S, rowidx, trp, perm, trow);
+        f4j_dev_free(ctx, ri);
     }
-    f4j_dev_free(ctx, keys);
-    f4j_dev_free(ctx, rowidx);
+    if (rc) {
+        f4j_dev_free(ctx, trp);
+        f4j_dev_free(ctx, perm);
+        f4j_dev_free(ctx, trow);
+        return rc;
+    }
     S->t_rowptr = trp;
     S->t_perm = perm;
     S->t_rowidx = trow;
     return F4J_OK;
-fail:
-    f4j_dev_free(ctx, trp);
-    f4j_dev_free(ctx, perm);
-    f4j_dev_free(ctx, trow);
-    f4j_dev_free(ctx, keys);
-    f4j_dev_free(ctx, rowidx);
-    return rc;
 }
 
 // Row of each nonzero, cached in the handle.
@@ -973,7 +1332,7 @@ static int ensure_rowidx(f4j_ctx* ctx, f4j_csr S) {
     int* ri = nullptr;
     int rc = f4j_dev_alloc(ctx, (size_t)S->nnz * 4, (void**)&ri);
     if (rc) return rc;
-    k_expand_rows<<<grid1(S->rows * 32), 256, 0, ctx->stream>>>(S->rows, (const int*)S->rowptr->ptr, ri);
+    k_expand_rows<<<(unsigned)f4j_cdiv(S->rows, 256), 256, 0, ctx->stream>>>(S->rows, (const int*)S->rowptr->ptr, ri);
     F4J_LAUNCHED(ctx);
     S->rowidx = ri;
     return F4J_OK;
@@ -1151,7 +1510,8 @@ extern "C" int f4j_csr_from_coo(f4j_ctx* ctx, int64_t rows, int64_t cols, int64_
     // inclusive scan; column indices and values copied unchanged
     F4J_CUDA(cudaMemsetAsync(rp, 0, (size_t)(rows + 1) * 4, ctx->stream));
     if (nnz) {
-        k_count_rows_checked<<<grid1(nnz), 256, 0, ctx->stream>>>(nnz, (const int*)rowidx->ptr, rows, rp, (int*)ws);
+        (f4j_aligned16(rowidx->ptr) ? k_count_rows_checked<true> : k_count_rows_checked<false>)
+            <<<grid1(f4j_cdiv(nnz, 8)), 256, 0, ctx->stream>>>(nnz, (const int*)rowidx->ptr, rows, rp, (int*)ws);
         F4J_LAUNCHED(ctx);
         const bool vec = ((reinterpret_cast<uintptr_t>(colidx->ptr) | reinterpret_cast<uintptr_t>(S->colidx->ptr)) &
                           15) == 0;

@@ -633,3 +633,37 @@ def test_spmv_balanced_lanes_edge_shapes(f4j, oracle, rows, lam, p_empty):
     assert np.array_equal(S.mult(f4j.Vector(x)).data, ref)
     y = S.mult(f4j.Vector(x), mode="fma").data
     assert np.all(np.abs(y - ref) <= fma_bound(oracle, rp, ci, v, x[:, None])[:, 0])
+
+
+@pytest.mark.parametrize("rows,cols,nnz,kind", [
+    (50, 1, 40, "uniform"), (3000, 7, 9000, "uniform"),                   # a column is a bucket
+    (5000, 1024, 40961, "uniform"), (5000, 1025, 40960, "uniform"),       # the most columns of that form, one more
+    (2000, (1 << 20) + 1, 30000, "uniform"), (2000, 1 << 22, 30000, "uniform"),  # 2048 and 4096 columns a bucket
+    (2000, (1 << 22) + 1, 30000, "uniform"),                              # the radix sort
+    (20000, 5000, 200000, "one column"), (20000, 5000, 200000, "few"),     # a bucket past shared memory
+    (40000, 9000, 30000, "gaps"),                                         # empty rows and columns
+])
+def test_transpose_structure_is_the_stable_column_order(f4j, rows, cols, nnz, kind):
+    """CsrMatrix.T() and the transpose permutation at the edges of the bucketed column sort: the stable
+    order by column of the nonzeros in storage order."""
+    g = np.random.default_rng(rows + cols + nnz)
+    row = np.sort(g.integers(0, rows, nnz)) if kind != "gaps" else np.sort(g.integers(0, rows // 3, nnz) * 3)
+    col = g.integers(0, cols, nnz)
+    if kind == "one column":
+        col[g.random(nnz) < 0.8] = cols - 2
+    elif kind == "few":
+        col = np.minimum(g.pareto(0.6, nnz).astype(np.int64), cols - 1)
+    elif kind == "gaps":
+        col = col // 5 * 5
+    rp = np.zeros(rows + 1, np.int32)
+    np.cumsum(np.bincount(row, minlength=rows), out=rp[1:])
+    vals = g.standard_normal(nnz)
+    S = f4j.CsrMatrix((rows, cols), vals, rp, col.astype(np.int32), validate=False)
+    perm = np.argsort(col, kind="stable")
+    trp = np.zeros(cols + 1, np.int32)
+    np.cumsum(np.bincount(col, minlength=cols), out=trp[1:])
+    assert np.array_equal(S.transposePermutation(), perm)
+    T = S.T()
+    assert np.array_equal(T.rowPointers, trp)
+    assert np.array_equal(T.colIndices, row[perm])
+    assert np.array_equal(T.data, vals[perm])
