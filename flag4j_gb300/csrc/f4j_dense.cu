@@ -87,6 +87,7 @@ __global__ void __launch_bounds__(TM * TN) k_gemm_exact(int64_t m, int64_t n, in
             else rb[i] = re;
         }
     };
+    const ExactOps ops;
     double cr = 0.0, ci = 0.0;
     fetch(0);
     for (int64_t k0 = 0; k0 < k; k0 += BK) {
@@ -108,12 +109,12 @@ __global__ void __launch_bounds__(TM * TN) k_gemm_exact(int64_t m, int64_t n, in
         auto step = [&](int kk) {
             if constexpr (CPLX) {
                 const double2 a = sA[kk][ty], b = sB[kk][tx];
-                const double pr = __dsub_rn(__dmul_rn(a.x, b.x), __dmul_rn(a.y, b.y));
-                const double pi = __dadd_rn(__dmul_rn(a.x, b.y), __dmul_rn(a.y, b.x));
-                cr = __dadd_rn(cr, pr);
-                ci = __dadd_rn(ci, pi);
+                const double pr = ops.sub(ops.mul(a.x, b.x), ops.mul(a.y, b.y));
+                const double pi = ops.add(ops.mul(a.x, b.y), ops.mul(a.y, b.x));
+                cr = ops.add(pr, cr);
+                ci = ops.add(pi, ci);
             } else {
-                cr = __dadd_rn(cr, __dmul_rn(sA[kk][ty], sB[kk][tx]));
+                cr = ops.add(ops.mul(sA[kk][ty], sB[kk][tx]), cr);
             }
         };
         if (k - k0 >= BK) {
@@ -555,15 +556,16 @@ static int launch_exact(f4j_ctx* ctx, int64_t m, int64_t n, int64_t k, const dou
     return F4J_OK;
 }
 
-// The FP64 units bound this kernel whatever the tile (1024^3: 4.09 ms for every
-// tile from 4 x 8 to 64 x 1), so the tile only has to put warps on every SM
+// The FP64 units bound this kernel whatever the tile (1024^3 with DMUL and DADD:
+// 4.09 ms for every tile from 4 x 8 to 64 x 1; with ExactOps 3.49 ms, 96 % of
+// two lanes per SM and clock), so the tile only has to put warps on every SM
 // sub-partition and leave few lanes idle: 8 x 8 (two warps) unless one side is
 // at most 6, where a tile of that side's width keeps the lanes busy.  Measured,
-// us, the earlier 64 x 64 tile / 8 x 8: 96 x 80 x 64 162 / 8.7, 700 x 500 x 600
-// 1497 / 849, 1024^3 4894 / 4090.  8 x 8 / 16 x 2 or 2 x 16: 8192 x 1 x 1000
-// 264 / 99, 2 x 8192 x 500 134 / 58, 4000 x 6 x 400 66 / 53, 4000 x 12 x 400
-// 109 / 81 but 1000 x 1 x 1000 92 / 96.  16 x 2 / 32 x 1: 30000 x 1 x 300
-// 80 / 52, 8192 x 1 x 1000 99 / 103.
+// us, the earlier 64 x 64 tile / 8 x 8: 96 x 80 x 64 162 / 10.3, 700 x 500 x 600
+// 1497 / 721, 1024^3 4894 / 3490.  The narrow tiles, with DMUL and DADD: 8 x 8
+// / 16 x 2 or 2 x 16: 8192 x 1 x 1000 264 / 99, 2 x 8192 x 500 134 / 58, 4000 x
+// 6 x 400 66 / 53, 4000 x 12 x 400 109 / 81 but 1000 x 1 x 1000 92 / 96.
+// 16 x 2 / 32 x 1: 30000 x 1 x 300 80 / 52, 8192 x 1 x 1000 99 / 103.
 template <bool CPLX>
 static int pick_exact(f4j_ctx* ctx, int64_t m, int64_t n, int64_t k, const double* A, int opA, const double* B,
                       int opB, double* C) {

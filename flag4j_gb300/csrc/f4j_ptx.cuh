@@ -78,6 +78,28 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
     return mbar_wait_ns(bar, parity, status, code, F4J_WAIT_NS);
 }
 
+// Separately rounded FP64 products and sums as fused multiply-adds: RN(a b) =
+// fma(a, b, -0) and RN(a + b) = fma(a, 1, b), signed zeros included.  GB300
+// issues an FMA of three registers every 68 clocks per SM sub-partition and a
+// DMUL, a DADD, or an FMA the assembler can turn into one (a constant operand)
+// every 80 (152 x 6 blocks of 256 threads on shared-memory operands), so the
+// constants 1 and -0 are kept in per-lane registers the compiler cannot see
+// through (a uniform register or constant-bank operand is the slow form too).
+// Latency is the other way round (one warp per sub-partition, 96 x 80 x 64: 9.6
+// us with DMUL and DADD, 10.3 so), which shows below one warp only; the FMAs
+// are ahead from two warps up.  gridDim.z is 1 in every kernel that uses this.
+struct ExactOps {
+    double one, nz;
+    __device__ __forceinline__ ExactOps() {
+        const unsigned zero = (gridDim.z - 1) * threadIdx.x;  // differs by lane for all the assembler knows
+        asm("mov.b64 %0, {%1, %2};" : "=d"(one) : "r"(zero), "r"(0x3FF00000u + zero));
+        asm("mov.b64 %0, {%1, %2};" : "=d"(nz) : "r"(zero), "r"(0x80000000u + zero));
+    }
+    __device__ __forceinline__ double mul(double a, double b) const { return __fma_rn(a, b, nz); }
+    __device__ __forceinline__ double add(double a, double b) const { return __fma_rn(a, one, b); }
+    __device__ __forceinline__ double sub(double a, double b) const { return __fma_rn(b, -one, a); }
+};
+
 // Asynchronous 4- / 8-byte copies global -> shared (no register staging; the
 // source and destination are aligned to the copy size), and the wait for all
 // of this thread's copies.  Other lanes see the data after a __syncwarp.

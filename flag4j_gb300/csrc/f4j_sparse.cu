@@ -39,19 +39,19 @@ namespace {
 // RealCsrDenseMatMult.standardVector rounds them (acc starts at +0.0), so y is
 // bit-identical.  GB300's FP64 pipe (2 lane-operations per clock per SM, two
 // per nonzero) bounds the exact mode; the random 8-byte gathers of x (one L2
-// sector each) come next.  No shared memory, so L1 keeps its full size for
+// sector each) come next.  Gathering the next group's x under the current
+// group's sums (two groups in registers, 2 to 4 blocks per SM) was slower, 147
+// to 237 us against 116 at 2^20 rows x 16: the warps lost hide more.  No shared memory, so L1 keeps its full size for
 // the gathers.
 // FUSED (the opt-in FMA mode) accumulates fma(v, x, acc) in the same order,
 // one FP64 instruction per nonzero, within the reference's componentwise bound.
 constexpr int SPMV_RPW_MAX = 256;  // rows per warp for large matrices
 constexpr int SPMV_BLOCK = 256;
 
-// Blocks per SM: 5 for the exact mode (48 registers, no spills), 4 for FMA
-// (whose 48-register build spills).
-template <bool FUSED>
-struct SpmvOcc {
-    static constexpr int BLOCKS = FUSED ? 4 : 5;
-};
+// Blocks per SM: 4 (64 registers) in both modes; 5 (48) spill.  Exact mode at
+// 2^20 rows x 16, us: separate multiplies and adds at 5 blocks 118-119, FMA
+// forms (ExactOps) at 5 blocks 120-122, at 4 blocks 115-116.
+constexpr int SPMV_BLOCKS = 4;
 
 // 32-byte read-only loads (one sector): 8 column indices, 4 values.  The
 // address must be 32-byte aligned.
@@ -65,7 +65,7 @@ __device__ __forceinline__ void ld_nc_v4_f64(const double* p, double& a, double&
 }
 
 template <bool FUSED, bool VEC>
-__global__ void __launch_bounds__(SPMV_BLOCK, SpmvOcc<FUSED>::BLOCKS)
+__global__ void __launch_bounds__(SPMV_BLOCK, SPMV_BLOCKS)
     k_spmv(int64_t rows, int64_t nnz, int rpw, const int* __restrict__ rowptr, const int* __restrict__ colidx,
            const double* __restrict__ vals, const double* __restrict__ x, double* __restrict__ y) {
     const int lane = threadIdx.x & 31;
@@ -92,6 +92,7 @@ __global__ void __launch_bounds__(SPMV_BLOCK, SpmvOcc<FUSED>::BLOCKS)
     int64_t r = a;
     int rend = __ldg(rowptr + a + 1);
     int rnext = a + 1 < b ? __ldg(rowptr + a + 2) : qe;
+    const ExactOps ops;
     double acc = 0.0;
     while (rend == qs) {  // empty rows before the lane's first nonzero
         y[r] = 0.0;
@@ -123,13 +124,13 @@ __global__ void __launch_bounds__(SPMV_BLOCK, SpmvOcc<FUSED>::BLOCKS)
         }
         if (!FUSED) {
 #pragma unroll
-            for (int u = 0; u < 8; u++) v[u] = __dmul_rn(v[u], xv[u]);
+            for (int u = 0; u < 8; u++) v[u] = ops.mul(v[u], xv[u]);
         }
 #pragma unroll
         for (int u = 0; u < 8; u++) {
             const int q = qb + u;
             if (q < qs || q >= qe) continue;
-            acc = FUSED ? __fma_rn(v[u], xv[u], acc) : __dadd_rn(acc, v[u]);
+            acc = FUSED ? __fma_rn(v[u], xv[u], acc) : ops.add(v[u], acc);
             while (q + 1 == rend) {  // row r ends here (and any empty rows after it)
                 y[r] = acc;
                 acc = 0.0;
@@ -151,7 +152,9 @@ __global__ void __launch_bounds__(SPMV_BLOCK, SpmvOcc<FUSED>::BLOCKS)
 // is half the exact mode's, so the X gathers' latency decides its speed: it
 // runs 8 blocks per SM (32 registers) to keep more of them in flight; the
 // exact mode runs 6 (40 registers), its best balance of loads in flight per
-// warp against warps.
+// warp against warps.  Exact mode at 2^20 rows x 16 nonzeros, 32 columns: 1.79
+// ms, 95 % of the FP64 pipe's two lanes per SM and clock (2.07 ms with DMUL
+// and DADD for ExactOps); 64 columns 3.54 ms (4.02), 5 columns .82 ms (.93).
 template <bool VEC2, bool PERM, bool FUSED = false>
 __global__ void __launch_bounds__(256, FUSED ? 8 : 6)
     k_spmm(int64_t rows, int64_t ncols, int G, const int* __restrict__ rowptr, const int* __restrict__ colidx,
@@ -161,6 +164,7 @@ __global__ void __launch_bounds__(256, FUSED ? 8 : 6)
     const int lane = threadIdx.x % G;
     const int64_t row = gid;
     if (row >= rows) return;
+    const ExactOps ops;
     const int q0 = rowptr[row], q1 = rowptr[row + 1];
     constexpr int W = VEC2 ? 2 : 1;
     for (int64_t cbase = (int64_t)lane * W; cbase < ncols; cbase += (int64_t)G * W) {
@@ -185,8 +189,8 @@ __global__ void __launch_bounds__(256, FUSED ? 8 : 6)
                         a0 = __fma_rn(v[u], xv[u].x, a0);
                         a1 = __fma_rn(v[u], xv[u].y, a1);
                     } else {
-                        a0 = __dadd_rn(a0, __dmul_rn(v[u], xv[u].x));
-                        a1 = __dadd_rn(a1, __dmul_rn(v[u], xv[u].y));
+                        a0 = ops.add(ops.mul(v[u], xv[u].x), a0);
+                        a1 = ops.add(ops.mul(v[u], xv[u].y), a1);
                     }
                 }
             } else {
@@ -194,7 +198,7 @@ __global__ void __launch_bounds__(256, FUSED ? 8 : 6)
 #pragma unroll
                 for (int u = 0; u < UN; u++) xv[u] = __ldg(X + (int64_t)c[u] * ncols + cbase);
 #pragma unroll
-                for (int u = 0; u < UN; u++) a0 = FUSED ? __fma_rn(v[u], xv[u], a0) : __dadd_rn(a0, __dmul_rn(v[u], xv[u]));
+                for (int u = 0; u < UN; u++) a0 = FUSED ? __fma_rn(v[u], xv[u], a0) : ops.add(ops.mul(v[u], xv[u]), a0);
             }
         }
         for (; q < q1; q++) {
@@ -202,11 +206,11 @@ __global__ void __launch_bounds__(256, FUSED ? 8 : 6)
             const double v = PERM ? __ldg(&vals[__ldg(&perm[q])]) : __ldg(&vals[q]);
             if (VEC2) {
                 const double2 xv = __ldg(reinterpret_cast<const double2*>(X + (int64_t)c * ncols + cbase));
-                a0 = FUSED ? __fma_rn(v, xv.x, a0) : __dadd_rn(a0, __dmul_rn(v, xv.x));
-                a1 = FUSED ? __fma_rn(v, xv.y, a1) : __dadd_rn(a1, __dmul_rn(v, xv.y));
+                a0 = FUSED ? __fma_rn(v, xv.x, a0) : ops.add(ops.mul(v, xv.x), a0);
+                a1 = FUSED ? __fma_rn(v, xv.y, a1) : ops.add(ops.mul(v, xv.y), a1);
             } else {
                 const double xe = __ldg(X + (int64_t)c * ncols + cbase);
-                a0 = FUSED ? __fma_rn(v, xe, a0) : __dadd_rn(a0, __dmul_rn(v, xe));
+                a0 = FUSED ? __fma_rn(v, xe, a0) : ops.add(ops.mul(v, xe), a0);
             }
         }
         if (VEC2) *reinterpret_cast<double2*>(Y + row * ncols + cbase) = make_double2(a0, a1);
@@ -226,6 +230,7 @@ __global__ void __launch_bounds__(256)
     const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
     const int lane = threadIdx.x % G;
     if (row >= rows) return;
+    const ExactOps ops;
     const int q0 = rowptr[row], q1 = rowptr[row + 1];
     for (int64_t c0 = lane; c0 < ncols; c0 += G) {
         double ar = 0.0, ai = 0.0;
@@ -240,19 +245,19 @@ __global__ void __launch_bounds__(256)
             }
 #pragma unroll
             for (int u = 0; u < UN; u++) {
-                const double pr = __dsub_rn(__dmul_rn(x[u].x, v[u].x), __dmul_rn(x[u].y, v[u].y));
-                const double pi = __dadd_rn(__dmul_rn(x[u].x, v[u].y), __dmul_rn(x[u].y, v[u].x));
-                ar = __dadd_rn(ar, pr);
-                ai = __dadd_rn(ai, pi);
+                const double pr = ops.sub(ops.mul(x[u].x, v[u].x), ops.mul(x[u].y, v[u].y));
+                const double pi = ops.add(ops.mul(x[u].x, v[u].y), ops.mul(x[u].y, v[u].x));
+                ar = ops.add(pr, ar);
+                ai = ops.add(pi, ai);
             }
         }
         for (; q < q1; q++) {
             const double2 v = __ldg(&vals[q]);
             const double2 x = __ldg(&X[(int64_t)__ldg(&colidx[q]) * ncols + c0]);
-            const double pr = __dsub_rn(__dmul_rn(x.x, v.x), __dmul_rn(x.y, v.y));
-            const double pi = __dadd_rn(__dmul_rn(x.x, v.y), __dmul_rn(x.y, v.x));
-            ar = __dadd_rn(ar, pr);
-            ai = __dadd_rn(ai, pi);
+            const double pr = ops.sub(ops.mul(x.x, v.x), ops.mul(x.y, v.y));
+            const double pi = ops.add(ops.mul(x.x, v.y), ops.mul(x.y, v.x));
+            ar = ops.add(pr, ar);
+            ai = ops.add(pi, ai);
         }
         Y[row * ncols + c0] = make_double2(ar, ai);
     }
@@ -1933,10 +1938,9 @@ extern "C" int f4j_spmv_ex(f4j_ctx* ctx, f4j_csr S, f4j_buf x, f4j_buf y, int mo
     int64_t l0 = ctx->launches;
     if (S->rows) {
         // rows per warp: as many as fill every SM's resident blocks of 8 warps
-        // once (173 exact / 216 FMA at 2^20 rows), so the SMs finish together;
+        // once (216 at 2^20 rows), so the SMs finish together;
         // more rows per warp balance the lanes better, up to 256; at least 32
-        const int bps = mode == F4J_SPARSE_FMA ? SpmvOcc<true>::BLOCKS : SpmvOcc<false>::BLOCKS;
-        const int64_t slots = (int64_t)ctx->sm_count * bps * (SPMV_BLOCK / 32);
+        const int64_t slots = (int64_t)ctx->sm_count * SPMV_BLOCKS * (SPMV_BLOCK / 32);
         int64_t rpw64 = f4j_cdiv(S->rows, slots);
         const int rpw = (int)(rpw64 < 32 ? 32 : (rpw64 > SPMV_RPW_MAX ? SPMV_RPW_MAX : rpw64));
         const unsigned blocks = (unsigned)f4j_cdiv(f4j_cdiv(S->rows, rpw), SPMV_BLOCK / 32);
