@@ -321,6 +321,8 @@ __global__ void __launch_bounds__(256, 4) k_crt_planes(const CrtOperand a, const
                                                        const CrtCfg* __restrict__ cfgs) {
     __shared__ double sre[SP_TR][SP_TQ + 1];
     __shared__ double sim[CPLX ? SP_TR : 1][SP_TQ + 1];
+    chain_wait();
+    chain_trigger();
     if (plan->nonfinite) return;
     const int s = plan->s, nmod = cfgs[plan->crt].nmod, nsq = cfgs[plan->crt].nsq;
     if (blockIdx.z == 0) crt_planes_body<CPLX>(a, klen, Kh, Kp, s, nmod, nsq, sre, sim);
@@ -463,13 +465,9 @@ __global__ void __launch_bounds__(CG_THREADS, 1) __cluster_dims__(2, 1, 1)
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
 
-    if (p.plan->nonfinite) return;  // the gated plain path computes this product (both CTAs of a pair)
-    const CrtCfg* __restrict__ cfg = p.cfgs + p.plan->crt;
-    const int nmod = cfg->nmod, nsq = cfg->nsq;
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const uint32_t rank = cluster_rank();
     const int tiles_m = p.tm1 - p.tm0, tiles_n = p.tn1 - p.tn0, ntiles = tiles_m * tiles_n;
-    const int nunits = ntiles * nmod;
     const int pair = blockIdx.x / 2, npairs = gridDim.x / 2;
 
     if (threadIdx.x == 0) {
@@ -500,6 +498,13 @@ __global__ void __launch_bounds__(CG_THREADS, 1) __cluster_dims__(2, 1, 1)
     cluster_sync_all();
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
+    chain_wait();  // the setup above runs under the planes kernel's last blocks
+    chain_trigger();
+    // nonfinite: the gated plain path computes this product
+    const bool off = p.plan->nonfinite != 0;
+    const CrtCfg* __restrict__ cfg = p.cfgs + (off ? 0 : p.plan->crt);
+    const int nmod = cfg->nmod, nsq = cfg->nsq;
+    const int nunits = off ? 0 : ntiles * nmod;
 
     if (warp == 0) {
         // ---------------- TMA producer: lane 0 loads the slot's A tile, lane 1 its B tile
@@ -542,7 +547,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) __cluster_dims__(2, 1, 1)
         // tensor pipe queues only a couple of MMAs, so what this thread does
         // between them (waits, slot arithmetic, commits) shows as idle pipe: ring
         // cursors instead of divisions, one barrier test per slot on the fast path.
-        if (rank == 0 && lane == 0) {
+        if (rank == 0 && lane == 0 && pair < nunits) {
             const uint64_t desc0 = umma_desc_sw128(ring);
             const uint32_t hi = (uint32_t)(desc0 >> 32), lo0 = (uint32_t)desc0;
             const uint32_t idesc = umma_idesc_e4m3_f32(256, 256);
@@ -923,6 +928,8 @@ __device__ __forceinline__ void crt_combine_body(const CrtCombineParams& p, cons
 template <bool CPLX>
 __global__ void __launch_bounds__(256, 4) k_crt_combine(const __grid_constant__ CrtCombineParams p) {
     __shared__ CrtCfg c;
+    chain_wait();
+    chain_trigger();
     if (p.plan->nonfinite) return;
     {
         const int* src = reinterpret_cast<const int*>(p.cfgs + p.plan->crt);

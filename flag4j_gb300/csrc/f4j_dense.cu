@@ -198,6 +198,7 @@ __global__ void __launch_bounds__(DM_THREADS, 1)
     __shared__ __align__(8) uint64_t full[DM_ST], empty[DM_ST];
     __shared__ int abort_flag;
 
+    chain_wait();
     if (p.gate && *(volatile const int*)p.gate == 0) return;
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int nk = (int)((p.k + DM_BK - 1) / DM_BK);
@@ -637,11 +638,11 @@ int f4j_gemm_dmma(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, cons
     if (cplx) {
         F4J_CUDA(cudaFuncSetAttribute(k_gemm_dmma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         f4j_prof_begin(ctx);
-        k_gemm_dmma<true><<<grid, DM_THREADS, smem, ctx->stream>>>(ta, tb, p);
+        f4j_launch(gate && !ctx->prof, k_gemm_dmma<true>, grid, DM_THREADS, smem, ctx->stream, ta, tb, p);
     } else {
         F4J_CUDA(cudaFuncSetAttribute(k_gemm_dmma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         f4j_prof_begin(ctx);
-        k_gemm_dmma<false><<<grid, DM_THREADS, smem, ctx->stream>>>(ta, tb, p);
+        f4j_launch(gate && !ctx->prof, k_gemm_dmma<false>, grid, DM_THREADS, smem, ctx->stream, ta, tb, p);
     }
     f4j_prof_end(ctx);
     F4J_LAUNCHED(ctx);

@@ -106,6 +106,25 @@ int f4j_cuda_fail(cudaError_t e, const char* what);
         if (e__ != cudaSuccess) return f4j_cuda_fail(e__, #call);   \
     } while (0)
 
+// A kernel launch.  after: directly behind another kernel of the same stream that
+// belongs to the same chain (chain_wait in f4j_ptx.cuh), so that its blocks may
+// become resident before that one has ended.  Errors surface in F4J_LAUNCHED.
+template <typename... P, typename... Q>
+inline void f4j_launch(bool after, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                       Q&&... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = after ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // After a kernel launch: record it and surface launch errors.
 #define F4J_LAUNCHED(ctx)                                                    \
     do {                                                                     \

@@ -78,6 +78,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
     return mbar_wait_ns(bar, parity, status, code, F4J_WAIT_NS);
 }
 
+// Kernels launched back to back (f4j_launch with after): a kernel lets the next one's
+// blocks become resident once all of its own have started (chain_trigger), and
+// waits for the previous one's completion and writes (chain_wait) before it
+// reads or writes anything of it.  Every kernel of a chain passes chain_wait
+// before it ends, so a kernel's completion implies that of all before it.
+// Without the launch attribute both do nothing.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Separately rounded FP64 products and sums as fused multiply-adds: RN(a b) =
 // fma(a, b, -0) and RN(a + b) = fma(a, 1, b), signed zeros included.  GB300
 // issues an FMA of three registers every 68 clocks per SM sub-partition and a

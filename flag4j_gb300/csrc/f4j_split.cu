@@ -169,6 +169,7 @@ __global__ void k_stats_rows(const double* __restrict__ X, int64_t rows, int64_t
                              int* __restrict__ cnt_out, int* __restrict__ bad_out) {
     int64_t r = (int64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     int lane = threadIdx.x % 32;
+    chain_trigger();
     if (r >= rows) return;
     unsigned long long mx = 0;
     long long es = 0;
@@ -183,6 +184,7 @@ __global__ void k_stats_rows(const double* __restrict__ X, int64_t rows, int64_t
         cnt_out[r] = cnt;
         if (bad) atomicExch(bad_out, 1);
     }
+    chain_wait();  // the other operand's statistics share nothing with these: they may run at once
 }
 
 // One block of 256 threads per stored row.
@@ -195,6 +197,7 @@ __global__ void __launch_bounds__(256) k_stats_row_blocks(const double* __restri
     __shared__ int scnt[8], sbad[8];
     const int64_t r = blockIdx.x;
     const int warp = threadIdx.x / 32;
+    chain_trigger();
     unsigned long long mx = 0;
     long long es = 0;
     int cnt = 0, bad = 0;
@@ -216,6 +219,7 @@ __global__ void __launch_bounds__(256) k_stats_row_blocks(const double* __restri
     esum_out[r] = es;
     cnt_out[r] = cnt;
     if (bad) atomicExch(bad_out, 1);
+    chain_wait();
 }
 
 // Thread per stored column, block (bx, by) over chunks of `chunk` rows: stats
@@ -250,7 +254,9 @@ __device__ __forceinline__ void stats_cols_body(const double* __restrict__ X, in
 __global__ void k_stats_cols(const double* __restrict__ X, int64_t rows, int64_t cols, int64_t ld, int cplx,
                              int chunk, unsigned long long* __restrict__ mx_out, long long* __restrict__ esum_out,
                              int* __restrict__ cnt_out, int* __restrict__ bad_out) {
+    chain_trigger();
     stats_cols_body(X, rows, cols, ld, cplx, chunk, blockIdx.x, blockIdx.y, mx_out, esum_out, cnt_out, bad_out);
+    chain_wait();
 }
 
 // Exponent bound e (max|x| < 2^e) of target t, and its spread (x256).
@@ -523,6 +529,8 @@ __global__ void __launch_bounds__(256) k_finalize_pick(int64_t ta, int64_t tb, i
                                                        int* __restrict__ eb, int* misc, const SliceModel model, int s_req,
                                                        const SplitPlan* __restrict__ tab,
                                                        const CrtPick pick, SplitPlan* __restrict__ plan) {
+    chain_wait();
+    chain_trigger();
     const int64_t nba = (ta + 255) / 256;
     const bool is_b = (int64_t)blockIdx.x >= nba;
     const int64_t t = ((int64_t)blockIdx.x - (is_b ? nba : 0)) * 256 + threadIdx.x;
@@ -1315,11 +1323,12 @@ static int split_kcb_cap(int64_t tiles, int64_t nkb, int* nchunks) {
 // wait for their own loads, one after the other.  Measured, us, warp / block per
 // row: 700 x 2500 14.7 / 8.4, 2111 x 1543 11.0 / 13.0.
 static void launch_stats_rows(const double* X, int64_t rows, int64_t cols, int cplx, int sm_count,
-                              unsigned long long* mx, long long* es, int* cn, int* bad, cudaStream_t st) {
+                              unsigned long long* mx, long long* es, int* cn, int* bad, cudaStream_t st,
+                              bool after = false) {
     if (rows < 8 * (int64_t)sm_count && cols >= 512)
-        k_stats_row_blocks<<<(unsigned)rows, 256, 0, st>>>(X, cols, cplx, mx, es, cn, bad);
+        f4j_launch(after, k_stats_row_blocks, (unsigned)rows, 256, 0, st, X, cols, cplx, mx, es, cn, bad);
     else
-        k_stats_rows<<<(unsigned)f4j_cdiv(rows, 8), 256, 0, st>>>(X, rows, cols, cplx, mx, es, cn, bad);
+        f4j_launch(after, k_stats_rows, (unsigned)f4j_cdiv(rows, 8), 256, 0, st, X, rows, cols, cplx, mx, es, cn, bad);
 }
 
 // Column statistics of a stored rows x cols operand whose rows are ld elements
@@ -1327,13 +1336,14 @@ static void launch_stats_rows(const double* X, int64_t rows, int64_t cols, int c
 // four blocks per SM: a 1024-wide operand otherwise runs as 16 blocks.  The
 // chunk count stays within grid.y.
 static void launch_stats_cols(const double* X, int64_t rows, int64_t cols, int64_t ld, int cplx, int sm_count,
-                              unsigned long long* mx, long long* es, int* cn, int* bad, cudaStream_t st) {
+                              unsigned long long* mx, long long* es, int* cn, int* bad, cudaStream_t st,
+                              bool after = false) {
     const int64_t bx = f4j_cdiv(cols, 256);
     int64_t chunk = 256;
     while (chunk > 16 && bx * f4j_cdiv(rows, chunk) < 4 * (int64_t)sm_count) chunk /= 2;
     while (f4j_cdiv(rows, chunk) > 65535) chunk *= 2;
-    k_stats_cols<<<dim3((unsigned)bx, (unsigned)f4j_cdiv(rows, chunk)), 256, 0, st>>>(X, rows, cols, ld, cplx,
-                                                                                      (int)chunk, mx, es, cn, bad);
+    f4j_launch(after, k_stats_cols, dim3((unsigned)bx, (unsigned)f4j_cdiv(rows, chunk)), 256, 0, st, X, rows, cols, ld,
+               cplx, (int)chunk, mx, es, cn, bad);
 }
 
 // Offsets in the small workspace of one split GEMM (M rows of op(A), n
@@ -1697,8 +1707,10 @@ static int crt_setup(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, C
 
 // The products of tile rows [tm0, tm1) x tile columns [tn0, tn1) and their
 // reconstruction into C, on `stream`; y holds rows [row0, row0 + S.yrows).
+// after: `stream`'s last launch is the planes' or an earlier crt_launch's, and no
+// other stream has kernels for the blocks that wait to keep off the SMs.
 static int crt_launch(f4j_ctx* ctx, const CrtSetup& S, bool cplx, int64_t n, double* C, cudaStream_t stream, int tm0,
-                      int tm1, int tn0, int tn1, int row0) {
+                      int tm1, int tn0, int tn1, int row0, bool after) {
     const int64_t r0 = (int64_t)tm0 * CG_T, r1 = (int64_t)tm1 * CG_T < S.M ? (int64_t)tm1 * CG_T : S.M;
     // complex launches cover every tile column
     const int64_t c0 = cplx ? 0 : (int64_t)tn0 * CG_T, c1 = cplx || (int64_t)tn1 * CG_T > n ? n : (int64_t)tn1 * CG_T;
@@ -1712,7 +1724,7 @@ static int crt_launch(f4j_ctx* ctx, const CrtSetup& S, bool cplx, int64_t n, dou
     const cudaStream_t saved = ctx->stream;
     ctx->stream = stream;
     f4j_prof_begin(ctx);
-    k_crt_gemm<<<2 * pairs, CG_THREADS, S.smem, stream>>>(S.ta, S.tb, g);
+    f4j_launch(after, k_crt_gemm, 2 * pairs, CG_THREADS, S.smem, stream, S.ta, S.tb, g);
     f4j_prof_end(ctx);
     ctx->stream = saved;
     F4J_LAUNCHED(ctx);
@@ -1726,7 +1738,8 @@ static int crt_launch(f4j_ctx* ctx, const CrtSetup& S, bool cplx, int64_t n, dou
     int64_t by = f4j_cdiv(gy, 3), cap = 16 * (int64_t)ctx->sm_count / gx;
     cap = cap < 1 ? 1 : (cap > 65535 ? 65535 : cap);
     by = by < cap ? by : cap;
-    (cplx ? k_crt_combine<true> : k_crt_combine<false>)<<<dim3((unsigned)gx, (unsigned)by), dim3(bx, 256 / bx), 0, stream>>>(cp);
+    f4j_launch(after, cplx ? k_crt_combine<true> : k_crt_combine<false>, dim3((unsigned)gx, (unsigned)by),
+               dim3(bx, 256 / bx), 0, stream, cp);
     F4J_LAUNCHED(ctx);
     return F4J_OK;
 }
@@ -1749,26 +1762,26 @@ static int crt_gemm(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, co
         launch_stats_cols(A, k, M, M, cplx, ctx->sm_count, S.mxa, S.esa, S.cna, S.misc, ctx->stream);
     F4J_LAUNCHED(ctx);
     if (b_rows)
-        launch_stats_rows(B, n, k, cplx, ctx->sm_count, S.mxb, S.esb, S.cnb, S.misc, ctx->stream);
+        launch_stats_rows(B, n, k, cplx, ctx->sm_count, S.mxb, S.esb, S.cnb, S.misc, ctx->stream, true);
     else
-        launch_stats_cols(B, k, n, n, cplx, ctx->sm_count, S.mxb, S.esb, S.cnb, S.misc, ctx->stream);
+        launch_stats_cols(B, k, n, n, cplx, ctx->sm_count, S.mxb, S.esb, S.cnb, S.misc, ctx->stream, true);
     F4J_LAUNCHED(ctx);
-    k_finalize_pick<<<(unsigned)(f4j_cdiv(M, 256) + f4j_cdiv(n, 256)), 256, 0, ctx->stream>>>(
-        M, n, 0, S.mxa, S.esa, S.cna, S.mxb, S.esb, S.cnb, S.ea, S.eb, S.misc, slice_model(k, S.klen), env_slices(), nullptr,
-        S.pick, S.plan);
+    f4j_launch(true, k_finalize_pick, (unsigned)(f4j_cdiv(M, 256) + f4j_cdiv(n, 256)), 256, 0, ctx->stream, M, n, 0,
+               S.mxa, S.esa, S.cna, S.mxb, S.esb, S.cnb, S.ea, S.eb, S.misc, slice_model(k, S.klen), env_slices(), nullptr,
+               S.pick, S.plan);
     F4J_LAUNCHED(ctx);
     {
         const CrtOperand oa{A, a_rows ? k : M, a_rows ? 0 : 1, opA == F4J_OP_C ? 1 : 0, 0, M, M, 0, S.ea, S.plA};
         const CrtOperand ob{B, b_rows ? k : n, b_rows ? 0 : 1, opB == F4J_OP_C ? 1 : 0, 1, n, S.N, S.half, S.eb, S.plB};
         const dim3 grid((unsigned)(S.Kh / SP_TQ), slice_grid_y(M > n ? M : n), 2);
-        if (cplx) k_crt_planes<true><<<grid, 256, 0, ctx->stream>>>(oa, ob, k, S.Kh, S.Kp, S.plan, S.cfgs);
-        else k_crt_planes<false><<<grid, 256, 0, ctx->stream>>>(oa, ob, k, S.Kh, S.Kp, S.plan, S.cfgs);
+        f4j_launch(true, cplx ? k_crt_planes<true> : k_crt_planes<false>, grid, 256, 0, ctx->stream, oa, ob, k, S.Kh, S.Kp,
+                   S.plan, S.cfgs);
         F4J_LAUNCHED(ctx);
     }
     f4j_prof_end(ctx);
     for (int t0 = 0; t0 < S.tiles_m; t0 += (int)S.blk) {
         const int t1 = t0 + (int)S.blk < S.tiles_m ? t0 + (int)S.blk : S.tiles_m;
-        rc = crt_launch(ctx, S, cplx, n, C, ctx->stream, t0, t1, 0, S.tiles_n, t0 * CG_T);
+        rc = crt_launch(ctx, S, cplx, n, C, ctx->stream, t0, t1, 0, S.tiles_n, t0 * CG_T, !ctx->prof);
         if (rc) return rc;
     }
     *plan_out = S.plan;
@@ -2024,7 +2037,7 @@ static int host_split_pipelined(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, i
             const cudaStream_t ps = ctx->part_stream[id];
             F4J_CUDA(cudaStreamWaitEvent(ps, ctx->part_prep_ev[id], 0));
             launched = id + 1;
-            int r = crt ? crt_launch(ctx, R, cplx, n, dC, ps, tm0, tm1, tn0, tn1, 0)
+            int r = crt ? crt_launch(ctx, R, cplx, n, dC, ps, tm0, tm1, tn0, tn1, 0, false)
                         : split_launch(ctx, L, ps, tm0, tm1, tn0, tn1);
             if (r) return r;
             const int64_t r0 = (int64_t)tm0 * tile, r1 = (int64_t)tm1 * tile < m ? (int64_t)tm1 * tile : m;

@@ -133,3 +133,39 @@ def test_residue_form_within_its_bound(f4j, oracle, case):
         assert not C.any()
     if case == "tiny_row":
         assert not C[:, 3].any()
+
+
+def test_residue_form_launches_in_order(f4j):
+    """Products queued back to back without a wait, each from the one before (its kernels start while the
+    previous kernel's last blocks run), with a non-finite operand that stands the form down in between: bit
+    for bit the products of a queue that waits after each."""
+    from flag4j_gb300 import _lib
+    from flag4j_gb300.device import check
+    ctx = f4j.default_context()
+    g = np.random.default_rng(5)
+    shapes = [(300, 1100, 900), (300, 1500, 1100), (300, 260, 1500), (300, 2048, 260)]
+    X0 = g.standard_normal((300, 900))
+    Bs = [g.standard_normal((k, n)) for _, n, k in shapes]
+    bad = Bs[1].copy()
+    bad[3, 4] = np.nan
+    outs = []
+    for wait in (True, False):
+        dX, dB, dbad = ctx.from_numpy(X0), [ctx.from_numpy(B) for B in Bs], ctx.from_numpy(bad)
+        dC = [ctx.alloc(C_bytes(m, n, False)) for m, n, _ in shapes]
+        dD = ctx.alloc(C_bytes(300, 1500, False))
+        for _ in range(3):
+            src = dX
+            for (m, n, k), b, c in zip(shapes, dB, dC):
+                if n == 1500:  # the same sizes with a NaN: the plain product, from the same workspace
+                    check(ctx.lib.f4j_dgemm(ctx.handle, m, n, k, src.handle, 0, dbad.handle, 0, dD.handle,
+                                            _lib.MODE_AUTO, None))
+                check(ctx.lib.f4j_dgemm(ctx.handle, m, n, k, src.handle, 0, b.handle, 0, c.handle, _lib.MODE_AUTO,
+                                        None))
+                if wait:
+                    ctx.sync()
+                src = c
+        outs.append([c.to_numpy(np.float64, m * n) for c, (m, n, _) in zip(dC, shapes)] +
+                    [dD.to_numpy(np.float64, 300 * 1500)])
+    for w, q in zip(*outs):
+        assert np.array_equal(w, q, equal_nan=True)
+    assert np.isnan(outs[0][-1]).any() and not np.isnan(outs[0][0]).any()
