@@ -659,6 +659,30 @@ __global__ void __launch_bounds__(CG_THREADS, 1) __cluster_dims__(2, 1, 1)
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(empty_addr[a]);
         };
+        // The warp's 128 columns of accumulator a, reduced mod the p in (np, ip), to
+        // halves.  TMEM is released before the last 64 columns are reduced, so the
+        // next unit's products wait for half of the arithmetic only (64 raw columns
+        // are what fits the 168 registers beside the other accumulator's halves).
+        auto drain = [&](int a, uint32_t (&r)[64], f32x2 np, f32x2 ip) {
+            uint32_t v[2][32];
+            auto reduce = [&](int part) {
+#pragma unroll
+                for (int i = 0; i < 16; i++)
+                    r[part * 16 + i] = crt_halves(crt_mod2(pack2(v[part & 1][2 * i], v[part & 1][2 * i + 1]), np, ip));
+            };
+            const uint32_t t = tq + a * 256;
+            tmem_ld32(t, v[0]);
+            tmem_ld32(t + 32, v[1]);
+            tmem_ld_wait();
+            reduce(0);
+            tmem_ld32(t + 64, v[0]);
+            reduce(1);
+            tmem_ld32(t + 96, v[1]);
+            tmem_ld_wait();
+            release(a);
+            reduce(2);
+            reduce(3);
+        };
         for (int u = pair; u < nunits && ok; u += npairs) {
             const int l = u / ntiles;
             int tm, tn;
@@ -697,28 +721,10 @@ __global__ void __launch_bounds__(CG_THREADS, 1) __cluster_dims__(2, 1, 1)
                     uint32_t xr[64], yr[64];
                     wait_full(0);
                     if (!ok) break;
-#pragma unroll
-                    for (int part = 0; part < 4; part++) {
-                        uint32_t v[32];
-                        tmem_ld32(tq + part * 32, v);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int i = 0; i < 16; i++)
-                            xr[part * 16 + i] = crt_halves(crt_mod2(pack2(v[2 * i], v[2 * i + 1]), np, ip));
-                    }
-                    release(0);
+                    drain(0, xr, np, ip);
                     wait_full(1);
                     if (!ok) break;
-#pragma unroll
-                    for (int part = 0; part < 4; part++) {
-                        uint32_t v[32];
-                        tmem_ld32(tq + 256 + part * 32, v);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int i = 0; i < 16; i++)
-                            yr[part * 16 + i] = crt_halves(crt_mod2(pack2(v[2 * i], v[2 * i + 1]), nb, ib));
-                    }
-                    release(1);
+                    drain(1, yr, nb, ib);
 #pragma unroll
                     for (int g = 0; g < 8; g++) {
                         f32x2 c[8];
@@ -731,16 +737,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) __cluster_dims__(2, 1, 1)
                     uint32_t xr[64];
                     wait_full(turn);
                     if (!ok) break;
-#pragma unroll
-                    for (int part = 0; part < 4; part++) {
-                        uint32_t v[32];
-                        tmem_ld32(tq + turn * 256 + part * 32, v);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int i = 0; i < 16; i++)
-                            xr[part * 16 + i] = crt_halves(crt_mod2(pack2(v[2 * i], v[2 * i + 1]), np, ip));
-                    }
-                    release(turn);
+                    drain(turn, xr, np, ip);
 #pragma unroll
                     for (int g = 0; g < 8; g++) {
                         f32x2 c[8];
