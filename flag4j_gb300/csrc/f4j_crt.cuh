@@ -335,7 +335,10 @@ constexpr int CG_BK = 128;                  // K bytes per ring slot (one 128-by
 constexpr int CG_TILE = 128 * CG_BK;        // 16 KB
 constexpr int CG_SLOT = 2 * CG_TILE;        // an A tile and a B tile
 constexpr int CG_RING = 7;
-constexpr int CG_THREADS = 320;             // warp 0 TMA, warp 1 MMA, warps 2..9 epilogue
+constexpr int CG_THREADS = 384;             // warp 0 TMA, warp 1 MMA, two idle, warps 4..11 epilogue
+// Registers a thread: all start with 168; the first warpgroup gives up what the
+// epilogue warpgroups take, 128 x 40 + 256 x 232 = 384 x 168.
+constexpr int CG_REGS_LOAD = 40, CG_REGS_EPI = 232;
 constexpr int CG_KB = CRT_KC / CG_BK;       // K blocks per accumulation
 constexpr int CG_GROUP_M = 8;
 
@@ -411,6 +414,27 @@ __device__ __forceinline__ void umma2_f8_k128(uint32_t d, uint32_t a_lo, uint32_
             : "memory");
     }
 }
+// One K block of a square's three products: x += a0 b0, y += a0 b1 + a1 b0.  The
+// tile a0 is read from shared memory once for its two products of a K = 32 step
+// (the MMA's A collector): the MMAs read 64 bytes a clock and the loads write 45
+// of an SM's 128, and the MMAs took 580 clocks a K block for the 512 they take
+// alone.  GEMM at 4096^3 1303 -> 1264 us, 8192^3 10.9 -> 10.5 ms.  Not unrolled:
+// the kernel starts with a cold instruction cache (1024^3: 1.5 us).
+__device__ __forceinline__ void umma2_f8_square(uint32_t x, uint32_t y, uint32_t a0, uint32_t b0, uint32_t a1,
+                                                uint32_t b1, uint32_t hi, uint32_t idesc) {
+#pragma unroll 1
+    for (int k = 0; k < 4; k++) {
+        asm volatile(
+            "{\n\t.reg .pred t;\n\t.reg .b64 a0, b0, a1, b1;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+            "mov.b64 a0, {%2, %6};\n\tmov.b64 b0, {%3, %6};\n\t"
+            "mov.b64 a1, {%4, %6};\n\tmov.b64 b1, {%5, %6};\n\t"
+            "tcgen05.mma.cta_group::2.kind::f8f6f4.collector::a::fill [%0], a0, b0, %7, t;\n\t"
+            "tcgen05.mma.cta_group::2.kind::f8f6f4.collector::a::lastuse [%1], a0, b1, %7, t;\n\t"
+            "tcgen05.mma.cta_group::2.kind::f8f6f4 [%1], a1, b0, %7, t;\n\t}" ::"r"(x),
+            "r"(y), "r"(a0 + 2 * k), "r"(b0 + 2 * k), "r"(a1 + 2 * k), "r"(b1 + 2 * k), "r"(hi), "r"(idesc)
+            : "memory");
+    }
+}
 // Arrive on the barrier of both CTAs once this thread's MMAs have completed.
 __device__ __forceinline__ void umma2_commit(uint64_t* bar) {
     asm volatile(
@@ -454,7 +478,11 @@ __device__ __forceinline__ f32x2 crt_floats(uint32_t h) {
 // 256 columns: X (x0 y0) and Y (x0 y1 + x1 y0) of a square, in turn the
 // singles'.  X's products run two K blocks ahead of Y's at the start and the end of
 // a square, so X is drained under Y's last products and Y under the next
-// unit's first.
+// unit's first.  In between the three products of a K block go together
+// (umma2_f8_square).  Epilogue warps with 232 registers read an accumulator whole
+// before they reduce it; with 168 and a copy of the code for each kind of modulus
+// the GEMM took, us, 49.7 for 47.8 at 1024^3, 56 / 54.7 at 1500 x 900 x 700, 355 /
+// 344 at 2048 x 2048 x 4096.
 __global__ void __launch_bounds__(CG_THREADS, 1) __cluster_dims__(2, 1, 1)
     k_crt_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ CrtGemmParams p) {
@@ -506,150 +534,158 @@ __global__ void __launch_bounds__(CG_THREADS, 1) __cluster_dims__(2, 1, 1)
     const int nmod = cfg->nmod, nsq = cfg->nsq;
     const int nunits = off ? 0 : ntiles * nmod;
 
-    if (warp == 0) {
-        // ---------------- TMA producer: lane 0 loads the slot's A tile, lane 1 its B tile
-        int s = 0, round = 0;  // next slot, and how often the ring has been filled
-        bool ok = true;
-        const uint32_t full0 = cluster_map(&full[0], 0);
-        const CUtensorMap* map = lane == 0 ? &tmA : &tmB;
-        for (int u = pair; u < nunits && ok; u += npairs) {
-            const int l = u / ntiles;
-            int tm, tn;
-            crt_tile(u - l * ntiles, tiles_m, tiles_n, tm, tn);
-            const int row = (lane == 0 ? p.tm0 + tm : p.tn0 + tn) * CG_T + (int)rank * 128;
-            const int nd = l < nsq ? 2 : 1;
-            for (int kb = 0; kb < p.nkb && ok; kb++) {
-                for (int d = 0; d < nd; d++) {
-                    if (lane == 0) {
-                        if (round > 0)
-                            ok = mbar_wait(&empty[s], (round & 1) ^ 1, p.status, 21) && !*(volatile int*)&abort_flag;
-                        if (!ok) abort_flag = 1;
-                        else if (rank == 0) mbar_arrive_expect_tx(&full[s], 2 * CG_SLOT);
-                    }
-                    ok = __shfl_sync(0xffffffffu, ok, 0);
-                    if (!ok) break;
-                    if (lane < 2)
-                        tma_load_3d_pair(ring + s * CG_SLOT + lane * CG_TILE, map, full0 + 8 * s, kb * CG_BK, row,
-                                         d ? nmod + l : l);
-                    if (++s == CG_RING) s = 0, round++;
-                }
-            }
-        }
-        // copies still in flight signal the first CTA's barriers: it waits for them (bounded), and the
-        // cluster barrier below keeps both CTAs until then
-        if (rank == 0 && lane == 0)
-            for (int q = 0; q < CG_RING; q++) {
-                const int fills = round + (q < s ? 1 : 0);
-                if (fills) mbar_wait(&full[q], (fills - 1) & 1, nullptr, 0);
-            }
-    } else if (warp == 1) {
-        // ---------------- MMA issuer: one thread of the pair's first CTA.  The
-        // tensor pipe queues only a couple of MMAs, so what this thread does
-        // between them (waits, slot arithmetic, commits) shows as idle pipe: ring
-        // cursors instead of divisions, one barrier test per slot on the fast path.
-        if (rank == 0 && lane == 0 && pair < nunits) {
-            const uint64_t desc0 = umma_desc_sw128(ring);
-            const uint32_t hi = (uint32_t)(desc0 >> 32), lo0 = (uint32_t)desc0;
-            const uint32_t idesc = umma_idesc_e4m3_f32(256, 256);
-            constexpr uint32_t SLOT16 = CG_SLOT >> 4, TILE16 = CG_TILE >> 4;
-            struct Cursor {
-                uint32_t s = 0, par = 0;
-                __device__ __forceinline__ void next() {
-                    if (++s == CG_RING) s = 0, par ^= 1;
-                }
-            };
-            Cursor cur;  // first slot not yet consumed
-            uint32_t turn = 0, fill0 = 0, fill1 = 0;
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(CG_REGS_LOAD));
+        if (warp == 0) {
+            // ---------------- TMA producer: lane 0 loads the slot's A tile, lane 1 its B tile
+            int s = 0, round = 0;  // next slot, and how often the ring has been filled
             bool ok = true;
-            auto acquire = [&](uint32_t a, uint32_t fills) {  // the epilogue has drained accumulator a
-                if (fills > 0) ok = ok && mbar_wait_cluster(&accempty[a], (fills - 1) & 1, p.status, 22);
-                tc_fence_after();
-            };
-            auto landed = [&](const Cursor& c) {
-                if (!mbar_try_wait(&full[c.s], c.par)) {
-                    ok = ok && mbar_wait(&full[c.s], c.par, p.status, 23) && !*(volatile int*)&abort_flag;
-                }
-            };
-            auto mma = [&](uint32_t acc, uint32_t sa, uint32_t sb, bool first) {
-                umma2_f8_k128(tmem + acc * 256, lo0 + sa * SLOT16, lo0 + sb * SLOT16 + TILE16, hi, idesc,
-                              first ? 0u : 1u);
-            };
+            const uint32_t full0 = cluster_map(&full[0], 0);
+            const CUtensorMap* map = lane == 0 ? &tmA : &tmB;
             for (int u = pair; u < nunits && ok; u += npairs) {
                 const int l = u / ntiles;
-                for (int k0 = 0; k0 < p.nkb && ok; k0 += CG_KB) {
-                    const int nk = p.nkb - k0 < CG_KB ? p.nkb - k0 : CG_KB;
-                    if (l < nsq) {
-                        acquire(0, fill0);
-                        Cursor cx = cur;
-                        auto step_x = [&](bool first) {
-                            landed(cx);
-                            if (!ok) return;
-                            mma(0, cx.s, cx.s, first);
-                            cx.next();
-                            cx.next();
-                        };
-                        step_x(true);
-                        int x = 1;  // K blocks of X issued
-                        for (int kb = 0; kb < nk && ok; kb++) {
-                            // X ahead of Y by two blocks at the start and the end only: in between a
-                            // K block's slots are freed at once, so more of the ring is loads in flight
-                            const int lead = kb == 0 ? 3 : kb + 2 < nk ? kb + 1 : nk;
-                            const int xend = lead < nk ? lead : nk;
-                            if (x < xend) {
-                                for (; x < xend && ok; x++) step_x(false);
-                                if (ok && x == nk) umma2_commit(&accfull[0]);
-                            }
-                            if (kb == 0) {
-                                if (ok && nk == 1) umma2_commit(&accfull[0]);
-                                acquire(1, fill1);
-                            }
-                            const uint32_t s0 = cur.s;
-                            cur.next();
-                            landed(cur);
-                            if (!ok) break;
-                            mma(1, s0, cur.s, kb == 0);
-                            mma(1, cur.s, s0, false);
-                            umma2_commit(&empty[s0]);
-                            umma2_commit(&empty[cur.s]);
-                            cur.next();
+                int tm, tn;
+                crt_tile(u - l * ntiles, tiles_m, tiles_n, tm, tn);
+                const int row = (lane == 0 ? p.tm0 + tm : p.tn0 + tn) * CG_T + (int)rank * 128;
+                const int nd = l < nsq ? 2 : 1;
+                for (int kb = 0; kb < p.nkb && ok; kb++) {
+                    for (int d = 0; d < nd; d++) {
+                        if (lane == 0) {
+                            if (round > 0)
+                                ok = mbar_wait(&empty[s], (round & 1) ^ 1, p.status, 21) && !*(volatile int*)&abort_flag;
+                            if (!ok) abort_flag = 1;
+                            else if (rank == 0) mbar_arrive_expect_tx(&full[s], 2 * CG_SLOT);
                         }
+                        ok = __shfl_sync(0xffffffffu, ok, 0);
                         if (!ok) break;
-                        umma2_commit(&accfull[1]);
-                        fill0++;
-                        fill1++;
-                    } else {
-                        acquire(turn, turn ? fill1 : fill0);
-                        for (int kb = 0; kb < nk; kb++) {
-                            landed(cur);
-                            if (!ok) break;
-                            mma(turn, cur.s, cur.s, kb == 0);
-                            umma2_commit(&empty[cur.s]);
-                            cur.next();
-                        }
-                        if (!ok) break;
-                        umma2_commit(&accfull[turn]);
-                        if (turn) fill1++;
-                        else fill0++;
-                        turn ^= 1;
+                        if (lane < 2)
+                            tma_load_3d_pair(ring + s * CG_SLOT + lane * CG_TILE, map, full0 + 8 * s, kb * CG_BK, row,
+                                             d ? nmod + l : l);
+                        if (++s == CG_RING) s = 0, round++;
                     }
                 }
             }
-            if (!ok) abort_flag = 1;
-            umma2_commit(&mma_done);
-            mbar_wait_cluster(&mma_done, 0, p.status, 24);
+            // copies still in flight signal the first CTA's barriers: it waits for them (bounded), and the
+            // cluster barrier below keeps both CTAs until then
+            if (rank == 0 && lane == 0)
+                for (int q = 0; q < CG_RING; q++) {
+                    const int fills = round + (q < s ? 1 : 0);
+                    if (fills) mbar_wait(&full[q], (fills - 1) & 1, nullptr, 0);
+                }
+        } else if (warp == 1) {
+            // ---------------- MMA issuer: one thread of the pair's first CTA.  The
+            // tensor pipe queues only a couple of MMAs, so what this thread does
+            // between them (waits, slot arithmetic, commits) shows as idle pipe: ring
+            // cursors instead of divisions, one barrier test per slot on the fast path.
+            if (rank == 0 && lane == 0 && pair < nunits) {
+                const uint64_t desc0 = umma_desc_sw128(ring);
+                const uint32_t hi = (uint32_t)(desc0 >> 32), lo0 = (uint32_t)desc0;
+                const uint32_t idesc = umma_idesc_e4m3_f32(256, 256);
+                constexpr uint32_t SLOT16 = CG_SLOT >> 4, TILE16 = CG_TILE >> 4;
+                struct Cursor {
+                    uint32_t s = 0, par = 0;
+                    __device__ __forceinline__ void next() {
+                        if (++s == CG_RING) s = 0, par ^= 1;
+                    }
+                };
+                Cursor cur;  // first slot not yet consumed
+                uint32_t turn = 0, fill0 = 0, fill1 = 0;
+                bool ok = true;
+                auto acquire = [&](uint32_t a, uint32_t fills) {  // the epilogue has drained accumulator a
+                    if (fills > 0) ok = ok && mbar_wait_cluster(&accempty[a], (fills - 1) & 1, p.status, 22);
+                    tc_fence_after();
+                };
+                auto landed = [&](const Cursor& c) {
+                    if (!mbar_try_wait(&full[c.s], c.par)) {
+                        ok = ok && mbar_wait(&full[c.s], c.par, p.status, 23) && !*(volatile int*)&abort_flag;
+                    }
+                };
+                auto mma = [&](uint32_t acc, uint32_t sa, uint32_t sb, bool first) {
+                    umma2_f8_k128(tmem + acc * 256, lo0 + sa * SLOT16, lo0 + sb * SLOT16 + TILE16, hi, idesc,
+                                  first ? 0u : 1u);
+                };
+                for (int u = pair; u < nunits && ok; u += npairs) {
+                    const int l = u / ntiles;
+                    for (int k0 = 0; k0 < p.nkb && ok; k0 += CG_KB) {
+                        const int nk = p.nkb - k0 < CG_KB ? p.nkb - k0 : CG_KB;
+                        if (l < nsq) {
+                            acquire(0, fill0);
+                            Cursor cx = cur;
+                            int x = 0;  // K blocks of X issued
+                            for (int kb = 0; kb < nk && ok; kb++) {
+                                // X ahead of Y by two K blocks at the start and the end only: in between a
+                                // K block's slots are freed at once, so more of the ring is loads in flight
+                                const int lead = kb == 0 ? (nk < 3 ? nk : 3) : (kb + 2 < nk ? 0 : nk);
+                                if (x < lead) {
+                                    for (; x < lead; x++) {
+                                        landed(cx);
+                                        if (!ok) break;
+                                        mma(0, cx.s, cx.s, x == 0);
+                                        cx.next();
+                                        cx.next();
+                                    }
+                                    if (!ok) break;
+                                    if (x == nk) umma2_commit(&accfull[0]);
+                                    if (kb == 0) acquire(1, fill1);
+                                }
+                                const uint32_t s0 = cur.s;
+                                if (x == kb) landed(cur);
+                                cur.next();
+                                landed(cur);
+                                if (!ok) break;
+                                if (x == kb) {  // the middle
+                                    const uint32_t a0 = lo0 + s0 * SLOT16, a1 = lo0 + cur.s * SLOT16;
+                                    umma2_f8_square(tmem, tmem + 256, a0, a0 + TILE16, a1, a1 + TILE16, hi, idesc);
+                                    x++;
+                                    cx = cur;
+                                    cx.next();
+                                } else {
+                                    mma(1, s0, cur.s, kb == 0);
+                                    mma(1, cur.s, s0, false);
+                                }
+                                umma2_commit(&empty[s0]);
+                                umma2_commit(&empty[cur.s]);
+                                cur.next();
+                            }
+                            if (!ok) break;
+                            umma2_commit(&accfull[1]);
+                            fill0++;
+                            fill1++;
+                        } else {
+                            acquire(turn, turn ? fill1 : fill0);
+                            for (int kb = 0; kb < nk; kb++) {
+                                landed(cur);
+                                if (!ok) break;
+                                mma(turn, cur.s, cur.s, kb == 0);
+                                umma2_commit(&empty[cur.s]);
+                                cur.next();
+                            }
+                            if (!ok) break;
+                            umma2_commit(&accfull[turn]);
+                            if (turn) fill1++;
+                            else fill0++;
+                            turn ^= 1;
+                        }
+                    }
+                }
+                if (!ok) abort_flag = 1;
+                umma2_commit(&mma_done);
+                mbar_wait_cluster(&mma_done, 0, p.status, 24);
+            }
         }
     } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(CG_REGS_EPI));
         // ---------------- epilogue warps: lane quarter q of the CTA's 128 rows, column half h
-        const int q = warp % 4, h = (warp - 2) / 4;
+        const int q = warp % 4, h = warp / 4 - 1;
         const uint32_t tq = tmem + ((uint32_t)(32 * q) << 16) + h * 128;
-        uint32_t filled[2] = {0, 0};
+        uint32_t filled = 0;  // parity of accumulator a's fills so far in bit a
         int turn = 0;
         bool ok = true;
         const uint32_t empty_addr[2] = {cluster_map(&accempty[0], 0), cluster_map(&accempty[1], 0)};
         auto wait_full = [&](int a) {
             bool w = true;
-            if (lane == 0) w = mbar_wait_cluster(&accfull[a], filled[a] & 1, p.status, 25);
-            filled[a]++;
+            if (lane == 0) w = mbar_wait_cluster(&accfull[a], filled >> a & 1, p.status, 25);
+            filled ^= 1u << a;
             ok = __shfl_sync(0xffffffffu, w, 0) && !*(volatile int*)&abort_flag;
             if (!ok) abort_flag = 1;
             tc_fence_after();
@@ -660,28 +696,19 @@ __global__ void __launch_bounds__(CG_THREADS, 1) __cluster_dims__(2, 1, 1)
             if (lane == 0) mbar_arrive_cluster(empty_addr[a]);
         };
         // The warp's 128 columns of accumulator a, reduced mod the p in (np, ip), to
-        // halves.  TMEM is released before the last 64 columns are reduced, so the
-        // next unit's products wait for half of the arithmetic only (64 raw columns
-        // are what fits the 168 registers beside the other accumulator's halves).
+        // halves.  TMEM is released once they are in registers: the next unit's
+        // products do not wait for the arithmetic.
         auto drain = [&](int a, uint32_t (&r)[64], f32x2 np, f32x2 ip) {
-            uint32_t v[2][32];
-            auto reduce = [&](int part) {
+            uint32_t v[4][32];
 #pragma unroll
-                for (int i = 0; i < 16; i++)
-                    r[part * 16 + i] = crt_halves(crt_mod2(pack2(v[part & 1][2 * i], v[part & 1][2 * i + 1]), np, ip));
-            };
-            const uint32_t t = tq + a * 256;
-            tmem_ld32(t, v[0]);
-            tmem_ld32(t + 32, v[1]);
-            tmem_ld_wait();
-            reduce(0);
-            tmem_ld32(t + 64, v[0]);
-            reduce(1);
-            tmem_ld32(t + 96, v[1]);
+            for (int part = 0; part < 4; part++) tmem_ld32(tq + a * 256 + part * 32, v[part]);
             tmem_ld_wait();
             release(a);
-            reduce(2);
-            reduce(3);
+#pragma unroll
+            for (int part = 0; part < 4; part++)
+#pragma unroll
+                for (int i = 0; i < 16; i++)
+                    r[part * 16 + i] = crt_halves(crt_mod2(pack2(v[part][2 * i], v[part][2 * i + 1]), np, ip));
         };
         for (int u = pair; u < nunits && ok; u += npairs) {
             const int l = u / ntiles;
@@ -697,55 +724,51 @@ __global__ void __launch_bounds__(CG_THREADS, 1) __cluster_dims__(2, 1, 1)
             auto put = [&](int c16, const f32x2 (&c)[8], bool add) {
                 if (row >= p.M || col0 + c16 >= p.ldy) return;
                 int16_t* dst = yrow + c16;
-                uint32_t w[8];
+                f32x2 sum[8];
+#pragma unroll
+                for (int i = 0; i < 8; i++) sum[i] = 0ull;
                 if (add) {
                     const uint4 o0 = reinterpret_cast<const uint4*>(dst)[0], o1 = reinterpret_cast<const uint4*>(dst)[1];
                     const uint32_t old[8] = {o0.x, o0.y, o0.z, o0.w, o1.x, o1.y, o1.z, o1.w};
 #pragma unroll
                     for (int i = 0; i < 8; i++)  // signed halves: flip the top bit for the unsigned form
-                        w[i] = crt_halves(crt_mod2(fma2(c[i], uw, crt_floats(old[i] ^ 0x80008000u)), np, ip));
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 8; i++) w[i] = crt_halves(crt_mod2(fma2(c[i], uw, 0ull), np, ip));
+                        sum[i] = crt_floats(old[i] ^ 0x80008000u);
                 }
+                uint32_t w[8];
+#pragma unroll
+                for (int i = 0; i < 8; i++) w[i] = crt_halves(crt_mod2(fma2(c[i], uw, sum[i]), np, ip));
                 asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst),
                              "r"(w[0] ^ 0x80008000u), "r"(w[1] ^ 0x80008000u), "r"(w[2] ^ 0x80008000u),
                              "r"(w[3] ^ 0x80008000u), "r"(w[4] ^ 0x80008000u), "r"(w[5] ^ 0x80008000u),
                              "r"(w[6] ^ 0x80008000u), "r"(w[7] ^ 0x80008000u)
                              : "memory");
             };
+            const bool square = l < nsq;
+            const f32x2 nb = dup2(c_crt.m[l].nb[0]), b = dup2(-c_crt.m[l].nb[0]), ib = dup2(c_crt.m[l].inv[0]);
             for (int k0 = 0; k0 < p.nkb && ok; k0 += CG_KB) {
-                if (l < nsq) {
-                    const f32x2 nb = dup2(c_crt.m[l].nb[0]), b = dup2(-c_crt.m[l].nb[0]), ib = dup2(c_crt.m[l].inv[0]);
-                    // both accumulators are reduced to halves first, so TMEM is free again early
-                    uint32_t xr[64], yr[64];
-                    wait_full(0);
-                    if (!ok) break;
-                    drain(0, xr, np, ip);
+                // both accumulators are reduced to halves first, so TMEM is free again early
+                uint32_t xr[64], yr[64];
+                const int a = square ? 0 : turn;
+                wait_full(a);
+                if (!ok) break;
+                drain(a, xr, np, ip);
+                if (square) {
                     wait_full(1);
                     if (!ok) break;
                     drain(1, yr, nb, ib);
-#pragma unroll
-                    for (int g = 0; g < 8; g++) {
-                        f32x2 c[8];
-#pragma unroll
-                        for (int i = 0; i < 8; i++)
-                            c[i] = fma2(b, crt_floats(yr[g * 8 + i]), crt_floats(xr[g * 8 + i]));
-                        put(g * 16, c, k0 > 0);
-                    }
                 } else {
-                    uint32_t xr[64];
-                    wait_full(turn);
-                    if (!ok) break;
-                    drain(turn, xr, np, ip);
-#pragma unroll
-                    for (int g = 0; g < 8; g++) {
-                        f32x2 c[8];
-#pragma unroll
-                        for (int i = 0; i < 8; i++) c[i] = crt_floats(xr[g * 8 + i]);
-                        put(g * 16, c, k0 > 0);
-                    }
                     turn ^= 1;
+                }
+#pragma unroll
+                for (int g = 0; g < 8; g++) {
+                    f32x2 c[8];
+#pragma unroll
+                    for (int i = 0; i < 8; i++) c[i] = crt_floats(xr[g * 8 + i]);
+                    if (square) {
+#pragma unroll
+                        for (int i = 0; i < 8; i++) c[i] = fma2(b, crt_floats(yr[g * 8 + i]), c[i]);
+                    }
+                    put(g * 16, c, k0 > 0);
                 }
                 __syncwarp();  // rows past M skip their stores; the TMEM reads are warp-wide
             }
