@@ -547,8 +547,20 @@ __global__ void k_scan_add(int64_t n, int* __restrict__ data, const int* __restr
     if (blockIdx.x == 0) return;
     const int add = sums[blockIdx.x - 1];
     const int64_t base = (int64_t)blockIdx.x * SCAN_TILE;
-    for (int i = threadIdx.x; i < SCAN_TILE; i += blockDim.x)
-        if (base + i < n) data[base + i] += add;
+    constexpr int U = 8;  // in flight a thread: one at a time, 2^20 entries took 11.5 us for 4.2
+    for (int i = threadIdx.x; i < SCAN_TILE; i += U * blockDim.x) {
+        int v[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int64_t at = base + i + u * (int)blockDim.x;
+            v[u] = i + u * (int)blockDim.x < SCAN_TILE && at < n ? data[at] : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int64_t at = base + i + u * (int)blockDim.x;
+            if (i + u * (int)blockDim.x < SCAN_TILE && at < n) data[at] = v[u] + add;
+        }
+    }
 }
 
 // ---------------- stable LSD radix sort of (key, value) pairs, 8-bit digits
@@ -629,25 +641,54 @@ __global__ void __launch_bounds__(RS_T) k_radix_scatter(int64_t n, const unsigne
 // from global memory by their place instead took half of both passes.
 // Against an LSD radix sort of (column, index) pairs, three passes of two random
 // 4-byte writes at 2^20 columns, and the rows gathered after it: 2^20 rows and
-// columns, 16.8 M nonzeros, 0.93 -> 0.42 ms (scatter 148, bucket 185, histogram
-// and scan 67, rows 19 us).
+// columns, 16.8 M nonzeros, 0.93 -> 0.38 ms (scatter 137, bucket 185, histogram
+// and places 38, rows 19 us).  Both passes are instruction-bound (153 and 204 warp
+// instructions per 32 items).
 constexpr int TP_NB = 1024, TP_BITS = 10;
 constexpr int TP1_T = 256, TP1_WARPS = TP1_T / 32, TP1_TILE = 4096;  // pass 1: items per block
 constexpr int TP2_T = 512, TP2_WARPS = TP2_T / 32;
 constexpr int TP2_CNT = TP2_WARPS * TP_NB;
 constexpr int TP2_CAP = 18432;           // bucket items that pass 2 places in shared memory
 
-__global__ void __launch_bounds__(512) k_tp_hist(int64_t n, const int* __restrict__ col, int shift, int nb,
-                                                 int* __restrict__ hist, int nblocks) {
+// hist[block][bucket], rows of nbp (nb rounded up to a multiple of four).
+__global__ void __launch_bounds__(512) k_tp_hist(int64_t n, const int* __restrict__ col, int shift, int nbp,
+                                                 int* __restrict__ hist) {
     __shared__ int h[TP_NB];
-    for (int i = threadIdx.x; i < nb; i += 512) h[i] = 0;
+    for (int i = threadIdx.x; i < nbp; i += 512) h[i] = 0;
     __syncthreads();
     const int64_t base = (int64_t)blockIdx.x * TP1_TILE;
     const int cnt = (int)(n - base < TP1_TILE ? n - base : TP1_TILE);
 #pragma unroll 8
     for (int i = threadIdx.x; i < cnt; i += 512) atomicAdd(&h[__ldg(col + base + i) >> shift], 1);
     __syncthreads();
-    for (int i = threadIdx.x; i < nb; i += 512) hist[(int64_t)i * nblocks + blockIdx.x] = h[i];
+    for (int i = threadIdx.x; i < nbp; i += 512) hist[(int64_t)blockIdx.x * nbp + i] = h[i];
+}
+
+// The places of pass 1 come from prefixes down the columns of hist: chunks of
+// TP_CHUNK blocks here (in place, exclusive; the chunk's total to part), the
+// chunks and the buckets in k_tp_starts.  Bucket-major counts and one scan over
+// all of them wrote and read four bytes at a time: 2^20 columns, 16.8 M
+// nonzeros, histogram and scan 69 us for 38,
+// and the places read with them 12 us of k_tp_scatter's.
+constexpr int TP_CHUNK = 64;
+__global__ void __launch_bounds__(64) k_tp_chunks(int nblocks, int nbp, int* __restrict__ hist, int* __restrict__ part) {
+    const int b = 4 * (64 * blockIdx.y + threadIdx.x), r0 = blockIdx.x * TP_CHUNK;
+    if (b >= nbp) return;
+    const int r1 = r0 + TP_CHUNK < nblocks ? r0 + TP_CHUNK : nblocks;
+    int4 run = make_int4(0, 0, 0, 0);
+    constexpr int U = 16;
+    for (int r = r0; r < r1; r += U) {
+        int4 v[U];
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            v[u] = r + u < r1 ? *reinterpret_cast<const int4*>(hist + (int64_t)(r + u) * nbp + b) : make_int4(0, 0, 0, 0);
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (r + u < r1) *reinterpret_cast<int4*>(hist + (int64_t)(r + u) * nbp + b) = run;
+            run.x += v[u].x, run.y += v[u].y, run.z += v[u].z, run.w += v[u].w;
+        }
+    }
+    *reinterpret_cast<int4*>(part + (int64_t)blockIdx.x * nbp + b) = run;
 }
 
 // Exclusive prefix of v over the block's WARPS warps; *total their sum.
@@ -671,10 +712,36 @@ __device__ __forceinline__ int tp_block_excl(int v, int* sh, int* total) {
     return before + x - v;
 }
 
+// part: exclusive prefix over the chunks, in place; start[b]: the bucket's first
+// place, start[nb]: all items.  One block, a thread per bucket.
+__global__ void __launch_bounds__(TP_NB) k_tp_starts(int chunks, int nb, int nbp, int* __restrict__ part,
+                                                     int* __restrict__ start) {
+    __shared__ int sh[TP_NB / 32];
+    const int b = threadIdx.x;
+    int run = 0;
+    if (b < nbp) {
+        constexpr int U = 16;
+        for (int r = 0; r < chunks; r += U) {
+            int v[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) v[u] = r + u < chunks ? part[(int64_t)(r + u) * nbp + b] : 0;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                if (r + u < chunks) part[(int64_t)(r + u) * nbp + b] = run;
+                run += v[u];
+            }
+        }
+    }
+    int total;
+    const int at = tp_block_excl<TP_NB / 32>(run, sh, &total);
+    if (b < nb) start[b] = at;
+    if (b == 0) start[nb] = total;
+}
+
 // cnt[w * nkp + key]: how many of warp w's items have the key (nkp: keys rounded
 // up to a multiple of four, the rest zero).  Turns it into the place of the
-// warp's first one in (key, item) order; start(key, first, count) sees each
-// key's first place and count.  A thread takes four adjacent keys, so that one
+// warp's first one in (key, item) order; start(key, first) sees each key's first
+// place.  A thread takes four adjacent keys, so that one
 // block scan covers 4 x threads of them.
 template <int WARPS, typename F>
 __device__ __forceinline__ void tp_places(int* cnt, int nw, int nkp, int* sh, F start) {
@@ -693,7 +760,7 @@ __device__ __forceinline__ void tp_places(int* cnt, int nw, int nkp, int* sh, F 
         at.x = run + tp_block_excl<WARPS>(c.x + c.y + c.z + c.w, sh, &total);
         at.y = at.x + c.x, at.z = at.y + c.y, at.w = at.z + c.z;
         if (in) {
-            start(key, at, c);
+            start(key, at);
             for (int w = 0; w < nw; w++) {
                 int4* p = reinterpret_cast<int4*>(cnt + w * nkp + key);
                 const int4 t = *p;
@@ -724,13 +791,26 @@ __device__ __forceinline__ int tp_rank(int* mine, int key, int bits) {
     return at + r;
 }
 
+// What the passes write at each place of the order: source index and row, and for
+// f4j_csr_transpose (col non-null) the transpose's own copy of the row.  The
+// values stay with k_gather: read here, by the 16 warps an SM holds, they took
+// 460 us for its 163.
+struct TpOut {
+    int *perm, *row, *col;
+    __device__ __forceinline__ void put(int64_t at, int q, int r) const {
+        perm[at] = q;
+        row[at] = r;
+        if (col) col[at] = r;
+    }
+};
+
 // Item words: source index in the low qbits, row in the next rbits, column
 // within the bucket above.
 __global__ void __launch_bounds__(TP1_T) k_tp_scatter(int64_t n, const int* __restrict__ col,
                                                       const int* __restrict__ row, int shift, int nb, int qbits,
-                                                      int rbits, const int* __restrict__ incl, int nblocks,
-                                                      unsigned long long* __restrict__ items, int* __restrict__ perm,
-                                                      int* __restrict__ t_row) {
+                                                      int rbits, const int* __restrict__ hist,
+                                                      const int* __restrict__ part, const int* __restrict__ start,
+                                                      unsigned long long* __restrict__ items, const TpOut to) {
     extern __shared__ unsigned long long tp_smem[];
     unsigned long long* place = tp_smem;                      // (column, row) at each place of the tile
     int* cnt = reinterpret_cast<int*>(place + TP1_TILE);       // [warp][bucket]
@@ -745,13 +825,14 @@ __global__ void __launch_bounds__(TP1_T) k_tp_scatter(int64_t n, const int* __re
     const int nkp = (nb + 3) & ~3;
     int* mine = cnt + warp * nkp;
     const int i0 = warp * PART + lane;
-    // this block's last place of four buckets, for tp_places (nb <= 4 x threads)
+    // this block's first place of four buckets, for tp_places (nb <= 4 x threads; start has nbp entries)
     static_assert(TP_NB <= 4 * TP1_T, "four buckets a thread");
-    int last[4];
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-        const int b = 4 * threadIdx.x + u;
-        last[u] = b < nb ? __ldg(incl + (int64_t)b * nblocks + blockIdx.x) : 0;
+    int4 out = make_int4(0, 0, 0, 0);
+    if (4 * (int)threadIdx.x < nkp) {
+        const int4 x = reinterpret_cast<const int4*>(hist + (int64_t)blockIdx.x * nkp)[threadIdx.x];
+        const int4 y = reinterpret_cast<const int4*>(part + (int64_t)(blockIdx.x / TP_CHUNK) * nkp)[threadIdx.x];
+        const int4 z = reinterpret_cast<const int4*>(start)[threadIdx.x];
+        out = make_int4(x.x + y.x + z.x, x.y + y.y + z.y, x.z + y.z + z.z, x.w + y.w + z.w);
     }
     int c[PER], r[PER];
 #pragma unroll
@@ -767,9 +848,8 @@ __global__ void __launch_bounds__(TP1_T) k_tp_scatter(int64_t n, const int* __re
     for (int u = 0; u < PER; u++)
         if (c[u] >= 0) atomicAdd(&mine[c[u] >> shift], 1);
     __syncthreads();
-    tp_places<TP1_WARPS>(cnt, TP1_WARPS, nkp, sh, [&](int b, int4 first, int4 k) {
-        *reinterpret_cast<int4*>(delta + b) = make_int4(last[0] - k.x - first.x, last[1] - k.y - first.y,
-                                                        last[2] - k.z - first.z, last[3] - k.w - first.w);
+    tp_places<TP1_WARPS>(cnt, TP1_WARPS, nkp, sh, [&](int b, int4 first) {
+        *reinterpret_cast<int4*>(delta + b) = make_int4(out.x - first.x, out.y - first.y, out.z - first.z, out.w - first.w);
     });
 #pragma unroll
     for (int u = 0; u < PER; u++) {
@@ -789,25 +869,23 @@ __global__ void __launch_bounds__(TP1_T) k_tp_scatter(int64_t n, const int* __re
             items[dst] = q | (w & 0xffffffffull) << qbits |
                          (unsigned long long)(cc & ((1 << shift) - 1)) << (qbits + rbits);
         } else {  // one column a bucket: this is the whole order
-            perm[dst] = (int)q;
-            t_row[dst] = (int)w;
+            to.put(dst, (int)q, (int)w);
         }
     }
 }
 
-// Bucket blockIdx.x: columns [b << shift, (b + 1) << shift), items
-// [incl[b nblocks - 1], incl[(b + 1) nblocks - 1]) of the pass 1 output.
+// Bucket b = blockIdx.x: columns [b << shift, (b + 1) << shift), items
+// [start[b], start[b + 1]) of the pass 1 output.
 __global__ void __launch_bounds__(TP2_T) k_tp_bucket(int64_t cols, int shift, int qbits, int rbits, int nw,
-                                                     const int* __restrict__ incl, int nblocks,
+                                                     const int* __restrict__ start,
                                                      const unsigned long long* __restrict__ items,
-                                                     int* __restrict__ t_rowptr, int* __restrict__ perm,
-                                                     int* __restrict__ t_row) {
+                                                     int* __restrict__ t_rowptr, const TpOut to) {
     extern __shared__ unsigned long long tp_smem[];
     unsigned long long* place = tp_smem;                 // item at each place of the bucket
     int* cnt = reinterpret_cast<int*>(place + TP2_CAP);   // [warp][column]
     __shared__ int sh[TP2_WARPS];
     const int b = blockIdx.x, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    const int64_t s0 = b ? __ldg(incl + (int64_t)b * nblocks - 1) : 0, s1 = __ldg(incl + (int64_t)(b + 1) * nblocks - 1);
+    const int64_t s0 = __ldg(start + b), s1 = __ldg(start + b + 1);
     const int m = (int)(s1 - s0);
     const int64_t c0 = (int64_t)b << shift;
     const int nk = (int)(cols - c0 < (1 << shift) ? cols - c0 : 1 << shift);
@@ -831,7 +909,7 @@ __global__ void __launch_bounds__(TP2_T) k_tp_bucket(int64_t cols, int shift, in
             if (key[u] >= 0) atomicAdd(&mine[key[u]], 1);
     }
     __syncthreads();
-    tp_places<TP2_WARPS>(cnt, nw, nkp, sh, [&](int c, int4 first, int4) {
+    tp_places<TP2_WARPS>(cnt, nw, nkp, sh, [&](int c, int4 first) {
         const int f[4] = {first.x, first.y, first.z, first.w};
 #pragma unroll
         for (int u = 0; u < 4; u++)
@@ -852,8 +930,7 @@ __global__ void __launch_bounds__(TP2_T) k_tp_bucket(int64_t cols, int shift, in
             if (placed) {
                 place[at] = w[u];
             } else {  // more items than shared memory holds: straight to their places
-                perm[s0 + at] = (int)(w[u] & qmask);
-                t_row[s0 + at] = (int)(w[u] >> qbits & rmask);
+                to.put(s0 + at, (int)(w[u] & qmask), (int)(w[u] >> qbits & rmask));
             }
         }
     }
@@ -861,16 +938,14 @@ __global__ void __launch_bounds__(TP2_T) k_tp_bucket(int64_t cols, int shift, in
     __syncthreads();
     for (int p = threadIdx.x; p < m; p += TP2_T) {
         const unsigned long long w = place[p];
-        perm[s0 + p] = (int)(w & qmask);
-        t_row[s0 + p] = (int)(w >> qbits & rmask);
+        to.put(s0 + p, (int)(w & qmask), (int)(w >> qbits & rmask));
     }
 }
 
 // Row pointers when every bucket is one column (shift 0).
-__global__ void k_tp_rowptr(int nb, const int* __restrict__ incl, int nblocks, int* __restrict__ t_rowptr) {
+__global__ void k_tp_rowptr(int nb, const int* __restrict__ start, int* __restrict__ t_rowptr) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c > nb) return;
-    t_rowptr[c] = c ? incl[(int64_t)c * nblocks - 1] : 0;
+    if (c <= nb) t_rowptr[c] = start[c];
 }
 
 // ---------------- COO sort by (row, col), stable
@@ -1222,7 +1297,7 @@ static int bits_for(int64_t maxval) {
 // most-significant-bits-first buckets (see k_tp_scatter); shift: columns per
 // bucket, qbits / rbits: bits of a source index and of a row.
 static int transpose_buckets(f4j_ctx* ctx, f4j_csr S, int shift, int qbits, int rbits, const int* rowidx, int* trp,
-                             int* perm, int* trow) {
+                             const TpOut& to) {
     const int64_t nnz = S->nnz, cols = S->cols;
     const int* col = (const int*)S->colidx->ptr;
     const int nb = (int)((cols - 1) >> shift) + 1;
@@ -1233,24 +1308,23 @@ static int transpose_buckets(f4j_ctx* ctx, f4j_csr S, int shift, int qbits, int 
     F4J_CUDA(cudaFuncSetAttribute(k_tp_bucket, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));
     int* hist = nullptr;
     unsigned long long* items = nullptr;
-    int rc = f4j_dev_alloc(ctx, (size_t)nb * nblocks * 4, (void**)&hist);
+    const int nbp = (nb + 3) & ~3, chunks = (int)f4j_cdiv(nblocks, TP_CHUNK);
+    int rc = f4j_dev_alloc(ctx, ((size_t)(nblocks + chunks + 1) * nbp + 4) * 4, (void**)&hist);
     if (!rc && shift) rc = f4j_dev_alloc(ctx, (size_t)nnz * 8, (void**)&items);
     if (!rc) {
-        k_tp_hist<<<nblocks, 512, 0, ctx->stream>>>(nnz, col, shift, nb, hist, nblocks);
-        ctx->launches++;
-        rc = scan_inclusive(ctx, hist, (int64_t)nb * nblocks);
-    }
-    if (!rc) {
-        k_tp_scatter<<<nblocks, TP1_T, smem1, ctx->stream>>>(nnz, col, rowidx, shift, nb, qbits, rbits, hist, nblocks,
-                                                             items, perm, trow);
+        int *part = hist + (size_t)nblocks * nbp, *start = part + (size_t)chunks * nbp;
+        k_tp_hist<<<nblocks, 512, 0, ctx->stream>>>(nnz, col, shift, nbp, hist);
+        k_tp_chunks<<<dim3(chunks, (unsigned)f4j_cdiv(nbp, 256)), 64, 0, ctx->stream>>>(nblocks, nbp, hist, part);
+        k_tp_starts<<<1, TP_NB, 0, ctx->stream>>>(chunks, nb, nbp, part, start);
+        k_tp_scatter<<<nblocks, TP1_T, smem1, ctx->stream>>>(nnz, col, rowidx, shift, nb, qbits, rbits, hist, part, start,
+                                                             items, to);
         if (shift) {
             const int nw = TP2_WARPS < TP2_CNT >> shift ? TP2_WARPS : TP2_CNT >> shift;
-            k_tp_bucket<<<nb, TP2_T, smem2, ctx->stream>>>(cols, shift, qbits, rbits, nw, hist, nblocks, items, trp,
-                                                           perm, trow);
+            k_tp_bucket<<<nb, TP2_T, smem2, ctx->stream>>>(cols, shift, qbits, rbits, nw, start, items, trp, to);
         } else {
-            k_tp_rowptr<<<grid1(nb + 1), 256, 0, ctx->stream>>>(nb, hist, nblocks, trp);
+            k_tp_rowptr<<<grid1(nb + 1), 256, 0, ctx->stream>>>(nb, start, trp);
         }
-        ctx->launches += 2;
+        ctx->launches += 5;
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) rc = f4j_cuda_fail(e, "transpose structure");
     }
@@ -1289,8 +1363,10 @@ static int transpose_radix(f4j_ctx* ctx, f4j_csr S, const int* rowidx, int* trp,
     return rc;
 }
 
-// Builds the cached transpose structure of S (RealCsrOps.transpose order).
-static int ensure_transpose(f4j_ctx* ctx, f4j_csr S) {
+// Builds the cached transpose structure of S (RealCsrOps.transpose order).  t_col:
+// an array for a copy of its column indices, made on the way where that can be
+// (*copied).
+static int ensure_transpose(f4j_ctx* ctx, f4j_csr S, int* t_col = nullptr, bool* copied = nullptr) {
     if (S->t_perm) return F4J_OK;
     const int64_t nnz = S->nnz, rows = S->rows, cols = S->cols;
     int *trp = nullptr, *perm = nullptr, *trow = nullptr, *ri = nullptr;
@@ -1313,10 +1389,11 @@ static int ensure_transpose(f4j_ctx* ctx, f4j_csr S) {
         int shift = 0;
         while (((cols - 1) >> shift) >= TP_NB) shift++;
         const int qbits = bits_for(nnz - 1), rbits = bits_for(rows - 1);
+        const bool buckets = shift <= 12 && qbits + rbits + shift <= 64;
         if (!rc)
-            rc = shift <= 12 && qbits + rbits + shift <= 64
-                     ? transpose_buckets(ctx, S, shift, qbits, rbits, rowidx, trp, perm, trow)
-                     : transpose_radix(ctx, S, rowidx, trp, perm, trow);
+            rc = buckets ? transpose_buckets(ctx, S, shift, qbits, rbits, rowidx, trp, TpOut{perm, trow, t_col})
+                         : transpose_radix(ctx, S, rowidx, trp, perm, trow);
+        if (!rc && t_col) *copied = buckets;
         f4j_dev_free(ctx, ri);
     }
     if (rc) {
@@ -1895,14 +1972,19 @@ extern "C" int f4j_csr_transpose(f4j_ctx* ctx, f4j_csr S, f4j_csr* out) {
     F4J_CHECK_CTX(ctx);
     if (!S || !out) return f4j_fail(F4J_ERR_ARG, "null argument");
     F4J_CUDA(cudaSetDevice(ctx->device));
-    int rc = ensure_transpose(ctx, S);
-    if (rc) return rc;
     f4j_csr T;
-    rc = alloc_owned_csr(ctx, S->cols, S->rows, S->nnz, &T);
+    int rc = alloc_owned_csr(ctx, S->cols, S->rows, S->nnz, &T);
     if (rc) return rc;
+    bool copied = false;
+    rc = ensure_transpose(ctx, S, (int*)T->colidx->ptr, &copied);
+    if (rc) {
+        f4j_csr_free(ctx, T);
+        return rc;
+    }
     F4J_CUDA(cudaMemcpyAsync(T->rowptr->ptr, S->t_rowptr, (size_t)(S->cols + 1) * 4, cudaMemcpyDeviceToDevice,
                              ctx->stream));
-    F4J_CUDA(cudaMemcpyAsync(T->colidx->ptr, S->t_rowidx, (size_t)S->nnz * 4, cudaMemcpyDeviceToDevice, ctx->stream));
+    if (!copied)
+        F4J_CUDA(cudaMemcpyAsync(T->colidx->ptr, S->t_rowidx, (size_t)S->nnz * 4, cudaMemcpyDeviceToDevice, ctx->stream));
     if (S->nnz) {
         k_gather<double><<<grid1(S->nnz), 256, 0, ctx->stream>>>(S->nnz, (const int*)S->t_perm,
                                                                  (const double*)S->vals->ptr, (double*)T->vals->ptr);

@@ -667,3 +667,25 @@ def test_transpose_structure_is_the_stable_column_order(f4j, rows, cols, nnz, ki
     assert np.array_equal(T.rowPointers, trp)
     assert np.array_equal(T.colIndices, row[perm])
     assert np.array_equal(T.data, vals[perm])
+
+
+@pytest.mark.parametrize("rows,cols,nnz", [
+    (700, 900, 20000),                                   # a column is a bucket
+    (9000, 60001, 64 * 4096), (9000, 60001, 64 * 4096 + 1),  # one chunk of histogram rows, one row more
+    (30000, 5003, 130 * 4096 + 77),                      # several chunks, buckets past shared memory
+    (2000, (1 << 22) + 1, 30000),                        # the radix sort
+])
+def test_transpose_of_a_new_matrix_and_again_from_its_structure(f4j, rows, cols, nnz):
+    """CsrMatrix.T() as the first call on a handle (its column indices come with the structure) and again
+    from the cached structure: both the stable order by column."""
+    g = np.random.default_rng(nnz)
+    row, col = np.sort(g.integers(0, rows, nnz)), g.integers(0, cols, nnz)
+    rp = np.zeros(rows + 1, np.int32)
+    np.cumsum(np.bincount(row, minlength=rows), out=rp[1:])
+    vals = g.standard_normal(nnz)
+    S = f4j.CsrMatrix((rows, cols), vals, rp, col.astype(np.int32), validate=False)
+    perm = np.argsort(col, kind="stable")
+    for T in (S.T(), S.T()):
+        assert np.array_equal(np.diff(T.rowPointers), np.bincount(col, minlength=cols))
+        assert np.array_equal(T.colIndices, row[perm])
+        assert np.array_equal(T.data, vals[perm])
