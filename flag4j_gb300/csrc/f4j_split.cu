@@ -1572,22 +1572,26 @@ static int split_report(f4j_ctx* ctx, const SplitPlan* plan, f4j_report* rep) {
 // forced small slice count, and with F4J_MODE_SPLIT (any_form false) not the
 // shapes f4j_dgemm_split_noalloc accepts: its result is that mode's bit for
 // bit, and its scratch holds slice planes only.
-// Narrow and short products stay with the slices: the residue planes cost
-// about twice as much per element, the tiles are 256 wide, and reconstructing
-// C is work per entry that the slices do not have.  Measured on GB300, us,
-// slices / residues: 256^3 68 / 52, 512^3 74 / 60, 1024^3 123 / 108, 1024 x
-// 1024 x 512 95 / 92, 1500 x 1500 x 512 113 / 131, 4096 x 4096 x 512 503 / 528,
-// 2500 x 700 x 600 200 / 130, 4096 x 4096 x 768 774 / 584, 256 x 256 x 4096
-// 91 / 98, 300 x 3000 x 1000 133 / 140, 256 x 8192 x 8192 1107 / 1097, 384 x
-// 8192 x 8192 1750 / 1410, 8192^3 19200 / 12000; complex 384 x 192 x 300
-// 86 / 69, 2000 x 2000 x 100 259 / 284.
+// The slices keep what fits one of their 128-wide tiles, short sums (the residue
+// planes cost about twice as much per element, and reconstructing C is work per
+// entry that the slices do not have), and on large C also sums that are one
+// power-of-two K chunk of theirs, four or eight blocks of 64.  Measured on GB300,
+// us, slices / residues: 256^3 70 / 43, 512^3 74 / 54, 1024^3 123 / 91, 1500 x 1500
+// x 256 89 / 109, x 288 156 / 113, x 512 114 / 120, x 544 181 / 123; 8192 x 8192 x
+// 256 1188 / 1840, x 288 1774 / 1843, x 352 1910 / 1859, x 512 1730 / 1851, x 544
+// 2321 / 1930; 128 x 4096 x 4096 278 / 338, 129 x 2048 x 4096 212 / 201, 129 x 2048 x
+// 512 80 / 63, 192 x 8192 x 512 141 / 140, 256 x 8192 x 8192 1127 / 1107, 300 x 300 x
+// 8000 679 / 147; complex 256 x 256 x 2048 111 / 109, 300 x 3000 x 500 208 / 185,
+// 200 x 2000 x 2000 343 / 275.
 static bool crt_wanted(bool cplx, int64_t m, int64_t n, int64_t k, int slices_req, bool any_form) {
     const int req = slices_req > 0 ? slices_req : env_slices();
     if (req > 0 && req < 8) return false;
     const int64_t N = cplx ? 2 * n : n, klen = cplx ? 2 * k : k;
     const int64_t lo = m < N ? m : N, hi = m < N ? N : m;
-    if (lo < 384 && !(lo >= 256 && hi <= 1024 && klen <= 2048)) return false;
-    if (klen < (lo * hi <= (1 << 20) ? 256 : 576) || klen > (1 << 22)) return false;
+    const int64_t blocks = f4j_cdiv(klen, BKB);
+    if (lo <= 128 || klen < 256 || klen > (1 << 22)) return false;
+    if (lo * hi > 3 << 19 && blocks <= 8 && (blocks & (blocks - 1)) == 0) return false;
+    if (lo * hi > 1 << 24 && klen < 320) return false;
     if (!any_form && !cplx && F4J_NOALLOC_NEED(m, n, f4j_cdiv(k, BKB) * BKB) <= F4J_NOALLOC_SCRATCH_BYTES)
         return false;
     return crt_config(S_MAX, klen) >= 0;

@@ -169,3 +169,26 @@ def test_residue_form_launches_in_order(f4j):
     for w, q in zip(*outs):
         assert np.array_equal(w, q, equal_nan=True)
     assert np.isnan(outs[0][-1]).any() and not np.isnan(outs[0][0]).any()
+
+
+@pytest.mark.parametrize("m,n,k", [
+    (129, 700, 256), (700, 129, 300), (129, 2048, 288), (255, 257, 4100),   # one tile wide, just past a slice tile
+    (1254, 1254, 512), (1300, 1300, 288), (1300, 1300, 449), (1300, 1300, 513),  # short sums of a large C
+    (4100, 4100, 320),
+])
+def test_narrow_and_short_products_take_the_residue_form(f4j, m, n, k):
+    """AUTO at the edges of the shapes that the residue form takes: exact on integers, which the slices are
+    not, for every order of the operands."""
+    from flag4j_gb300 import _lib
+    from flag4j_gb300.device import check
+    ctx = f4j.default_context()
+    A, B = ints((m, k), m), ints((k, n), n + 1)
+    want = int_product(A, B)
+    for opA, opB in ((0, 0), (0, 1), (1, 0), (1, 1)):
+        dA = ctx.from_numpy(A if opA == 0 else np.ascontiguousarray(A.T))
+        dB = ctx.from_numpy(B if opB == 0 else np.ascontiguousarray(B.T))
+        dC, rep = ctx.alloc(C_bytes(m, n, False)), _lib.f4j_report()
+        check(ctx.lib.f4j_dgemm(ctx.handle, m, n, k, dA.handle, opA, dB.handle, opB, dC.handle, _lib.MODE_AUTO,
+                                ctypes.byref(rep)))
+        assert rep.mode_used == _lib.MODE_SPLIT
+        assert np.array_equal(dC.to_numpy(np.float64, m * n).reshape(m, n), want), (opA, opB)
