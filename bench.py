@@ -2,13 +2,14 @@
 
 One step = one FP64-accurate GEMM C = A B at 8192^3 (real float64, entries
 u 2^e, u ~ U[-1,1), integer e ~ U[-8, 8] per row of A / column of B) through
-the split path: exponent statistics, FP8 slicing and the tcgen05 slice GEMM.
+the split path: exponent statistics, FP8 residue planes, the tcgen05 residue
+GEMM and the reconstruction.
 value = 2 m n k / step time (TFLOP/s, FP64-equivalent), inputs resident in
 HBM (A, B: 512 MiB each, larger than L2, so no flush is needed).  The same JSON
 line carries the plain DMMA path, errors against the double-double check for
 phi in {0, 8, 32}, the Complex128 4096^3 product, CSR SpMV/SpMM GB/s at 2^20
 rows (Poisson(16) row lengths), the dense adjoint step ratio, the roofline of
-the slice GEMM kernel, the CPU baseline and an end-to-end number through the
+the residue GEMM kernel, the CPU baseline and an end-to-end number through the
 host-buffer API (host<->device copies inside the timed region).  After all GPU
 timing, the oracle's restatements of the reference's loops are timed on this
 host beside the sparse, complex and adjoint rows (their cpu_baseline keys).
@@ -227,6 +228,16 @@ def fp8_peak_tflops():
         return v, "%s (fp8 measurement failed: %s)" % (src, type(ex).__name__)
 
 
+def residue_products(s, klen):
+    """FP8 products of a residue-form GEMM with s slices' precision (F = 4 + 5 (s - 1) bits) and sums of klen
+    terms: the cheapest choice of moduli whose product holds klen 2^(2F) and a sign; a square of a base costs
+    three products, a base one (crt_config in f4j_crt.cuh)."""
+    bases = (49, 47, 43, 41, 37, 32, 31, 29, 27, 25, 23, 19, 17, 13, 11)
+    need = 2.0 * (4 + 5 * (s - 1)) + math.log2(klen) + 1.01
+    return min(nmod + 2 * nsq for nmod in range(9, len(bases) + 1) for nsq in range(nmod + 1)
+               if sum(math.log2(b) for b in bases[:nmod] + bases[:nsq]) >= need)
+
+
 def fp8_peak_from_file():
     """2 x the dense bf16 burst rate in MEASURED_PEAKS.json (FP8 runs at twice bf16 on the tensor pipe);
     the recipe's 1.9 PFLOP/s bf16 fallback when the file is absent."""
@@ -236,17 +247,17 @@ def fp8_peak_from_file():
     return 2 * 1900.0, "2 x fallback bf16 1.9 PFLOP/s"
 
 
-# DRAM bytes of one k_split_gemm launch at 8192^3 by slice count, from one ncu
-# capture each (dram__bytes_read.sum + dram__bytes_write.sum, 1 pass):
+# DRAM bytes of one k_crt_gemm launch at 8192^3, s = 10, from one ncu capture
+# (dram__bytes_read.sum + dram__bytes_write.sum, 1 pass):
 #   ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum,gpu__time_duration.sum --clock-control none
-#       -k regex:k_split_gemm -s 2 -c 1 python bench.py --skip-extras --steps 2 --warmup 3
-SPLIT_GEMM_DRAM_BYTES_8192 = {11: 15.077633e9 + 0.636095e9, 10: 12.27e9 + 0.65615e9}
+#       -k regex:k_crt_gemm -s 2 -c 1 python bench.py --skip-extras --steps 2 --warmup 3
+CRT_GEMM_DRAM_BYTES_8192 = {10: 32.655e9 + 2.352e9}
 
 # DRAM bytes of one 2^20-row, 32-column SpMM launch (k_spmm), exact and FMA
 # modes, from the ncu capture in profiles/k_spmm_1M_rows_32cols.md
-SPMM_DRAM_BYTES_1M = {"exact": 3.255e9 + 0.266e9, "fma": 3.257e9 + 0.265e9}
+SPMM_DRAM_BYTES_1M = {"exact": 3.256e9 + 0.265e9, "fma": 3.257e9 + 0.265e9}
 # FP64-pipe activity of the same launches (sm__pipe_fp64_cycles_active, of active cycles)
-SPMM_FP64_PIPE_1M = {"exact": 0.839, "fma": 0.933}
+SPMM_FP64_PIPE_1M = {"exact": 0.976, "fma": 0.933}
 
 
 def fp64_peak_tflops():
@@ -653,9 +664,9 @@ def run_ours(args):
                        "note": "f4j_report accuracy fields: sampled Dot2 error of this result, k u bound of a plain "
                                "FP64 product on the same scale, the CPU kernel Flag4j's dispatcher would run"}
 
-    # dominant kernel time: the tcgen05 slice GEMM alone (same inputs), for the roofline
+    # dominant kernel time: the tcgen05 residue GEMM alone (same inputs), for the roofline
     s = rep.slices
-    prods = s * (s + 1) // 2
+    prods = residue_products(s, n)
     kp = math.ceil(n / 128) * 128
     fp8_flops = prods * 2.0 * n * n * kp
     out["split"] = {"slices": s, "frac_bits": rep.frac_bits, "exp_spread_bits": round(rep.exp_spread, 3),
@@ -731,7 +742,8 @@ def run_ours(args):
         out["complex"]["e2e"] = {"value": zf / (zhe * 1e-3) / 1e12, "unit": "TFLOP/s", "ms": zhe,
                                  "h2d_bytes_per_step": Azh.nbytes + Bzh.nbytes, "d2h_bytes_per_step": Czh.nbytes,
                                  "path": "f4j_zgemm_host on page-locked host A, B, C (interleaved complex): B up "
-                                         "whole, then A in 4 row parts, each sliced and multiplied as it arrives "
+                                         "whole, then A in 4 row parts, each brought to residues and multiplied as it "
+                                         "arrives "
                                          "and its rows of C downloaded behind its product"}
         del Azh, Bzh, Czh
         # ---- dense adjoint step: A (n/2 x n/4), B (n/4 x n/2), split
@@ -750,7 +762,7 @@ def run_ours(args):
         del Aa, Ba, Wa, Ca, dA, dB
         out["spmm"] = sparse_section(E, full)
 
-    # ---- roofline of the dominant kernel (the tcgen05 slice GEMM), timed alone
+    # ---- roofline of the dominant kernel (the tcgen05 residue GEMM), timed alone
     # with CUDA events around its launch on the context stream
     A, B = E.dev(A_h), E.dev(B_h)
     kms, prep_ms = E.kernel_ms(lambda: E.gemm(A, B, C, n, n, n, L.MODE_SPLIT), max(3, args.steps // 2), True)
@@ -763,14 +775,14 @@ def run_ours(args):
     fp8_peak, fp8_src = fp8_peak_from_file()
     fp8_run, fp8_run_src = fp8_peak_tflops() if not args.skip_extras else (None, None)
     achieved = fp8_flops / (kms * 1e-3) / 1e12
-    traffic = SPLIT_GEMM_DRAM_BYTES_8192.get(s) if n == 8192 else None
+    traffic = CRT_GEMM_DRAM_BYTES_8192.get(s) if n == 8192 else None
     roofline = {"bound": "tensor", "achieved": achieved, "peak": fp8_peak, "unit": "TFLOP/s",
                 "frac": achieved / fp8_peak, "traffic": traffic,
-                "traffic_note": "DRAM bytes per launch from one ncu capture of the 8192^3 launch (read + write); "
-                                "the kernel is tensor-bound, 0.76 GB/ms of DRAM" if traffic else None,
-                "kernel": "k_split_gemm (tcgen05 kind::f8f6f4)",
+                "traffic_note": "DRAM bytes per launch from one ncu capture of the 8192^3 launch (read + write)"
+                                if traffic else None,
+                "kernel": "k_crt_gemm (tcgen05 kind::f8f6f4, cta_group::2)",
                 "kernel_ms": kms, "kernel_share_of_step": kms / ms_local,
-                "basis": "FP8 MMA flops per launch: s(s+1)/2 slice products x 2 n n Kp",
+                "basis": "FP8 MMA flops per launch: the moduli's products (three a square, one a single) x 2 n n Kp",
                 "peak_source": fp8_src + ", of measured",
                 "cublaslt_fp8_this_run": fp8_run, "frac_of_cublaslt_fp8_this_run":
                     achieved / fp8_run if fp8_run else None, "cublaslt_fp8_source": fp8_run_src}
@@ -836,7 +848,7 @@ def run_ours(args):
         return
     line = {"metric": METRIC, "value": value, "unit": "TFLOP/s", "n_gpus": ws, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak",
-            "vs_baseline": None, "dtype": "f64 (FP8 E4M3 slices, exact FP32/int64 accumulation)",
+            "vs_baseline": None, "dtype": "f64 (FP8 E4M3 residue digits, exact FP32/integer accumulation)",
             "data": "synthetic (seeded PCG64)",
             "config": headline_config(n, ws),
             "roofline": roofline, "cpu_baseline": cb,
@@ -844,7 +856,7 @@ def run_ours(args):
                     "h2d_bytes_per_step": Ah.nbytes + Bh.nbytes, "d2h_bytes_per_step": Ch.nbytes,
                     "path": "f4j_dgemm_host (split) on page-locked host A, B, C (f4j_host_alloc): uploads back "
                             "to back (A's first 1024 rows, B in 4 column parts, the rest of A in 3 row parts), "
-                            "each part sliced as it arrives, B's column parts multiplied by A's first rows and "
+                            "each part brought to residues as it arrives, B's column parts multiplied by A's first rows and "
                             "A's later parts by all of B, each block of C downloaded behind its product (the "
                             "slice count from the first parts, checked against all of A and B)"},
             "e2e_pageable_pinned_per_call": {"value": ws * flops / (e2e_pg_ms * 1e-3) / 1e12, "unit": "TFLOP/s",
