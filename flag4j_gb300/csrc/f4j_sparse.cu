@@ -292,78 +292,73 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// SDDMM with 64 columns, flat over the nonzeros: a block takes 64 consecutive
-// nonzeros whatever their rows, a group of 4 lanes one nonzero.  The block's
-// distinct rows of A (rows are sorted, so equal rows are adjacent) are staged
-// in shared memory once, so a lane holds only its 16 values of the row of B
-// in registers (60 registers and 4 blocks per SM, against 74 and about 20
-// warps per SM with A in registers too).  Lane l4 of a group owns the
-// 16-byte pairs l4, l4 + 4, ..., l4 + 28 of the 64 columns: the group's four
-// lanes read 64 contiguous bytes per step from shared memory and from B, and
-// the padded row stride (33 pairs) puts neighbouring rows in other banks.
-// 16 FMAs and a 2-step tree sum per lane: 18 FP64 warp instructions per 8
-// nonzeros.  The B loads are issued first, so they are in flight while the
-// block stages A.  rowidx: the row of each nonzero.
-constexpr int SD_NNZ = 64;        // nonzeros per block (256 threads)
-constexpr int SD_PAIRS = 33;      // padded row stride of the staged rows, in 16-byte pairs
+// SDDMM with 64 columns, flat over the nonzeros: a warp takes SD_WARP
+// consecutive nonzeros, eight at a time, a group of 4 lanes one nonzero.  Lane
+// l4 of a group owns the 16-byte pairs l4, l4 + 4, ..., l4 + 28 of the 64 columns,
+// so the group's four lanes read 64 contiguous bytes a step.  The FP64 pipe
+// bounds it: 16 FMAs a nonzero and lane, and three adds for four nonzeros (their
+// sums are exchanged so that each lane ends up with one; two adds each take 72
+// instructions for these 67).  What keeps the pipe fed: a pair of the next
+// nonzero's row of B is loaded as soon as the current one has been used, its
+// indices a step earlier, and nothing waits for a barrier.  The rows of A come
+// through L1 (rowidx is sorted: neighbouring groups read the same row; B does not
+// allocate there).  2^18 rows x 16: 0.50 ms at 3 or 4 blocks an SM, 0.55 at 2; with
+// A staged in shared memory by blocks of 64 nonzeros, two barriers each, 0.56.
+// rowidx: the row of each nonzero.
+constexpr int SD_WARP = 64;
+__device__ __forceinline__ double2 ld_nc_stream(const double2* p) {
+    double2 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+    return v;
+}
 __global__ void __launch_bounds__(256, 4)
-    k_sddmm64s(int64_t nnz, const int* __restrict__ rowidx, const int* __restrict__ colidx,
-               const double* __restrict__ A, const double* __restrict__ B, double* __restrict__ out) {
-    __shared__ double2 sA[SD_NNZ * SD_PAIRS];
-    __shared__ int slot[SD_NNZ], srow[SD_NNZ], s_nrows;
-    const int64_t q0 = (int64_t)blockIdx.x * SD_NNZ;
-    const int tid = threadIdx.x, g = tid >> 2, l4 = tid & 3;
-    const int64_t q = q0 + g;
+    k_sddmm64(int64_t nnz, const int* __restrict__ rowidx, const int* __restrict__ colidx,
+              const double* __restrict__ A, const double* __restrict__ B, double* __restrict__ out) {
+    const int lane = threadIdx.x % 32, g = lane >> 2, l4 = lane & 3;
+    const int64_t w0 = ((int64_t)blockIdx.x * 8 + threadIdx.x / 32) * SD_WARP;
+    if (w0 >= nnz) return;
+    auto at = [&](int step) {  // past the end: the last nonzero again, not stored
+        const int64_t q = w0 + step * 8 + g;
+        return q < nnz ? q : nnz - 1;
+    };
+    auto row_of = [&](const double* X, int i) { return reinterpret_cast<const double2*>(X + (int64_t)i * 64) + l4; };
+    const double2* arow = row_of(A, __ldg(rowidx + at(0)));
+    const double2* brow = row_of(B, __ldg(colidx + at(0)));
+    int rn = __ldg(rowidx + at(1)), cn = __ldg(colidx + at(1));
     double2 b[8];
-    if (q < nnz) {
-        const double2* brow = reinterpret_cast<const double2*>(B + (int64_t)__ldg(&colidx[q]) * 64) + l4;
 #pragma unroll
-        for (int u = 0; u < 8; u++) b[u] = __ldg(brow + 4 * u);
-    } else {
+    for (int u = 0; u < 8; u++) b[u] = ld_nc_stream(brow + 4 * u);
+#pragma unroll 1
+    for (int s0 = 0; s0 < SD_WARP / 8; s0 += 4) {
+        double p[4];
 #pragma unroll
-        for (int u = 0; u < 8; u++) b[u] = make_double2(0.0, 0.0);
-    }
-    if (tid < 32) {  // warp 0: slots of the block's nonzeros (two per lane) and the distinct rows
-        int r[2];
-        bool head[2];
+        for (int j = 0; j < 4; j++) {
+            const int step = s0 + j;
+            const double2* an = row_of(A, rn);
+            brow = row_of(B, cn);
+            if (step + 2 < SD_WARP / 8) {
+                rn = __ldg(rowidx + at(step + 2));
+                cn = __ldg(colidx + at(step + 2));
+            }
+            double s = 0.0;
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int t = tid + 32 * h;
-            const int64_t qq = q0 + t;
-            r[h] = qq < nnz ? __ldg(&rowidx[qq]) : -1;
-            head[h] = qq < nnz && (t == 0 || __ldg(&rowidx[qq - 1]) != r[h]);
+            for (int u = 0; u < 8; u++) {
+                const double2 a = __ldg(arow + 4 * u);
+                s = fma(a.y, b[u].y, fma(a.x, b[u].x, s));
+                if (step + 1 < SD_WARP / 8) b[u] = ld_nc_stream(brow + 4 * u);
+            }
+            p[j] = s;
+            arow = an;
         }
-        const unsigned b0 = __ballot_sync(0xffffffffu, head[0]), b1 = __ballot_sync(0xffffffffu, head[1]);
-        const unsigned below = (1u << tid) - 1u;
-        const int n0 = __popc(b0);
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int t = tid + 32 * h;
-            const int idx = (h ? n0 + __popc(b1 & below) : __popc(b0 & below)) + (head[h] ? 1 : 0) - 1;
-            slot[t] = idx;
-            if (head[h]) srow[idx] = r[h];
-        }
-        if (tid == 0) s_nrows = n0 + __popc(b1);
+        // four sums of four lanes: lane l4 ends with the nonzero of step s0 + l4
+        const bool h2 = l4 & 2, h1 = l4 & 1;
+        const double u0 = __shfl_xor_sync(0xffffffffu, h2 ? p[0] : p[2], 2);
+        const double u1 = __shfl_xor_sync(0xffffffffu, h2 ? p[1] : p[3], 2);
+        const double t0 = (h2 ? p[2] : p[0]) + u0, t1 = (h2 ? p[3] : p[1]) + u1;
+        const double r = (h1 ? t1 : t0) + __shfl_xor_sync(0xffffffffu, h1 ? t0 : t1, 1);
+        const int64_t q = w0 + (s0 + l4) * 8 + g;
+        if (q < nnz) out[q] = r;
     }
-    __syncthreads();
-    const int nrows = s_nrows;
-    for (int i = tid; i < nrows * 32; i += 256) {
-        const int rr = i >> 5, pr = i & 31;
-        sA[rr * SD_PAIRS + pr] = __ldg(reinterpret_cast<const double2*>(A + (int64_t)srow[rr] * 64) + pr);
-    }
-    __syncthreads();
-    double s = 0.0;
-    if (q < nnz) {
-        const double2* arow = sA + slot[g] * SD_PAIRS + l4;
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const double2 a = arow[4 * u];
-            s = fma(a.y, b[u].y, fma(a.x, b[u].x, s));
-        }
-    }
-    s += __shfl_xor_sync(0xffffffffu, s, 2);
-    s += __shfl_xor_sync(0xffffffffu, s, 1);
-    if (q < nnz && l4 == 0) out[q] = s;
 }
 
 // ------------------------------------------------------------------ structure
@@ -2153,7 +2148,7 @@ extern "C" int f4j_sddmm(f4j_ctx* ctx, f4j_csr S, f4j_buf A, f4j_buf B, int64_t 
         if (ncols == 64 && ((reinterpret_cast<uintptr_t>(A->ptr) | reinterpret_cast<uintptr_t>(B->ptr)) & 15) == 0) {
             int rc = ensure_rowidx(ctx, S);
             if (rc) return rc;
-            k_sddmm64s<<<(unsigned)f4j_cdiv(S->nnz, SD_NNZ), 256, 0, ctx->stream>>>(
+            k_sddmm64<<<(unsigned)f4j_cdiv(S->nnz, 8 * SD_WARP), 256, 0, ctx->stream>>>(
                 S->nnz, (const int*)S->rowidx, (const int*)S->colidx->ptr, (const double*)A->ptr,
                 (const double*)B->ptr, (double*)out->ptr);
         } else

@@ -689,3 +689,24 @@ def test_transpose_of_a_new_matrix_and_again_from_its_structure(f4j, rows, cols,
         assert np.array_equal(np.diff(T.rowPointers), np.bincount(col, minlength=cols))
         assert np.array_equal(T.colIndices, row[perm])
         assert np.array_equal(T.data, vals[perm])
+
+
+@pytest.mark.parametrize("nnz", [1, 7, 8, 63, 64, 65, 511, 512, 513, 1000])
+def test_sddmm_64_columns_at_the_edges_of_a_warp(f4j, nnz):
+    """dS at 64 columns for nonzero counts around a step (8), a warp (64) and a block (512) of the kernel, with
+    rows of every length in one matrix: within 2 ncols u sum|a||b| of the double product."""
+    from flag4j_gb300.device import check
+    g = np.random.default_rng(nnz)
+    rows, cols = 40, 2000
+    row = np.sort(g.integers(0, rows, nnz))
+    col = np.concatenate([np.sort(g.choice(cols, n, replace=False)) for n in np.bincount(row, minlength=rows)])
+    rp = np.zeros(rows + 1, np.int32)
+    np.cumsum(np.bincount(row, minlength=rows), out=rp[1:])
+    S = f4j.CsrMatrix((rows, cols), np.ones(nnz), rp, col.astype(np.int32))
+    A, B = g.standard_normal((rows, 64)), g.standard_normal((cols, 64))
+    ctx = f4j.default_context()
+    dA, dB, out = ctx.from_numpy(A), ctx.from_numpy(B), ctx.alloc(8 * nnz)
+    check(ctx.lib.f4j_sddmm(ctx.handle, S.handle(ctx), dA.handle, dB.handle, 64, out.handle, None))
+    got = out.to_numpy(np.float64, nnz)
+    terms = A[row].astype(np.longdouble) * B[col].astype(np.longdouble)
+    assert np.all(np.abs(got - terms.sum(1)) <= 2 * 64 * U * np.abs(terms).sum(1))
