@@ -292,62 +292,95 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// SDDMM with 64 columns, flat over the nonzeros: a warp takes SD_WARP
-// consecutive nonzeros, eight at a time, a group of 4 lanes one nonzero.  Lane
-// l4 of a group owns the 16-byte pairs l4, l4 + 4, ..., l4 + 28 of the 64 columns,
-// so the group's four lanes read 64 contiguous bytes a step.  The FP64 pipe
-// bounds it: 16 FMAs a nonzero and lane, and three adds for four nonzeros (their
-// sums are exchanged so that each lane ends up with one; two adds each take 72
-// instructions for these 67).  What keeps the pipe fed: a pair of the next
-// nonzero's row of B is loaded as soon as the current one has been used, its
-// indices a step earlier, and nothing waits for a barrier.  The rows of A come
-// through L1 (rowidx is sorted: neighbouring groups read the same row; B does not
-// allocate there).  2^18 rows x 16: 0.50 ms at 3 or 4 blocks an SM, 0.55 at 2; with
-// A staged in shared memory by blocks of 64 nonzeros, two barriers each, 0.56.
+// SDDMM of up to 64 columns of rows ld entries apart (add: on top of the columns
+// before), flat over the nonzeros: a warp takes SD_WARP consecutive nonzeros, eight at a time, a group of 4 lanes one nonzero.  A unit
+// is a 16-byte pair of columns (PAIRS: an even number of columns, aligned
+// operands) or one column; lane l4 of a group owns the units l4, l4 + 4, ..., at
+// most U of them, so the group's four lanes read 64 (32) contiguous bytes a
+// step.  The FP64 pipe bounds it: with 64 columns 16 FMAs a nonzero and lane and
+// three adds for four nonzeros (their sums are exchanged so that each lane ends
+// up with one; two adds each take 72 instructions for these 67).  What keeps the
+// pipe fed: a unit of the next nonzero's row of B is loaded as soon as the current
+// one has been used, its indices a step earlier, and nothing waits for a barrier.
+// The rows of A come through L1 (rowidx is sorted: neighbouring groups read the
+// same row; B does not allocate there).  Narrower rows add up in
+// two sums a lane, from 33 columns in four: no larger an error than k_sddmm's 16
+// sums (rms over 10^6 entries, 16, 32 and
+// 48 columns: 3.93, 3.26 and 2.77e-17 for 4.09, 3.26 and 2.84e-17 of sum |a||b|).
 // rowidx: the row of each nonzero.
-constexpr int SD_WARP = 64;
+// Measured: 64 columns, 2^18 rows x 16, 0.50 ms at 3 or 4 blocks an SM, 0.55 at 2,
+// 0.56 with A staged in shared memory by blocks of 64 nonzeros.  k_sddmm / this, us,
+// 2^20 rows x 16: 1 column 4129 / 288, 4 3966 / 346, 8 3968 / 544, 16 3968 / 702, 32
+// 3966 / 1135, 33 3966 / 2309, 48 3965 / 1861, 63 3966 / 2453, 66 5971 / 2810, 96 5761 /
+// 3756, 128 5760 / 4925; 2^17 rows: 193 1256 / 1089, 200 1205 / 981, 256 1203 / 1255,
+// 512 2116 / 2564: past SD_FLAT_COLS its parts' indexes and sums cost more than
+// k_sddmm's tree.
+constexpr int SD_WARP = 64, SD_FLAT_COLS = 200;
 __device__ __forceinline__ double2 ld_nc_stream(const double2* p) {
     double2 v;
     asm volatile("ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
     return v;
 }
+__device__ __forceinline__ double ld_nc_stream(const double* p) {
+    double v;
+    asm volatile("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+template <int U, bool PAIRS>
 __global__ void __launch_bounds__(256, 4)
-    k_sddmm64(int64_t nnz, const int* __restrict__ rowidx, const int* __restrict__ colidx,
-              const double* __restrict__ A, const double* __restrict__ B, double* __restrict__ out) {
+    k_sddmm_flat(int64_t nnz, int ncols, int64_t ld, bool add, const int* __restrict__ rowidx,
+                 const int* __restrict__ colidx, const double* __restrict__ A, const double* __restrict__ B,
+                 double* __restrict__ out) {
+    using V = typename std::conditional<PAIRS, double2, double>::type;
+    constexpr bool WHOLE = PAIRS && U == 8;  // 64 columns, no unit left over (the launch sees to it)
+    constexpr int SUMS = WHOLE || (!PAIRS && U == 1) ? 1 : (U > (PAIRS ? 4 : 8) ? 4 : 2);
     const int lane = threadIdx.x % 32, g = lane >> 2, l4 = lane & 3;
+    const int units = WHOLE ? 32 : (PAIRS ? ncols / 2 : ncols);
     const int64_t w0 = ((int64_t)blockIdx.x * 8 + threadIdx.x / 32) * SD_WARP;
     if (w0 >= nnz) return;
     auto at = [&](int step) {  // past the end: the last nonzero again, not stored
         const int64_t q = w0 + step * 8 + g;
         return q < nnz ? q : nnz - 1;
     };
-    auto row_of = [&](const double* X, int i) { return reinterpret_cast<const double2*>(X + (int64_t)i * 64) + l4; };
-    const double2* arow = row_of(A, __ldg(rowidx + at(0)));
-    const double2* brow = row_of(B, __ldg(colidx + at(0)));
+    auto row_of = [&](const double* X, int64_t i) {
+        return reinterpret_cast<const V*>(X + i * ld) + l4;
+    };
+    auto mine = [&](int u) { return WHOLE || 4 * u + l4 < units; };
+    const V* arow = row_of(A, __ldg(rowidx + at(0)));
+    const V* brow = row_of(B, __ldg(colidx + at(0)));
     int rn = __ldg(rowidx + at(1)), cn = __ldg(colidx + at(1));
-    double2 b[8];
+    V b[U];
 #pragma unroll
-    for (int u = 0; u < 8; u++) b[u] = ld_nc_stream(brow + 4 * u);
+    for (int u = 0; u < U; u++) b[u] = mine(u) ? ld_nc_stream(brow + 4 * u) : V{};
 #pragma unroll 1
     for (int s0 = 0; s0 < SD_WARP / 8; s0 += 4) {
         double p[4];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const int step = s0 + j;
-            const double2* an = row_of(A, rn);
+            const V* an = row_of(A, rn);
             brow = row_of(B, cn);
             if (step + 2 < SD_WARP / 8) {
                 rn = __ldg(rowidx + at(step + 2));
                 cn = __ldg(colidx + at(step + 2));
             }
-            double s = 0.0;
+            double s[SUMS] = {};
 #pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const double2 a = __ldg(arow + 4 * u);
-                s = fma(a.y, b[u].y, fma(a.x, b[u].x, s));
-                if (step + 1 < SD_WARP / 8) b[u] = ld_nc_stream(brow + 4 * u);
+            for (int u = 0; u < U; u++) {
+                const V a = mine(u) ? __ldg(arow + 4 * u) : V{};
+                if constexpr (PAIRS) {
+                    double &x = s[2 * u % SUMS], &y = s[(2 * u + 1) % SUMS];
+                    x = fma(a.x, b[u].x, x);
+                    y = fma(a.y, b[u].y, y);
+                } else {
+                    double& x = s[u % SUMS];
+                    x = fma(a, b[u], x);
+                }
+                if (step + 1 < SD_WARP / 8 && mine(u)) b[u] = ld_nc_stream(brow + 4 * u);
             }
-            p[j] = s;
+            p[j] = s[0];
+            if constexpr (SUMS == 2) p[j] = s[0] + s[1];
+            if constexpr (SUMS == 4) p[j] = (s[0] + s[1]) + (s[2] + s[3]);
             arow = an;
         }
         // four sums of four lanes: lane l4 ends with the nonzero of step s0 + l4
@@ -357,7 +390,7 @@ __global__ void __launch_bounds__(256, 4)
         const double t0 = (h2 ? p[2] : p[0]) + u0, t1 = (h2 ? p[3] : p[1]) + u1;
         const double r = (h1 ? t1 : t0) + __shfl_xor_sync(0xffffffffu, h1 ? t0 : t1, 1);
         const int64_t q = w0 + (s0 + l4) * 8 + g;
-        if (q < nnz) out[q] = r;
+        if (q < nnz) out[q] = add ? out[q] + r : r;
     }
 }
 
@@ -2145,16 +2178,42 @@ extern "C" int f4j_sddmm(f4j_ctx* ctx, f4j_csr S, f4j_buf A, f4j_buf B, int64_t 
     int64_t l0 = ctx->launches;
     if (S->rows && S->nnz) {
         f4j_prof_begin(ctx);
-        if (ncols == 64 && ((reinterpret_cast<uintptr_t>(A->ptr) | reinterpret_cast<uintptr_t>(B->ptr)) & 15) == 0) {
-            int rc = ensure_rowidx(ctx, S);
-            if (rc) return rc;
-            k_sddmm64<<<(unsigned)f4j_cdiv(S->nnz, 8 * SD_WARP), 256, 0, ctx->stream>>>(
-                S->nnz, (const int*)S->rowidx, (const int*)S->colidx->ptr, (const double*)A->ptr,
-                (const double*)B->ptr, (double*)out->ptr);
-        } else
+        // no room for the row of each nonzero: k_sddmm, which needs none
+        int rc = ncols >= 1 && ncols <= SD_FLAT_COLS ? ensure_rowidx(ctx, S) : F4J_ERR_OOM;
+        if (rc && rc != F4J_ERR_OOM) return rc;
+        if (rc == F4J_OK) {
+            using Kernel = void (*)(int64_t, int, int64_t, bool, const int*, const int*, const double*, const double*,
+                                    double*);
+            static const Kernel pairs[8] = {k_sddmm_flat<1, true>, k_sddmm_flat<2, true>, k_sddmm_flat<3, true>,
+                                            k_sddmm_flat<4, true>, k_sddmm_flat<5, true>, k_sddmm_flat<6, true>,
+                                            k_sddmm_flat<7, true>, k_sddmm_flat<8, true>};
+            static const Kernel ones[5] = {k_sddmm_flat<1, false>, k_sddmm_flat<2, false>, k_sddmm_flat<4, false>,
+                                           k_sddmm_flat<8, false>, k_sddmm_flat<16, false>};
+            const double *a = (const double*)A->ptr, *b = (const double*)B->ptr;
+            const bool even = ncols % 2 == 0 && f4j_aligned16(a) && f4j_aligned16(b);
+            // more than 64 columns: equal parts of at most 56, whose sums k_sddmm_flat
+            // keeps in four, added up in order
+            const int64_t part = ncols <= 64 ? 64 : f4j_cdiv(f4j_cdiv(ncols, f4j_cdiv(ncols, 56)), 8) * 8;
+            for (int64_t c0 = 0; c0 < ncols; c0 += part) {
+                const int w = (int)(ncols - c0 < part ? ncols - c0 : part);
+                Kernel k;
+                if (even && w > 4 && (w <= 56 || w == 64)) {  // up to four columns: a lane's pair leaves lanes idle
+                    k = pairs[(w + 7) / 8 - 1];
+                } else {
+                    int i = 0;
+                    while ((4 << i) < w) i++;
+                    k = ones[i];
+                }
+                k<<<(unsigned)f4j_cdiv(S->nnz, 8 * SD_WARP), 256, 0, ctx->stream>>>(
+                    S->nnz, w, ncols, c0 > 0, (const int*)S->rowidx, (const int*)S->colidx->ptr, a + c0, b + c0,
+                    (double*)out->ptr);
+                if (c0 + part < ncols) ctx->launches++;
+            }
+        } else {
             k_sddmm<<<(unsigned)f4j_cdiv(S->rows * 32, 256), 256, 0, ctx->stream>>>(
                 S->rows, ncols, (const int*)S->rowptr->ptr, (const int*)S->colidx->ptr, (const double*)A->ptr,
                 (const double*)B->ptr, (double*)out->ptr);
+        }
         f4j_prof_end(ctx);
         F4J_LAUNCHED(ctx);
     }

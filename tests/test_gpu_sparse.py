@@ -710,3 +710,24 @@ def test_sddmm_64_columns_at_the_edges_of_a_warp(f4j, nnz):
     got = out.to_numpy(np.float64, nnz)
     terms = A[row].astype(np.longdouble) * B[col].astype(np.longdouble)
     assert np.all(np.abs(got - terms.sum(1)) <= 2 * 64 * U * np.abs(terms).sum(1))
+
+
+@pytest.mark.parametrize("ncols", [1, 2, 3, 4, 6, 8, 9, 16, 17, 24, 32, 33, 40, 48, 56, 58, 63, 66, 96, 129, 200, 201])
+def test_sddmm_every_width(f4j, ncols):
+    """dS for every width of a lane's share, the parts of wide rows and the first width past them: within 2
+    ncols u sum|a||b|."""
+    from flag4j_gb300.device import check
+    g = np.random.default_rng(ncols)
+    rows, cols, nnz = 37, 500, 1003
+    row = np.sort(g.integers(0, rows, nnz))
+    col = np.concatenate([np.sort(g.choice(cols, n, replace=False)) for n in np.bincount(row, minlength=rows)])
+    rp = np.zeros(rows + 1, np.int32)
+    np.cumsum(np.bincount(row, minlength=rows), out=rp[1:])
+    S = f4j.CsrMatrix((rows, cols), np.ones(nnz), rp, col.astype(np.int32))
+    A, B = g.standard_normal((rows, ncols)), g.standard_normal((cols, ncols))
+    ctx = f4j.default_context()
+    terms = A[row].astype(np.longdouble) * B[col].astype(np.longdouble)
+    dA, dB, out = ctx.from_numpy(A), ctx.from_numpy(B), ctx.alloc(8 * nnz)
+    check(ctx.lib.f4j_sddmm(ctx.handle, S.handle(ctx), dA.handle, dB.handle, ncols, out.handle, None))
+    got = out.to_numpy(np.float64, nnz)
+    assert np.all(np.abs(got - terms.sum(1)) <= 2 * ncols * U * np.abs(terms).sum(1))
