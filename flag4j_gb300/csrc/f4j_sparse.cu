@@ -155,14 +155,20 @@ __global__ void __launch_bounds__(SPMV_BLOCK, SPMV_BLOCKS)
 // warp against warps.  Exact mode at 2^20 rows x 16 nonzeros, 32 columns: 1.79
 // ms, 95 % of the FP64 pipe's two lanes per SM and clock (2.07 ms with DMUL
 // and DADD for ExactOps); 64 columns 3.54 ms (4.02), 5 columns .82 ms (.93).
-template <bool VEC2, bool PERM, bool FUSED = false>
-__global__ void __launch_bounds__(256, FUSED ? 8 : 6)
+// MIXED (exact mode, rows of different lengths in a warp): every group of eight
+// nonzeros under predicates, its sums in pairs that the warp leaves together, so
+// a warp takes its longest row's FP64 instructions, where whole groups and a
+// loop over the rest took the most of both: 2^20 rows x 16, us, 2 columns 228 / 191, 8
+// 819 / 626, 16 1326 / 1092.  5 blocks an SM (48 registers; 6 spill, 2 % slower).
+// With one row a warp the predicated rest costs more than the loop (32 columns
+// 1792 / 2225, without the pairs).
+template <bool VEC2, bool PERM, bool FUSED = false, bool MIXED = false>
+__global__ void __launch_bounds__(256, FUSED ? 8 : (MIXED ? 5 : 6))
     k_spmm(int64_t rows, int64_t ncols, int G, const int* __restrict__ rowptr, const int* __restrict__ colidx,
            const double* __restrict__ vals, const int* __restrict__ perm, const double* __restrict__ X,
            double* __restrict__ Y) {
-    const int64_t gid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
-    const int lane = threadIdx.x % G;
-    const int64_t row = gid;
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, row = t / G;
+    const int lane = (int)(t - row * G);
     if (row >= rows) return;
     const ExactOps ops;
     const int q0 = rowptr[row], q1 = rowptr[row + 1];
@@ -171,6 +177,27 @@ __global__ void __launch_bounds__(256, FUSED ? 8 : 6)
         double a0 = 0.0, a1 = 0.0;
         int q = q0;
         constexpr int UN = 8;  // nonzeros whose X rows are in flight together
+        if constexpr (MIXED) {
+            for (; q < q1; q += UN) {
+                double v[UN], xv[UN];
+#pragma unroll
+                for (int u = 0; u < UN; u++) {
+                    v[u] = xv[u] = 0.0;
+                    if (q + u < q1) {
+                        v[u] = PERM ? __ldg(&vals[__ldg(&perm[q + u])]) : __ldg(&vals[q + u]);
+                        xv[u] = __ldg(X + (int64_t)__ldg(&colidx[q + u]) * ncols + cbase);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < UN; u += 2) {
+                    if (q + u >= q1) break;
+                    a0 = ops.add(ops.mul(v[u], xv[u]), a0);
+                    if (q + u + 1 < q1) a0 = ops.add(ops.mul(v[u + 1], xv[u + 1]), a0);
+                }
+            }
+            Y[row * ncols + cbase] = a0;
+            continue;
+        }
         for (; q + UN <= q1; q += UN) {
             int c[UN];
             double v[UN];
@@ -1448,16 +1475,30 @@ static int ensure_rowidx(f4j_ctx* ctx, f4j_csr S) {
     return F4J_OK;
 }
 
-static int launch_spmm(f4j_ctx* ctx, int64_t rows, int64_t ncols, const int* rp, const int* ci, const double* v,
-                       const int* perm, const double* X, double* Y, bool fused = false) {
+static int launch_spmm(f4j_ctx* ctx, int64_t rows, int64_t nnz, int64_t ncols, const int* rp, const int* ci,
+                       const double* v, const int* perm, const double* X, double* Y, bool fused = false) {
     if (rows == 0 || ncols == 0) return F4J_OK;
-    // one row per warp from 17 columns on (the FP64 instructions of a warp then
-    // never wait on a second row of another length); 128-bit X loads only
-    // where a warp of 2-column lanes is still needed for the width
-    const bool vec2 = ncols > 32 && (ncols % 2 == 0) && f4j_aligned16(X) && f4j_aligned16(Y);
-    const int64_t per_lane = vec2 ? 2 : 1;
-    int G = 1;
-    while (G < 32 && G * per_lane < ncols) G *= 2;
+    // Lanes of a row: a power of two up to a warp, two columns a lane (128-bit X
+    // loads) above 32 columns, or one lane a column, rows straddling warps, where
+    // that power of two (64 columns a pass) would leave too many lanes idle.  2^20 rows
+    // x 16, us, power of two / a lane a column: exact mode 5 columns 625 / 416, 9 1119 /
+    // 691, 15 1121 / 1115, 17 1792 / 1246, 24 1792 / 1628, 28 1793 / 1943, 33 3562 / 2217, 48
+    // 3538 / 2997, 52 3536 / 3405, 56 3538 / 3617, 72 7054 / 4486, 112 7054 / 6964; FMA mode
+    // 5 423 / 284, 13 683 / 655, 15 685 / 738, 17 927 / 812, 20 931 / 899, 22 935 / 984, 33
+    // 1820 / 1370, 48 1807 / 1621, 52 1808 / 1887, 96 3591 / 2812.  Rows of mostly less
+    // than two nonzeros (the transpose of a wide matrix) are writes of zeros, for
+    // which more lanes and predicates are only work: S^T of 19026 x 593791 x 6, 76
+    // columns, with its SDDMM 201 / 352.
+    const bool filled = nnz >= 2 * rows;
+    int64_t lanes = 1;  // what the first form occupies
+    while (lanes < 32 && lanes < ncols) lanes *= 2;
+    if (ncols > 32) lanes = f4j_cdiv(ncols, 64) * 64;
+    const bool flat = filled &&
+                      (fused ? ncols <= 14 || (ncols <= 32 ? ncols * 8 <= lanes * 5 : ncols * 4 <= lanes * 3)
+                             : ncols <= 16 || ncols * 4 <= lanes * 3) &&
+                      f4j_cdiv(rows * ncols, 256) <= INT32_MAX;
+    const bool vec2 = !flat && ncols > 32 && (ncols % 2 == 0) && f4j_aligned16(X) && f4j_aligned16(Y);
+    const int G = (int)(flat ? ncols : (lanes < 32 ? lanes : 32));
     const int64_t threads = rows * G;
     const unsigned blocks = (unsigned)f4j_cdiv(threads, 256);
     f4j_prof_begin(ctx);
@@ -1469,7 +1510,10 @@ static int launch_spmm(f4j_ctx* ctx, int64_t rows, int64_t ncols, const int* rp,
         if (perm) k_spmm<true, true><<<blocks, 256, 0, ctx->stream>>>(rows, ncols, G, rp, ci, v, perm, X, Y);
         else k_spmm<true, false><<<blocks, 256, 0, ctx->stream>>>(rows, ncols, G, rp, ci, v, perm, X, Y);
     } else {
-        if (perm) k_spmm<false, true><<<blocks, 256, 0, ctx->stream>>>(rows, ncols, G, rp, ci, v, perm, X, Y);
+        if (filled && G % 32) {  // a warp holds rows of different lengths
+            if (perm) k_spmm<false, true, false, true><<<blocks, 256, 0, ctx->stream>>>(rows, ncols, G, rp, ci, v, perm, X, Y);
+            else k_spmm<false, false, false, true><<<blocks, 256, 0, ctx->stream>>>(rows, ncols, G, rp, ci, v, perm, X, Y);
+        } else if (perm) k_spmm<false, true><<<blocks, 256, 0, ctx->stream>>>(rows, ncols, G, rp, ci, v, perm, X, Y);
         else k_spmm<false, false><<<blocks, 256, 0, ctx->stream>>>(rows, ncols, G, rp, ci, v, perm, X, Y);
     }
     f4j_prof_end(ctx);
@@ -2092,7 +2136,7 @@ extern "C" int f4j_spmm_ex(f4j_ctx* ctx, f4j_csr S, f4j_buf X, int64_t ncols, f4
     if (!f4j_aligned(X->ptr, 8) || !f4j_aligned(Y->ptr, 8)) return f4j_fail(F4J_ERR_ARG, "X and Y must be 8-byte aligned");
     F4J_CUDA(cudaSetDevice(ctx->device));
     int64_t l0 = ctx->launches;
-    int rc = launch_spmm(ctx, S->rows, ncols, (const int*)S->rowptr->ptr, (const int*)S->colidx->ptr,
+    int rc = launch_spmm(ctx, S->rows, S->nnz, ncols, (const int*)S->rowptr->ptr, (const int*)S->colidx->ptr,
                          (const double*)S->vals->ptr, nullptr, (const double*)X->ptr, (double*)Y->ptr,
                          mode == F4J_SPARSE_FMA);
     if (rc) return rc;
@@ -2153,7 +2197,7 @@ extern "C" int f4j_spmm_t(f4j_ctx* ctx, f4j_csr S, f4j_buf dC, int64_t ncols, f4
     int64_t l0 = ctx->launches;
     int rc = ensure_transpose(ctx, S);
     if (rc) return rc;
-    rc = launch_spmm(ctx, S->cols, ncols, (const int*)S->t_rowptr, (const int*)S->t_rowidx,
+    rc = launch_spmm(ctx, S->cols, S->nnz, ncols, (const int*)S->t_rowptr, (const int*)S->t_rowidx,
                      (const double*)S->vals->ptr, (const int*)S->t_perm, (const double*)dC->ptr, (double*)dX->ptr);
     if (rc) return rc;
     if (rep) {

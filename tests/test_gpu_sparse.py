@@ -731,3 +731,25 @@ def test_sddmm_every_width(f4j, ncols):
     check(ctx.lib.f4j_sddmm(ctx.handle, S.handle(ctx), dA.handle, dB.handle, ncols, out.handle, None))
     got = out.to_numpy(np.float64, nnz)
     assert np.all(np.abs(got - terms.sum(1)) <= 2 * ncols * U * np.abs(terms).sum(1))
+
+
+@pytest.mark.parametrize("ncols", [1, 2, 3, 5, 8, 9, 13, 14, 15, 16, 17, 20, 21, 24, 25, 33, 48, 49, 53, 65, 96, 97,
+                                   102, 103, 129, 200])
+def test_spmm_every_width_bit_identical(f4j, oracle, ncols):
+    """S X and S^T X (exact mode bit for bit, FMA mode within its bound) at widths on both sides of every rule
+    for a row's lanes, on rows of very different lengths, empty ones among them."""
+    g = np.random.default_rng(ncols)
+    for rows, cols in ((211, 300), (211, 9000)):  # S^T with several and with less than two nonzeros a row
+        lens = np.minimum(g.pareto(0.8, rows).astype(np.int64) * 3, 300)
+        lens[::7] = 0
+        rp = np.zeros(rows + 1, np.int32)
+        np.cumsum(lens, out=rp[1:])
+        ci = np.concatenate([np.sort(g.choice(cols, n, replace=False)) for n in lens]).astype(np.int32)
+        v, X, W = g.standard_normal(len(ci)), g.standard_normal((cols, ncols)), g.standard_normal((rows, ncols))
+        S = f4j.CsrMatrix((rows, cols), v, rp, ci)
+        ref = oracle.spmm(rp, ci, v, X)
+        assert np.array_equal(S.mult(f4j.Matrix(X)).toNumpy(), ref)
+        fma = S.mult(f4j.Matrix(X), mode="fma").toNumpy()
+        assert np.all(np.abs(fma - ref) <= fma_bound(oracle, rp, ci, v, X))
+        trp, tci, tv, _ = oracle.csr_transpose(rows, cols, rp, ci, v)
+        assert np.array_equal(S.multTransposeLeft(f4j.Matrix(W)).toNumpy(), oracle.spmm(trp, tci, tv, W))
