@@ -143,8 +143,9 @@ __global__ void __launch_bounds__(SPMV_BLOCK, SPMV_BLOCKS)
 }
 
 // ------------------------------------------------------------------ SpMM
-// A group of G lanes owns one row; each lane owns 2 adjacent columns
-// (128-bit loads of X rows) and sums over the row's nonzeros in storage order.
+// A group of G lanes owns one row; each lane owns a column, or two adjacent ones
+// (VEC2: 128-bit loads of X rows), and sums over the row's nonzeros in storage
+// order.  G need not divide a warp (launch_spmm).
 // For S^T products the same kernel reads values through the transpose
 // permutation and row indices from the cached S^T structure.
 // FUSED (the opt-in FMA mode): one fma(v, x, acc) per nonzero and column, in
@@ -154,7 +155,7 @@ __global__ void __launch_bounds__(SPMV_BLOCK, SPMV_BLOCKS)
 // exact mode runs 6 (40 registers), its best balance of loads in flight per
 // warp against warps.  Exact mode at 2^20 rows x 16 nonzeros, 32 columns: 1.79
 // ms, 95 % of the FP64 pipe's two lanes per SM and clock (2.07 ms with DMUL
-// and DADD for ExactOps); 64 columns 3.54 ms (4.02), 5 columns .82 ms (.93).
+// and DADD for ExactOps); 64 columns 3.54 ms (4.02).
 // MIXED (exact mode, rows of different lengths in a warp): every group of eight
 // nonzeros under predicates, its sums in pairs that the warp leaves together, so
 // a warp takes its longest row's FP64 instructions, where whole groups and a

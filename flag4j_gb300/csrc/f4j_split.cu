@@ -1,6 +1,8 @@
 // f4j_split.cu -- FP64-accurate split-precision GEMM on tcgen05 FP8 tensor cores.
 //
-// Scheme (Ozaki-style error-free slicing):
+// Two forms of one fixed-point product: residues modulo small coprime numbers
+// (f4j_crt.cuh, included below; most products, crt_wanted) and slices.  The slice
+// form (Ozaki-style error-free slicing):
 //  1. k_stats_*: per row of op(A) and per column of op(B), the power-of-two
 //     bound 2^e > max|x| and the exponent spread (bits between the largest and
 //     the mean element exponent).  The host picks the slice count s from the
@@ -1844,8 +1846,8 @@ static void host_part_bounds(int tiles_m, int parts, int* bound, int first = 8) 
 // (f4j_dgemm_host / f4j_zgemm_host, op(A) = N).  The uploads go back to back
 // on their own stream: A's first row part, then B in column parts (complex: B
 // whole, since a column part of B lands in both halves of the [Re | Im]
-// concatenation), then the rest of A in row parts.  Each part's statistics and slicing run on the context stream as
-// soon as it is up; each column part of B is then multiplied by A's first
+// concatenation), then the rest of A in row parts.  Each part's statistics and
+// slicing (crt: residue planes) run on the context stream as soon as it is up; each column part of B is then multiplied by A's first
 // rows, and each later row part of A by all of B.  Every product is one launch
 // on its own stream, its block of C going down behind it.  The slice count
 // cannot wait for all of A and B, so it is picked from A's first rows and B's
