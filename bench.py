@@ -914,7 +914,7 @@ def run_sddmm_only(args):
     A, B, o = E.dev(synth.normal(rows, 64, 9)), E.dev(synth.normal(rows, 64, 8)), E.ctx.alloc(8 * len(v))
     ms = E.timed(lambda: E.check(E.lib.f4j_sddmm(E.ctx.handle, hS, A.handle, B.handle, 64, o.handle, None)),
                  args.steps, args.warmup)
-    print(json.dumps({"kernel": "k_sddmm64s", "rows": rows, "nnz": len(v), "ms": ms,
+    print(json.dumps({"kernel": "k_sddmm_flat", "rows": rows, "nnz": len(v), "ms": ms,
                       "fp64_lane_ops_per_s": 64.0 * len(v) / (ms * 1e-3)}))
     del S
 
