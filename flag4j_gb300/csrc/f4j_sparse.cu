@@ -2223,8 +2223,12 @@ extern "C" int f4j_sddmm(f4j_ctx* ctx, f4j_csr S, f4j_buf A, f4j_buf B, int64_t 
     int64_t l0 = ctx->launches;
     if (S->rows && S->nnz) {
         f4j_prof_begin(ctx);
-        // no room for the row of each nonzero: k_sddmm, which needs none
-        int rc = ncols >= 1 && ncols <= SD_FLAT_COLS ? ensure_rowidx(ctx, S) : F4J_ERR_OOM;
+        // no room for the row of each nonzero, or a stream capture, which an allocation
+        // kept in the handle must not be part of: k_sddmm, which needs none
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (!S->rowidx && ncols != 64) F4J_CUDA(cudaStreamIsCapturing(ctx->stream, &cap));
+        int rc = ncols >= 1 && ncols <= SD_FLAT_COLS && cap == cudaStreamCaptureStatusNone ? ensure_rowidx(ctx, S)
+                                                                                          : F4J_ERR_OOM;
         if (rc && rc != F4J_ERR_OOM) return rc;
         if (rc == F4J_OK) {
             using Kernel = void (*)(int64_t, int, int64_t, bool, const int*, const int*, const double*, const double*,
