@@ -120,7 +120,6 @@ extern "C" int f4j_destroy(f4j_ctx* ctx) {
         if (ctx->ws[i]) cudaFree(ctx->ws[i]);
     for (int i = 0; i < 2; i++)
         if (ctx->plan_tab[i]) cudaFree(ctx->plan_tab[i]);
-    if (ctx->crt_tab) cudaFree(ctx->crt_tab);
     if (ctx->d_status) cudaFree(ctx->d_status);
     if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
     lock.unlock();

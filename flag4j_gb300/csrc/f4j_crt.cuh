@@ -81,13 +81,11 @@ __constant__ CrtMods c_crt{};
 
 // One configuration: which moduli, and the constants of the reconstruction.
 struct CrtCfg {
-    int nmod, nsq;   // moduli; the first nsq are squares
-    int cost;        // FP8 products: nmod + 2 nsq
+    int nmod, nsq;   // moduli; the first nsq are squares (nmod + 2 nsq FP8 products)
     int words;       // words of the reconstruction: 4 while M < 2^127, else 5
     float bits;      // log2 M
     int sh;          // the words below hold 2^sh times their number: 2^sh M in [2^(32 words - 2), 2^(32 words - 1))
     float qinv;      // 2^(32 words - 18) / (2^sh M), for the quotient by M
-    int pad;
     float p[CRT_NB], invp[CRT_NB], u[CRT_NB];  // modulus, 1 / p, (M / p)^-1 mod p (balanced)
     int32_t c[CRT_NB];                         // P / p, P the product of the group's moduli
     int32_t z0[CRT_NG];                        // 2 P: makes a group's sum positive, and vanishes modulo M
@@ -95,6 +93,108 @@ struct CrtCfg {
     uint32_t NM[CRT_WORDS];                    // 2^(32 words) - M
 };
 __host__ __device__ constexpr int crt_group(int l) { return l / 2 < CRT_NG ? l / 2 : CRT_NG - 1; }
+
+// Every configuration worth having, by rising cost in FP8 products: squares of the
+// first nsq bases, the last `drop` bases left out.  Built by the compiler, for the
+// host and as a constant of the device code: no kernel can meet it half written, and
+// no product's first call allocates or copies for it.  Exact arithmetic on 32-bit
+// words: M and M / P are products of the other moduli.
+struct CrtTable {
+    CrtCfg cfg[CRT_CFGS] = {};
+    int n = 0;
+
+    static constexpr void mul(uint32_t (&a)[CRT_WORDS], uint32_t m) {
+        uint64_t carry = 0;
+        for (int j = 0; j < CRT_WORDS; j++) {
+            const uint64_t t = (uint64_t)a[j] * m + carry;
+            a[j] = (uint32_t)t;
+            carry = t >> 32;
+        }
+    }
+    // log2 x, x >= 1: the integer part by halving, the rest as 2 / ln 2 times the
+    // series of artanh at (f - 1) / (f + 1) <= 1/3
+    static constexpr double log2_of(double x) {
+        int e = 0;
+        while (x >= 2.0) x *= 0.5, e++;
+        const double t = (x - 1.0) / (x + 1.0);
+        double sum = 0, pw = t;
+        for (int i = 1; i < 40; i += 2, pw *= t * t) sum += pw / i;
+        return e + 2.0 * 1.44269504088896340736 * sum;
+    }
+    static constexpr int inverse(int r, int p) {  // r^-1 mod p, coprime
+        int a = r % p, b = p, u = 1, v = 0;
+        while (a > 1) {
+            const int q = b / a, b1 = b - q * a, v1 = v - q * u;
+            b = a, a = b1, v = u, u = v1;
+        }
+        return u < 0 ? u + p : u;
+    }
+
+    constexpr CrtTable() {
+        double best = 0;
+        for (int cost = 9; cost <= 3 * CRT_NB; cost++) {
+            int bj = -1, bd = 0;
+            double bbits = 0;
+            for (int d = 0; d <= 6; d++) {
+                const int nmod = CRT_NB - d, j2 = cost - nmod;
+                if (j2 < 0 || j2 % 2 || j2 / 2 > nmod) continue;
+                double bits = 0;
+                for (int i = 0; i < nmod; i++) bits += (i < j2 / 2 ? 2 : 1) * log2_of(crt_base(i));
+                if (bits > bbits) bbits = bits, bj = j2 / 2, bd = d;
+            }
+            if (bj < 0 || bbits <= best || n >= CRT_CFGS) continue;
+            best = bbits;
+            fill(cfg[n++], CRT_NB - bd, bj, bbits);
+        }
+    }
+    static constexpr void fill(CrtCfg& c, int nmod, int nsq, double bits) {
+        c.nmod = nmod;
+        c.nsq = nsq;
+        c.bits = (float)bits;
+        c.words = bits < 127.0 ? 4 : 5;
+        int p[CRT_NB] = {};
+        for (int l = 0; l < nmod; l++) p[l] = l < nsq ? crt_base(l) * crt_base(l) : crt_base(l);
+        uint32_t M[CRT_WORDS] = {1};
+        for (int l = 0; l < nmod; l++) {
+            mul(M, (uint32_t)p[l]);
+            int r = 1, cl = 1;
+            for (int i = 0; i < nmod; i++) {
+                if (i == l) continue;
+                r = (int)((int64_t)r * p[i] % p[l]);  // M / p mod p
+                if (crt_group(i) == crt_group(l)) cl *= p[i];
+            }
+            const int inv = inverse(r, p[l]);
+            c.p[l] = (float)p[l];
+            c.invp[l] = 1.0f / (float)p[l];
+            c.u[l] = (float)(2 * inv > p[l] ? inv - p[l] : inv);
+            c.c[l] = cl;
+        }
+        c.sh = 0;
+        while (!(M[c.words - 1] >> 30)) mul(M, 2), c.sh++;
+        uint64_t borrow = 1;  // two's complement over `words` words
+        double frac = 0;      // 2^sh M / 2^(32 words)
+        for (int j = 0; j < c.words; j++) {
+            const uint64_t t = (uint64_t)(uint32_t)~M[j] + borrow;
+            c.NM[j] = (uint32_t)t;
+            borrow = t >> 32;
+            frac = (frac + M[j]) / 4294967296.0;
+        }
+        c.qinv = (float)(1.0 / 262144.0 / frac);  // 2^-18 / frac
+        for (int g = 0; 2 * g < nmod && g < CRT_NG; g++) {  // without a modulus: z stays 0
+            uint32_t W[CRT_WORDS] = {1};
+            int P = 1;
+            for (int i = 0; i < nmod; i++) {
+                if (crt_group(i) == g) P *= p[i];
+                else mul(W, (uint32_t)p[i]);
+            }
+            for (int i = 0; i < c.sh; i++) mul(W, 2);
+            c.z0[g] = 2 * P;
+            for (int j = 0; j < CRT_WORDS; j++) c.W[g][j] = W[j];
+        }
+    }
+};
+constexpr CrtTable crt_host{};
+__device__ const CrtTable crt_dev{};
 
 constexpr float CRT_MAGIC = 12582912.0f;  // 1.5 * 2^23: x + CRT_MAGIC rounds |x| < 2^22 to an integer
 
@@ -322,14 +422,14 @@ __device__ __forceinline__ void crt_planes_body(const CrtOperand& o, int64_t kle
 // rolled loop); its 4.2 GB take 0.62.
 template <bool CPLX>
 __global__ void __launch_bounds__(256, 4) k_crt_planes(const CrtOperand a, const CrtOperand b, int64_t klen,
-                                                       int64_t Kh, int64_t Kp, const SplitPlan* __restrict__ plan,
-                                                       const CrtCfg* __restrict__ cfgs) {
+                                                       int64_t Kh, int64_t Kp,
+                                                       const SplitPlan* __restrict__ plan) {
     __shared__ double sre[SP_TR][SP_TQ + 1];
     __shared__ double sim[CPLX ? SP_TR : 1][SP_TQ + 1];
     chain_wait();
     chain_trigger();
     if (plan->nonfinite) return;
-    const int s = plan->s, nmod = cfgs[plan->crt].nmod, nsq = cfgs[plan->crt].nsq;
+    const int s = plan->s, nmod = crt_dev.cfg[plan->crt].nmod, nsq = crt_dev.cfg[plan->crt].nsq;
     if (blockIdx.z == 0) crt_planes_body<CPLX>(a, klen, Kh, Kp, s, nmod, nsq, sre, sim);
     else crt_planes_body<CPLX>(b, klen, Kh, Kp, s, nmod, nsq, sre, sim);
 }
@@ -355,7 +455,6 @@ struct CrtGemmParams {
     int16_t* y;             // [nmod][rows][ldy]
     int* status;
     const SplitPlan* plan;
-    const CrtCfg* cfgs;
 };
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -535,7 +634,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) __cluster_dims__(2, 1, 1)
     chain_trigger();
     // nonfinite: the gated plain path computes this product
     const bool off = p.plan->nonfinite != 0;
-    const CrtCfg* __restrict__ cfg = p.cfgs + (off ? 0 : p.plan->crt);
+    const CrtCfg* __restrict__ cfg = crt_dev.cfg + (off ? 0 : p.plan->crt);
     const int nmod = cfg->nmod, nsq = cfg->nsq;
     const int nunits = off ? 0 : ntiles * nmod;
 
@@ -878,7 +977,6 @@ struct CrtCombineParams {
     const int* eb;
     double* C;
     const SplitPlan* plan;
-    const CrtCfg* cfgs;
 };
 
 // Two adjacent entries of C (X: exponent of the row's unit, eb: the columns').
@@ -962,7 +1060,7 @@ __global__ void __launch_bounds__(256, 4) k_crt_combine(const __grid_constant__ 
     chain_trigger();
     if (p.plan->nonfinite) return;
     {
-        const int* src = reinterpret_cast<const int*>(p.cfgs + p.plan->crt);
+        const int* src = reinterpret_cast<const int*>(crt_dev.cfg + p.plan->crt);
         for (int i = threadIdx.y * blockDim.x + threadIdx.x; i < (int)(sizeof(CrtCfg) / 4); i += 256)
             reinterpret_cast<int*>(&c)[i] = src[i];
     }
@@ -978,95 +1076,10 @@ __global__ void __launch_bounds__(256, 4) k_crt_combine(const __grid_constant__ 
 }
 
 // ------------------------------------------------------------------ host side
-// Every configuration worth having, by rising cost: squares of the first nsq
-// bases, the last `drop` bases left out.  Exact arithmetic on 32-bit words: M
-// and M / P are products of the other moduli.
-struct CrtTable {
-    CrtCfg cfg[CRT_CFGS];
-    int n = 0;
-};
-
-static void crt_words_mul(uint32_t (&a)[CRT_WORDS], uint32_t m) {
-    uint64_t carry = 0;
-    for (int j = 0; j < CRT_WORDS; j++) {
-        const uint64_t t = (uint64_t)a[j] * m + carry;
-        a[j] = (uint32_t)t;
-        carry = t >> 32;
-    }
-}
-
-static const CrtTable& crt_table() {
-    static const CrtTable table = [] {
-        CrtTable T;
-        float best = 0;
-        for (int cost = 9; cost <= 3 * CRT_NB; cost++) {
-            int bj = -1, bd = 0;
-            double bbits = 0;
-            for (int d = 0; d <= 6; d++) {
-                const int nmod = CRT_NB - d, j2 = cost - nmod;
-                if (j2 < 0 || j2 % 2 || j2 / 2 > nmod) continue;
-                double bits = 0;
-                for (int i = 0; i < nmod; i++) bits += (i < j2 / 2 ? 2 : 1) * log2((double)crt_base(i));
-                if (bits > bbits) bbits = bits, bj = j2 / 2, bd = d;
-            }
-            if (bj < 0 || bbits <= best || T.n >= CRT_CFGS) continue;
-            best = (float)bbits;
-            CrtCfg& c = T.cfg[T.n++];
-            c = CrtCfg{};
-            c.nmod = CRT_NB - bd;
-            c.nsq = bj;
-            c.cost = cost;
-            c.bits = (float)bbits;
-            c.words = bbits < 127.0 ? 4 : 5;
-            const auto mod = [&](int l) { return l < c.nsq ? crt_base(l) * crt_base(l) : crt_base(l); };
-            const int top = 32 * c.words;
-            c.sh = top - 1 - (int)ceil(bbits);  // M is never a power of two
-            uint32_t M[CRT_WORDS] = {1};
-            for (int l = 0; l < c.nmod; l++) {
-                const int pl = mod(l);
-                crt_words_mul(M, (uint32_t)pl);
-                int inv = 1, r = 1, cl = 1;
-                for (int i = 0; i < c.nmod; i++) {
-                    if (i == l) continue;
-                    r = (int)((int64_t)r * mod(i) % pl);  // M / p mod p
-                    if (crt_group(i) == crt_group(l)) cl *= mod(i);
-                }
-                while ((int64_t)inv * r % pl != 1 % pl) inv++;
-                c.p[l] = (float)pl;
-                c.invp[l] = 1.0f / (float)pl;
-                c.u[l] = (float)(2 * inv > pl ? inv - pl : inv);
-                c.c[l] = cl;
-            }
-            for (int i = 0; i < c.sh; i++) crt_words_mul(M, 2);
-            uint64_t borrow = 1;  // two's complement over `words` words
-            for (int j = 0; j < c.words; j++) {
-                const uint64_t t = (uint64_t)(uint32_t)~M[j] + borrow;
-                c.NM[j] = (uint32_t)t;
-                borrow = t >> 32;
-            }
-            for (int g = 0; g < CRT_NG; g++) {
-                uint32_t W[CRT_WORDS] = {1};
-                int P = 1;
-                for (int i = 0; i < c.nmod; i++) {
-                    if (crt_group(i) == g) P *= mod(i);
-                    else crt_words_mul(W, (uint32_t)mod(i));
-                }
-                if (2 * g >= c.nmod) continue;  // no modulus: z stays 0
-                for (int i = 0; i < c.sh; i++) crt_words_mul(W, 2);
-                c.z0[g] = 2 * P;
-                for (int j = 0; j < CRT_WORDS; j++) c.W[g][j] = W[j];
-            }
-            c.qinv = (float)exp2((double)(top - 18) - bbits - c.sh);
-        }
-        return T;
-    }();
-    return table;
-}
-
 // The cheapest configuration that holds a sum of klen products of F-bit
 // integers with its sign (|C'| <= klen 2^(2F) < M / 2), or -1.
 static int crt_config(int s, int64_t klen) {
-    const CrtTable& T = crt_table();
+    const CrtTable& T = crt_host;
     const double need = 2.0 * (4 + 5 * (s - 1)) + log2((double)(klen > 1 ? klen : 1)) + 1.01;
     for (int i = 0; i < T.n; i++)
         if (T.cfg[i].bits >= need) return i;

@@ -73,7 +73,6 @@ struct f4j_ctx {
     void* plan_tab[2];
     long long plan_key[2][4];
     bool plan_valid[2];
-    void* crt_tab;     // constants of the residue form's configurations (created on first use)
     bool parts_init;
     bool host_pin;     // host-buffer products page-lock their arrays per call (f4j_set_host_pinning)
     int* d_status;     // device status words (bounded-wait timeouts, validation)

@@ -1613,22 +1613,6 @@ static int make_crt_map(CUtensorMap* map, const void* base, uint64_t Kp, uint64_
     return F4J_OK;
 }
 
-// The configurations' constants on the device, uploaded on the context's first use.
-static int crt_device_table(f4j_ctx* ctx, const CrtCfg** out) {
-    if (!ctx->crt_tab) {
-        const CrtTable& T = crt_table();
-        F4J_CUDA(cudaMalloc(&ctx->crt_tab, sizeof T.cfg));
-        cudaError_t e = cudaMemcpy(ctx->crt_tab, T.cfg, sizeof T.cfg, cudaMemcpyHostToDevice);
-        if (e != cudaSuccess) {
-            cudaFree(ctx->crt_tab);
-            ctx->crt_tab = nullptr;
-            return f4j_cuda_fail(e, "residue constants");
-        }
-    }
-    *out = (const CrtCfg*)ctx->crt_tab;
-    return F4J_OK;
-}
-
 // Residues of C (2 bytes per modulus and entry) up to this size are kept for
 // all of C; a larger product goes in row blocks of it.
 constexpr size_t CRT_Y_BYTES = size_t(4) << 30;
@@ -1638,7 +1622,6 @@ struct CrtSetup {
     int64_t half, M, N, Kh, Kp, klen, ldy, blk, yrows;  // blk: tile rows per row block of C, yrows its rows
     int tiles_m, tiles_n, planes, nmod;
     CrtPick pick;
-    const CrtCfg* cfgs;
     SmallLayout Lo;
     size_t plane_a, plane_b;
     char* w;
@@ -1667,12 +1650,10 @@ static int crt_setup(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, C
     for (int s = 0; s <= S_MAX; s++) {
         S->pick.cfg[s] = (int8_t)(s < 2 || s > s_max ? -1 : crt_config(s, S->klen));
         if (S->pick.cfg[s] < 0) continue;
-        const CrtCfg& c = crt_table().cfg[S->pick.cfg[s]];
+        const CrtCfg& c = crt_host.cfg[S->pick.cfg[s]];
         S->planes = c.nmod + c.nsq > S->planes ? c.nmod + c.nsq : S->planes;
         S->nmod = c.nmod > S->nmod ? c.nmod : S->nmod;
     }
-    int rc = crt_device_table(ctx, &S->cfgs);
-    if (rc) return rc;
     S->Lo = small_layout(S->M, n, cplx ? 2 * n : n);
     S->plane_a = (size_t)S->M * S->Kp;
     S->plane_b = (size_t)S->N * S->Kp;
@@ -1683,7 +1664,7 @@ static int crt_setup(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, C
     S->blk = fit < 1 ? 1 : (fit > S->tiles_m ? S->tiles_m : fit);
     S->yrows = S->blk * CG_T < S->M ? S->blk * CG_T : S->M;
     void *ws1, *ws0;
-    rc = f4j_workspace(ctx, ctx->ws_base + 1, S->Lo.total, &ws1);
+    int rc = f4j_workspace(ctx, ctx->ws_base + 1, S->Lo.total, &ws1);
     if (rc) return rc;
     const size_t pa = al1k(S->plane_a * S->planes), pb = al1k(S->plane_b * S->planes);
     rc = f4j_workspace(ctx, ctx->ws_base, pa + pb + (size_t)S->nmod * S->yrows * S->ldy * 2, &ws0);
@@ -1724,7 +1705,7 @@ static int crt_launch(f4j_ctx* ctx, const CrtSetup& S, bool cplx, int64_t n, dou
         r1 > row0 + S.yrows || (cplx && (tn0 != 0 || tn1 != S.tiles_n)))
         return f4j_fail(F4J_ERR_ARG, "residue GEMM tile range [%d, %d) x [%d, %d)", tm0, tm1, tn0, tn1);
     CrtGemmParams g{(int)S.M, (int)S.N, (int)f4j_cdiv(S.Kp, CG_BK), tm0, tm1, tn0, tn1, row0, (int)S.yrows, S.ldy, S.y,
-                    ctx->d_status + F4J_ST_TIMEOUT, S.plan, S.cfgs};
+                    ctx->d_status + F4J_ST_TIMEOUT, S.plan};
     const int64_t units = (int64_t)(tm1 - tm0) * (tn1 - tn0) * S.nmod;
     const int pairs = (int)(units < ctx->sm_count / 2 ? units : ctx->sm_count / 2);
     const cudaStream_t saved = ctx->stream;
@@ -1735,7 +1716,7 @@ static int crt_launch(f4j_ctx* ctx, const CrtSetup& S, bool cplx, int64_t n, dou
     ctx->stream = saved;
     F4J_LAUNCHED(ctx);
     CrtCombineParams cp{(int)(r0 - row0), row0, (int)(r1 - r0), (int)S.yrows, (int)c0, (int)c1, (int)n, S.half, S.ldy,
-                        S.y, S.ea, S.eb, C, S.plan, S.cfgs};
+                        S.y, S.ea, S.eb, C, S.plan};
     const int64_t per_row = f4j_cdiv(c1 - c0, 2);
     unsigned bx = 32;  // threads along a row
     while (bx < 256 && bx < per_row) bx *= 2;
@@ -1781,7 +1762,7 @@ static int crt_gemm(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, co
         const CrtOperand ob{B, b_rows ? k : n, b_rows ? 0 : 1, opB == F4J_OP_C ? 1 : 0, 1, n, S.N, S.half, S.eb, S.plB};
         const dim3 grid((unsigned)(S.Kh / SP_TQ), slice_grid_y(M > n ? M : n), 2);
         f4j_launch(true, cplx ? k_crt_planes<true> : k_crt_planes<false>, grid, 256, 0, ctx->stream, oa, ob, k, S.Kh, S.Kp,
-                   S.plan, S.cfgs);
+                   S.plan);
         F4J_LAUNCHED(ctx);
     }
     f4j_prof_end(ctx);
@@ -2027,7 +2008,7 @@ static int host_split_pipelined(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, i
             const dim3 grid((unsigned)(Kh / SP_TQ), slice_grid_y(rows));
             if (crt) {
                 const CrtOperand o{dA + r0 * k * w2, k, 0, 0, 0, rows, M, 0, ea + r0, slA + r0 * Kp};
-                planes_k<<<grid, 256, 0, st>>>(o, o, k, Kh, Kp, plan, R.cfgs);
+                planes_k<<<grid, 256, 0, st>>>(o, o, k, Kh, Kp, plan);
             } else {
                 split_k<<<grid, 256, 0, st>>>(dA + r0 * k * w2, rows, k, 0, 0, 0, rows, k, Kh, Kp, M, ea + r0, plan,
                                               slA + r0 * Kp);
@@ -2086,7 +2067,7 @@ static int host_split_pipelined(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, i
             if (crt) {
                 const CrtOperand o{src, b_rows ? k : n, b_rows ? 0 : 1, conjb, 1, cw, R.N, R.half, eb + c0,
                                    slB + c0 * Kp};
-                planes_k<<<grid, 256, 0, st>>>(o, o, k, Kh, Kp, plan, R.cfgs);
+                planes_k<<<grid, 256, 0, st>>>(o, o, k, Kh, Kp, plan);
             } else {
                 split_k<<<grid, 256, 0, st>>>(src, b_rows ? cw : k, b_rows ? k : n, b_rows ? 0 : 1, conjb, 1, cw, k,
                                               Kh, Kp, N, eb + c0, plan, slB + c0 * Kp);
