@@ -335,7 +335,9 @@ __global__ void __launch_bounds__(256)
 // two sums a lane, from 33 columns in four: no larger an error than k_sddmm's 16
 // sums (rms over 10^6 entries, 16, 32 and
 // 48 columns: 3.93, 3.26 and 2.77e-17 for 4.09, 3.26 and 2.84e-17 of sum |a||b|).
-// rowidx: the row of each nonzero.
+// rowidx: the row of each nonzero, the first one's in rowidx[0].  A view of a larger
+// pattern has rowptr[0] > 0, and its column indices and results stand from there;
+// rows that hold fewer than nnz nonzeros leave the rest of out alone.
 // Measured: 64 columns, 2^18 rows x 16, 0.50 ms at 3 or 4 blocks an SM, 0.55 at 2,
 // 0.56 with A staged in shared memory by blocks of 64 nonzeros.  k_sddmm / this, us,
 // 2^20 rows x 16: 1 column 4129 / 288, 4 3966 / 346, 8 3968 / 544, 16 3968 / 702, 32
@@ -354,20 +356,50 @@ __device__ __forceinline__ double ld_nc_stream(const double* p) {
     asm volatile("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
     return v;
 }
+// The nonzeros w0 .. w0 + SD_WARP - 1 of a view (see k_sddmm_flat), a warp on one at
+// a time.
+__device__ __noinline__ void sddmm_view(int64_t w0, int first, int held, int ncols, int64_t ld, bool add,
+                                        const int* rowidx, const int* colidx, const double* A, const double* B,
+                                        double* out) {
+    for (int64_t i = w0; i < held && i < w0 + SD_WARP; i++) {
+        const double *a = A + rowidx[i] * ld, *b = B + colidx[first + i] * ld;
+        double s = 0.0;
+        for (int c = threadIdx.x % 32; c < ncols; c += 32) s = fma(a[c], b[c], s);
+        for (int off = 16; off; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+        if (threadIdx.x % 32 == 0) out[first + i] = add ? out[first + i] + s : s;
+    }
+}
 template <int U, bool PAIRS>
 __global__ void __launch_bounds__(256, 4)
-    k_sddmm_flat(int64_t nnz, int ncols, int64_t ld, bool add, const int* __restrict__ rowidx,
-                 const int* __restrict__ colidx, const double* __restrict__ A, const double* __restrict__ B,
-                 double* __restrict__ out) {
+    k_sddmm_flat(int64_t rows, int64_t nnz0, int ncols, int64_t ld, bool add, const int* __restrict__ rowptr,
+                 const int* __restrict__ rowidx, const int* __restrict__ colidx, const double* __restrict__ A,
+                 const double* __restrict__ B, double* __restrict__ out) {
     using V = typename std::conditional<PAIRS, double2, double>::type;
     constexpr bool WHOLE = PAIRS && U == 8;  // 64 columns, no unit left over (the launch sees to it)
     constexpr int SUMS = WHOLE || (!PAIRS && U == 1) ? 1 : (U > (PAIRS ? 4 : 8) ? 4 : 2);
     const int lane = threadIdx.x % 32, g = lane >> 2, l4 = lane & 3;
     const int units = WHOLE ? 32 : (PAIRS ? ncols / 2 : ncols);
-    const int64_t w0 = ((int64_t)blockIdx.x * 8 + threadIdx.x / 32) * SD_WARP;
+    // 16 units a lane are short of registers: with 32-bit indices, or the view's
+    // offsets in the loop, 63 columns take 2.6 to 2.8 ms for 2.4
+    using Q = typename std::conditional<U == 16, int64_t, unsigned>::type;
+    Q nnz = (Q)nnz0;  // below 2^31
+    const Q w0 = ((Q)blockIdx.x * 8 + threadIdx.x / 32) * SD_WARP;
     if (w0 >= nnz) return;
+    const int first = __ldg(rowptr);
+    const Q held = (Q)(__ldg(rowptr + rows) - first);
+    if constexpr (U == 16) {
+        if (first != 0 || held != nnz) {
+            sddmm_view(w0, first, (int)(held < nnz ? held : nnz), ncols, ld, add, rowidx, colidx, A, B, out);
+            return;
+        }
+    } else {
+        if (held < nnz) nnz = held;
+        if (w0 >= nnz) return;
+        colidx += first;
+        out += first;
+    }
     auto at = [&](int step) {  // past the end: the last nonzero again, not stored
-        const int64_t q = w0 + step * 8 + g;
+        const Q q = w0 + step * 8 + g;
         return q < nnz ? q : nnz - 1;
     };
     auto row_of = [&](const double* X, int64_t i) {
@@ -417,7 +449,7 @@ __global__ void __launch_bounds__(256, 4)
         const double u1 = __shfl_xor_sync(0xffffffffu, h2 ? p[1] : p[3], 2);
         const double t0 = (h2 ? p[2] : p[0]) + u0, t1 = (h2 ? p[3] : p[1]) + u1;
         const double r = (h1 ? t1 : t0) + __shfl_xor_sync(0xffffffffu, h1 ? t0 : t1, 1);
-        const int64_t q = w0 + (s0 + l4) * 8 + g;
+        const Q q = w0 + (s0 + l4) * 8 + g;
         if (q < nnz) out[q] = add ? out[q] + r : r;
     }
 }
@@ -511,17 +543,17 @@ __global__ void k_validate_csr(int64_t rows, int64_t cols, int64_t nnz, const in
     }
 }
 
-// Row of each nonzero.  A warp covers 32 consecutive rows: their nonzeros are
-// written in order, each lane finding its row among the 32 by bisection over
+// Row of each of the nnz nonzeros, the first one's in rowidx[0] (rowptr[0] may be
+// above 0).  A warp covers 32 consecutive rows: their nonzeros are written in order, each lane finding its row among the 32 by bisection over
 // the lanes (a warp per row left half its lanes idle at 16 nonzeros a row and
 // started 2^20 warps: 93 us for 16.8 M nonzeros).
-__global__ void k_expand_rows(int64_t rows, const int* __restrict__ rowptr, int* __restrict__ rowidx) {
+__global__ void k_expand_rows(int64_t rows, int64_t nnz, const int* __restrict__ rowptr, int* __restrict__ rowidx) {
     const int64_t w0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32) * 32;
     const int lane = threadIdx.x % 32;
     if (w0 >= rows) return;
     const int64_t r = w0 + lane;
     const int end = __ldg(rowptr + (r < rows ? r + 1 : rows));  // rows past the last end where it ends
-    const int q1 = __shfl_sync(0xffffffffu, end, 31);
+    const int first = __ldg(rowptr), q1 = __shfl_sync(0xffffffffu, end, 31);
     for (int base = __ldg(rowptr + w0); base < q1; base += 32) {
         const int q = base + lane;
         int lo = 0;  // first row of the 32 that ends after q
@@ -530,7 +562,7 @@ __global__ void k_expand_rows(int64_t rows, const int* __restrict__ rowptr, int*
             const int e = __shfl_sync(0xffffffffu, end, lo + step - 1);
             if (e <= q) lo += step;
         }
-        if (q < q1) rowidx[q] = (int)(w0 + lo);
+        if (q < q1 && q - first < nnz) rowidx[q - first] = (int)(w0 + lo);
     }
 }
 
@@ -1437,7 +1469,7 @@ static int ensure_transpose(f4j_ctx* ctx, f4j_csr S, int* t_col = nullptr, bool*
         if (!rowidx) {
             rc = f4j_dev_alloc(ctx, (size_t)nnz * 4, (void**)&ri);
             if (!rc) {
-                k_expand_rows<<<(unsigned)f4j_cdiv(rows, 256), 256, 0, ctx->stream>>>(rows, (const int*)S->rowptr->ptr, ri);
+                k_expand_rows<<<(unsigned)f4j_cdiv(rows, 256), 256, 0, ctx->stream>>>(rows, nnz, (const int*)S->rowptr->ptr, ri);
                 ctx->launches++;
             }
             rowidx = ri;
@@ -1470,7 +1502,8 @@ static int ensure_rowidx(f4j_ctx* ctx, f4j_csr S) {
     int* ri = nullptr;
     int rc = f4j_dev_alloc(ctx, (size_t)S->nnz * 4, (void**)&ri);
     if (rc) return rc;
-    k_expand_rows<<<(unsigned)f4j_cdiv(S->rows, 256), 256, 0, ctx->stream>>>(S->rows, (const int*)S->rowptr->ptr, ri);
+    k_expand_rows<<<(unsigned)f4j_cdiv(S->rows, 256), 256, 0, ctx->stream>>>(S->rows, S->nnz,
+                                                                             (const int*)S->rowptr->ptr, ri);
     F4J_LAUNCHED(ctx);
     S->rowidx = ri;
     return F4J_OK;
@@ -2231,8 +2264,8 @@ extern "C" int f4j_sddmm(f4j_ctx* ctx, f4j_csr S, f4j_buf A, f4j_buf B, int64_t 
                                                                                           : F4J_ERR_OOM;
         if (rc && rc != F4J_ERR_OOM) return rc;
         if (rc == F4J_OK) {
-            using Kernel = void (*)(int64_t, int, int64_t, bool, const int*, const int*, const double*, const double*,
-                                    double*);
+            using Kernel = void (*)(int64_t, int64_t, int, int64_t, bool, const int*, const int*, const int*,
+                                    const double*, const double*, double*);
             static const Kernel pairs[8] = {k_sddmm_flat<1, true>, k_sddmm_flat<2, true>, k_sddmm_flat<3, true>,
                                             k_sddmm_flat<4, true>, k_sddmm_flat<5, true>, k_sddmm_flat<6, true>,
                                             k_sddmm_flat<7, true>, k_sddmm_flat<8, true>};
@@ -2254,8 +2287,8 @@ extern "C" int f4j_sddmm(f4j_ctx* ctx, f4j_csr S, f4j_buf A, f4j_buf B, int64_t 
                     k = ones[i];
                 }
                 k<<<(unsigned)f4j_cdiv(S->nnz, 8 * SD_WARP), 256, 0, ctx->stream>>>(
-                    S->nnz, w, ncols, c0 > 0, (const int*)S->rowidx, (const int*)S->colidx->ptr, a + c0, b + c0,
-                    (double*)out->ptr);
+                    S->rows, S->nnz, w, ncols, c0 > 0, (const int*)S->rowptr->ptr, (const int*)S->rowidx,
+                    (const int*)S->colidx->ptr, a + c0, b + c0, (double*)out->ptr);
                 if (c0 + part < ncols) ctx->launches++;
             }
         } else {

@@ -753,3 +753,35 @@ def test_spmm_every_width_bit_identical(f4j, oracle, ncols):
         assert np.all(np.abs(fma - ref) <= fma_bound(oracle, rp, ci, v, X))
         trp, tci, tv, _ = oracle.csr_transpose(rows, cols, rp, ci, v)
         assert np.array_equal(S.multTransposeLeft(f4j.Matrix(W)).toNumpy(), oracle.spmm(trp, tci, tv, W))
+
+
+@pytest.mark.parametrize("first,tail", [(0, 0), (5, 0), (37, 64), (0, 900)])
+@pytest.mark.parametrize("ncols", [1, 7, 32, 64, 100])
+def test_sddmm_of_a_view_of_a_larger_pattern(f4j, first, tail, ncols):
+    """A handle on rows of a larger CSR (rowptr[0] > 0, arrays longer than the view) and one that declares room
+    for more nonzeros than its rows hold: the results stand at the view's own positions, nothing else is
+    written, and the call repeats."""
+    from flag4j_gb300.device import check
+    g = np.random.default_rng(first + 3 * ncols)
+    rows, cols = 300, 400
+    lens = g.integers(0, 9, rows)
+    held = int(lens.sum())
+    rp = np.full(rows + 1, first, np.int32)
+    rp[1:] += np.cumsum(lens).astype(np.int32)
+    row = np.repeat(np.arange(rows), lens)
+    size = first + held + tail
+    ci = g.integers(0, cols, size).astype(np.int32)
+    A, B = g.standard_normal((rows, ncols)), g.standard_normal((cols, ncols))
+    ctx = f4j.default_context()
+    bufs = [ctx.from_numpy(x) for x in (rp, ci, g.standard_normal(size))]
+    nnz = held if first else held + tail
+    h = ctypes.c_void_p()
+    check(ctx.lib.f4j_csr_wrap(ctx.handle, rows, cols, nnz, *[b.handle for b in bufs], 0, ctypes.byref(h)))
+    dA, dB, out = ctx.from_numpy(A), ctx.from_numpy(B), ctx.from_numpy(np.full(size, 7.0))
+    terms = A[row].astype(np.longdouble) * B[ci[first:first + held]].astype(np.longdouble)
+    for _ in range(2):
+        check(ctx.lib.f4j_sddmm(ctx.handle, h, dA.handle, dB.handle, ncols, out.handle, None))
+        got = out.to_numpy(np.float64, size)
+        assert np.all(got[:first] == 7.0) and np.all(got[first + held:] == 7.0)
+        assert np.all(np.abs(got[first:first + held] - terms.sum(1)) <= 2 * ncols * U * np.abs(terms).sum(1))
+    check(ctx.lib.f4j_csr_free(ctx.handle, h))
