@@ -1451,14 +1451,38 @@ static int transpose_radix(f4j_ctx* ctx, f4j_csr S, const int* rowidx, int* trp,
     return rc;
 }
 
-// Builds the cached transpose structure of S (RealCsrOps.transpose order).  t_col:
+// Whether calls on the context's stream become part of a graph.  What the stream
+// allocates then belongs to the graph and holds nothing until the graph runs, so
+// no handle may keep it.
+static int in_capture(f4j_ctx* ctx, bool* captured) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    F4J_CUDA(cudaStreamIsCapturing(ctx->stream, &st));
+    *captured = st != cudaStreamCaptureStatusNone;
+    return F4J_OK;
+}
+
+// Frees a structure that ensure_transpose made for this call alone.
+static void drop_transpose(f4j_ctx* ctx, f4j_csr S, bool once) {
+    if (!once) return;
+    f4j_dev_free(ctx, S->t_rowptr);
+    f4j_dev_free(ctx, S->t_perm);
+    f4j_dev_free(ctx, S->t_rowidx);
+    S->t_rowptr = S->t_perm = S->t_rowidx = nullptr;
+}
+
+// Builds the cached transpose structure of S (RealCsrOps.transpose order).  *once:
+// in a stream capture it is for this call alone, which drops it (drop_transpose)
+// behind its last use: the graph then makes and frees it each time it runs.  t_col:
 // an array for a copy of its column indices, made on the way where that can be
 // (*copied).
-static int ensure_transpose(f4j_ctx* ctx, f4j_csr S, int* t_col = nullptr, bool* copied = nullptr) {
+static int ensure_transpose(f4j_ctx* ctx, f4j_csr S, bool* once, int* t_col = nullptr, bool* copied = nullptr) {
+    *once = false;
     if (S->t_perm) return F4J_OK;
+    int rc = in_capture(ctx, once);
+    if (rc) return rc;
     const int64_t nnz = S->nnz, rows = S->rows, cols = S->cols;
     int *trp = nullptr, *perm = nullptr, *trow = nullptr, *ri = nullptr;
-    int rc = f4j_dev_alloc(ctx, (size_t)(cols + 1) * 4, (void**)&trp);
+    rc = f4j_dev_alloc(ctx, (size_t)(cols + 1) * 4, (void**)&trp);
     if (!rc) rc = f4j_dev_alloc(ctx, (size_t)nnz * 4, (void**)&perm);
     if (!rc) rc = f4j_dev_alloc(ctx, (size_t)nnz * 4, (void**)&trow);
     if (!rc && nnz == 0) {
@@ -2081,8 +2105,8 @@ extern "C" int f4j_csr_transpose(f4j_ctx* ctx, f4j_csr S, f4j_csr* out) {
     f4j_csr T;
     int rc = alloc_owned_csr(ctx, S->cols, S->rows, S->nnz, &T);
     if (rc) return rc;
-    bool copied = false;
-    rc = ensure_transpose(ctx, S, (int*)T->colidx->ptr, &copied);
+    bool once = false, copied = false;
+    rc = ensure_transpose(ctx, S, &once, (int*)T->colidx->ptr, &copied);
     if (rc) {
         f4j_csr_free(ctx, T);
         return rc;
@@ -2096,6 +2120,7 @@ extern "C" int f4j_csr_transpose(f4j_ctx* ctx, f4j_csr S, f4j_csr* out) {
                                                                  (const double*)S->vals->ptr, (double*)T->vals->ptr);
         F4J_LAUNCHED(ctx);
     }
+    drop_transpose(ctx, S, once);
     *out = T;
     return F4J_OK;
 }
@@ -2106,9 +2131,11 @@ extern "C" int f4j_csr_transpose_perm(f4j_ctx* ctx, f4j_csr S, f4j_buf perm_out)
     if (!S || !perm_out) return f4j_fail(F4J_ERR_ARG, "null argument");
     if (perm_out->bytes < (size_t)S->nnz * 4) return f4j_fail(F4J_ERR_ARG, "perm buffer too small");
     F4J_CUDA(cudaSetDevice(ctx->device));
-    int rc = ensure_transpose(ctx, S);
+    bool once = false;
+    int rc = ensure_transpose(ctx, S, &once);
     if (rc) return rc;
     F4J_CUDA(cudaMemcpyAsync(perm_out->ptr, S->t_perm, (size_t)S->nnz * 4, cudaMemcpyDeviceToDevice, ctx->stream));
+    drop_transpose(ctx, S, once);
     return F4J_OK;
 }
 
@@ -2229,10 +2256,12 @@ extern "C" int f4j_spmm_t(f4j_ctx* ctx, f4j_csr S, f4j_buf dC, int64_t ncols, f4
     if (dX->bytes < (size_t)S->cols * ncols * 8) return f4j_fail(F4J_ERR_ARG, "dX buffer too small");
     F4J_CUDA(cudaSetDevice(ctx->device));
     int64_t l0 = ctx->launches;
-    int rc = ensure_transpose(ctx, S);
+    bool once = false;
+    int rc = ensure_transpose(ctx, S, &once);
     if (rc) return rc;
     rc = launch_spmm(ctx, S->cols, S->nnz, ncols, (const int*)S->t_rowptr, (const int*)S->t_rowidx,
                      (const double*)S->vals->ptr, (const int*)S->t_perm, (const double*)dC->ptr, (double*)dX->ptr);
+    drop_transpose(ctx, S, once);
     if (rc) return rc;
     if (rep) {
         *rep = f4j_report{};
@@ -2258,10 +2287,9 @@ extern "C" int f4j_sddmm(f4j_ctx* ctx, f4j_csr S, f4j_buf A, f4j_buf B, int64_t 
         f4j_prof_begin(ctx);
         // no room for the row of each nonzero, or a stream capture, which an allocation
         // kept in the handle must not be part of: k_sddmm, which needs none
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (!S->rowidx && ncols != 64) F4J_CUDA(cudaStreamIsCapturing(ctx->stream, &cap));
-        int rc = ncols >= 1 && ncols <= SD_FLAT_COLS && cap == cudaStreamCaptureStatusNone ? ensure_rowidx(ctx, S)
-                                                                                          : F4J_ERR_OOM;
+        bool captured = false;
+        int rc = S->rowidx ? F4J_OK : in_capture(ctx, &captured);
+        if (!rc) rc = ncols >= 1 && ncols <= SD_FLAT_COLS && !captured ? ensure_rowidx(ctx, S) : F4J_ERR_OOM;
         if (rc && rc != F4J_ERR_OOM) return rc;
         if (rc == F4J_OK) {
             using Kernel = void (*)(int64_t, int64_t, int, int64_t, bool, const int*, const int*, const int*,

@@ -334,7 +334,10 @@ int f4j_gemm_check(f4j_ctx* ctx, int cplx, int64_t m, int64_t n, int64_t k, f4j_
 
 /* ---- CSR matrices ---------------------------------------------------------- */
 /* Wrap device arrays as a CSR matrix (rowptr int32[rows+1], colidx int32[nnz],
- * vals float64[nnz]); the handle borrows the buffers.  validate != 0 runs
+ * vals float64[nnz]); the handle borrows the buffers, whose values may change
+ * between calls while the pattern (rowptr, colidx) stays: what f4j_spmm_t,
+ * f4j_sddmm and f4j_csr_transpose derive from it is kept in the handle.
+ * validate != 0 runs
  * SparseValidation.validateCsr's checks on the GPU
  *   (src/main/java/org/flag4j/arrays/sparse/SparseValidation.java:151-206;
  *    constructor CsrMatrix.java:175-185). */
@@ -427,12 +430,18 @@ int f4j_spmm_ex(f4j_ctx* ctx, f4j_csr S, f4j_buf X, int64_t ncols, f4j_buf Y, in
 int f4j_zspmm(f4j_ctx* ctx, f4j_csr S, f4j_buf X, int64_t ncols, f4j_buf Y, f4j_report* report);
 /* dX(cols x ncols) = S^T dC without forming S^T: gathers through a cached
  * transpose permutation (built on first use); atomic-free.  Bit-identical to
- * S.T().mult(dC) in the reference. */
+ * S.T().mult(dC) in the reference.  On a stream that is being captured a handle
+ * without that structure keeps none: the graph builds and frees it each time it
+ * runs, so make one call before the capture. */
 int f4j_spmm_t(f4j_ctx* ctx, f4j_csr S, f4j_buf dC, int64_t ncols, f4j_buf dX,
                f4j_report* report);
 /* SDDMM on S's pattern: out[q] = dot(A[row(q), :], B[col(q), :]) over ncols
  * (A rows x ncols, B cols x ncols) -- the gradient dS = (dC X^T) restricted to
- * pattern(S) for C = S X.  No Flag4j counterpart. */
+ * pattern(S) for C = S X.  No Flag4j counterpart.  Up to 200 columns the rows of
+ * the nonzeros are cached in the handle on first use; with no room for them, or on
+ * a stream that is being captured before they are there, a kernel by rows runs
+ * instead (about 2 to 10 times the time at 16 nonzeros a row), so make one call
+ * before the capture. */
 int f4j_sddmm(f4j_ctx* ctx, f4j_csr S, f4j_buf A, f4j_buf B, int64_t ncols, f4j_buf out,
               f4j_report* report);
 
