@@ -720,7 +720,8 @@ __global__ void __launch_bounds__(RS_T) k_radix_scatter(int64_t n, const unsigne
 // its low column bits, row and source index, into at most TP_NB buckets of
 // 2^shift columns, in storage order inside each; pass 2 (k_tp_bucket, a block
 // per bucket) counts the bucket's columns, which gives its part of the row
-// pointers, and orders it by column.  Both rank stably the same way: each warp
+// pointers, and orders it by column.  A bucket far above the others goes in
+// segments, a block each (k_tp_segments).  Both rank stably the same way: each warp
 // owns a contiguous part of the items and a counter per bucket (column); the
 // counters are summed over the warps before, so a warp then only walks its own
 // items in order.  The lanes holding equal keys are found with one ballot per
@@ -731,17 +732,20 @@ __global__ void __launch_bounds__(RS_T) k_radix_scatter(int64_t n, const unsigne
 // 4-byte writes at 2^20 columns, and the rows gathered after it: 2^20 rows and
 // columns, 16.8 M nonzeros, 0.93 -> 0.38 ms (scatter 137, bucket 185, histogram
 // and places 38, rows 19 us).  Both passes are instruction-bound (153 and 204 warp
-// instructions per 32 items).
+// instructions per 32 items).  The kernels are a chain (chain_wait in f4j_ptx.cuh):
+// 65536 rows and columns x 8, T() 105 -> 92 us.
 constexpr int TP_NB = 1024, TP_BITS = 10;
 constexpr int TP1_T = 256, TP1_WARPS = TP1_T / 32, TP1_TILE = 4096;  // pass 1: items per block
 constexpr int TP2_T = 512, TP2_WARPS = TP2_T / 32;
 constexpr int TP2_CNT = TP2_WARPS * TP_NB;
 constexpr int TP2_CAP = 18432;           // bucket items that pass 2 places in shared memory
+constexpr int TP2_SEG = 16384;           // items of a segment of a big bucket
 
 // hist[block][bucket], rows of nbp (nb rounded up to a multiple of four).
 __global__ void __launch_bounds__(512) k_tp_hist(int64_t n, const int* __restrict__ col, int shift, int nbp,
                                                  int* __restrict__ hist) {
     __shared__ int h[TP_NB];
+    chain_trigger();
     for (int i = threadIdx.x; i < nbp; i += 512) h[i] = 0;
     __syncthreads();
     const int64_t base = (int64_t)blockIdx.x * TP1_TILE;
@@ -761,6 +765,8 @@ __global__ void __launch_bounds__(512) k_tp_hist(int64_t n, const int* __restric
 constexpr int TP_CHUNK = 64;
 __global__ void __launch_bounds__(64) k_tp_chunks(int nblocks, int nbp, int* __restrict__ hist, int* __restrict__ part) {
     const int b = 4 * (64 * blockIdx.y + threadIdx.x), r0 = blockIdx.x * TP_CHUNK;
+    chain_wait();
+    chain_trigger();
     if (b >= nbp) return;
     const int r1 = r0 + TP_CHUNK < nblocks ? r0 + TP_CHUNK : nblocks;
     int4 run = make_int4(0, 0, 0, 0);
@@ -800,12 +806,22 @@ __device__ __forceinline__ int tp_block_excl(int v, int* sh, int* total) {
     return before + x - v;
 }
 
+// The buckets that go in segments, of more than `above` items: big[0 .. n), the segments of big[i] are
+// seg0[i] .. seg0[i + 1) - 1 of all.
+// done[i]: its segments whose columns are counted.
+struct TpBig {
+    int above;
+    int *n, *big, *seg0, *done;
+};
+
 // part: exclusive prefix over the chunks, in place; start[b]: the bucket's first
-// place, start[nb]: all items.  One block, a thread per bucket.
+// place, start[nb]: all items; the big buckets.  One block, a thread per bucket.
 __global__ void __launch_bounds__(TP_NB) k_tp_starts(int chunks, int nb, int nbp, int* __restrict__ part,
-                                                     int* __restrict__ start) {
+                                                     int* __restrict__ start, const TpBig to) {
     __shared__ int sh[TP_NB / 32];
     const int b = threadIdx.x;
+    chain_wait();
+    chain_trigger();
     int run = 0;
     if (b < nbp) {
         constexpr int U = 16;
@@ -824,6 +840,18 @@ __global__ void __launch_bounds__(TP_NB) k_tp_starts(int chunks, int nb, int nbp
     const int at = tp_block_excl<TP_NB / 32>(run, sh, &total);
     if (b < nb) start[b] = at;
     if (b == 0) start[nb] = total;
+    // one scan for both counts: at most 2^18 segments, 2^10 big buckets
+    const int segs = b < nb && run > to.above ? (run - 1) / TP2_SEG + 1 : 0;
+    const int before = tp_block_excl<TP_NB / 32>(segs << 11 | (segs > 0), sh, &total);
+    if (segs) {
+        to.big[before & 2047] = b;
+        to.seg0[before & 2047] = before >> 11;
+        to.done[before & 2047] = 0;
+    }
+    if (b == 0) {
+        *to.n = total & 2047;
+        to.seg0[total & 2047] = total >> 11;
+    }
 }
 
 // cnt[w * nkp + key]: how many of warp w's items have the key (nkp: keys rounded
@@ -913,6 +941,8 @@ __global__ void __launch_bounds__(TP1_T) k_tp_scatter(int64_t n, const int* __re
     const int nkp = (nb + 3) & ~3;
     int* mine = cnt + warp * nkp;
     const int i0 = warp * PART + lane;
+    chain_wait();
+    chain_trigger();
     // this block's first place of four buckets, for tp_places (nb <= 4 x threads; start has nbp entries)
     static_assert(TP_NB <= 4 * TP1_T, "four buckets a thread");
     int4 out = make_int4(0, 0, 0, 0);
@@ -962,31 +992,19 @@ __global__ void __launch_bounds__(TP1_T) k_tp_scatter(int64_t n, const int* __re
     }
 }
 
-// Bucket b = blockIdx.x: columns [b << shift, (b + 1) << shift), items
-// [start[b], start[b + 1]) of the pass 1 output.
-__global__ void __launch_bounds__(TP2_T) k_tp_bucket(int64_t cols, int shift, int qbits, int rbits, int nw,
-                                                     const int* __restrict__ start,
-                                                     const unsigned long long* __restrict__ items,
-                                                     int* __restrict__ t_rowptr, const TpOut to) {
-    extern __shared__ unsigned long long tp_smem[];
-    unsigned long long* place = tp_smem;                 // item at each place of the bucket
-    int* cnt = reinterpret_cast<int*>(place + TP2_CAP);   // [warp][column]
-    __shared__ int sh[TP2_WARPS];
-    const int b = blockIdx.x, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    const int64_t s0 = __ldg(start + b), s1 = __ldg(start + b + 1);
-    const int m = (int)(s1 - s0);
-    const int64_t c0 = (int64_t)b << shift;
-    const int nk = (int)(cols - c0 < (1 << shift) ? cols - c0 : 1 << shift);
-    const int nkp = (nk + 3) & ~3;
-    const unsigned long long* in = items + s0;
+// Orders the m items at `in` by key, stably: put(place, item) for each; start(key,
+// first) sees each key's first place before that.  nw warps (all of them up to 2^10
+// columns a bucket) rank; each takes a multiple of 32 items.
+template <typename F, typename G>
+__device__ __forceinline__ void tp_order(const unsigned long long* __restrict__ in, int m, int up, int shift, int nw,
+                                         int nkp, int* cnt, int* sh, F start, G put) {
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     for (int i = threadIdx.x; i < nw * nkp / 4; i += TP2_T) reinterpret_cast<int4*>(cnt)[i] = make_int4(0, 0, 0, 0);
     __syncthreads();
-    // nw warps (all of them up to 2^10 columns a bucket) rank; each takes a multiple of 32 items
     const int part = ((m + nw - 1) / nw + 31) & ~31;
     int* mine = cnt + warp * nkp;
-    const int i0 = warp < nw ? (int)((int64_t)warp * part < m ? warp * part : m) : m;
-    const int i1 = (int64_t)i0 + part < m ? i0 + part : m;
-    const int up = qbits + rbits;
+    const int i0 = warp < nw && warp * part < m ? warp * part : m;
+    const int i1 = i0 + part < m ? i0 + part : m;
     constexpr int U = 8;  // loads in flight per lane
     for (int i = i0 + lane; i < i1; i += 32 * U) {
         int key[U];
@@ -997,15 +1015,7 @@ __global__ void __launch_bounds__(TP2_T) k_tp_bucket(int64_t cols, int shift, in
             if (key[u] >= 0) atomicAdd(&mine[key[u]], 1);
     }
     __syncthreads();
-    tp_places<TP2_WARPS>(cnt, nw, nkp, sh, [&](int c, int4 first) {
-        const int f[4] = {first.x, first.y, first.z, first.w};
-#pragma unroll
-        for (int u = 0; u < 4; u++)
-            if (c + u < nk) t_rowptr[c0 + c + u] = (int)s0 + f[u];
-    });
-    if (b == gridDim.x - 1 && threadIdx.x == 0) t_rowptr[cols] = (int)s1;
-    const bool placed = m <= TP2_CAP;
-    const unsigned long long qmask = (1ull << qbits) - 1, rmask = (1ull << rbits) - 1;
+    tp_places<TP2_WARPS>(cnt, nw, nkp, sh, start);
     for (int i = i0; i < i1; i += 32 * U) {
         unsigned long long w[U];
 #pragma unroll
@@ -1014,19 +1024,178 @@ __global__ void __launch_bounds__(TP2_T) k_tp_bucket(int64_t cols, int shift, in
         for (int u = 0; u < U; u++) {
             const bool has = i + 32 * u + lane < i1;
             const int at = tp_rank(mine, has ? (int)(w[u] >> up) : -1, shift);
-            if (!has) continue;
-            if (placed) {
-                place[at] = w[u];
-            } else {  // more items than shared memory holds: straight to their places
-                to.put(s0 + at, (int)(w[u] & qmask), (int)(w[u] >> qbits & rmask));
-            }
+            if (has) put(at, w[u]);
         }
     }
+}
+
+// Segment seg of all: its big bucket (an index of of.big) and its first item within that.
+__device__ __forceinline__ int tp_segment(const TpBig& of, int seg, int64_t& at) {
+    int lo = 0, hi = *of.n - 1;  // the last big bucket that starts at or before it
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) / 2;
+        if (__ldg(of.seg0 + mid) <= seg) lo = mid;
+        else hi = mid - 1;
+    }
+    at = (int64_t)(seg - __ldg(of.seg0 + lo)) * TP2_SEG;
+    return lo;
+}
+
+// The places of big bucket i's segments, once all are counted: seg_cnt becomes, down
+// each column, the exclusive prefix over them; the columns' totals give the bucket's
+// row pointers.  A thread takes four adjacent columns of a row.
+__device__ __forceinline__ void tp_seg_places(int64_t cols, int shift, const int* start, const TpBig& of, int i,
+                                              int* seg_cnt, int* sh, int* t_rowptr) {
+    const int nkp = ((1 << shift) + 3) & ~3;
+    const int b = of.big[i], g0 = of.seg0[i], g1 = of.seg0[i + 1];
+    int before = start[b];
+    for (int k0 = 0; k0 < nkp; k0 += 4 * TP2_T) {
+        const int c = k0 + 4 * (int)threadIdx.x;
+        int4 run = make_int4(0, 0, 0, 0);
+        if (c < nkp) {
+            constexpr int U = 8;
+            for (int g = g0; g < g1; g += U) {
+                int4 v[U];
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                    v[u] = g + u < g1 ? __ldcg(reinterpret_cast<const int4*>(seg_cnt + (int64_t)(g + u) * nkp + c))
+                                      : make_int4(0, 0, 0, 0);
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    if (g + u < g1) *reinterpret_cast<int4*>(seg_cnt + (int64_t)(g + u) * nkp + c) = run;
+                    run.x += v[u].x, run.y += v[u].y, run.z += v[u].z, run.w += v[u].w;
+                }
+            }
+        }
+        int total;
+        int at = before + tp_block_excl<TP2_WARPS>(run.x + run.y + run.z + run.w, sh, &total);
+        before += total;
+        const int each[4] = {run.x, run.y, run.z, run.w};
+        const int64_t c0 = ((int64_t)b << shift) + c;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            if (c + u < 1 << shift && c0 + u < cols) t_rowptr[c0 + u] = at;
+            at += each[u];
+        }
+    }
+}
+
+// The blocks of pass 2 after the buckets': they count the columns of the big
+// buckets' segments, seg_cnt[segment][column], and the one that counts a bucket's
+// last goes on to its places; k_tp_seg_order then moves the items.  A block a bucket
+// left most of the work to one SM where the columns are skewed (a graph's vertices by
+// degree, a dense band).  T() at 2^20 rows and columns, 16.8 M nonzeros, us, a radix
+// sort / a block a bucket / this: 80 % of them in 1024 columns 2231 / 27785 / 745, in
+// one column 9539 / 14892 / 657, columns by a power law 5708 / 20739 / 742; evenly
+// spread 1478 / 604 / 611.
+__device__ __forceinline__ void tp_segments(int first, int stride, int64_t cols, int shift, int up, const int* start,
+                                            const unsigned long long* items, int* t_rowptr, const TpBig& of,
+                                            int* seg_cnt, int* cnt, int* sh) {
+    __shared__ int last;
+    const int nkp = ((1 << shift) + 3) & ~3, segs = of.seg0[*of.n];
+    for (int seg = first; seg < segs; seg += stride) {
+        int64_t at;
+        const int i = tp_segment(of, seg, at), b = of.big[i];
+        const int64_t s0 = start[b] + at, s1 = start[b + 1];
+        const int m = (int)(s1 - s0 < TP2_SEG ? s1 - s0 : TP2_SEG);
+        for (int c = threadIdx.x; c < nkp; c += TP2_T) cnt[c] = 0;
+        __syncthreads();
+#pragma unroll 8
+        for (int j = threadIdx.x; j < m; j += TP2_T) atomicAdd(&cnt[__ldg(items + s0 + j) >> up], 1);
+        __syncthreads();
+        for (int c = threadIdx.x; c < nkp; c += TP2_T) seg_cnt[(int64_t)seg * nkp + c] = cnt[c];
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) last = atomicAdd(of.done + i, 1) + 1 == of.seg0[i + 1] - of.seg0[i];
+        __syncthreads();
+        if (last) {
+            __threadfence();
+            tp_seg_places(cols, shift, start, of, i, seg_cnt, sh, t_rowptr);
+        }
+        __syncthreads();
+    }
+}
+
+// Bucket b = blockIdx.x < nb: columns [b << shift, (b + 1) << shift), items
+// [start[b], start[b + 1]) of the pass 1 output.  The blocks from nb on: tp_segments.
+__global__ void __launch_bounds__(TP2_T) k_tp_bucket(int nb, int64_t cols, int shift, int qbits, int rbits, int nw,
+                                                     const int* __restrict__ start,
+                                                     const unsigned long long* __restrict__ items,
+                                                     int* __restrict__ t_rowptr, const TpOut to, const TpBig of,
+                                                     int* __restrict__ seg_cnt) {
+    extern __shared__ unsigned long long tp_smem[];
+    unsigned long long* place = tp_smem;                 // item at each place of the bucket
+    int* cnt = reinterpret_cast<int*>(place + TP2_CAP);   // [warp][column]
+    __shared__ int sh[TP2_WARPS];
+    const int up = qbits + rbits;
+    const int b = blockIdx.x;
+    chain_wait();
+    chain_trigger();
+    if (b >= nb) {
+        tp_segments(b - nb, gridDim.x - nb, cols, shift, up, start, items, t_rowptr, of, seg_cnt, cnt, sh);
+        return;
+    }
+    const int64_t s0 = __ldg(start + b), s1 = __ldg(start + b + 1);
+    if (b == nb - 1 && threadIdx.x == 0) t_rowptr[cols] = (int)s1;
+    if (s1 - s0 > of.above) return;
+    const int m = (int)(s1 - s0);
+    const bool placed = m <= TP2_CAP;  // else more items than shared memory holds: straight to their places
+    const int64_t c0 = (int64_t)b << shift;
+    const int nk = (int)(cols - c0 < (1 << shift) ? cols - c0 : 1 << shift);
+    const unsigned long long qmask = (1ull << qbits) - 1, rmask = (1ull << rbits) - 1;
+    auto start_of = [&](int c, int4 first) {
+        const int f[4] = {first.x, first.y, first.z, first.w};
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (c + u < nk) t_rowptr[c0 + c + u] = (int)s0 + f[u];
+    };
+    tp_order(items + s0, m, up, shift, nw, (nk + 3) & ~3, cnt, sh, start_of, [&](int at, unsigned long long w) {
+        if (placed) place[at] = w;
+        else to.put(s0 + at, (int)(w & qmask), (int)(w >> qbits & rmask));
+    });
     if (!placed) return;
     __syncthreads();
     for (int p = threadIdx.x; p < m; p += TP2_T) {
         const unsigned long long w = place[p];
         to.put(s0 + p, (int)(w & qmask), (int)(w >> qbits & rmask));
+    }
+}
+
+// The big buckets' segments, each ordered by a block and written to its places.
+__global__ void __launch_bounds__(TP2_T) k_tp_seg_order(int64_t cols, int shift, int qbits, int rbits, int nw,
+                                                        const int* __restrict__ start,
+                                                        const unsigned long long* __restrict__ items,
+                                                        const int* __restrict__ t_rowptr, const TpOut to, const TpBig of,
+                                                        const int* __restrict__ seg_cnt) {
+    extern __shared__ unsigned long long tp_smem[];
+    unsigned long long* place = tp_smem;
+    int* cnt = reinterpret_cast<int*>(place + TP2_SEG);
+    int* delta = cnt + TP2_CNT;  // place in the output less place in the segment, by column
+    __shared__ int sh[TP2_WARPS];
+    chain_wait();
+    const int nkp = ((1 << shift) + 3) & ~3, up = qbits + rbits, segs = of.seg0[*of.n];
+    const unsigned long long qmask = (1ull << qbits) - 1, rmask = (1ull << rbits) - 1;
+    for (int seg = blockIdx.x; seg < segs; seg += gridDim.x) {
+        int64_t at;
+        const int b = of.big[tp_segment(of, seg, at)];
+        const int64_t s0 = __ldg(start + b) + at, s1 = __ldg(start + b + 1);
+        const int m = (int)(s1 - s0 < TP2_SEG ? s1 - s0 : TP2_SEG);
+        const int64_t c0 = (int64_t)b << shift;
+        auto start_of = [&](int c, int4 first) {
+            const int4 d = *reinterpret_cast<const int4*>(seg_cnt + (int64_t)seg * nkp + c);
+            const int v[4] = {d.x - first.x, d.y - first.y, d.z - first.z, d.w - first.w};
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (c0 + c + u < cols) delta[c + u] = v[u] + t_rowptr[c0 + c + u];
+        };
+        tp_order(items + s0, m, up, shift, nw, nkp, cnt, sh, start_of,
+                 [&](int p, unsigned long long w) { place[p] = w; });
+        __syncthreads();
+        for (int p = threadIdx.x; p < m; p += TP2_T) {
+            const unsigned long long w = place[p];
+            to.put((int64_t)p + delta[w >> up], (int)(w & qmask), (int)(w >> qbits & rmask));
+        }
+        __syncthreads();
     }
 }
 
@@ -1393,22 +1562,40 @@ static int transpose_buckets(f4j_ctx* ctx, f4j_csr S, int shift, int qbits, int 
     const size_t smem1 = (size_t)TP1_TILE * 10 + (size_t)(TP1_WARPS + 1) * TP_NB * 4;
     const size_t smem2 = (size_t)TP2_CAP * 8 + (size_t)TP2_CNT * 4;
     F4J_CUDA(cudaFuncSetAttribute(k_tp_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1));
+    const size_t smem3 = (size_t)TP2_SEG * 8 + (size_t)(TP2_CNT + (4 << TP_BITS)) * 4;
     F4J_CUDA(cudaFuncSetAttribute(k_tp_bucket, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));
+    F4J_CUDA(cudaFuncSetAttribute(k_tp_seg_order, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3));
     int* hist = nullptr;
     unsigned long long* items = nullptr;
     const int nbp = (nb + 3) & ~3, chunks = (int)f4j_cdiv(nblocks, TP_CHUNK);
-    int rc = f4j_dev_alloc(ctx, ((size_t)(nblocks + chunks + 1) * nbp + 4) * 4, (void**)&hist);
+    // big buckets: of more items than shared memory places and twice the others' mean (evenly filled
+    // ones are as fast whole: 2^20 rows x 20, us, whole / in segments: 3000 columns 687 / 825, 2^20 998 /
+    // 1044; x 64 2519 / 2771, 4587 / 3265).  At most this many, and segments of them, whose counts take
+    // the place of hist, which is done with by then
+    const int64_t above = f4j_cdiv(2 * nnz, nb) > TP2_CAP ? f4j_cdiv(2 * nnz, nb) : TP2_CAP;
+    const int64_t bigs = shift ? nnz / (above + 1) : 0, segs = bigs ? nnz / TP2_SEG + bigs : 0;
+    const size_t rows_hist = (size_t)nblocks * nbp, rows_seg = (size_t)segs * (((1 << shift) + 3) & ~3);
+    const size_t head = rows_hist > rows_seg ? rows_hist : rows_seg;
+    int rc = f4j_dev_alloc(ctx, (head + (size_t)(chunks + 4) * nbp + 12) * 4, (void**)&hist);
     if (!rc && shift) rc = f4j_dev_alloc(ctx, (size_t)nnz * 8, (void**)&items);
     if (!rc) {
-        int *part = hist + (size_t)nblocks * nbp, *start = part + (size_t)chunks * nbp;
+        int *part = hist + head, *start = part + (size_t)chunks * nbp;
+        const TpBig big{(int)above, start + nbp + 4, start + nbp + 8, start + 2 * nbp + 8, start + 3 * nbp + 12};
         k_tp_hist<<<nblocks, 512, 0, ctx->stream>>>(nnz, col, shift, nbp, hist);
-        k_tp_chunks<<<dim3(chunks, (unsigned)f4j_cdiv(nbp, 256)), 64, 0, ctx->stream>>>(nblocks, nbp, hist, part);
-        k_tp_starts<<<1, TP_NB, 0, ctx->stream>>>(chunks, nb, nbp, part, start);
-        k_tp_scatter<<<nblocks, TP1_T, smem1, ctx->stream>>>(nnz, col, rowidx, shift, nb, qbits, rbits, hist, part, start,
-                                                             items, to);
+        f4j_launch(true, k_tp_chunks, dim3(chunks, (unsigned)f4j_cdiv(nbp, 256)), 64, 0, ctx->stream, nblocks, nbp, hist, part);
+        f4j_launch(true, k_tp_starts, 1, TP_NB, 0, ctx->stream, chunks, nb, nbp, part, start, big);
+        f4j_launch(true, k_tp_scatter, nblocks, TP1_T, smem1, ctx->stream, nnz, col, rowidx, shift, nb, qbits, rbits, hist,
+                   part, start, items, to);
         if (shift) {
             const int nw = TP2_WARPS < TP2_CNT >> shift ? TP2_WARPS : TP2_CNT >> shift;
-            k_tp_bucket<<<nb, TP2_T, smem2, ctx->stream>>>(cols, shift, qbits, rbits, nw, start, items, trp, to);
+            const int most = (int)(segs < ctx->sm_count ? segs : ctx->sm_count);
+            f4j_launch(true, k_tp_bucket, nb + most, TP2_T, smem2, ctx->stream, nb, cols, shift, qbits, rbits, nw, start,
+                       items, trp, to, big, hist);
+            if (most) {
+                f4j_launch(true, k_tp_seg_order, most, TP2_T, smem3, ctx->stream, cols, shift, qbits, rbits, nw, start, items,
+                           trp, to, big, hist);
+                ctx->launches++;
+            }
         } else {
             k_tp_rowptr<<<grid1(nb + 1), 256, 0, ctx->stream>>>(nb, start, trp);
         }

@@ -785,3 +785,39 @@ def test_sddmm_of_a_view_of_a_larger_pattern(f4j, first, tail, ncols):
         assert np.all(got[:first] == 7.0) and np.all(got[first + held:] == 7.0)
         assert np.all(np.abs(got[first:first + held] - terms.sum(1)) <= 2 * ncols * U * np.abs(terms).sum(1))
     check(ctx.lib.f4j_csr_free(ctx.handle, h))
+
+
+@pytest.mark.parametrize("cols,sizes", [
+    (5000, [18432, 18433, 16384, 32768]),            # the most a block places, one more, whole segments
+    (5000, [32769, 0, 40001, 18432, 65536 + 5]),     # segments with one item in the last
+    (1500, [30000, 100, 20000]),                     # two columns a bucket
+    (1 << 20, [200000, 3, 19000, 50000]), ((1 << 20) - 900, [70000, 1, 0, 90000]),
+    (1 << 22, [60000, 30000, 5, 20000]), ((1 << 22) - 4000, [0, 0, 0, 120000]),  # 4096 columns a bucket
+])
+@pytest.mark.parametrize("spread", ["even", "one column"])
+def test_transpose_of_skewed_columns(f4j, cols, sizes, spread):
+    """Buckets of columns with more nonzeros than a block places: stable column order, whatever their number,
+    their sizes and the columns inside (the last bucket, which may be short, among them)."""
+    g = np.random.default_rng(cols + sum(sizes))
+    shift = 0
+    while (cols - 1) >> shift >= 1024:
+        shift += 1
+    nb = ((cols - 1) >> shift) + 1
+    at = [3, 4, nb // 2, nb - 2, nb - 1]
+    col = [g.integers(0, cols, 5000)]
+    for b, n in zip(at[-len(sizes):], sizes):
+        c0, c1 = b << shift, min((b + 1) << shift, cols)
+        col.append(np.full(n, c1 - 1) if spread == "one column" else g.integers(c0, c1, n))
+    col = g.permutation(np.concatenate(col))
+    rows, nnz = 3000, len(col)
+    row = np.sort(g.integers(0, rows, nnz))
+    rp = np.zeros(rows + 1, np.int32)
+    np.cumsum(np.bincount(row, minlength=rows), out=rp[1:])
+    vals = g.standard_normal(nnz)
+    S = f4j.CsrMatrix((rows, cols), vals, rp, col.astype(np.int32), validate=False)
+    perm = np.argsort(col, kind="stable")
+    T = S.T()
+    assert np.array_equal(np.diff(T.rowPointers), np.bincount(col, minlength=cols))
+    assert np.array_equal(T.colIndices, row[perm])
+    assert np.array_equal(T.data, vals[perm])
+    assert np.array_equal(S.transposePermutation(), perm)
