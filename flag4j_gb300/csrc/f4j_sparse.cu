@@ -156,13 +156,15 @@ __global__ void __launch_bounds__(SPMV_BLOCK, SPMV_BLOCKS)
 // warp against warps.  Exact mode at 2^20 rows x 16 nonzeros, 32 columns: 1.79
 // ms, 95 % of the FP64 pipe's two lanes per SM and clock (2.07 ms with DMUL
 // and DADD for ExactOps); 64 columns 3.54 ms (4.02).
-// MIXED (exact mode, rows of different lengths in a warp): every group of eight
-// nonzeros under predicates, its sums in pairs that the warp leaves together, so
-// a warp takes its longest row's FP64 instructions, where whole groups and a
-// loop over the rest took the most of both: 2^20 rows x 16, us, 2 columns 228 / 191, 8
-// 819 / 626, 16 1326 / 1092.  5 blocks an SM (48 registers; 6 spill, 2 % slower).
-// With one row a warp the predicated rest costs more than the loop (32 columns
-// 1792 / 2225, without the pairs).
+// MIXED (exact mode, rows of different lengths in a warp): a group of eight
+// nonzeros that is not whole in every row still running goes under predicates, its
+// sums in pairs that the warp leaves together, so a warp takes its longest row's
+// FP64 instructions, where whole groups and a loop over the rest took the most of
+// both: 2^20 rows x 16, us, 2 columns 228 / 181, 8 819 / 594, 16 1326 / 1069.  Groups
+// whole in all of them go without predicates, which is what long rows take: 80 % of
+// 4.2 M nonzeros in 1024 rows, 8 columns 694 with predicates throughout, 613 so.  5
+// blocks an SM (48 registers; 6 spill, 2 % slower).  With one row a warp the
+// predicated rest costs more than the loop (32 columns 1792 / 2225, without the pairs).
 template <bool VEC2, bool PERM, bool FUSED = false, bool MIXED = false>
 __global__ void __launch_bounds__(256, FUSED ? 8 : (MIXED ? 5 : 6))
     k_spmm(int64_t rows, int64_t ncols, int G, const int* __restrict__ rowptr, const int* __restrict__ colidx,
@@ -181,6 +183,16 @@ __global__ void __launch_bounds__(256, FUSED ? 8 : (MIXED ? 5 : 6))
         if constexpr (MIXED) {
             for (; q < q1; q += UN) {
                 double v[UN], xv[UN];
+                if (__all_sync(__activemask(), q + UN <= q1)) {
+#pragma unroll
+                    for (int u = 0; u < UN; u++) {
+                        v[u] = PERM ? __ldg(&vals[__ldg(&perm[q + u])]) : __ldg(&vals[q + u]);
+                        xv[u] = __ldg(X + (int64_t)__ldg(&colidx[q + u]) * ncols + cbase);
+                    }
+#pragma unroll
+                    for (int u = 0; u < UN; u++) a0 = ops.add(ops.mul(v[u], xv[u]), a0);
+                    continue;
+                }
 #pragma unroll
                 for (int u = 0; u < UN; u++) {
                     v[u] = xv[u] = 0.0;

@@ -821,3 +821,22 @@ def test_transpose_of_skewed_columns(f4j, cols, sizes, spread):
     assert np.array_equal(T.colIndices, row[perm])
     assert np.array_equal(T.data, vals[perm])
     assert np.array_equal(S.transposePermutation(), perm)
+
+
+@pytest.mark.parametrize("ncols", [1, 3, 8, 16, 24])
+@pytest.mark.parametrize("lens", ["eights", "one long", "long neighbours"])
+def test_spmm_whole_groups_and_long_rows_bit_identical(f4j, oracle, ncols, lens):
+    """Rows that share a warp: all of whole groups of eight nonzeros, one far longer than the others, and
+    long ones that end at different places."""
+    g = np.random.default_rng(ncols)
+    rows, cols = 130, 6000
+    n = {"eights": 8 * g.integers(0, 5, rows), "one long": g.integers(0, 12, rows),
+         "long neighbours": g.integers(990, 1010, rows)}[lens]
+    if lens == "one long":
+        n[41] = 5003
+    rp = np.zeros(rows + 1, np.int32)
+    np.cumsum(n, out=rp[1:])
+    ci = np.concatenate([np.sort(g.choice(cols, k, replace=False)) for k in n]).astype(np.int32)
+    v, X = g.standard_normal(len(ci)), g.standard_normal((cols, ncols))
+    S = f4j.CsrMatrix((rows, cols), v, rp, ci)
+    assert np.array_equal(S.mult(f4j.Matrix(X)).toNumpy(), oracle.spmm(rp, ci, v, X))
