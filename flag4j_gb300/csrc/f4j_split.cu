@@ -261,6 +261,17 @@ __global__ void k_stats_cols(const double* __restrict__ X, int64_t rows, int64_t
     chain_wait();
 }
 
+// 256 num / cnt to the nearest integer, halves up, for 0 < num < 2^11 cnt: a float
+// quotient, which is off by one at most, and the exact remainder's verdict on it
+// (GB300's FP64 division would be the longest wait of the kernel that calls this).
+__host__ __device__ inline int spread_x256(long long num, int cnt) {
+    int q = (int)((float)num / (float)cnt * 256.0f + 0.5f);
+    const long long twice = 2ll * cnt, rem = 512 * num + cnt - twice * q;
+    if (rem < 0) q--;
+    if (rem >= twice) q++;
+    return q;
+}
+
 // Exponent bound e (max|x| < 2^e) of target t, and its spread (x256).
 __device__ __forceinline__ int finalize_target(int64_t t, int64_t targets, int dup,
                                                const unsigned long long* __restrict__ mx,
@@ -276,11 +287,9 @@ __device__ __forceinline__ int finalize_target(int64_t t, int64_t targets, int d
             // in the fixed-point form instead of being rounded at 2^(-1022 - F)
             int E = (int)(b >> 52);
             e = E ? E - 1022 : (63 - __clzll((long long)b)) - 1073;
-            // (e - 1) - mean exponent, from its exact numerator: 32 bits carry it to
-            // 2^-8 for any spread, and GB300's FP64 division would be the longest
-            // wait of this kernel
+            // (e - 1) - mean exponent, from its exact numerator
             const long long num = (long long)(e - 1) * cnt[t] - esum[t];
-            sp = num > 0 ? (int)((float)num / (float)cnt[t] * 256.0f + 0.5f) : 0;
+            sp = num > 0 ? spread_x256(num, cnt[t]) : 0;
         }
         e_out[t] = e;
         if (dup) e_out[t + targets] = e;
