@@ -1,5 +1,6 @@
 // f4j_core.cu -- contexts, device buffers, errors, timers and the dense
 // front ends of libflag4j_cuda.so.
+#include <cstdlib>
 #include <mutex>
 
 #include "f4j_internal.cuh"
@@ -281,6 +282,40 @@ int f4j_workspace(f4j_ctx* ctx, int slot, size_t bytes, void** out) {
     }
     *out = ctx->ws[slot];
     return F4J_OK;
+}
+
+int f4j_workspace_optional(f4j_ctx* ctx, int slot, size_t bytes, void** out) {
+    if (slot < 0 || slot >= 8) return f4j_fail(F4J_ERR_ARG, "workspace slot %d", slot);
+    const size_t held = ctx->ws_bytes[slot], want = bytes + bytes / 8;
+    if (bytes <= held && held) {
+        *out = ctx->ws[slot];
+        return F4J_OK;
+    }
+    const char* cap = getenv("F4J_WORKSPACE_MB");
+    const size_t limit = cap ? (size_t)strtoull(cap, nullptr, 10) << 20 : SIZE_MAX;
+    size_t room = 0, total = 0;
+    if (want <= limit) {
+        F4J_CUDA(cudaMemGetInfo(&room, &total));
+        room += held;
+    }
+    // asked before, with as much room: no allocation, no free and no wait this time
+    f4j_ctx::Refusal& no = ctx->ws_refused[slot];
+    if (want > limit || (no.want && want >= no.want && room <= no.room))
+        return f4j_fail(F4J_ERR_OOM, "workspace of %zu bytes: no room", want);
+    void* p = nullptr;
+    const cudaError_t e = cudaMalloc(&p, want);  // beside the slot's own, which stays if this fails
+    if (e == cudaSuccess) {
+        F4J_CUDA(cudaStreamSynchronize(ctx->stream));
+        if (ctx->ws[slot]) cudaFree(ctx->ws[slot]);
+        ctx->ws[slot] = *out = p;
+        ctx->ws_bytes[slot] = want;
+        return F4J_OK;
+    }
+    cudaGetLastError();
+    if (held && room >= want && f4j_workspace(ctx, slot, bytes, out) == F4J_OK) return F4J_OK;
+    no.want = want;
+    no.room = room;
+    return f4j_fail(F4J_ERR_OOM, "workspace of %zu bytes: %s", want, cudaGetErrorString(e));
 }
 
 int f4j_dev_alloc(f4j_ctx* ctx, size_t bytes, void** out) {

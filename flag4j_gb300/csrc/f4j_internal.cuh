@@ -56,6 +56,9 @@ struct f4j_ctx {
     void* ws[8];       // grow-only workspaces (slot ws_base + 0: split bulk, ws_base + 1: split
     size_t ws_bytes[8];  // small/stats; 2: sparse; 4-5: the second product of an adjoint;
                          // 3, 6, 7: A, B, C of f4j_dgemm_host)
+    struct Refusal {
+        size_t want, room;
+    } ws_refused[8];   // what f4j_workspace_optional could not have, and the room there was (0: nothing)
     int ws_base;       // first split workspace slot (0, or 4 while an adjoint's second product is queued)
     cudaStream_t aux_stream;  // second stream of an adjoint (created on first use)
     cudaEvent_t ev_fork, ev_join;
@@ -146,6 +149,10 @@ inline void f4j_launch(bool after, void (*kernel)(P...), dim3 grid, dim3 block, 
 // Workspace slot of at least `bytes` (stream-ordered reuse; growing syncs the
 // stream and discards the slot's previous contents).
 int f4j_workspace(f4j_ctx* ctx, int slot, size_t bytes, void** out);
+// The same for a caller that can do without: F4J_ERR_OOM leaves the slot as it is,
+// and costs no allocation, free or wait again while there is no more room than the
+// last time.  F4J_WORKSPACE_MB in the environment caps what it asks for.
+int f4j_workspace_optional(f4j_ctx* ctx, int slot, size_t bytes, void** out);
 // Device allocation helpers (stream-ordered pool).
 int f4j_dev_alloc(f4j_ctx* ctx, size_t bytes, void** out);
 void f4j_dev_free(f4j_ctx* ctx, void* p);

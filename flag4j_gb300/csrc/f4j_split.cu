@@ -1676,7 +1676,7 @@ static int crt_setup(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, C
     int rc = f4j_workspace(ctx, ctx->ws_base + 1, S->Lo.total, &ws1);
     if (rc) return rc;
     const size_t pa = al1k(S->plane_a * S->planes), pb = al1k(S->plane_b * S->planes);
-    rc = f4j_workspace(ctx, ctx->ws_base, pa + pb + (size_t)S->nmod * S->yrows * S->ldy * 2, &ws0);
+    rc = f4j_workspace_optional(ctx, ctx->ws_base, pa + pb + (size_t)S->nmod * S->yrows * S->ldy * 2, &ws0);
     if (rc) return rc;
     char* w = S->w = (char*)ws1;
     S->mxa = (unsigned long long*)(w + S->Lo.mxa);
@@ -2191,19 +2191,7 @@ static int gemm_host(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, c
     // n == 1 runs the device path's matrix-vector kernel
     const bool split = k > 0 && n > 1 && f4j_resolve_mode(cplx, m, n, k, mode) == F4J_MODE_SPLIT;
     // the residue form's parts are whole 256 x 256 tiles and need all of C's residues at once
-    const bool crt = split && crt_wanted(cplx, m, n, k, 0, mode == F4J_MODE_AUTO);
-    const int tile = crt ? CG_T : BM;
-    const int tiles_m = (int)f4j_cdiv(m, tile);
-    const int want = env_host_parts("F4J_HOST_PARTS", F4J_HOST_PARTS);
-    const int parts = tiles_m < want ? tiles_m : want;
-    const int bparts = env_host_parts("F4J_HOST_BPARTS", F4J_HOST_BPARTS);
-    const int64_t ncat = cplx ? 2 * n : n;  // slice rows of B (the [Re | Im] concatenation when complex)
-    const int tiles_n = (int)f4j_cdiv(ncat, tile);
-    // pipelined when A has two row parts or B two column parts (real only)
-    const bool piped = parts >= 2 || (!cplx && bparts >= 2 && tiles_n >= 2);
-    int kchunks = 0;
-    if (!crt) split_kcb_cap(tiles_m * (int64_t)tiles_n, (cplx ? 2 : 1) * f4j_cdiv(k, BKB), &kchunks);
-    const bool blocks = crt && (size_t)CRT_NB * 2 * (m + CG_T) * (ncat + 16) > CRT_Y_BYTES;
+    bool crt = split && crt_wanted(cplx, m, n, k, 0, mode == F4J_MODE_AUTO);
     auto in_turn = [&]() -> int {  // upload, multiply, download
         if (ab) F4J_CUDA(cudaMemcpyAsync(dA, A, ab, cudaMemcpyHostToDevice, ctx->stream));
         if (bb) F4J_CUDA(cudaMemcpyAsync(dB, B, bb, cudaMemcpyHostToDevice, ctx->stream));
@@ -2215,7 +2203,7 @@ static int gemm_host(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, c
         return f4j_report_accuracy(ctx, cplx, m, n, k, (const double*)dA, opA, (const double*)dB, opB,
                                    (const double*)dC, check_samples, check_flags, rep);
     };
-    if (!split || opA != F4J_OP_N || !piped || kchunks || blocks) return in_turn();  // split K runs as one launch
+    if (!split || opA != F4J_OP_N) return in_turn();
     if (!ctx->parts_init) {
         for (int i = 0; i < F4J_HOST_STREAMS; i++) {
             F4J_CUDA(cudaStreamCreateWithFlags(&ctx->part_stream[i], cudaStreamNonBlocking));
@@ -2231,9 +2219,25 @@ static int gemm_host(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, c
     bool recompute = false;
     const SplitPlan* plan = nullptr;
     float spread = 0.0f;
-    rc = host_split_pipelined(ctx, cplx, m, n, k, A, B, opB, C, (double*)dA, (double*)dB, (double*)dC, crt, parts,
-                              bparts, &recompute, &plan, &spread);
-    if (rc == F4J_ERR_OOM && crt) return in_turn();  // no room for the residue planes
+    for (;;) {
+        const int tile = crt ? CG_T : BM;
+        const int tiles_m = (int)f4j_cdiv(m, tile);
+        const int want = env_host_parts("F4J_HOST_PARTS", F4J_HOST_PARTS);
+        const int parts = tiles_m < want ? tiles_m : want;
+        const int bparts = env_host_parts("F4J_HOST_BPARTS", F4J_HOST_BPARTS);
+        const int64_t ncat = cplx ? 2 * n : n;  // slice rows of B (the [Re | Im] concatenation when complex)
+        const int tiles_n = (int)f4j_cdiv(ncat, tile);
+        // pipelined when A has two row parts or B two column parts (real only)
+        const bool piped = parts >= 2 || (!cplx && bparts >= 2 && tiles_n >= 2);
+        int kchunks = 0;
+        if (!crt) split_kcb_cap(tiles_m * (int64_t)tiles_n, (cplx ? 2 : 1) * f4j_cdiv(k, BKB), &kchunks);
+        const bool blocks = crt && (size_t)CRT_NB * 2 * (m + CG_T) * (ncat + 16) > CRT_Y_BYTES;
+        if (!piped || kchunks || blocks) return in_turn();  // split K runs as one launch
+        rc = host_split_pipelined(ctx, cplx, m, n, k, A, B, opB, C, (double*)dA, (double*)dB, (double*)dC, crt, parts,
+                                  bparts, &recompute, &plan, &spread);
+        if (rc != F4J_ERR_OOM || !crt) break;
+        crt = false;  // no room for the residue planes: slices, as the device path takes then
+    }
     if (rc) return rc;
     if (recompute) {
         // all of A and B ask for another slice count than their first parts

@@ -236,7 +236,11 @@ int f4j_buf_wrap(f4j_ctx* ctx, void* ptr, size_t bytes, f4j_buf* out);
  *    src/main/java/org/flag4j/linalg/ops/dispatch/ReDeMatMultDispatcher.java:157-237)
  * and, with opB = F4J_OP_T, Matrix.multTranspose
  *   (Matrix.java:655-663, RealDenseMatrixMultiplyDispatcher.java:148-154).
- * A is stored m x k (opA N) or k x m (opA T); B k x n (N) or n x k (T). */
+ * A is stored m x k (opA N) or k x m (opA T); B k x n (N) or n x k (T).
+ * A split product's residue form needs about 2.5 times the slices' workspace, and
+ * 30 bytes an entry of C (up to 4 GiB).  Where the device has no room for it, or
+ * F4J_WORKSPACE_MB in the environment allows less, the slices compute the product:
+ * within the same bound, but not the same last bits. */
 int f4j_dgemm(f4j_ctx* ctx, int64_t m, int64_t n, int64_t k, f4j_buf A, int opA, f4j_buf B,
               int opB, f4j_buf C, int mode, f4j_report* report);
 /* f4j_dgemm from and to host memory: A, B, C are host pointers (row-major;

@@ -1,0 +1,82 @@
+"""The residue form's workspace: what a product does when it cannot have it, and that the host-buffer products
+agree with the device's in AUTO, whichever form that is."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from test_gpu_capture import capturing_context
+
+pytestmark = pytest.mark.gpu
+
+
+def product(ctx, A, B, mode, host=False):
+    from flag4j_gb300.device import check
+    m, k = A.shape
+    n = B.shape[1]
+    if host:
+        C = np.empty((m, n), A.dtype)
+        fn = ctx.lib.f4j_zgemm_host if np.iscomplexobj(A) else ctx.lib.f4j_dgemm_host
+        check(fn(ctx.handle, m, n, k, A.ctypes.data, 0, B.ctypes.data, 0, C.ctypes.data, mode, None))
+        return C
+    dA, dB, dC = ctx.from_numpy(A), ctx.from_numpy(B), ctx.alloc(A.dtype.itemsize * m * n)
+    fn = ctx.lib.f4j_zgemm if np.iscomplexobj(A) else ctx.lib.f4j_dgemm
+    check(fn(ctx.handle, m, n, k, dA.handle, 0, dB.handle, 0, dC.handle, mode, None))
+    return dC.to_numpy(A.dtype, m * n).reshape(m, n)
+
+
+def operands(m, n, k, seed=1, cplx=False):
+    g = np.random.default_rng(seed)
+    mk = lambda *s: g.standard_normal(s) + 1j * g.standard_normal(s) if cplx else g.standard_normal(s)
+    return mk(m, k), mk(k, n)
+
+
+@pytest.mark.parametrize("m,n,k", [(2111, 1777, 700), (2000, 2000, 640)])
+def test_no_room_for_the_residues_takes_the_slices(f4j, monkeypatch, m, n, k):
+    """With its workspace capped an AUTO product is the sliced one, on the device and from host arrays; with the
+    cap gone the same context takes the residues."""
+    from flag4j_gb300 import _lib
+    A, B = operands(m, n, k)
+    ctx = f4j.Context(0)
+    sliced = product(ctx, A, B, _lib.MODE_SPLIT)  # f4j_dgemm_split_noalloc accepts these shapes
+    monkeypatch.setenv("F4J_WORKSPACE_MB", "48")
+    other = f4j.Context(0)
+    for _ in range(2):
+        assert np.array_equal(product(other, A, B, _lib.MODE_AUTO), sliced)
+        assert np.array_equal(product(other, A, B, _lib.MODE_AUTO, host=True), sliced)
+    monkeypatch.delenv("F4J_WORKSPACE_MB")
+    residues = product(other, A, B, _lib.MODE_AUTO)
+    assert not np.array_equal(residues, sliced)
+    assert np.array_equal(residues, product(ctx, A, B, _lib.MODE_AUTO))
+    assert np.array_equal(residues, product(ctx, A, B, _lib.MODE_AUTO, host=True))
+
+
+def test_a_refused_workspace_costs_nothing_again(f4j, monkeypatch):
+    """Once refused, a product neither allocates nor frees nor waits: it can be captured."""
+    import torch
+    from flag4j_gb300 import _lib
+    from flag4j_gb300.device import check
+    A, B = operands(2000, 1900, 640)
+    monkeypatch.setenv("F4J_WORKSPACE_MB", "48")
+    with capturing_context(f4j) as (ctx, capture):
+        want = product(ctx, A, B, _lib.MODE_AUTO)
+        dA, dB, dC = ctx.from_numpy(A), ctx.from_numpy(B), ctx.alloc(8 * 2000 * 1900)
+        dC.zero()
+        ctx.sync()
+        graph = capture(lambda: check(ctx.lib.f4j_dgemm(ctx.handle, 2000, 1900, 640, dA.handle, 0, dB.handle, 0, dC.handle,
+                                                        _lib.MODE_AUTO, None)))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(dC.to_numpy(np.float64, 2000 * 1900).reshape(2000, 1900), want)
+
+
+@pytest.mark.parametrize("m,n,k,cplx", [
+    (300, 300, 300, False), (1024, 1024, 1024, False), (1300, 700, 512, False), (129, 2048, 300, False),  # SPLIT: slices
+    (2111, 1777, 700, False), (1300, 1300, 449, False), (600, 500, 400, True),  # complex
+])
+def test_host_product_is_the_device_product_in_auto(f4j, m, n, k, cplx):
+    """f4j_dgemm_host and f4j_zgemm_host in AUTO: bit for bit f4j_dgemm's and f4j_zgemm's AUTO."""
+    from flag4j_gb300 import _lib
+    A, B = operands(m, n, k, m + k, cplx)
+    ctx = f4j.default_context()
+    assert np.array_equal(product(ctx, A, B, _lib.MODE_AUTO, host=True), product(ctx, A, B, _lib.MODE_AUTO))
