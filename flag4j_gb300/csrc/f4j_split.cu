@@ -1625,6 +1625,12 @@ static int make_crt_map(CUtensorMap* map, const void* base, uint64_t Kp, uint64_
 // Residues of C (2 bytes per modulus and entry) up to this size are kept for
 // all of C; a larger product goes in row blocks of it.
 constexpr size_t CRT_Y_BYTES = size_t(4) << 30;
+// A host-buffer product in parts keeps all of C's up to this size: its parts run at
+// once.  Up, through and down in turn it is slower than in slices: ms, slices in
+// parts / residues in turn / in parts: 12000 x 12100 x 1024 11.0 / 12.0 / 9.8, 16384 x
+// 16384 x 1024 20.3 / 21.0 / 17.8, 26000 x 26000 x 1024 51.8 / - / 48.0; past this
+// size not any more: 36000 x 36000 x 1024 99.7 / 98.4 / -.
+constexpr size_t CRT_HOST_Y_BYTES = size_t(32) << 30;
 
 // A residue-form product's sizes and workspace.
 struct CrtSetup {
@@ -1644,7 +1650,7 @@ struct CrtSetup {
     size_t smem;
 };
 
-static int crt_setup(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, CrtSetup* S) {
+static int crt_setup(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, size_t y_bytes, CrtSetup* S) {
     S->half = cplx ? f4j_cdiv(n, 8) * 8 : 0;  // the imaginary half's first row of B_cat^T
     S->M = m;
     S->N = cplx ? 2 * S->half : n;
@@ -1669,7 +1675,7 @@ static int crt_setup(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, C
     S->ldy = f4j_cdiv(S->N, 16) * 16;  // rows of y start on 32-byte sectors
     S->tiles_m = (int)f4j_cdiv(S->M, CG_T);
     S->tiles_n = (int)f4j_cdiv(S->N, CG_T);
-    const int64_t fit = (int64_t)(CRT_Y_BYTES / ((size_t)S->nmod * S->ldy * 2)) / CG_T;
+    const int64_t fit = (int64_t)(y_bytes / ((size_t)S->nmod * S->ldy * 2)) / CG_T;
     S->blk = fit < 1 ? 1 : (fit > S->tiles_m ? S->tiles_m : fit);
     S->yrows = S->blk * CG_T < S->M ? S->blk * CG_T : S->M;
     void *ws1, *ws0;
@@ -1746,7 +1752,7 @@ static int crt_launch(f4j_ctx* ctx, const CrtSetup& S, bool cplx, int64_t n, dou
 static int crt_gemm(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, const double* A, int opA,
                     const double* B, int opB, double* C, const SplitPlan** plan_out) {
     CrtSetup S;
-    int rc = crt_setup(ctx, cplx, m, n, k, &S);
+    int rc = crt_setup(ctx, cplx, m, n, k, CRT_Y_BYTES, &S);
     if (rc) return rc;
     const int64_t M = S.M;
     F4J_CUDA(cudaMemsetAsync(S.w, 0, S.Lo.plan, ctx->stream));
@@ -1880,7 +1886,7 @@ static int host_split_pipelined(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, i
     CrtSetup R;
     int rc = F4J_OK;
     if (crt) {
-        rc = crt_setup(ctx, cplx, m, n, k, &R);
+        rc = crt_setup(ctx, cplx, m, n, k, CRT_HOST_Y_BYTES, &R);
         if (rc) return rc;
         if (R.blk < R.tiles_m) return f4j_fail(F4J_ERR_ARG, "residue-form product in parts and row blocks");
     }
@@ -2231,11 +2237,12 @@ static int gemm_host(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, c
         const bool piped = parts >= 2 || (!cplx && bparts >= 2 && tiles_n >= 2);
         int kchunks = 0;
         if (!crt) split_kcb_cap(tiles_m * (int64_t)tiles_n, (cplx ? 2 : 1) * f4j_cdiv(k, BKB), &kchunks);
-        const bool blocks = crt && (size_t)CRT_NB * 2 * (m + CG_T) * (ncat + 16) > CRT_Y_BYTES;
-        if (!piped || kchunks || blocks) return in_turn();  // split K runs as one launch
+        const size_t y = crt ? (size_t)CRT_NB * 2 * (m + CG_T) * (ncat + 16) : 0;
+        if (!piped || kchunks || y > CRT_HOST_Y_BYTES) return in_turn();  // split K runs as one launch
         rc = host_split_pipelined(ctx, cplx, m, n, k, A, B, opB, C, (double*)dA, (double*)dB, (double*)dC, crt, parts,
                                   bparts, &recompute, &plan, &spread);
         if (rc != F4J_ERR_OOM || !crt) break;
+        if (y > CRT_Y_BYTES) return in_turn();  // row blocks may fit
         crt = false;  // no room for the residue planes: slices, as the device path takes then
     }
     if (rc) return rc;

@@ -80,3 +80,24 @@ def test_host_product_is_the_device_product_in_auto(f4j, m, n, k, cplx):
     A, B = operands(m, n, k, m + k, cplx)
     ctx = f4j.default_context()
     assert np.array_equal(product(ctx, A, B, _lib.MODE_AUTO, host=True), product(ctx, A, B, _lib.MODE_AUTO))
+
+
+@pytest.mark.parametrize("m,n,k,cplx", [
+    (12000, 12100, 330, False),    # C's residues past 4 GiB: row blocks on the device, all at once from the host
+    (2200000, 160, 330, False),    # and more than 65535 blocks of rows of A
+    (8100, 9000, 170, True),
+])
+def test_large_results_in_row_blocks(f4j, m, n, k, cplx):
+    """Integer operands whose sums stay below 2^53: C is the exact product, and the host-buffer product the same."""
+    from flag4j_gb300 import _lib
+    from flag4j_gb300.device import check
+    g = np.random.default_rng(m)
+    mk = lambda *s: g.integers(-30000, 30000, s, dtype=np.int32).astype(np.float64)
+    A, B = mk(m, k), mk(k, n)
+    if cplx:
+        A, B = A + 1j * mk(m, k), B + 1j * mk(k, n)
+    ctx = f4j.Context(0)  # its workspace goes with it
+    want = A @ B
+    assert np.array_equal(product(ctx, A, B, _lib.MODE_AUTO), want)
+    assert np.array_equal(product(ctx, A, B, _lib.MODE_AUTO, host=True), want)
+    ctx.close()
