@@ -360,7 +360,8 @@ int ref_kernel(const f4j_dispatch_config& d, bool cplx, int64_t m, int64_t n, in
 
 }  // namespace
 
-int f4j_resolve_mode(bool cplx, int64_t m, int64_t n, int64_t k, int mode) {
+int f4j_resolve_mode(bool cplx, int64_t m, int64_t n, int64_t k, int mode, bool* any_form) {
+    if (any_form) *any_form = false;
     if (mode != F4J_MODE_AUTO) return mode;
     f4j_dispatch_config d;
     {
@@ -373,7 +374,9 @@ int f4j_resolve_mode(bool cplx, int64_t m, int64_t n, int64_t k, int mode) {
     // products of a few microseconds of work keep the reference's order too
     const double work = (cplx ? 8.0 : 2.0) * (double)m * (double)n * (double)k;
     if (work <= (double)(1 << 24)) return F4J_MODE_EXACT;
-    return d.gpu_gemm_mode == F4J_MODE_AUTO ? F4J_MODE_SPLIT : d.gpu_gemm_mode;
+    if (d.gpu_gemm_mode != F4J_MODE_AUTO) return d.gpu_gemm_mode;
+    if (any_form) *any_form = true;
+    return F4J_MODE_SPLIT;
 }
 
 extern "C" int f4j_config_load(const char* dir) {

@@ -521,11 +521,8 @@ int f4j_gemm_impl(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, cons
     // AUTO follows the dispatcher configuration: the reference's small-product
     // rule and products of a few microseconds of work run Flag4j's own order
     // (bit-identical); larger ones take the configured GPU path (f4j_config.cu).
-    const bool any_form = mode == F4J_MODE_AUTO;
-    if (mode == F4J_MODE_AUTO) {
-        mode = f4j_resolve_mode(cplx, m, n, k, mode);
-        if (mode == F4J_MODE_AUTO) mode = F4J_MODE_SPLIT;
-    }
+    bool any_form = false;
+    mode = f4j_resolve_mode(cplx, m, n, k, mode, &any_form);
     int rc = F4J_OK;
     int used = mode;
     if (k == 0) {

@@ -181,7 +181,9 @@ static inline bool f4j_aligned(const void* p, uintptr_t n) { return (reinterpret
 
 // The mode a dense product runs in: F4J_MODE_AUTO resolved by the dispatcher
 // configuration (f4j_config.cu); other modes unchanged.
-int f4j_resolve_mode(bool cplx, int64_t m, int64_t n, int64_t k, int mode);
+// *any_form: nobody asked for SPLIT by name, so the faster of its forms may run also
+// where f4j_dgemm_split_noalloc fixes that mode's bits.
+int f4j_resolve_mode(bool cplx, int64_t m, int64_t n, int64_t k, int mode, bool* any_form = nullptr);
 
 // Fills a dense product's report with its accuracy fields (check_samples,
 // check_flags as the caller set them; see f4j_report).
@@ -211,8 +213,7 @@ int f4j_check_sampled(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, 
                       double* max_rel);
 int f4j_gemm_exact(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, const double* A,
                    int opA, const double* B, int opB, double* C);
-// any_form: the caller did not ask for F4J_MODE_SPLIT itself, so the faster of
-// the split forms may run also where f4j_dgemm_split_noalloc fixes the bits.
+// any_form: as f4j_resolve_mode gives it.
 int f4j_gemm_split(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, const double* A,
                    int opA, const double* B, int opB, double* C, int slices_req, bool any_form,
                    f4j_report* rep, const int** gate);

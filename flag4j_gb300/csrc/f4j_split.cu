@@ -2195,9 +2195,10 @@ static int gemm_host(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, c
     if (!rc) rc = f4j_workspace(ctx, 7, cb, &dC);
     if (rc) return rc;
     // n == 1 runs the device path's matrix-vector kernel
-    const bool split = k > 0 && n > 1 && f4j_resolve_mode(cplx, m, n, k, mode) == F4J_MODE_SPLIT;
+    bool any_form = false;
+    const bool split = k > 0 && n > 1 && f4j_resolve_mode(cplx, m, n, k, mode, &any_form) == F4J_MODE_SPLIT;
     // the residue form's parts are whole 256 x 256 tiles and need all of C's residues at once
-    bool crt = split && crt_wanted(cplx, m, n, k, 0, mode == F4J_MODE_AUTO);
+    bool crt = split && crt_wanted(cplx, m, n, k, 0, any_form);
     auto in_turn = [&]() -> int {  // upload, multiply, download
         if (ab) F4J_CUDA(cudaMemcpyAsync(dA, A, ab, cudaMemcpyHostToDevice, ctx->stream));
         if (bb) F4J_CUDA(cudaMemcpyAsync(dB, B, bb, cudaMemcpyHostToDevice, ctx->stream));

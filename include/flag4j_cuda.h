@@ -52,13 +52,16 @@ extern "C" {
 #define F4J_MODE_PLAIN 0 /* FP64 DMMA tensor-core GEMM (mma.sync f64)                   */
 #define F4J_MODE_SPLIT 1 /* FP64-accurate split GEMM: FP8 on tcgen05, exact FP32.  Two forms
                             by shape: slices, or residues modulo small coprime numbers
-                            (from about 400 x 400 x 600).  Shapes that
-                            f4j_dgemm_split_noalloc accepts run its slices, bit for bit  */
+                            (both sides above 128, sums of 256 terms and more).  Shapes
+                            that f4j_dgemm_split_noalloc accepts (1024 x 1024 x 1344, say)
+                            run its slices, bit for bit                                 */
 #define F4J_MODE_AUTO 2  /* the dispatcher configuration's choice (f4j_config_load): EXACT
                             below smallThreshold entries or 2^24 flops; otherwise
-                            gpuGemmMode, by default SPLIT (the faster form for the shape,
-                            also where F4J_MODE_SPLIT keeps to slices) for finite inputs
-                            and PLAIN when a NaN/Inf is present                         */
+                            gpuGemmMode, by default SPLIT for finite inputs and PLAIN when
+                            a NaN/Inf is present.  By default the faster form runs also
+                            where F4J_MODE_SPLIT keeps to slices (1024^3: 90 us for 123),
+                            so the last bits may differ from that mode's; with
+                            gpuGemmMode = split they are that mode's                    */
 #define F4J_MODE_EXACT 3 /* Flag4j's own order: k-ascending, no FMA -> bit-identical     */
 
 typedef struct f4j_ctx f4j_ctx;

@@ -71,3 +71,23 @@ def test_split_mode_keeps_the_slices_of_the_no_allocation_shapes(f4j, m, n, k, f
     for host in (False, True):
         good, of = rounded_once(A, B, product(f4j, A, B, _lib.MODE_SPLIT, host=host))
         assert (good == of) == (form == "residues"), (good, of, host)
+
+
+def test_auto_with_split_configured_by_name_is_split(f4j, tmp_path):
+    """gpuGemmMode = split: AUTO's bits are F4J_MODE_SPLIT's, from the device and from host arrays, where the
+    default takes the residues."""
+    from flag4j_gb300 import _lib, configs
+    A, B = ints45((700, 300), 1), ints45((300, 600), 2)
+    sliced = product(f4j, A, B, _lib.MODE_SPLIT)
+    try:
+        (tmp_path / "GeneralConfigs.properties").write_text("gpuGemmMode = split\n")
+        configs.load(tmp_path)
+        for host in (False, True):
+            assert np.array_equal(product(f4j, A, B, _lib.MODE_AUTO, host=host), sliced)
+        (tmp_path / "GeneralConfigs.properties").write_text("gpuGemmMode = auto\n")
+        configs.load(tmp_path)
+        for host in (False, True):
+            C = product(f4j, A, B, _lib.MODE_AUTO, host=host)
+            assert not np.array_equal(C, sliced) and len(set(rounded_once(A, B, C))) == 1
+    finally:
+        configs.reset()
