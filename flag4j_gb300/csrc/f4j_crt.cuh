@@ -15,7 +15,7 @@
 // A product of 8192 terms at F = 49 needs 112 bits: eight squares and seven
 // single moduli, 31 FP8 products where the slices take 55 (66 -> 34 or 35 at
 // F = 54), and no slice product is dropped: C' is exact and C is C' 2^(..)
-// rounded once.
+// rounded once (where that is subnormal, to 53 bits first).
 //
 //  k_crt_planes   Y of each element, then its residues' digits, one E4M3 plane
 //                 per digit (K-major, as the slice planes).
@@ -24,7 +24,7 @@
 //                 over at most 8192 terms), reduced mod p and multiplied by the
 //                 modulus's weight (M / p)^-1: an int16 plane per modulus.
 //  k_crt_combine  sum_l y_l (M / p_l) in 32-bit words, reduced mod M, rounded to
-//                 double once and scaled.
+//                 double and scaled.
 //
 // Included by f4j_split.cu.
 #pragma once
@@ -888,17 +888,8 @@ __global__ void __launch_bounds__(CG_THREADS, 1) __cluster_dims__(2, 1, 1)
 }
 
 // ------------------------------------------------------------------ reconstruction
-// round(sign mag 2^X) of a 192-bit magnitude (w2, w1, w0), to nearest even.
-__device__ __forceinline__ double crt_round(unsigned long long w2, unsigned long long w1, unsigned long long w0,
-                                            bool neg, int X) {
-    if (w2) {  // five-limb sums only
-        const int z = 64 - __clzll((long long)w2);  // 1..64 bits to drop from the bottom
-        const unsigned long long lost = z == 64 ? w0 : w0 << (64 - z);
-        w0 = z == 64 ? w1 : (w0 >> z) | (w1 << (64 - z));
-        w1 = z == 64 ? w2 : (w1 >> z) | (w2 << (64 - z));
-        w0 |= lost ? 1ull : 0ull;
-        X += z;
-    }
+// round(sign mag 2^X) of a 128-bit magnitude (w1, w0), to nearest even.
+__device__ __forceinline__ double crt_round(unsigned long long w1, unsigned long long w0, bool neg, int X) {
     if (!w1) {
         if (!w0) return 0.0;
         w1 = w0;
@@ -947,10 +938,8 @@ __device__ __forceinline__ double crt_value(unsigned long long (&a)[L], const Cr
             carry = carry && x[j] == 0;
         }
     }
-    if (x[L - 1] == 0) {  // much cancellation, or zero
-        const unsigned long long w2 = L == 5 ? x[L - 1] : 0ull;
-        return crt_round(w2, (unsigned long long)x[3] << 32 | x[2], (unsigned long long)x[1] << 32 | x[0], neg, X);
-    }
+    if (x[L - 1] == 0)  // much cancellation, or zero
+        return crt_round((unsigned long long)x[3] << 32 | x[2], (unsigned long long)x[1] << 32 | x[0], neg, X);
     // top 64 bits, 53 of them to nearest even
     const int z = __clz((int)x[L - 1]);
     const uint32_t y3 = __funnelshift_l(x[L - 2], x[L - 1], z), y2 = __funnelshift_l(x[L - 3], x[L - 2], z);
