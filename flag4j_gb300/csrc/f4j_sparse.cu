@@ -476,14 +476,17 @@ __global__ void k_count(int64_t n, const int* __restrict__ idx, int* __restrict_
 // one count per in-range row index in counts_plus1[r + 1], and the first
 // position of an out-of-range one in *first_bad.  A thread takes eight
 // consecutive entries and adds each run of equal rows at once (COO input is
-// usually row-sorted): 16.8 M entries of 16 a row 71 -> 25 us against one entry
-// a lane with equal rows matched across the warp.  VEC: 16-byte loads.
+// usually row-sorted); neighbouring threads whose eight are all of one row add
+// together, or the threads of a row of millions would queue at one counter.  16.8 M
+// entries, us, one entry a lane with equal rows matched across the warp / eight a
+// thread / this: 16 a row 71 / 16 / 19, all in one row 334 / 1313 / 48.  VEC: 16-byte
+// loads.
 template <bool VEC>
 __global__ void k_count_rows_checked(int64_t n, const int* __restrict__ idx, int64_t limit,
                                      int* __restrict__ counts_plus1, int* __restrict__ first_bad) {
+    const int lane = threadIdx.x & 31;
     const int64_t i0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
-    if (i0 >= n) return;
-    const int m = n - i0 < 8 ? (int)(n - i0) : 8;
+    const int m = n - i0 < 8 ? (n > i0 ? (int)(n - i0) : 0) : 8;
     int v[8];
     if (VEC && m == 8) {
         const int4 a = reinterpret_cast<const int4*>(idx + i0)[0], b = reinterpret_cast<const int4*>(idx + i0)[1];
@@ -491,6 +494,18 @@ __global__ void k_count_rows_checked(int64_t n, const int* __restrict__ idx, int
     } else {
 #pragma unroll
         for (int u = 0; u < 8; u++) v[u] = u < m ? idx[i0 + u] : -1;
+    }
+    bool whole = m > 0 && v[0] >= 0 && v[0] < limit;  // one row
+#pragma unroll
+    for (int u = 1; u < 8; u++) whole = whole && (u >= m || v[u] == v[0]);
+    const int before = __shfl_up_sync(0xffffffffu, whole ? v[0] : -1, 1);
+    const bool joins = whole && lane > 0 && before == v[0];
+    const unsigned later = __ballot_sync(0xffffffffu, !joins) & ~((2u << lane) - 1u);
+    const int end = later ? __ffs((int)later) - 1 : 32;  // the lanes from this one on that join it end here
+    const int last = __shfl_sync(0xffffffffu, m, end - 1);
+    if (whole) {
+        if (!joins) atomicAdd(&counts_plus1[v[0] + 1], 8 * (end - 1 - lane) + last);
+        return;
     }
     int run = 0;
 #pragma unroll

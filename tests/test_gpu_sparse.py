@@ -840,3 +840,34 @@ def test_spmm_whole_groups_and_long_rows_bit_identical(f4j, oracle, ncols, lens)
     v, X = g.standard_normal(len(ci)), g.standard_normal((cols, ncols))
     S = f4j.CsrMatrix((rows, cols), v, rp, ci)
     assert np.array_equal(S.mult(f4j.Matrix(X)).toNumpy(), oracle.spmm(rp, ci, v, X))
+
+
+@pytest.mark.parametrize("rows,nnz,kind", [
+    (7, 8 * 32 * 3, "one"), (7, 8 * 32 * 3 + 5, "one"), (7, 3, "one"), (900, 60000, "long"), (900, 59997, "long"),
+    (5000, 40003, "short"), (300, 30011, "unsorted"),
+])
+def test_coo_row_counts_of_rows_that_span_threads(f4j, rows, nnz, kind):
+    """Row counts where a row covers a thread's entries, a warp's, many warps', or ends inside one of them."""
+    g = np.random.default_rng(nnz)
+    if kind == "one":
+        row = np.full(nnz, rows - 2)
+    elif kind == "long":
+        row = np.sort(np.minimum(g.pareto(0.6, nnz).astype(np.int64) * 7, rows - 1))
+    else:
+        row = g.integers(0, rows, nnz)
+        row = np.sort(row) if kind == "short" else row
+    col, v = g.integers(0, 999, nnz).astype(np.int32), g.standard_normal(nnz)
+    for shift in (0, 1):  # aligned for wide loads, and not
+        C = f4j.CooMatrix((rows, 999), v[shift:], row[shift:].astype(np.int32), col[shift:]).toCsr()
+        assert np.array_equal(np.diff(C.rowPointers), np.bincount(row[shift:], minlength=rows))
+        assert np.array_equal(C.colIndices, col[shift:]) and np.array_equal(C.data, v[shift:])
+
+
+@pytest.mark.parametrize("at", [0, 7, 8, 255, 256, 1000])
+def test_coo_row_out_of_range_beside_long_rows(f4j, at):
+    """An out-of-range row index among entries of one row is reported at its own position."""
+    nnz = 1001
+    row = np.full(nnz, 3, np.int32)
+    row[at] = 9
+    with pytest.raises(f4j.IllegalArgumentException):
+        f4j.CooMatrix((9, 50), np.ones(nnz), row, np.zeros(nnz, np.int32)).toCsr()
