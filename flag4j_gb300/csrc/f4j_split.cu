@@ -1631,6 +1631,13 @@ constexpr size_t CRT_Y_BYTES = size_t(4) << 30;
 // 16384 x 1024 20.3 / 21.0 / 17.8, 26000 x 26000 x 1024 51.8 / - / 48.0; past this
 // size not any more: 36000 x 36000 x 1024 99.7 / 98.4 / -.
 constexpr size_t CRT_HOST_Y_BYTES = size_t(32) << 30;
+// Below this much of A, B and C together a residue-form product from host arrays
+// goes in turn: its parts' many small launches take longer than the copies they
+// overlap.  Host arrays, us, in parts / in turn: 300^3 137 / 73, 1024^3 309 / 246, 1300^3
+// (41 MB) 427 / 390, 1800 x 1800 x 600 (43) 426 / 424, 3173 x 795 x 1037 (53) 479 / 478,
+// 1500^3 (54) 469 / 475, 1024 x 1024 x 4096 (75) 539 / 621; complex 700 x 900 x 800 (31)
+// 363 / 332, 1024^3 (50) 469 / 475.
+constexpr size_t CRT_HOST_PARTS_BYTES = size_t(48) << 20;
 
 // A residue-form product's sizes and workspace.
 struct CrtSetup {
@@ -2239,7 +2246,8 @@ static int gemm_host(f4j_ctx* ctx, bool cplx, int64_t m, int64_t n, int64_t k, c
         int kchunks = 0;
         if (!crt) split_kcb_cap(tiles_m * (int64_t)tiles_n, (cplx ? 2 : 1) * f4j_cdiv(k, BKB), &kchunks);
         const size_t y = crt ? (size_t)CRT_NB * 2 * (m + CG_T) * (ncat + 16) : 0;
-        if (!piped || kchunks || y > CRT_HOST_Y_BYTES) return in_turn();  // split K runs as one launch
+        const bool small = crt && ab + bb + cb < CRT_HOST_PARTS_BYTES;
+        if (!piped || kchunks || small || y > CRT_HOST_Y_BYTES) return in_turn();  // split K runs as one launch
         rc = host_split_pipelined(ctx, cplx, m, n, k, A, B, opB, C, (double*)dA, (double*)dB, (double*)dC, crt, parts,
                                   bparts, &recompute, &plan, &spread);
         if (rc != F4J_ERR_OOM || !crt) break;

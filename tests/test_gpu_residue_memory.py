@@ -10,18 +10,18 @@ from test_gpu_capture import capturing_context
 pytestmark = pytest.mark.gpu
 
 
-def product(ctx, A, B, mode, host=False):
+def product(ctx, A, B, mode, opB=0, host=False):
     from flag4j_gb300.device import check
     m, k = A.shape
-    n = B.shape[1]
+    n = B.shape[1 if opB == 0 else 0]
     if host:
         C = np.empty((m, n), A.dtype)
         fn = ctx.lib.f4j_zgemm_host if np.iscomplexobj(A) else ctx.lib.f4j_dgemm_host
-        check(fn(ctx.handle, m, n, k, A.ctypes.data, 0, B.ctypes.data, 0, C.ctypes.data, mode, None))
+        check(fn(ctx.handle, m, n, k, A.ctypes.data, 0, B.ctypes.data, opB, C.ctypes.data, mode, None))
         return C
     dA, dB, dC = ctx.from_numpy(A), ctx.from_numpy(B), ctx.alloc(A.dtype.itemsize * m * n)
     fn = ctx.lib.f4j_zgemm if np.iscomplexobj(A) else ctx.lib.f4j_dgemm
-    check(fn(ctx.handle, m, n, k, dA.handle, 0, dB.handle, 0, dC.handle, mode, None))
+    check(fn(ctx.handle, m, n, k, dA.handle, 0, dB.handle, opB, dC.handle, mode, None))
     return dC.to_numpy(A.dtype, m * n).reshape(m, n)
 
 
@@ -70,16 +70,22 @@ def test_a_refused_workspace_costs_nothing_again(f4j, monkeypatch):
         assert np.array_equal(dC.to_numpy(np.float64, 2000 * 1900).reshape(2000, 1900), want)
 
 
-@pytest.mark.parametrize("m,n,k,cplx", [
-    (300, 300, 300, False), (1024, 1024, 1024, False), (1300, 700, 512, False), (129, 2048, 300, False),  # SPLIT: slices
-    (2111, 1777, 700, False), (1300, 1300, 449, False), (600, 500, 400, True),  # complex
+@pytest.mark.parametrize("m,n,k,opB,cplx", [
+    (300, 300, 300, 0, False), (1024, 1024, 1024, 0, False), (1300, 700, 512, 1, False),    # in turn; SPLIT: slices
+    (129, 2048, 300, 0, False), (1300, 1300, 449, 0, False), (600, 500, 400, 2, True),
+    (2111, 1777, 700, 0, False), (1777, 2111, 900, 1, False), (513, 400, 8193, 1, False),   # in parts
+    (1500, 1300, 900, 0, True), (1300, 1500, 901, 1, True), (1301, 1400, 1000, 2, True),
 ])
-def test_host_product_is_the_device_product_in_auto(f4j, m, n, k, cplx):
+def test_host_product_is_the_device_product_in_auto(f4j, m, n, k, opB, cplx):
     """f4j_dgemm_host and f4j_zgemm_host in AUTO: bit for bit f4j_dgemm's and f4j_zgemm's AUTO."""
     from flag4j_gb300 import _lib
     A, B = operands(m, n, k, m + k, cplx)
+    B = B if opB == 0 else np.ascontiguousarray(B.T if opB == 1 else B.conj().T)
     ctx = f4j.default_context()
-    assert np.array_equal(product(ctx, A, B, _lib.MODE_AUTO, host=True), product(ctx, A, B, _lib.MODE_AUTO))
+    dev, host = (product(ctx, A, B, _lib.MODE_AUTO, opB=opB, host=h) for h in (False, True))
+    assert np.array_equal(host, dev)
+    want = A[:40] @ (B if opB == 0 else B.T if opB == 1 else B.conj().T)
+    assert np.abs(dev[:40] - want).max() <= 1e-9
 
 
 @pytest.mark.parametrize("m,n,k,cplx", [
