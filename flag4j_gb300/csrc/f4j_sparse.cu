@@ -1599,7 +1599,8 @@ static int transpose_buckets(f4j_ctx* ctx, f4j_csr S, int shift, int qbits, int 
     // ones are as fast whole: 2^20 rows x 20, us, whole / in segments: 3000 columns 687 / 825, 2^20 998 /
     // 1044; x 64 2519 / 2771, 4587 / 3265).  At most this many, and segments of them, whose counts take
     // the place of hist, which is done with by then
-    const int64_t above = f4j_cdiv(2 * nnz, nb) > TP2_CAP ? f4j_cdiv(2 * nnz, nb) : TP2_CAP;
+    int64_t above = f4j_cdiv(2 * nnz, nb) > TP2_CAP ? f4j_cdiv(2 * nnz, nb) : TP2_CAP;
+    above = above < INT32_MAX ? above : INT32_MAX;
     const int64_t bigs = shift ? nnz / (above + 1) : 0, segs = bigs ? nnz / TP2_SEG + bigs : 0;
     const size_t rows_hist = (size_t)nblocks * nbp, rows_seg = (size_t)segs * (((1 << shift) + 3) & ~3);
     const size_t head = rows_hist > rows_seg ? rows_hist : rows_seg;
