@@ -2517,7 +2517,8 @@ extern "C" int f4j_sddmm(f4j_ctx* ctx, f4j_csr S, f4j_buf A, f4j_buf B, int64_t 
             const double *a = (const double*)A->ptr, *b = (const double*)B->ptr;
             const bool even = ncols % 2 == 0 && f4j_aligned16(a) && f4j_aligned16(b);
             // more than 64 columns: equal parts of at most 56, whose sums k_sddmm_flat
-            // keeps in four, added up in order
+            // keeps in four, added up in order.  57 to 63 columns go singly: eight
+            // pairs a lane are built for 64 alone, where no unit is left over
             const int64_t part = ncols <= 64 ? 64 : f4j_cdiv(f4j_cdiv(ncols, f4j_cdiv(ncols, 56)), 8) * 8;
             for (int64_t c0 = 0; c0 < ncols; c0 += part) {
                 const int w = (int)(ncols - c0 < part ? ncols - c0 : part);
