@@ -757,7 +757,7 @@ __global__ void __launch_bounds__(RS_T) k_radix_scatter(int64_t n, const unsigne
 // from global memory by their place instead took half of both passes.
 // Against an LSD radix sort of (column, index) pairs, three passes of two random
 // 4-byte writes at 2^20 columns, and the rows gathered after it: 2^20 rows and
-// columns, 16.8 M nonzeros, 0.93 -> 0.38 ms (scatter 137, bucket 185, histogram
+// columns, 16.8 M nonzeros, 0.93 -> 0.39 ms (scatter 138, bucket 191, histogram
 // and places 38, rows 19 us).  Both passes are instruction-bound (153 and 204 warp
 // instructions per 32 items).  The kernels are a chain (chain_wait in f4j_ptx.cuh):
 // 65536 rows and columns x 8, T() 105 -> 92 us.
