@@ -80,7 +80,7 @@ extern "C" int f4j_create(int device, f4j_ctx** out) {
         cudaGetLastError();
     }
     e = cudaMalloc(&c->d_status, F4J_ST_WORDS * sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(c->d_status, 0, F4J_ST_WORDS * sizeof(int));
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->d_status, 0, F4J_ST_WORDS * sizeof(int), c->stream);
     if (e != cudaSuccess) {
         cudaStreamDestroy(c->stream);
         delete c;
